@@ -16,7 +16,7 @@ DEBUG_LIB_PATH = os.path.join(_HERE, "libmsda_sm100_dbg.so")
 
 F32, F16, BF16 = 0, 1, 2
 TUNE_STAGE, TUNE_CTAS_PER_SM, TUNE_CTAS_PER_SM_BWD, TUNE_INTERLEAVE, TUNE_SPIN_LIMIT = 0, 1, 2, 3, 4
-TUNE_PRECISE_AMP, TUNE_DEBUG_ROW_LIMIT, TUNE_PACK_ROWS = 5, 6, 7
+TUNE_PRECISE_AMP, TUNE_DEBUG_ROW_LIMIT, TUNE_PACK_ROWS, TUNE_SORT = 5, 6, 7, 8
 
 # name -> (restype, argtypes); kept in step with the headers under include/
 _vp, _ip, _i, _sz = ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
@@ -25,6 +25,8 @@ SIGNATURES = {
     "msda_sm100_forward": (_i, [_vp, _ip, _ip, _vp, _vp, _vp] + _DIMS7 + [_i, _vp]),
     "msda_sm100_backward": (_i, [_vp, _ip, _ip, _vp, _vp, _vp, _vp, _vp, _vp] + _DIMS7 + [_i, _vp]),
     "msda_sm100_backward_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
+    "msda_sm100_backward_sorted_workspace_bytes": (_sz, _DIMS7 + [_i]),
+    "gka_sm100_backward_sorted_workspace_bytes": (_sz, _DIMS7 + [_i]),
     "msda_sm100_backward_ws": (_i, [_vp, _ip, _ip, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz]
                                + _DIMS7 + [_i, _vp]),
     "msda_sm100_fused_forward": (_i, [_vp, _ip, _ip, _vp, _vp, _vp, _vp] + _DIMS7 + [_i, _vp]),

@@ -194,7 +194,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> multi_scale_deformable_attn_backw
     const int dt = dtype_code(value.scalar_type());
     at::Tensor workspace;
     void* ws_ptr = nullptr;
-    size_t ws_bytes = msda_sm100_backward_workspace_bytes(d.B, d.K, d.H, d.D, dt);
+    size_t ws_bytes = msda_sm100_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
     if (ws_bytes > 0) {
         workspace = at::empty({static_cast<int64_t>(ws_bytes / sizeof(float))},
                               value.options().dtype(at::kFloat));
@@ -313,7 +313,7 @@ std::tuple<at::Tensor, at::Tensor> geometric_kernel_attention_backward(
     const int dt = dtype_code(value.scalar_type());
     at::Tensor workspace;
     void* ws_ptr = nullptr;
-    const size_t ws_bytes = msda_sm100_backward_workspace_bytes(d.B, d.K, d.H, d.D, dt);
+    const size_t ws_bytes = gka_sm100_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
     if (ws_bytes > 0) {
         workspace = at::empty({static_cast<int64_t>(ws_bytes / sizeof(float))},
                               value.options().dtype(at::kFloat));

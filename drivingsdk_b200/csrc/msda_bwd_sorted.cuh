@@ -1,0 +1,939 @@
+// Backward over samples sorted by the pixel cell they fall into, shared by the bilinear operator
+// (MSDA, CPS = 4 corners per sample) and the nearest-pixel operator (CPS = 1).
+//
+// The task-ordered backward (msda_bwd_kernel.cuh) gathers and reduces every corner row of every
+// sample: 8 row transfers between L2 and an SM per sample, of which the reductions retire at
+// the sector rate of L2. Samples of one cell share their four corner rows. Walking the samples
+// cell by cell keeps the corner rows and their gradient sums in registers, and what is left per
+// sample is one row of grad_out; corner rows are loaded and their sums reduced once per run of
+// samples in a cell (and only the new two when the walk moves one cell to the right).
+//
+//   1 sort     cluster of CTAs = (batch, head, level): counting sort by cell in shared memory;
+//              dropped samples get their zero gradients.
+//   2 main     warp = a ticket of consecutive sorted samples, in 32 / LPR streams: a stream is
+//              LPR lanes, each lane four channels of all corners.
+// The main kernel compares the cells themselves, so the order is only a matter of speed.
+// Work is cut by samples, not by cells: a map whose samples all fall into one cell is as
+// balanced as any other.
+#pragma once
+
+#include <type_traits>
+
+#include "msda_launch.h"
+#include "msda_tile.cuh"
+
+namespace msda {
+
+constexpr int kSortThreads = 1024;
+constexpr uint32_t kSortCells = 24 * 1024;   // counters of one CTA: 96 KB, two CTAs per SM
+constexpr uint32_t kMaxStream = 256;         // most consecutive sorted samples in one stream
+
+// Level table of one CTA.
+struct SortLevels {
+    float4 geo[kMaxLevels];   // width, height, width (bits), first key (bits)
+};
+
+// All threads of the CTA must call it. False: a level table in device memory is inconsistent
+// (status bit set); nothing may be touched then.
+__device__ __forceinline__ bool load_sort_levels(const Params& p, SortLevels& lv) {
+    if (!device_level_table_ok(p)) return false;
+    for (int l = threadIdx.x; l < p.L; l += blockDim.x) {
+        const int h = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l];
+        const int w = p.use_table ? p.lv.w[l] : p.shapes_dev[2 * l + 1];
+        const int start = p.use_table ? p.lv.start[l] : p.start_dev[l];
+        lv.geo[l] = make_float4(static_cast<float>(w), static_cast<float>(h), __int_as_float(w),
+                                __int_as_float(start));
+    }
+    __syncthreads();
+    return true;
+}
+
+// Task, level and sample-in-task of sample number `id`.
+struct SampleId {
+    uint32_t task, b, h;
+    int level;
+};
+__device__ __forceinline__ SampleId sample_id(const Params& p, const SortParams& sp, uint32_t id) {
+    SampleId r;
+    r.task = fd_div(id, p.fd_lp);
+    r.level = static_cast<int>(fd_div(id - r.task * p.LP, sp.fd_p));
+    r.b = fd_div(r.task, p.fd_qh);
+    r.h = r.task - fd_div(r.task, p.fd_h) * p.H;
+    return r;
+}
+
+template <typename TL>
+__device__ __forceinline__ float2 load_pair(const TL* p);
+template <>
+__device__ __forceinline__ float2 load_pair<float>(const float* p) {
+    return __ldg(reinterpret_cast<const float2*>(p));
+}
+template <>
+__device__ __forceinline__ float2 load_pair<__half>(const __half* p) {
+    return __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
+}
+template <>
+__device__ __forceinline__ float2 load_pair<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
+    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
+// The sample's cell in its level, or kNoRow for a sample that takes no part.
+template <int CPS>
+__device__ __forceinline__ uint32_t sample_cell(float2 xy, int W, int H) {
+    if constexpr (CPS == 4) {
+        const float wf = static_cast<float>(W), hf = static_cast<float>(H);
+        const float x = xy.x * wf - 0.5f;
+        const float y = xy.y * hf - 0.5f;
+        if (!((x > -1.f) && (y > -1.f) && (x < wf) && (y < hf))) return kNoRow;
+        return static_cast<uint32_t>(__float2int_rd(y) + 1) * static_cast<uint32_t>(W + 1) +
+               static_cast<uint32_t>(__float2int_rd(x) + 1);
+    } else {
+        const int x = min(max(__float2int_rz(xy.x), 0), W - 1);
+        const int y = min(max(__float2int_rz(xy.y), 0), H - 1);
+        return static_cast<uint32_t>(y * W + x);
+    }
+}
+
+// Counters in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_address(const uint32_t* p, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_count(uint32_t addr) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], 1;" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_take(uint32_t addr) {
+    uint32_t r;
+    asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(r) : "r"(addr) : "memory");
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_read(uint32_t addr) {
+    uint32_t r;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(r) : "r"(addr) : "memory");
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Counting sort of one (batch, head, level)'s samples by cell, with the counters in the shared
+// memory of a cluster of CTAs: atomics there are faster than in L2 (a version with one L2 counter
+// per cell took 72 + 42 us at the encoder shape, bound by the rate of L2 atomics). The CTAs of a
+// cluster share the queries and the cells of a level: each counts and places its queries'
+// samples, whoever holds the counter. Where cells hold many samples each CTA keeps to itself:
+// it sorts its own queries (whose runs are then that much shorter). The CTAs' results follow
+// each other in the order in which they get there.
+template <typename TL, int CPS>
+__global__ void __launch_bounds__(kSortThreads, 2)
+sort_cells_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
+    extern __shared__ uint32_t s_count[];   // [kSortCells]
+    __shared__ uint32_t warp_sum[32];
+    __shared__ uint32_t block_sum;           // samples this CTA's counters hold
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (blockIdx.x == 0 && tid == 0) *sp.ticket = 0u;
+    if (!device_level_table_ok(p)) {         // the same answer in every CTA
+        if (tid == 0) sp.regions[blockIdx.x / sp.parts] = make_uint2(0u, 0u);
+        return;
+    }
+
+    uint32_t unit = blockIdx.x;
+    const uint32_t part = unit % sp.parts;   // rank in the cluster
+    unit /= sp.parts;
+    const uint32_t l = unit % p.L;
+    unit /= p.L;
+    const uint32_t h = unit % p.H, b = unit / p.H;
+    const int H = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l];
+    const int W = p.use_table ? p.lv.w[l] : p.shapes_dev[2 * l + 1];
+    const uint32_t cells = (CPS == 4) ? static_cast<uint32_t>(H + 1) * static_cast<uint32_t>(W + 1)
+                                      : static_cast<uint32_t>(H) * static_cast<uint32_t>(W);
+    const uint32_t samples = static_cast<uint32_t>(p.Q) * p.P;
+    // on its own: at least sixteen samples per cell are left to each CTA, and the counters fit
+    const bool alone = sp.parts == 1 || (samples / sp.parts >= 16u * cells && cells <= kSortCells);
+    const uint32_t q0 = static_cast<uint32_t>(static_cast<uint64_t>(p.Q) * part / sp.parts);
+    const uint32_t q1 = static_cast<uint32_t>(static_cast<uint64_t>(p.Q) * (part + 1) / sp.parts);
+    const uint32_t n = (q1 - q0) * p.P;
+    // sample i of the range: point i % P of query q0 + i / P
+    const uint32_t first = ((b * p.Q + q0) * p.H + h) * p.LP + l * p.P;
+    const uint32_t stride = static_cast<uint32_t>(p.H) * p.LP;
+    const TL* loc = static_cast<const TL*>(p.loc);
+    auto id_of = [&](uint32_t i) {
+        const uint32_t q = fd_div(i, sp.fd_p);
+        return first + q * stride + (i - q * p.P);
+    };
+
+    // cells held by one CTA at a time, by all of the cluster (or by this CTA alone) in a pass
+    const uint32_t holders = alone ? 1u : sp.parts;
+    const uint32_t held = min(kSortCells, (cells + holders - 1) / holders);
+    const uint32_t pass_cells = held * holders;
+    const FastDiv by_held = sp.parts == 1 ? FastDiv{0u, 0u} : device_fastdiv(held);
+    auto sync = [&]() {
+        if (alone) __syncthreads();
+        else cluster_barrier();
+    };
+    const uint32_t region = (blockIdx.x / sp.parts) * samples;
+    uint32_t placed = 0;         // samples of the region placed by earlier passes
+    constexpr uint32_t kU = 4;   // samples in flight per thread
+    for (uint32_t lo = 0; lo < cells; lo += pass_cells) {
+        for (uint32_t i = tid; i < held; i += kSortThreads) s_count[i] = 0u;
+        sync();
+        for (uint32_t i0 = tid; i0 < n; i0 += kU * kSortThreads) {
+            float2 xy[kU];
+            uint32_t id[kU];
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u) {
+                const uint32_t i = i0 + u * kSortThreads;
+                id[u] = id_of(i < n ? i : 0u);
+                xy[u] = load_pair(loc + 2ull * id[u]);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u) {
+                if (i0 + u * kSortThreads >= n) break;
+                const uint32_t c = sample_cell<CPS>(xy[u], W, H);
+                if (c - lo < pass_cells) {
+                    if (alone) {
+                        atomicAdd(s_count + (c - lo), 1u);
+                    } else {
+                        const uint32_t rank = fd_div(c - lo, by_held);
+                        cluster_count(cluster_address(s_count + (c - lo - rank * held), rank));
+                    }
+                } else if (CPS == 4 && c == kNoRow && lo == 0) {
+                    store_pair(static_cast<TL*>(p.grad_loc) + 2ull * id[u], 0.f, 0.f);
+                    static_cast<TL*>(p.grad_attn)[id[u]] = Elem<TL>::from_f(0.f);
+                }
+            }
+        }
+        sync();
+        // counts -> first positions: a thread takes an odd number of neighbours (no bank conflicts)
+        const uint32_t per = ((held + kSortThreads - 1) / kSortThreads) | 1u;
+        const uint32_t begin = min(held, tid * per), stop = min(held, begin + per);
+        uint32_t sum = 0;
+        for (uint32_t i = begin; i < stop; ++i) sum += s_count[i];
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) warp_sum[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t mine = warp_sum[lane];
+            uint32_t w = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += v;
+            }
+            warp_sum[lane] = w - mine;
+            if (lane == 31) block_sum = w;
+        }
+        if (sp.parts == 1) __syncthreads();
+        else cluster_barrier();
+        // the samples of lower ranks come first
+        uint32_t at = region + placed + warp_sum[warp] + incl - sum;
+        for (uint32_t r = 0; r < sp.parts; ++r) {
+            const uint32_t m = sp.parts == 1 ? block_sum : cluster_read(cluster_address(&block_sum, r));
+            if (r < part) at += m;
+            placed += m;
+        }
+        for (uint32_t i = begin; i < stop; ++i) {
+            const uint32_t m = s_count[i];
+            s_count[i] = at;
+            at += m;
+        }
+        sync();
+        for (uint32_t i0 = tid; i0 < n; i0 += kU * kSortThreads) {
+            float2 xy[kU];
+            uint32_t id[kU], pos[kU];
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u) {
+                const uint32_t i = i0 + u * kSortThreads;
+                id[u] = id_of(i < n ? i : 0u);
+                xy[u] = load_pair(loc + 2ull * id[u]);
+                pos[u] = kNoRow;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u) {
+                if (i0 + u * kSortThreads >= n) break;
+                const uint32_t c = sample_cell<CPS>(xy[u], W, H);
+                if (c - lo < pass_cells) {
+                    if (alone) {
+                        pos[u] = atomicAdd(s_count + (c - lo), 1u);
+                    } else {
+                        const uint32_t rank = fd_div(c - lo, by_held);
+                        pos[u] = cluster_take(cluster_address(s_count + (c - lo - rank * held), rank));
+                    }
+                }
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u)
+                if (pos[u] != kNoRow) sp.sorted[pos[u]] = id[u];
+        }
+        // nobody leaves, or clears the counters, while others still use them
+        if (sp.parts == 1) __syncthreads();
+        else cluster_barrier();
+    }
+    if (tid == 0 && part == 0) sp.regions[blockIdx.x / sp.parts] = make_uint2(region, placed);
+}
+
+// ---------------------------------------------------------------------------
+// main kernels
+// ---------------------------------------------------------------------------
+// Two fp32 values in one 64-bit register pair, the operand form of the packed multiply-add: kept
+// in this form throughout, so that no moves are needed to assemble operands.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Four channels of a row, as two fp32 pairs.
+template <typename T>
+__device__ __forceinline__ void load_quad(const T* p, f32x2 (&q)[2]) {
+    if constexpr (sizeof(T) == 4) {
+        const ulonglong2 r = __ldg(reinterpret_cast<const ulonglong2*>(p));
+        q[0] = r.x;
+        q[1] = r.y;
+    } else {
+        const uint2 r = __ldg(reinterpret_cast<const uint2*>(p));
+        const uint32_t w[2] = {r.x, r.y};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if constexpr (std::is_same<T, __half>::value) {
+                const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                q[i] = pack2(v.x, v.y);
+            } else {
+                q[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+            }
+        }
+    }
+}
+__device__ __forceinline__ void red_quad(float* p, const f32x2 (&q)[2]) {
+    const float2 a = unpack2(q[0]), b = unpack2(q[1]);
+    red_add_f32x4(p, a.x, a.y, b.x, b.y);
+}
+
+// Sums each of N per-lane values over groups of LPR lanes (N a power of two <= LPR): halving
+// steps in which a lane gives half of its values away and keeps the other half, then plain
+// steps. Lane j of a group ends up with the sum of value j / (LPR / N).
+template <int N, int LPR, typename V>
+__device__ __forceinline__ V reduce_values(V (&d)[N], int j) {
+    if constexpr (N == 1) {
+#pragma unroll
+        for (int o = LPR / 2; o >= 1; o >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], o);
+        return d[0];
+    } else {
+        const bool up = (j & (LPR / 2)) != 0;
+        V half[N / 2];
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            half[i] = up ? d[N / 2 + i] : d[i];
+            half[i] += __shfl_xor_sync(0xffffffffu, up ? d[i] : d[N / 2 + i], LPR / 2);
+        }
+        return reduce_values<N / 2, LPR / 2>(half, j);
+    }
+}
+
+// One sorted sample, on its lane.
+struct SortedSample {
+    uint32_t row;    // row offset of the cell's top-left corner (wraps where that does not exist)
+    uint32_t cell;   // level width << 4 | existing corners
+    uint32_t task, id;
+    float lw, lh, a, wf, hf;
+    float w[4];
+    bool amplified;
+};
+// MSDA_DEBUG_BOUNDS build: the rows of the cell's existing corners against the extent of value and
+// grad_value (see debug_check_rows); an offending sample loses all its corners.
+__device__ __forceinline__ void debug_check_cell(const Params& p, SortedSample& s) {
+#ifdef MSDA_DEBUG_BOUNDS
+    const uint32_t step_x = static_cast<uint32_t>(p.H) * p.row_units;
+    bool bad = false;
+    for (int c = 0; c < 4; ++c) {
+        const uint32_t off = s.row + ((c & 1) ? step_x : 0u) + ((c & 2) ? (s.cell >> 4) * step_x : 0u);
+        bad |= ((s.cell >> c) & 1u) && (off >= p.limit_units || p.limit_units - off < p.row_units);
+    }
+    if (bad) {
+        atomicOr(p.status, kStatusOutOfBounds);
+        s.cell &= ~15u;
+    }
+#else
+    (void)p;
+    (void)s;
+#endif
+}
+
+// What a lane loads for a sample; fetched a round ahead of its use.
+struct RawSample {
+    uint32_t id;
+    float2 xy;
+    float a;
+};
+template <typename TL>
+__device__ __forceinline__ void load_raw(const Params& p, RawSample& r, bool live) {
+    r.xy = make_float2(0.f, 0.f);
+    r.a = 0.f;
+    if (live) {
+        r.xy = load_pair(static_cast<const TL*>(p.loc) + 2ull * r.id);
+        r.a = Elem<TL>::to_f(__ldg(static_cast<const TL*>(p.attn) + r.id));
+    }
+}
+template <int CPS>
+__device__ __forceinline__ SortedSample set_up_sample(const Params& p, const SortParams& sp,
+                                                      const SortLevels& lv, const RawSample& raw,
+                                                      bool live) {
+    SortedSample r;
+    r.row = r.cell = r.task = r.id = 0u;   // no corner, task 0: adds nothing
+    r.lw = r.lh = r.a = r.wf = r.hf = 0.f;
+    r.w[0] = r.w[1] = r.w[2] = r.w[3] = 0.f;
+    r.amplified = false;
+    if (!live) return r;
+    r.id = raw.id;
+    const SampleId s = sample_id(p, sp, r.id);
+    const float4 geo = lv.geo[s.level];
+    const int W = __float_as_int(geo.z);
+    const uint32_t row_base =
+        (s.b * static_cast<uint32_t>(p.K) + __float_as_uint(geo.w)) * p.H + s.h;
+    r.task = s.task;
+    r.a = raw.a;
+    r.wf = geo.x;
+    r.hf = geo.y;
+    if constexpr (CPS == 4) {
+        // sample_setup (msda_common.cuh) for a sample known to take part
+        const float x0f = floorf(raw.xy.x * geo.x - 0.5f);
+        const float y0f = floorf(raw.xy.y * geo.y - 0.5f);
+        r.lw = fmaf(raw.xy.x, geo.x, -(x0f + 0.5f));
+        r.lh = fmaf(raw.xy.y, geo.y, -(y0f + 0.5f));
+        const float hw = 1.f - r.lw, hh = 1.f - r.lh;
+        const uint32_t sides = (x0f >= 0.f ? 1u : 0u) | (x0f < geo.x - 1.f ? 2u : 0u);
+        r.cell = (static_cast<uint32_t>(W) << 4) | (y0f >= 0.f ? sides : 0u) |
+                 (y0f < geo.y - 1.f ? sides << 2 : 0u);
+        r.row = (row_base + static_cast<uint32_t>(__float2int_rz(y0f) * W + __float2int_rz(x0f)) * p.H) *
+                p.row_units;
+        const float top = hh * r.a, bottom = r.lh * r.a;
+        r.w[0] = top * hw;
+        r.w[1] = top * r.lw;
+        r.w[2] = bottom * hw;
+        r.w[3] = bottom * r.lw;
+        r.amplified = fmaxf(geo.x, geo.y) * fabsf(r.a) >= p.precise_amp;
+    } else {
+        const int x = min(max(__float2int_rz(raw.xy.x), 0), W - 1);
+        const int y = min(max(__float2int_rz(raw.xy.y), 0), __float2int_rz(geo.y) - 1);
+        r.row = (row_base + static_cast<uint32_t>(y * W + x) * p.H) * p.row_units;
+        r.cell = 1u;
+    }
+    debug_check_cell(p, r);
+    return r;
+}
+// Warps draw tickets in order; a ticket is up to `len` consecutive sorted samples of one region.
+struct Ticket {
+    uint32_t begin, end;   // positions; begin >= end: nothing
+};
+__device__ __forceinline__ bool next_ticket(const SortParams& sp, uint32_t len, int lane, Ticket& t) {
+    uint32_t n = 0;
+    if (lane == 0) n = atomicAdd(sp.ticket, 1u);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if (n >= sp.tickets) return false;
+    const uint32_t region = fd_div(n, sp.fd_tickets);
+    const uint2 r = __ldg(sp.regions + region);
+    t.begin = r.x + (n - region * sp.tickets_per_region) * len;
+    t.end = min(r.x + r.y, t.begin + len);
+    return true;
+}
+
+// Flags of a sorted sample in its stream (low bits; level width << 8 and existing corners << 4
+// above them).
+constexpr uint32_t kEnters = 1;      // its cell is not the previous sample's
+constexpr uint32_t kJumps = 2;       // ... and not the next one to the right either
+constexpr uint32_t kAmplified = 4;   // wants its dot products in double
+
+// Bilinear main kernel. T: type of value / grad_out; TL: type of locations, weights and their
+// gradients. LPR lanes cover a row (4 channels each, NV times; lanes past D are idle, D need not
+// be a power of two) and hold all four corners of a cell: value rows and gradient sums. A warp
+// walks 32 / LPR streams of sp.stream consecutive sorted samples side by side, in rounds of 32
+// samples whose set-up and final gradients are done lane = sample. The accumulation rows are
+// fp32.
+template <typename T, typename TL, int NV, int LPR>
+__global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 3)
+msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
+    constexpr int S = 32 / LPR;       // streams
+    constexpr int U = 2;              // rows of grad_out in flight per lane
+    // fp32 bilinear operator: some dot products need double precision (see sample_grad)
+    constexpr bool WIDE = sizeof(TL) == 4 && sizeof(T) == 4;
+    static_assert(LPR % U == 0, "a round is LPR steps");
+
+    __shared__ SortLevels lv;
+    // records of one round, stream index fastest (streams then read different banks):
+    // weights, each twice (operands of the packed multiply-add), later the dot products; those
+    // formed in double; offset of the grad_out row and flags; row offset of the top-left corner
+    __shared__ ulonglong2 s_w[kWarpsPerCta][32][2];
+    __shared__ double s_wide[WIDE ? kWarpsPerCta : 1][WIDE ? 32 : 1][4];
+    __shared__ uint2 s_rec[kWarpsPerCta][32];
+    __shared__ uint32_t s_row[kWarpsPerCta][32];
+    if (!load_sort_levels(p, lv)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane / LPR, j = lane % LPR;
+    const int my_stream = lane % S, my_step = lane / S;   // of this lane's sample in a round
+
+    const uint32_t step_x = static_cast<uint32_t>(p.H) * p.row_units;
+    bool on[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) on[k] = (j + k * LPR) * 4 < p.D;
+    const T* vlane = static_cast<const T*>(p.value) + j * 4;
+    const T* glane = static_cast<const T*>(p.grad_out) + j * 4;
+    float* alane = static_cast<float*>(p.grad_value) + j * 4;
+    const uint32_t ticket_len = sp.stream * S;
+
+    Ticket ticket;
+    while (next_ticket(sp, ticket_len, lane, ticket)) {
+        if (ticket.begin >= ticket.end) continue;
+        f32x2 acc[4][NV][2], val[4][NV][2];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) acc[c][k][0] = acc[c][k][1] = val[c][k][0] = val[c][k][1] = 0ull;
+        // cell of this lane's stream and the offset of the pixel row below it; no corner: nothing
+        // to flush
+        uint32_t cur = 0u, cell = 0u, below = 0u;
+
+        auto flush = [&](int c, bool yes) {
+            if (yes && ((cell >> c) & 1u)) {
+                float* at = alane + static_cast<size_t>(cur + ((c & 1) ? step_x : 0u) +
+                                                        ((c & 2) ? below : 0u)) * 4;
+#pragma unroll
+                for (int k = 0; k < NV; ++k)
+                    if (on[k]) red_quad(at + k * (LPR * 4), acc[c][k]);
+            }
+        };
+        auto fetch = [&](int c, bool yes) {
+            if (yes) {
+                const T* at = vlane + static_cast<size_t>(cur + ((c & 1) ? step_x : 0u) +
+                                                          ((c & 2) ? below : 0u)) * 4;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    val[c][k][0] = val[c][k][1] = 0ull;
+                    if (((cell >> c) & 1u) && on[k]) load_quad<T>(at + k * (LPR * 4), val[c][k]);
+                }
+            }
+        };
+        auto clear = [&](int c, bool yes) {
+            if (yes) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) acc[c][k][0] = acc[c][k][1] = 0ull;
+            }
+        };
+        // right corners become left ones
+        auto shift = [&](int c, bool yes) {
+            if (yes) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        acc[c][k][e] = acc[c + 1][k][e];
+                        val[c][k][e] = val[c + 1][k][e];
+                    }
+            }
+        };
+
+        // this lane's samples: at, at + LPR, ... below `end`
+        uint32_t at = ticket.begin + my_stream * sp.stream + my_step;
+        const uint32_t end = min(ticket.end, ticket.begin + (my_stream + 1) * sp.stream);
+        RawSample raw;
+        raw.id = at < end ? __ldg(sp.sorted + at) : 0u;
+        uint32_t next_id = at + LPR < end ? __ldg(sp.sorted + at + LPR) : 0u;
+        load_raw<TL>(p, raw, at < end);
+        for (; __any_sync(0xffffffffu, at < end); at += LPR) {
+            // ---- lane = sample: cell, corner weights --------------------------------------
+            RawSample next;
+            next.id = next_id;
+            load_raw<TL>(p, next, at + LPR < end);
+            next_id = at + 2 * LPR < end ? __ldg(sp.sorted + at + 2 * LPR) : 0u;
+            const SortedSample s = set_up_sample<4>(p, sp, lv, raw, at < end);
+            raw = next;
+            {
+                uint32_t prow = __shfl_up_sync(0xffffffffu, s.row, S);
+                uint32_t pcell = __shfl_up_sync(0xffffffffu, s.cell, S);
+                const uint32_t srow = __shfl_sync(0xffffffffu, cur, my_stream * LPR);
+                const uint32_t scell = __shfl_sync(0xffffffffu, cell, my_stream * LPR);
+                if (my_step == 0) {
+                    prow = srow;
+                    pcell = scell;
+                }
+                uint32_t flags = s.cell << 4;
+                if (s.row != prow || s.cell != pcell) {
+                    const bool right = s.row == prow + step_x && (s.cell >> 4) == (pcell >> 4) &&
+                                       ((pcell >> 1) & 5u) == (s.cell & 5u);
+                    flags |= right ? kEnters : (kEnters | kJumps);
+                }
+                if (WIDE && s.amplified) flags |= kAmplified;
+                s_w[warp][lane][0] = make_ulonglong2(pack2(s.w[0], s.w[0]), pack2(s.w[1], s.w[1]));
+                s_w[warp][lane][1] = make_ulonglong2(pack2(s.w[2], s.w[2]), pack2(s.w[3], s.w[3]));
+                s_rec[warp][lane] = make_uint2(s.task * p.row_units, flags);
+                s_row[warp][lane] = s.row;
+            }
+            __syncwarp();
+
+            // ---- lanes = (stream, four channels) ------------------------------------------
+#pragma unroll 1
+            for (int t0 = 0; t0 < LPR; t0 += U) {
+                uint32_t flags[U];
+                f32x2 go[U][NV][2];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint2 rec = s_rec[warp][(t0 + u) * S + g];
+                    flags[u] = rec.y;
+                    const T* row = glane + static_cast<size_t>(rec.x) * 4;
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        go[u][k][0] = go[u][k][1] = 0ull;
+                        if (on[k]) load_quad<T>(row + k * (LPR * 4), go[u][k]);
+                    }
+                }
+                float d[U * 4];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int slot = (t0 + u) * S + g;
+                    const uint32_t any = (S == 1) ? flags[u] : __reduce_or_sync(0xffffffffu, flags[u] & 7u);
+                    if (any & kEnters) {
+                        const bool enters = flags[u] & kEnters, jumps = flags[u] & kJumps;
+                        flush(0, enters);
+                        flush(2, enters);
+                        if (any & kJumps) {
+                            flush(1, jumps);
+                            flush(3, jumps);
+                            clear(0, jumps);
+                            clear(2, jumps);
+                        }
+                        shift(0, enters && !jumps);
+                        shift(2, enters && !jumps);
+                        clear(1, enters);
+                        clear(3, enters);
+                        cur = s_row[warp][slot];      // the same for a stream that stays
+                        cell = flags[u] >> 4;
+                        below = (cell >> 4) * step_x;
+                        if (any & kJumps) {
+                            fetch(0, jumps);
+                            fetch(2, jumps);
+                        }
+                        fetch(1, enters);
+                        fetch(3, enters);
+                    }
+                    f32x2 w[4];
+                    {
+                        const ulonglong2 w01 = s_w[warp][slot][0], w23 = s_w[warp][slot][1];
+                        w[0] = w01.x;
+                        w[1] = w01.y;
+                        w[2] = w23.x;
+                        w[3] = w23.y;
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        f32x2 a2 = 0ull;
+#pragma unroll
+                        for (int k = 0; k < NV; ++k)
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                acc[c][k][e] = fma2(w[c], go[u][k][e], acc[c][k][e]);
+                                a2 = (k + e == 0) ? mul2(val[c][k][e], go[u][k][e])
+                                                  : fma2(val[c][k][e], go[u][k][e], a2);
+                            }
+                        const float2 h = unpack2(a2);
+                        d[u * 4 + c] = h.x + h.y;
+                    }
+                    if constexpr (WIDE) {
+                        // A step with an amplified sample forms its dot products in double as
+                        // well; each sample takes the kind it asked for, so its gradients do
+                        // not depend on which samples share the step.
+                        if (any & kAmplified) {
+                            double dd[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                            for (int k = 0; k < NV; ++k)
+#pragma unroll
+                                for (int e = 0; e < 2; ++e) {
+                                    const float2 gf = unpack2(go[u][k][e]);
+                                    const double gx = gf.x, gy = gf.y;
+#pragma unroll
+                                    for (int c = 0; c < 4; ++c) {
+                                        const float2 vf = unpack2(val[c][k][e]);
+                                        dd[c] = fma(static_cast<double>(vf.x), gx, dd[c]);
+                                        dd[c] = fma(static_cast<double>(vf.y), gy, dd[c]);
+                                    }
+                                }
+                            const double r = reduce_values<4, LPR>(dd, j);
+                            if (j % (LPR / 4) == 0) s_wide[warp][slot][j / (LPR / 4)] = r;
+                        }
+                    }
+                }
+                __syncwarp();   // every lane has read the weights of these steps
+                constexpr int N = (U * 4 < LPR) ? U * 4 : LPR;   // dot products per reduction
+#pragma unroll
+                for (int q = 0; q < U * 4 / N; ++q) {
+                    float part[N];
+#pragma unroll
+                    for (int i = 0; i < N; ++i) part[i] = d[q * N + i];
+                    const float r = reduce_values<N, LPR>(part, j);
+                    if (j % (LPR / N) == 0) {
+                        const int v = q * N + j / (LPR / N);
+                        reinterpret_cast<float*>(s_w[warp][(t0 + v / 4) * S + g])[v % 4] = r;
+                    }
+                }
+            }
+            __syncwarp();
+
+            // ---- lane = sample: gradients of location and weight ---------------------------
+            if (at < end) {
+                using Acc = typename std::conditional<WIDE, double, float>::type;
+                const float4 h4 = *reinterpret_cast<const float4*>(s_w[warp][lane]);
+                Acc S4[4] = {h4.x, h4.y, h4.z, h4.w};
+                if constexpr (WIDE) {
+                    if (s.amplified) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) S4[c] = s_wide[warp][lane][c];
+                    }
+                }
+                const Acc lw = s.lw, lh = s.lh, wf = s.wf, hf = s.hf, a = s.a;
+                const Acc hw = Acc(1) - lw, hh = Acc(1) - lh;
+                const float ga = static_cast<float>(hh * hw * S4[0] + hh * lw * S4[1] +
+                                                    lh * hw * S4[2] + lh * lw * S4[3]);
+                const float gx = static_cast<float>(wf * a * (hh * (S4[1] - S4[0]) + lh * (S4[3] - S4[2])));
+                const float gy = static_cast<float>(hf * a * (hw * (S4[2] - S4[0]) + lw * (S4[3] - S4[1])));
+                store_pair(static_cast<TL*>(p.grad_loc) + 2ull * s.id, gx, gy);
+                static_cast<TL*>(p.grad_attn)[s.id] = Elem<TL>::from_f(ga);
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) flush(c, true);
+    }
+}
+
+// Nearest-pixel main kernel: one row per sample. LPR lanes cover a row (four channels each, NV
+// times), 32 / LPR samples of one pixel are worked on at a time and share its row.
+template <typename T, typename TL, int NV, int LPR>
+__global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 4)
+gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
+    constexpr int U = 4;            // rows of grad_out in flight per lane
+    constexpr int SL = 32 / LPR;    // samples per step
+    __shared__ SortLevels lv;
+    __shared__ float s_dot[kWarpsPerCta][32];
+    if (!load_sort_levels(p, lv)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = lane % LPR, g = lane / LPR;
+    float* dot = s_dot[warp];
+    bool on[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) on[k] = (j + k * LPR) * 4 < p.D;
+    const T* vlane = static_cast<const T*>(p.value) + j * 4;
+    const T* glane = static_cast<const T*>(p.grad_out) + j * 4;
+    float* alane = static_cast<float*>(p.grad_value) + j * 4;
+
+    Ticket ticket;
+    while (next_ticket(sp, sp.stream, lane, ticket)) {
+        const uint32_t base = ticket.begin, end = ticket.end;
+        if (base >= end) continue;
+        f32x2 acc[NV][2], val[NV][2];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) acc[k][0] = acc[k][1] = val[k][0] = val[k][1] = 0ull;
+        uint32_t cur = 0u, cell = 0u;
+        auto flush = [&]() {
+            if (cell & 1u) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float2 a = unpack2(acc[k][e]);
+#pragma unroll
+                        for (int o = LPR; o < 32; o <<= 1) {
+                            a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+                            a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+                        }
+                        acc[k][e] = pack2(a.x, a.y);
+                    }
+                    if (g == 0 && on[k])
+                        red_quad(alane + (static_cast<size_t>(cur) + k * LPR) * 4, acc[k]);
+                }
+            }
+        };
+        RawSample raw;
+        raw.id = base + lane < end ? __ldg(sp.sorted + base + lane) : 0u;
+        uint32_t next_id = base + 32 + lane < end ? __ldg(sp.sorted + base + 32 + lane) : 0u;
+        load_raw<TL>(p, raw, base + lane < end);
+        for (uint32_t at = base; at < end; at += 32) {
+            const int n = min(32, static_cast<int>(end - at));
+            RawSample next;
+            next.id = next_id;
+            load_raw<TL>(p, next, at + 32 + lane < end);
+            next_id = at + 64 + lane < end ? __ldg(sp.sorted + at + 64 + lane) : 0u;
+            const SortedSample s = set_up_sample<1>(p, sp, lv, raw, lane < n);
+            raw = next;
+            uint32_t prow = __shfl_up_sync(0xffffffffu, s.row, 1);
+            uint32_t pcell = __shfl_up_sync(0xffffffffu, s.cell, 1);
+            if (lane == 0) {
+                prow = cur;
+                pcell = cell;
+            }
+            const uint32_t m_other =
+                __ballot_sync(0xffffffffu, lane < n && (s.row != prow || s.cell != pcell));
+#pragma unroll 1
+            for (int first = 0; first < n;) {
+                // samples [first, last) share a pixel
+                const uint32_t later = m_other & ~((2u << first) - 1u);
+                const int last = later != 0u ? __ffs(later) - 1 : n;
+                if ((m_other >> first) & 1u) {
+                    flush();
+                    cur = __shfl_sync(0xffffffffu, s.row, first);
+                    cell = __shfl_sync(0xffffffffu, s.cell, first);
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        acc[k][0] = acc[k][1] = val[k][0] = val[k][1] = 0ull;
+                        if (on[k] && (cell & 1u))
+                            load_quad<T>(vlane + (static_cast<size_t>(cur) + k * LPR) * 4, val[k]);
+                    }
+                }
+#pragma unroll 1
+                for (int i0 = first; i0 < last; i0 += U * SL) {
+                    f32x2 go[U][NV][2];
+                    float w[U], d[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int i = i0 + u * SL + g;
+                        const uint32_t task = __shfl_sync(0xffffffffu, s.task, i);
+                        w[u] = __shfl_sync(0xffffffffu, s.a, i);
+                        const bool live = i < last;
+                        const T* row = glane + static_cast<size_t>(task) * p.D;
+#pragma unroll
+                        for (int k = 0; k < NV; ++k) {
+                            go[u][k][0] = go[u][k][1] = 0ull;
+                            if (live && on[k]) load_quad<T>(row + k * (LPR * 4), go[u][k]);
+                        }
+                        if (!live) w[u] = 0.f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const f32x2 w2 = pack2(w[u], w[u]);
+                        f32x2 a2 = 0ull;
+#pragma unroll
+                        for (int k = 0; k < NV; ++k)
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                acc[k][e] = fma2(w2, go[u][k][e], acc[k][e]);
+                                a2 = (k + e == 0) ? mul2(val[k][e], go[u][k][e])
+                                                  : fma2(val[k][e], go[u][k][e], a2);
+                            }
+                        const float2 h = unpack2(a2);
+                        d[u] = h.x + h.y;
+                    }
+                    const float r = reduce_values<U, LPR>(d, j);
+                    const int i = i0 + (j / (LPR / U)) * SL + g;
+                    if (j % (LPR / U) == 0 && i < last) dot[i] = r;
+                }
+                first = last;
+            }
+            __syncwarp();
+            if (lane < n) static_cast<TL*>(p.grad_attn)[s.id] = Elem<TL>::from_f(dot[lane]);
+            __syncwarp();
+        }
+        flush();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// launch
+// ---------------------------------------------------------------------------
+// `streams` per warp, a round of 32 samples being 32 / streams steps of each.
+template <typename Kernel>
+static cudaError_t launch_sorted_main(Kernel kern, int streams, const Params& p, SortParams sp,
+                                      const LaunchShape& ls, cudaStream_t stream) {
+    int per_sm = ls.ctas_per_sm;
+    if (per_sm <= 0) {
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreadsPerCta, 0);
+        if (e != cudaSuccess) return e;
+        if (per_sm < 1) per_sm = 1;
+    }
+    const uint32_t cap = static_cast<uint32_t>(ls.sm_count) * per_sm;
+    // Long streams enter fewer cells, short ones level the load: eight tickets per resident
+    // warp, as long as a stream keeps one round.
+    const uint32_t want = sp.nsamples / (cap * kWarpsPerCta * 8u * streams);
+    const uint32_t round = 32u / streams;
+    sp.stream = want / round * round;
+    if (sp.stream < round) sp.stream = round;
+    if (sp.stream > kMaxStream) sp.stream = kMaxStream;
+    const uint32_t len = sp.stream * streams;
+    sp.tickets_per_region = (static_cast<uint32_t>(p.Q) * p.P + len - 1) / len;
+    sp.fd_tickets = make_fastdiv(sp.tickets_per_region);
+    sp.tickets = sp.nregions * sp.tickets_per_region;
+    const uint32_t need = (sp.tickets + kWarpsPerCta - 1) / kWarpsPerCta;
+    kern<<<need < cap ? need : cap, kThreadsPerCta, 0, stream>>>(p, sp);
+    return cudaGetLastError();
+}
+
+template <typename TL, int CPS>
+static cudaError_t launch_sort(const Params& p, SortParams& sp, const LaunchShape& ls,
+                               cudaStream_t stream) {
+    cudaError_t e;
+    auto kern = sort_cells_kernel<TL, CPS>;
+    const int smem = static_cast<int>(kSortCells * sizeof(uint32_t));
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    // the smallest cluster that gives most SMs work
+    const uint32_t levels = static_cast<uint32_t>(p.B) * p.H * p.L;
+    sp.parts = 1;
+    while (sp.parts < kMaxSortParts && levels * sp.parts < 3u * ls.sm_count / 2u) sp.parts *= 2;
+    sp.nregions = levels;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(levels * sp.parts);
+    cfg.blockDim = dim3(kSortThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = sp.parts;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, p, sp);
+}
+
+template <typename T, typename TL>
+static cudaError_t launch_sorted_bilinear(const Params& p, SortParams sp,
+                                          const LaunchShape& ls, cudaStream_t stream) {
+    cudaError_t e = launch_sort<TL, 4>(p, sp, ls, stream);
+    if (e != cudaSuccess) return e;
+    if (p.D <= 16) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 4>, 8, p, sp, ls, stream);
+    if (p.D <= 32) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 8>, 4, p, sp, ls, stream);
+    if (p.D <= 64) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 16>, 2, p, sp, ls, stream);
+    if (p.D <= 128) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 32>, 1, p, sp, ls, stream);
+    return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 2, 32>, 1, p, sp, ls, stream);
+}
+
+template <typename T>
+static cudaError_t launch_sorted_nearest(const Params& p, SortParams sp,
+                                         const LaunchShape& ls, cudaStream_t stream) {
+    cudaError_t e = launch_sort<T, 1>(p, sp, ls, stream);
+    if (e != cudaSuccess) return e;
+    if (p.D <= 16) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 4>, 1, p, sp, ls, stream);
+    if (p.D <= 32) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 8>, 1, p, sp, ls, stream);
+    if (p.D <= 64) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 16>, 1, p, sp, ls, stream);
+    if (p.D <= 128) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 32>, 1, p, sp, ls, stream);
+    return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 2, 32>, 1, p, sp, ls, stream);
+}
+
+}  // namespace msda

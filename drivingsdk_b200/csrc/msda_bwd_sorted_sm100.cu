@@ -1,0 +1,16 @@
+// MSDA backward over cell-sorted samples for sm_100a (msda_bwd_sorted.cuh), all types.
+#include "msda_bwd_sorted.cuh"
+
+namespace msda {
+
+cudaError_t launch_backward_sorted(const Params& p, const SortParams& sp, int dtype,
+                                   const LaunchShape& ls, cudaStream_t stream) {
+    switch (dtype) {
+        case 0: return launch_sorted_bilinear<float, float>(p, sp, ls, stream);
+        case 1: return launch_sorted_bilinear<__half, __half>(p, sp, ls, stream);
+        case 2: return launch_sorted_bilinear<__nv_bfloat16, __nv_bfloat16>(p, sp, ls, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace msda

@@ -28,6 +28,7 @@ std::atomic<int> g_tune_spin{msda::kSpinLimit};
 std::atomic<int> g_tune_precise_amp{8};
 std::atomic<int> g_tune_debug_rows{0};
 std::atomic<int> g_tune_pack{1};
+std::atomic<int> g_tune_sort{1};
 std::atomic<long long> g_launches{0};
 thread_local int t_last_cuda_error = 0;
 thread_local cudaEvent_t t_prof[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -111,6 +112,16 @@ RowPlan plan_rows(int D, int dtype, bool ptrs_16B_aligned) {
     return rp;
 }
 
+// One past the last valid row offset.
+uint32_t debug_limit(unsigned long long rows, unsigned long long units) {
+#ifdef MSDA_DEBUG_BOUNDS
+    // test hook of the bounds-checking build: pretend value / grad_value end after this many rows
+    const unsigned long long pretend = static_cast<unsigned long long>(g_tune_debug_rows.load());
+    if (pretend > 0 && pretend < rows) return static_cast<uint32_t>(pretend * units);
+#endif
+    return static_cast<uint32_t>(rows * units);
+}
+
 // Offsets of value rows travel as 32-bit counts of `row_units`: 16-byte pieces on the vector
 // path, elements on the scalar path.
 int set_row_units(Params& p, const RowPlan& rp, int dtype) {
@@ -120,13 +131,55 @@ int set_row_units(Params& p, const RowPlan& rp, int dtype) {
     const unsigned long long rows = static_cast<unsigned long long>(p.B) * p.K * p.H;
     if (rows * units >= 0xffffffffull) return MSDA_ERR_LIMIT;
     p.row_units = static_cast<uint32_t>(units);
-    p.limit_units = static_cast<uint32_t>(rows * units);
-#ifdef MSDA_DEBUG_BOUNDS
-    // test hook of the bounds-checking build: pretend value / grad_value end after this many rows
-    const unsigned long long pretend = static_cast<unsigned long long>(g_tune_debug_rows.load());
-    if (pretend > 0 && pretend < rows) p.limit_units = static_cast<uint32_t>(pretend * units);
-#endif
+    p.limit_units = debug_limit(rows, units);
     return MSDA_OK;
+}
+
+// Layout of the sorted backward's workspace: fp32 accumulation rows (16-bit tensors only),
+// ticket counter, regions, sorted sample numbers.
+struct SortPlan {
+    size_t ticket, regions, sorted, total;
+    uint32_t nsamples;
+};
+
+// False where the sorted backward does not apply: rows that are not whole groups of four
+// channels, more samples than 32-bit counters hold.
+bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, SortPlan* s) {
+    if (D % 4 != 0) return false;
+    const unsigned long long n = 1ull * B * Q * H * L * P;
+    // ... nor as many tickets (regions of a few samples each get one)
+    if (n + 1ull * B * H * L >= (1ull << 31) ||
+        1ull * B * Q * H * (D / 4) >= (1ull << 32))
+        return false;
+    auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+    s->nsamples = static_cast<uint32_t>(n);
+    s->ticket = dtype == MSDA_F32 ? 0 : up(static_cast<size_t>(B) * K * H * D * 4);
+    s->regions = s->ticket + 256;
+    s->sorted = s->regions + up(static_cast<size_t>(B) * H * L * sizeof(uint2));
+    s->total = s->sorted + up(n * 4);
+    return true;
+}
+
+// Where sorting pays: the gain is the rows that samples of one cell share, the cost a sort of
+// 15-25 ps per sample, so it takes enough samples per cell, fewer of them the longer the rows.
+// Measured on one level set from 64x100 down, uniform locations, old / sorted (us):
+//   D = 128  0.26 M samples, 1.9 per cell: 128 / 122   0.77 M, 5.6: 288 / 190   6.9 M, 51: 2412 / 1028
+//   D = 64   5.6 per cell: 154 / 145   17: 418 / 285   51: 1216 / 669
+//   D = 32   17 per cell: 204 / 233 (fp32), 233 / 209 (bf16)   51: 582 / 495, 654 / 411
+// (fp32 unless noted; with one query per pixel and samples around it, as in an encoder, 17 per cell
+// pays for fp32 at D = 32 too: 431 / 366). Below about 0.1 M samples two more launches cost more
+// than they save. The nearest-pixel operator has one row per sample and no double-precision
+// dot products: 519 / 397 at 24 x 107 k samples on 375 pixels.
+bool sort_pays(const SortPlan& s, int K, int H, int D, int dtype, int B, int mode) {
+    if (mode == kFused || g_tune_sort.load() == 0) return false;
+    if (g_tune_sort.load() == 2) return true;
+    if (s.nsamples < 100000u) return false;
+    const double per_cell = static_cast<double>(s.nsamples) / (static_cast<double>(B) * K * H);
+    if (mode == kNearest) return per_cell >= 16.0;
+    if (D > 64) return per_cell >= 3.0;
+    if (D > 32) return per_cell >= 6.0;
+    if (D > 16) return per_cell >= (dtype == MSDA_F32 ? 15.0 : 12.0) && s.nsamples >= 1000000u;
+    return per_cell >= (dtype == MSDA_F32 ? 50.0 : 25.0);
 }
 
 // Fills the parts of Params common to both directions.
@@ -228,6 +281,46 @@ int backward_impl(const void* value, const int32_t* shapes, const int32_t* start
 
     const long long nval = static_cast<long long>(B) * K * H * D;
     const bool acc_f32 = use_ws && dtype != MSDA_F32;
+    // the sorted form, where the caller brought the workspace for it
+    SortPlan plan;
+    if (use_ws && plan_sort(B, K, H, D, L, Q, P, dtype, &plan) &&
+        sort_pays(plan, K, H, D, dtype, B, mode) &&
+        workspace && workspace_bytes >= plan.total && aligned_to(workspace, 16) &&
+        aligned_to(value, 4 * e) && aligned_to(grad_out, 4 * e) &&
+        aligned_to(acc_f32 ? workspace : grad_value, 16) && aligned_to(loc, 2 * e)) {
+        char* ws = static_cast<char*>(workspace);
+        float* acc = static_cast<float*>(acc_f32 ? workspace : grad_value);
+        const unsigned long long quads = static_cast<unsigned long long>(D) / 4;
+        if (static_cast<unsigned long long>(B) * K * H * quads < 0xffffffffull) {
+            p.row_units = static_cast<uint32_t>(quads);
+            p.limit_units = debug_limit(static_cast<unsigned long long>(B) * K * H, quads);
+            p.grad_out = grad_out;
+            p.grad_value = acc;
+            p.grad_loc = grad_loc;
+            p.grad_attn = grad_attn;
+            msda::SortParams sp{};
+            sp.ticket = reinterpret_cast<uint32_t*>(ws + plan.ticket);
+            sp.regions = reinterpret_cast<uint2*>(ws + plan.regions);
+            sp.sorted = reinterpret_cast<uint32_t*>(ws + plan.sorted);
+            sp.nsamples = plan.nsamples;
+            sp.fd_p = msda::make_fastdiv(static_cast<uint32_t>(P));
+            const msda::LaunchShape shape{dev->sm_count, g_tune_cps_bwd.load()};
+            cudaError_t ce = cudaMemsetAsync(acc, 0, static_cast<size_t>(nval) * sizeof(float), stream);
+            if (ce != cudaSuccess) return fail_cuda(ce);
+            prof_record(2, stream);
+            ce = nearest ? msda::launch_gka_backward_sorted(p, sp, dtype, shape, stream)
+                                     : msda::launch_backward_sorted(p, sp, dtype, shape, stream);
+            prof_record(3, stream);
+            if (ce != cudaSuccess) return fail_cuda(ce);
+            g_launches.fetch_add(2, std::memory_order_relaxed);
+            if (acc_f32) {
+                ce = msda::launch_downcast(acc, grad_value, nval, dtype, stream);
+                if (ce != cudaSuccess) return fail_cuda(ce);
+                g_launches.fetch_add(1, std::memory_order_relaxed);
+            }
+            return MSDA_OK;
+        }
+    }
     void* acc = grad_value;
     size_t acc_bytes = static_cast<size_t>(nval) * e;
     if (acc_f32) {
@@ -401,6 +494,24 @@ size_t msda_sm100_backward_workspace_bytes(int B, int K, int H, int D, int dtype
     return static_cast<size_t>(B) * K * H * D * sizeof(float);
 }
 
+static size_t sorted_workspace(int B, int K, int H, int D, int L, int Q, int P, int dtype, int mode) {
+    SortPlan plan;
+    if (check_dims(B, K, H, D, L, Q, P, dtype) != MSDA_OK ||
+        !plan_sort(B, K, H, D, L, Q, P, dtype, &plan) || !sort_pays(plan, K, H, D, dtype, B, mode))
+        return msda_sm100_backward_workspace_bytes(B, K, H, D, dtype);
+    return plan.total;
+}
+
+size_t msda_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
+                                                  int dtype) {
+    return sorted_workspace(B, K, H, D, L, Q, P, dtype, kBilinear);
+}
+
+size_t gka_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
+                                                 int dtype) {
+    return sorted_workspace(B, K, H, D, L, Q, P, dtype, kNearest);
+}
+
 int msda_sm100_backward_ws(const void* value, const int32_t* spatial_shapes,
                            const int32_t* level_start_index, const void* sampling_locations,
                            const void* attention_weights, const void* grad_output,
@@ -456,6 +567,7 @@ int msda_sm100_tune(int knob, int value) {
         case MSDA_TUNE_PRECISE_AMP: target = &g_tune_precise_amp; break;
         case MSDA_TUNE_DEBUG_ROW_LIMIT: target = &g_tune_debug_rows; break;
         case MSDA_TUNE_PACK_ROWS: target = &g_tune_pack; break;
+        case MSDA_TUNE_SORT: target = &g_tune_sort; break;
         default: return MSDA_ERR_DIMS;
     }
     if (value < 0) return target->load();

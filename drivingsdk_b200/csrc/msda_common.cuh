@@ -38,8 +38,9 @@ constexpr int kStatusBadLevels = 4;     // device-resident level table inconsist
 constexpr int kStatusOutOfBounds = 16;  // MSDA_DEBUG_BOUNDS build: a computed row offset fell outside
                                         // value / grad_value; the access was skipped
 
-// Division by a runtime constant without a divide: q = (n * mul) >> shift, exact
-// for 0 <= n < 2^31 (round-up method with a 31 + ceil(log2 d) bit shift).
+// Division by a runtime constant without a divide: q = (n * mul) >> (31 + s) with
+// s = ceil(log2 d), exact for 0 <= n < 2^31 (round-up method); as (2n * mul) >> 32 >> s it is
+// one high multiplication and 32-bit shifts.
 struct FastDiv {
     uint32_t mul;
     uint32_t shift;
@@ -48,12 +49,18 @@ inline FastDiv make_fastdiv(uint32_t d) {
     uint32_t s = 0;
     while ((1ull << s) < d) ++s;
     FastDiv f;
-    f.shift = 31 + s;
-    f.mul = static_cast<uint32_t>(((1ull << f.shift) + d - 1) / d);
+    f.shift = s;
+    f.mul = static_cast<uint32_t>(((1ull << (31 + s)) + d - 1) / d);
+    return f;
+}
+__device__ __forceinline__ FastDiv device_fastdiv(uint32_t d) {
+    FastDiv f;
+    f.shift = d > 1u ? 32u - __clz(d - 1u) : 0u;
+    f.mul = static_cast<uint32_t>(((1ull << (31 + f.shift)) + d - 1) / d);
     return f;
 }
 __device__ __forceinline__ uint32_t fd_div(uint32_t n, const FastDiv& f) {
-    return static_cast<uint32_t>((static_cast<uint64_t>(n) * f.mul) >> f.shift);
+    return __umulhi(n + n, f.mul) >> f.shift;
 }
 
 // Kernel modes (template parameter): rows per sample, or the fused bilinear variant whose

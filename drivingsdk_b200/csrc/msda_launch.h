@@ -57,6 +57,26 @@ cudaError_t launch_gka_forward(const Params& p, int dtype, const RowPlan& rp,
 cudaError_t launch_gka_backward(const Params& p, int dtype, int acc_f32, const RowPlan& rp,
                                 const LaunchShape& ls, cudaStream_t stream);
 
+// Scratch of the backward over cell-sorted samples (msda_bwd_sorted.cuh); device memory, part of
+// the caller's workspace.
+constexpr uint32_t kMaxSortParts = 8;
+struct SortParams {
+    uint32_t* ticket;       // next ticket of the main kernel
+    uint2* regions;         // [B * H * L] {first position, samples} of each sorted region
+    uint32_t* sorted;       // [nsamples] sample numbers, cell by cell
+    uint32_t nsamples;
+    FastDiv fd_p;           // division by the points per level
+    // set by the launch:
+    uint32_t parts;         // CTAs per (batch, head, level) of the sort
+    uint32_t nregions, tickets, tickets_per_region;
+    FastDiv fd_tickets;     // division by tickets_per_region
+    uint32_t stream;        // sorted samples per stream
+};
+cudaError_t launch_backward_sorted(const Params& p, const SortParams& sp, int dtype,
+                                   const LaunchShape& ls, cudaStream_t stream);
+cudaError_t launch_gka_backward_sorted(const Params& p, const SortParams& sp, int dtype,
+                                       const LaunchShape& ls, cudaStream_t stream);
+
 // Fused variant (reference points + offsets + logits instead of locations + weights).
 cudaError_t launch_fused_forward(const Params& p, int dtype, const RowPlan& rp,
                                  const LaunchShape& ls, cudaStream_t stream);

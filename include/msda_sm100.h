@@ -96,6 +96,16 @@ int msda_sm100_backward_ws(const void* value, const int32_t* spatial_shapes,
                            void* workspace, size_t workspace_bytes, int B, int K, int H, int D,
                            int L, int Q, int P, int dtype, void* stream);
 
+/* Workspace with which msda_sm100_backward_ws() and gka_sm100_backward_ws() take their form over
+ * samples sorted by the cell they fall into, whose shared rows are loaded and reduced once. Any
+ * smaller workspace that satisfies the rule above selects the form that needs no sort. Equals
+ * msda_sm100_backward_workspace_bytes() where the sort would not apply (D not a multiple of
+ * four) or not pay (few samples per cell). */
+size_t msda_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
+                                                  int dtype);
+size_t gka_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
+                                                 int dtype);
+
 /* Backward for callers that cannot allocate device memory. It has no counterpart
  * in the reference (there the framework allocates the operator's workspace for
  * it). Who needs it: a host whose device memory is fully planned before the
@@ -256,7 +266,11 @@ int msda_sm100_device_status(int clear);
  *   MSDA_TUNE_PACK_ROWS      1 (default): the forward kernels of the bilinear operators keep a
  *                            record only for the corners that exist and walk those; 0 = one
  *                            record per (sample, corner), missing ones skipped one by one.
- *                            Same results either way. */
+ *                            Same results either way.
+ *   MSDA_TUNE_SORT           1 (default): the backward sorts its samples by cell where the
+ *                            workspace allows it and the size makes it pay; 0 = never;
+ *                            2 = wherever the workspace allows it (ask for its size with this
+ *                            set). Same results within rounding. */
 typedef enum msda_tune {
     MSDA_TUNE_STAGE = 0,
     MSDA_TUNE_CTAS_PER_SM = 1,
@@ -265,7 +279,8 @@ typedef enum msda_tune {
     MSDA_TUNE_SPIN_LIMIT = 4,
     MSDA_TUNE_PRECISE_AMP = 5,
     MSDA_TUNE_DEBUG_ROW_LIMIT = 6,
-    MSDA_TUNE_PACK_ROWS = 7
+    MSDA_TUNE_PACK_ROWS = 7,
+    MSDA_TUNE_SORT = 8
 } msda_tune;
 int msda_sm100_tune(int knob, int value);
 
