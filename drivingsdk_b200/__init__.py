@@ -62,6 +62,13 @@ __all__ = (list(_OP_NAMES) + list(_FUSED_NAMES) + list(_GKA_NAMES) + list(_DA_NA
 
 
 def __getattr__(name):
+    # looked up once: the name is a module attribute from then on
+    value = _load(name)
+    globals()[name] = value
+    return value
+
+
+def _load(name):
     if name in _OP_NAMES:
         mod = importlib.import_module(__name__ + ".ops.multi_scale_deformable_attn")
         return getattr(mod, name)

@@ -27,6 +27,7 @@ CUDA_SOURCES = ["msda_capi.cu", "msda_fwd_sm100.cu", "msda_bwd_sm100.cu", "gka_f
                 "gka_bwd_sm100.cu", "msda_bwd_sorted_sm100.cu", "gka_bwd_sorted_sm100.cu", "msda_fused_fwd_sm100.cu", "msda_fused_bwd_sm100.cu", "da_sm100.cu",
                 "msda_static_scratch.cu", "hw_probe_sm100.cu", "resnet_ops_sm100.cu", "dcn_sm100.cu",
                 "gemm_simt_sm100.cu", "gemm_tc_sm100.cu"]
+EXT_SOURCES = ["binding.cpp", "autograd.cpp"]
 CUDA_HEADERS = ["msda_common.cuh", "msda_tile.cuh", "msda_launch.h", "msda_fwd_kernel.cuh",
                 "msda_bwd_kernel.cuh", "msda_bwd_sorted.cuh", "gemm_sm100.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -86,11 +87,13 @@ def build_library(force=False, verbose_ptxas=False, debug_bounds=False) -> str:
 
 
 def build_extension(force=False) -> str:
-    src = os.path.join(CSRC, "binding.cpp")
-    deps = [src, os.path.join(ROOT, "include", "msda_sm100.h"),
-            os.path.join(ROOT, "include", "conv_ops_sm100.h"), LIB]
+    srcs = [os.path.join(CSRC, f) for f in EXT_SOURCES]
+    deps = srcs + [os.path.join(CSRC, "bindings.h"), os.path.join(ROOT, "include", "msda_sm100.h"),
+                   os.path.join(ROOT, "include", "conv_ops_sm100.h"), LIB]
     if not (force or _stale(EXT, deps)):
         return EXT
+    from concurrent.futures import ThreadPoolExecutor
+
     import torch
     from torch.utils import cpp_extension
 
@@ -101,13 +104,17 @@ def build_extension(force=False) -> str:
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda_lib = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "lib64")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-            "-DTORCH_EXTENSION_NAME=_C", "-DTORCH_API_INCLUDE_EXTENSION_H",
-            f"-D_GLIBCXX_USE_CXX11_ABI={abi}"] + inc + [src, "-o", EXT,
-            f"-L{PKG}", "-lmsda_sm100", f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
-            "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-L{cuda_lib}", "-lcudart",
-            "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}", f"-Wl,-rpath,{cuda_lib}"])
-    _run(cmd, "g++ binding")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_C",
+             "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={abi}"] + inc
+    os.makedirs(OBJ_DIR + "_ext", exist_ok=True)
+    objs = [os.path.join(OBJ_DIR + "_ext", os.path.basename(f)[:-4] + ".o") for f in srcs]
+    with ThreadPoolExecutor(max_workers=len(srcs)) as pool:
+        list(pool.map(lambda so: _run(["g++"] + flags + ["-c", so[0], "-o", so[1]],
+                                      "g++ " + os.path.basename(so[0])), zip(srcs, objs)))
+    _run(["g++", "-shared"] + objs + ["-o", EXT, f"-L{PKG}", "-lmsda_sm100", f"-L{torch_lib}", "-lc10",
+          "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-L{cuda_lib}",
+          "-lcudart", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}", f"-Wl,-rpath,{cuda_lib}"],
+         "g++ link")
     return EXT
 
 

@@ -42,6 +42,7 @@ SIGNATURES = {
     "msda_sm100_backward_static": (_i, [_vp, _ip, _ip, _vp, _vp, _vp, _vp, _vp, _vp] + _DIMS7
                                    + [_i, _vp]),
     "addrelu_sm100_forward": (_i, [_vp, _vp, _sz, _i, _vp]),
+    "addrelu_sm100_forward_out": (_i, [_vp, _vp, _vp, _sz, _i, _vp]),
     "addrelu_sm100_backward": (_i, [_vp, _vp, _vp, _sz, _i, _vp]),
     "maxpool_sm100_forward": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "dcn_sm100_columns_bytes": (_sz, [_vp]),

@@ -1,0 +1,223 @@
+// The differentiable operators, as C++ autograd functions. For calls of a few tens of
+// microseconds the host work of Python autograd functions (argument marshalling, autocast
+// decorators, the interpreter lock in the backward thread) is most of the time: 112 us per forward +
+// backward of 1000 queries against 40 us of kernels. Behaviour is that of the Python classes next
+// to them in drivingsdk_b200/ops (which callers may still subclass, patch or apply):
+//   * under autocast the attention operators run in float32 on cast inputs;
+//   * an empty operand raises the reference's Exception;
+//   * gradients are once-differentiable: using them in a graph raises.
+#include <ATen/autocast_mode.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/extension.h>
+
+#include "bindings.h"
+
+namespace sdk {
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+[[noreturn]] void raise_empty() {
+    pybind11::gil_scoped_acquire gil;
+    PyErr_SetString(PyExc_Exception, "Error! Input Tensor can not be a empty Tensor.\n");
+    throw pybind11::error_already_set();
+}
+
+// custom_fwd(cast_inputs=torch.float32)
+Tensor autocast_f32(const Tensor& t, bool on) {
+    return on && t.is_floating_point() && t.is_cuda() && t.scalar_type() != at::kDouble
+               ? t.to(at::kFloat)
+               : t;
+}
+
+// @once_differentiable: where a graph of the gradients is asked for, they carry a node that
+// raises when it is used.
+variable_list once(variable_list grads, const Tensor& grad_out) {
+    if (!at::GradMode::is_enabled() || !grad_out.requires_grad()) return grads;
+    variable_list in;
+    for (auto& g : grads) {
+        Tensor t = g;
+        if (t.defined()) {
+            t = t.detach();
+            t.requires_grad_(true);
+        }
+        in.push_back(t);
+    }
+    auto node = std::make_shared<torch::autograd::DelayedError>(
+        "trying to differentiate twice a function that was marked with @once_differentiable",
+        static_cast<int64_t>(in.size()));
+    return (*node)(std::move(in));
+}
+
+// int32 or int64 level tables, both alike
+void tables(Tensor& shapes, Tensor& starts) {
+    const auto kind = shapes.scalar_type();
+    if (kind == starts.scalar_type() && (kind == at::kInt || kind == at::kLong)) return;
+    shapes = shapes.to(at::kInt);
+    starts = starts.to(at::kInt);
+}
+
+struct Msda : Function<Msda> {
+    static Tensor forward(AutogradContext* ctx, Tensor value, Tensor shapes, Tensor starts,
+                          Tensor loc, Tensor attn) {
+        const bool cast = at::autocast::is_autocast_enabled(at::kCUDA);
+        value = autocast_f32(value, cast);
+        if (value.numel() == 0 || shapes.numel() == 0 || attn.numel() == 0) raise_empty();
+        tables(shapes, starts);
+        loc = loc.to(value.scalar_type());
+        attn = attn.to(value.scalar_type());
+        Tensor out = msda_forward(value, shapes, starts, loc, attn);
+        ctx->save_for_backward({value, shapes, starts, loc, attn});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        auto [gv, gl, ga] = [&] {
+            const at::NoGradGuard no_grad;
+            return msda_backward(s[0], s[1], s[2], s[3], s[4], g[0]);
+        }();
+        return once({gv, Tensor(), Tensor(), gl, ga}, g[0]);
+    }
+};
+
+struct Fused : Function<Fused> {
+    static Tensor forward(AutogradContext* ctx, Tensor value, Tensor shapes, Tensor starts,
+                          Tensor ref, Tensor off, Tensor logits) {
+        const bool cast = at::autocast::is_autocast_enabled(at::kCUDA);
+        value = autocast_f32(value, cast);
+        if (value.numel() == 0 || shapes.numel() == 0 || logits.numel() == 0) raise_empty();
+        tables(shapes, starts);
+        ref = ref.to(value.scalar_type());
+        off = off.to(value.scalar_type());
+        logits = logits.to(value.scalar_type());
+        Tensor out = msda_fused_forward(value, shapes, starts, ref, off, logits);
+        ctx->save_for_backward({value, shapes, starts, ref, off, logits});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        auto [gv, gr, go, gl] = [&] {
+            const at::NoGradGuard no_grad;
+            return msda_fused_backward(s[0], s[1], s[2], s[3], s[4], s[5], g[0]);
+        }();
+        return once({gv, Tensor(), Tensor(), gr, go, gl}, g[0]);
+    }
+};
+
+struct Gka : Function<Gka> {
+    static Tensor forward(AutogradContext* ctx, Tensor value, Tensor shapes, Tensor starts,
+                          Tensor loc, Tensor attn) {
+        TORCH_CHECK(value.dim() == 4, "geometric_kernel_attention: value [bs, keys, heads, dims] expected");
+        // written in full by the kernel
+        Tensor out = at::empty({value.size(0), attn.size(1), value.size(2) * value.size(3)}, value.options());
+        geometric_kernel_attention_forward(value, shapes, starts, loc, attn, out);
+        ctx->save_for_backward({value, shapes, starts, loc, attn});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        const at::NoGradGuard no_grad;
+        auto [gv, ga] = geometric_kernel_attention_backward(s[0], s[1], s[2], s[3], s[4], g[0]);
+        return {gv, Tensor(), Tensor(), Tensor(), ga};
+    }
+};
+
+struct Aggregation : Function<Aggregation> {
+    static Tensor forward(AutogradContext* ctx, Tensor feat, Tensor shape, Tensor start, Tensor loc,
+                          Tensor wts) {
+        if (feat.numel() == 0 || wts.numel() == 0) raise_empty();
+        feat = feat.contiguous();
+        shape = shape.contiguous().to(at::kInt);
+        start = start.contiguous().to(at::kInt);
+        loc = loc.contiguous();
+        wts = wts.contiguous();
+        Tensor out = deformable_aggregation(feat, shape, start, loc, wts);
+        ctx->save_for_backward({feat, shape, start, loc, wts});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        if (s[0].numel() == 0 || s[1].numel() == 0 || s[3].numel() == 0) raise_empty();
+        const at::NoGradGuard no_grad;
+        auto [gf, gl, gw] = deformable_aggregation_backward(s[0], s[1], s[2], s[3], s[4], g[0],
+                                                            Tensor(), Tensor(), Tensor());
+        return {gf, Tensor(), Tensor(), gl, gw};
+    }
+};
+
+// the reference overwrites x only from this size up (mx_driving/ops/npu_add_relu.py:22)
+constexpr int64_t kInPlaceMinNumel = 2000000;
+
+struct AddRelu : Function<AddRelu> {
+    static Tensor forward(AutogradContext* ctx, Tensor x, const Tensor& y, bool in_place) {
+        Tensor out;
+        if (in_place) {
+            out = npu_add_relu(x, y);
+            ctx->mark_dirty({x});
+        } else {
+            out = add_relu_out(x, y);
+        }
+        ctx->save_for_backward({out});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const at::NoGradGuard no_grad;
+        const Tensor r = npu_add_relu_grad(ctx->get_saved_variables()[0], g[0]);
+        return {r, r, Tensor()};
+    }
+};
+
+// inference only, as in the reference: the result knows its input, but has no derivative
+struct MaxPool : Function<MaxPool> {
+    static Tensor forward(AutogradContext*, const Tensor& x, int64_t kernel, int64_t stride,
+                          int64_t padding) {
+        return npu_max_pool2d(x, static_cast<int>(kernel), static_cast<int>(stride),
+                              static_cast<int>(padding));
+    }
+    static variable_list backward(AutogradContext*, variable_list) {
+        TORCH_CHECK_NOT_IMPLEMENTED(false, "npu_max_pool2d has no backward");
+    }
+};
+
+Tensor msda(const Tensor& value, const Tensor& shapes, const Tensor& starts, const Tensor& loc,
+            const Tensor& attn) {
+    return Msda::apply(value, shapes, starts, loc, attn);
+}
+Tensor fused(const Tensor& value, const Tensor& shapes, const Tensor& starts, const Tensor& ref,
+             const Tensor& off, const Tensor& logits) {
+    return Fused::apply(value, shapes, starts, ref, off, logits);
+}
+Tensor gka(const Tensor& value, const Tensor& shapes, const Tensor& starts, const Tensor& loc,
+           const Tensor& attn) {
+    return Gka::apply(value, shapes, starts, loc, attn);
+}
+Tensor aggregation(const Tensor& feat, const Tensor& shape, const Tensor& start, const Tensor& loc,
+                   const Tensor& wts) {
+    return Aggregation::apply(feat, shape, start, loc, wts);
+}
+Tensor add_relu(const Tensor& x, const Tensor& y) {
+    const bool in_place = x.numel() >= kInPlaceMinNumel && x.is_contiguous() &&
+                          !(x.is_leaf() && x.requires_grad());
+    return AddRelu::apply(x, y, in_place);
+}
+
+Tensor max_pool2d(const Tensor& x, int64_t kernel, int64_t stride, int64_t padding) {
+    return MaxPool::apply(x, kernel, stride, padding);
+}
+
+}  // namespace
+
+void register_autograd(pybind11::module& m) {
+    using release = pybind11::call_guard<pybind11::gil_scoped_release>;
+    m.def("msda_autograd", &msda, release(), "differentiable multi_scale_deformable_attn");
+    m.def("msda_fused_autograd", &fused, release(), "differentiable multi_scale_deformable_attn_fused");
+    m.def("gka_autograd", &gka, release(), "differentiable geometric_kernel_attention");
+    m.def("deformable_aggregation_autograd", &aggregation, release(), "differentiable deformable_aggregation");
+    m.def("max_pool2d_autograd", &max_pool2d, release(), "npu_max_pool2d, known to autograd");
+    m.def("add_relu_autograd", &add_relu, release(), "differentiable npu_add_relu");
+}
+
+}  // namespace sdk

@@ -28,6 +28,7 @@
 
 #include "../../include/conv_ops_sm100.h"
 #include "../../include/msda_sm100.h"
+#include "bindings.h"
 
 namespace {
 
@@ -43,21 +44,25 @@ int dtype_code(at::ScalarType t) {
     return MSDA_BF16;
 }
 
+// dtype argument of the msda / gka entry points, with what is known of the level tables.
+int dtype_and_tables(const at::Tensor& value, const at::Tensor& shapes) {
+    return dtype_code(value.scalar_type()) |
+           (shapes.scalar_type() == at::kLong ? MSDA_TABLES_INT64 : 0) |
+           (shapes.is_cuda() ? MSDA_TABLES_DEVICE : 0);
+}
+const int32_t* table(const at::Tensor& t) { return static_cast<const int32_t*>(t.data_ptr()); }
+
 struct Dims {
     int B, K, H, D, L, Q, P;
 };
 
+// The tables may be int32 or int64, both alike; the exported functions of the reference's
+// extension take int32 only (check_int32_tables).
 Dims check_inputs(const at::Tensor& value, const at::Tensor& shapes, const at::Tensor& starts,
                   const at::Tensor& loc, const at::Tensor& attn) {
     TORCH_CHECK(is_float_kind(value.scalar_type()),
                 "value: float16, bfloat16 or float32 tensor expected but got a tensor with dtype: ",
                 value.scalar_type());
-    TORCH_CHECK(shapes.scalar_type() == at::kInt,
-                "value_spatial_shapes: int32 tensor expected but got a tensor with dtype: ",
-                shapes.scalar_type());
-    TORCH_CHECK(starts.scalar_type() == at::kInt,
-                "value_level_start_index: int32 tensor expected but got a tensor with dtype: ",
-                starts.scalar_type());
     TORCH_CHECK(is_float_kind(loc.scalar_type()),
                 "sampling_locations: float16, bfloat16 or float32 tensor expected but got a tensor "
                 "with dtype: ", loc.scalar_type());
@@ -105,6 +110,15 @@ Dims check_inputs(const at::Tensor& value, const at::Tensor& shapes, const at::T
     return d;
 }
 
+void check_int32_tables(const at::Tensor& shapes, const at::Tensor& starts) {
+    TORCH_CHECK(shapes.scalar_type() == at::kInt,
+                "value_spatial_shapes: int32 tensor expected but got a tensor with dtype: ",
+                shapes.scalar_type());
+    TORCH_CHECK(starts.scalar_type() == at::kInt,
+                "value_level_start_index: int32 tensor expected but got a tensor with dtype: ",
+                starts.scalar_type());
+}
+
 // Debugging switch: read the device's sticky status word after every operator call. That
 // costs a device synchronisation per call, so it is off unless set_status_checks(true) was
 // called or the process started with MSDA_CHECK_STATUS=1.
@@ -140,9 +154,11 @@ bool set_status_checks(bool on) { return g_check_status.exchange(on); }
 
 }  // namespace
 
-at::Tensor multi_scale_deformable_attn(const at::Tensor& value_in, const at::Tensor& shapes_in,
-                                       const at::Tensor& starts_in, const at::Tensor& loc_in,
-                                       const at::Tensor& attn_in) {
+namespace sdk {
+
+at::Tensor msda_forward(const at::Tensor& value_in, const at::Tensor& shapes_in,
+                        const at::Tensor& starts_in, const at::Tensor& loc_in,
+                        const at::Tensor& attn_in) {
     const Dims d = check_inputs(value_in, shapes_in, starts_in, loc_in, attn_in);
     const c10::cuda::CUDAGuard guard(value_in.device());
     // the reference op marks its inputs auto-contiguous
@@ -156,14 +172,14 @@ at::Tensor multi_scale_deformable_attn(const at::Tensor& value_in, const at::Ten
     at::Tensor out = at::empty({d.B, d.Q, static_cast<int64_t>(d.H) * d.D}, value.options());
     if (out.numel() == 0) return out;
     const int rc = msda_sm100_forward(
-        value.data_ptr(), shapes.data_ptr<int32_t>(), starts.data_ptr<int32_t>(), loc.data_ptr(),
+        value.data_ptr(), table(shapes), table(starts), loc.data_ptr(),
         attn.data_ptr(), out.data_ptr(), d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
-        dtype_code(value.scalar_type()), at::cuda::getCurrentCUDAStream().stream());
+        dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "multi_scale_deformable_attn");
     return out;
 }
 
-std::tuple<at::Tensor, at::Tensor, at::Tensor> multi_scale_deformable_attn_backward(
+std::tuple<at::Tensor, at::Tensor, at::Tensor> msda_backward(
     const at::Tensor& value_in, const at::Tensor& shapes_in, const at::Tensor& starts_in,
     const at::Tensor& loc_in, const at::Tensor& attn_in, const at::Tensor& grad_out_in) {
     const Dims d = check_inputs(value_in, shapes_in, starts_in, loc_in, attn_in);
@@ -201,12 +217,28 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> multi_scale_deformable_attn_backw
         ws_ptr = workspace.data_ptr();
     }
     const int rc = msda_sm100_backward_ws(
-        value.data_ptr(), shapes.data_ptr<int32_t>(), starts.data_ptr<int32_t>(), loc.data_ptr(),
+        value.data_ptr(), table(shapes), table(starts), loc.data_ptr(),
         attn.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(), grad_loc.data_ptr(),
-        grad_attn.data_ptr(), ws_ptr, ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt,
-        at::cuda::getCurrentCUDAStream().stream());
+        grad_attn.data_ptr(), ws_ptr, ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
+        dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "multi_scale_deformable_attn_backward");
     return std::make_tuple(grad_value, grad_loc, grad_attn);
+}
+
+}  // namespace sdk
+
+at::Tensor multi_scale_deformable_attn(const at::Tensor& value, const at::Tensor& shapes,
+                                       const at::Tensor& starts, const at::Tensor& loc,
+                                       const at::Tensor& attn) {
+    check_int32_tables(shapes, starts);
+    return sdk::msda_forward(value, shapes, starts, loc, attn);
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> multi_scale_deformable_attn_backward(
+    const at::Tensor& value, const at::Tensor& shapes, const at::Tensor& starts,
+    const at::Tensor& loc, const at::Tensor& attn, const at::Tensor& grad_out) {
+    check_int32_tables(shapes, starts);
+    return sdk::msda_backward(value, shapes, starts, loc, attn, grad_out);
 }
 
 // ---------------------------------------------------------------------------
@@ -278,13 +310,14 @@ void geometric_kernel_attention_forward(const at::Tensor& value_in, const at::Te
     // integer pixel coordinates travel in value's dtype (exact up to 2048 in float16)
     const at::Tensor loc = loc_in.to(value.scalar_type()).contiguous();
     const at::Tensor attn = attn_in.to(value.scalar_type()).contiguous();
-    const at::Tensor shapes = shapes_in.to(at::kInt).contiguous();
-    const at::Tensor starts = starts_in.to(at::kInt).contiguous();
+    const bool alike = shapes_in.scalar_type() == starts_in.scalar_type();
+    const at::Tensor shapes = (alike ? shapes_in : shapes_in.to(at::kInt)).contiguous();
+    const at::Tensor starts = (alike ? starts_in : starts_in.to(at::kInt)).contiguous();
     if (output.numel() == 0) return;
     const int rc = gka_sm100_forward(
-        value.data_ptr(), shapes.data_ptr<int32_t>(), starts.data_ptr<int32_t>(), loc.data_ptr(),
+        value.data_ptr(), table(shapes), table(starts), loc.data_ptr(),
         attn.data_ptr(), output.data_ptr(), d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
-        dtype_code(value.scalar_type()), at::cuda::getCurrentCUDAStream().stream());
+        dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "geometric_kernel_attention_forward");
 }
 
@@ -301,8 +334,9 @@ std::tuple<at::Tensor, at::Tensor> geometric_kernel_attention_backward(
     const at::Tensor value = value_in.contiguous();
     const at::Tensor loc = loc_in.to(value.scalar_type()).contiguous();
     const at::Tensor attn = attn_in.to(value.scalar_type()).contiguous();
-    const at::Tensor shapes = shapes_in.to(at::kInt).contiguous();
-    const at::Tensor starts = starts_in.to(at::kInt).contiguous();
+    const bool alike = shapes_in.scalar_type() == starts_in.scalar_type();
+    const at::Tensor shapes = (alike ? shapes_in : shapes_in.to(at::kInt)).contiguous();
+    const at::Tensor starts = (alike ? starts_in : starts_in.to(at::kInt)).contiguous();
     const at::Tensor grad_out = grad_out_in.to(value.scalar_type()).contiguous();
     at::Tensor grad_value = at::empty_like(value);
     at::Tensor grad_attn = at::empty_like(attn);
@@ -320,10 +354,10 @@ std::tuple<at::Tensor, at::Tensor> geometric_kernel_attention_backward(
         ws_ptr = workspace.data_ptr();
     }
     const int rc = gka_sm100_backward_ws(
-        value.data_ptr(), shapes.data_ptr<int32_t>(), starts.data_ptr<int32_t>(), loc.data_ptr(),
+        value.data_ptr(), table(shapes), table(starts), loc.data_ptr(),
         attn.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(), grad_attn.data_ptr(), ws_ptr,
-        ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt,
-        at::cuda::getCurrentCUDAStream().stream());
+        ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
+        dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "geometric_kernel_attention_backward");
     return std::make_tuple(grad_value, grad_attn);
 }
@@ -474,9 +508,9 @@ at::Tensor msda_fused_forward(const at::Tensor& value_in, const at::Tensor& shap
     at::Tensor out = at::empty({d.B, d.Q, static_cast<int64_t>(d.H) * d.D}, value.options());
     if (out.numel() == 0) return out;
     const int rc = msda_sm100_fused_forward(
-        value.data_ptr(), shapes.data_ptr<int32_t>(), starts.data_ptr<int32_t>(), ref.data_ptr(),
+        value.data_ptr(), table(shapes), table(starts), ref.data_ptr(),
         off.data_ptr(), logits.data_ptr(), out.data_ptr(), d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
-        dtype_code(value.scalar_type()), at::cuda::getCurrentCUDAStream().stream());
+        dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "msda_fused_forward");
     return out;
 }
@@ -511,10 +545,10 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> msda_fused_backward(
         ws_ptr = workspace.data_ptr();
     }
     const int rc = msda_sm100_fused_backward_ws(
-        value.data_ptr(), shapes.data_ptr<int32_t>(), starts.data_ptr<int32_t>(), ref.data_ptr(),
+        value.data_ptr(), table(shapes), table(starts), ref.data_ptr(),
         off.data_ptr(), logits.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(),
         grad_ref.data_ptr<float>(), grad_off.data_ptr(), grad_logits.data_ptr(), ws_ptr, ws_bytes,
-        d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt, at::cuda::getCurrentCUDAStream().stream());
+        d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "msda_fused_backward");
     return std::make_tuple(grad_value, grad_ref.to(ref.scalar_type()), grad_off, grad_logits);
 }
@@ -540,6 +574,25 @@ at::Tensor npu_add_relu(at::Tensor& x, const at::Tensor& y_in) {
     raise_on_error(rc, "npu_add_relu");
     return x;
 }
+
+namespace sdk {
+at::Tensor add_relu_out(const at::Tensor& x_in, const at::Tensor& y_in) {
+    TORCH_CHECK(x_in.is_cuda() && y_in.is_cuda(),
+                "npu_add_relu: x and y must be CUDA tensors (this build has no CPU path)");
+    TORCH_CHECK(is_float_kind(x_in.scalar_type()) && x_in.scalar_type() == y_in.scalar_type(),
+                "npu_add_relu: x and y must share a dtype of float16, bfloat16 or float32");
+    TORCH_CHECK(x_in.sizes() == y_in.sizes(), "npu_add_relu: x and y must have the same shape");
+    const c10::cuda::CUDAGuard guard(x_in.device());
+    const at::Tensor x = x_in.contiguous(), y = y_in.contiguous();
+    at::Tensor out = at::empty(x.sizes(), x.options());
+    const int rc = addrelu_sm100_forward_out(x.data_ptr(), y.data_ptr(), out.data_ptr(),
+                                             static_cast<size_t>(x.numel()),
+                                             dtype_code(x.scalar_type()),
+                                             at::cuda::getCurrentCUDAStream().stream());
+    raise_on_error(rc, "npu_add_relu");
+    return out;
+}
+}  // namespace sdk
 
 at::Tensor npu_add_relu_grad(const at::Tensor& self_in, const at::Tensor& grad_output_in) {
     TORCH_CHECK(self_in.is_cuda() && grad_output_in.is_cuda(),
@@ -783,6 +836,10 @@ modulated_deformable_conv2d_backward(
                            g.mask.permute({0, 3, 1, 2}).to(mask.scalar_type()));
 }
 
+namespace sdk {
+void register_autograd(pybind11::module& m);   // autograd.cpp
+}
+
 int64_t dcn_use_tensor_cores(int64_t on) { return dcn_sm100_use_tensor_cores(static_cast<int>(on)); }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -826,6 +883,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           "device status word and raises if a kernel refused or abandoned work");
     m.def("device_status", [](bool clear) { return msda_sm100_device_status(clear ? 1 : 0); },
           "(clear) -> the device's sticky status bits (synchronises)");
+    sdk::register_autograd(m);
     m.def("dcn_use_tensor_cores", &dcn_use_tensor_cores,
           "1 / 0 selects the tcgen05 / fp32 FMA product kernels; returns the previous setting");
     m.def("npu_add_relu", &npu_add_relu, "x = relu(x + y) in place; returns x");

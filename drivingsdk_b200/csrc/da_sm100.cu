@@ -346,16 +346,9 @@ static cudaError_t da_launch(const DaParams& p, bool scalar, int lpr, int nv, in
                              cudaStream_t stream) {
     const size_t smem = static_cast<size_t>(p.warp_smem) * kWarpsPerCta;
     auto go = [&](auto kern) -> cudaError_t {
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(smem));
-            if (e != cudaSuccess) return e;
-        }
         int per_sm = 1;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern,
-                                                                      kThreadsPerCta, smem);
+        cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kThreadsPerCta, smem, &per_sm);
         if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
         const long long need = (p.ntasks + kWarpsPerCta - 1) / kWarpsPerCta;
         const long long cap = static_cast<long long>(sm_count) * per_sm;
         const int grid = static_cast<int>(need < cap ? need : cap);
@@ -450,12 +443,10 @@ int da_common(DaParams& p, const void* feat, const int32_t* shapes, const int32_
                                              : static_cast<unsigned long long>(pieces);
     if (static_cast<unsigned long long>(rows) * units >= 0xffffffffull) return MSDA_ERR_LIMIT;
     p.row_units = static_cast<uint32_t>(units);
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) {
-        t_da_cuda_error = static_cast<int>(e);
-        return MSDA_ERR_CUDA;
+    const int rc = msda::device_facts(sm_count, nullptr);
+    if (rc != MSDA_OK) {
+        t_da_cuda_error = msda_sm100_last_cuda_error();
+        return rc;
     }
     return MSDA_OK;
 }

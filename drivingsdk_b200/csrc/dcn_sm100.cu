@@ -323,10 +323,9 @@ int launch_sample_vec(const DcnParams& p, int sms, cudaStream_t stream) {
     const long long warps_needed = (static_cast<long long>(p.items) + items_per_warp - 1) / items_per_warp;
     const long long ctas_needed = (warps_needed + kThreads / 32 - 1) / (kThreads / 32);
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, dcn_sample_kernel<BACKWARD, VEC>, kThreads, 0);
+    cudaError_t e = msda::resident_ctas(
+        reinterpret_cast<const void*>(dcn_sample_kernel<BACKWARD, VEC>), kThreads, 0, &per_sm);
     if (e != cudaSuccess) return msda::note_cuda_error(e);
-    if (per_sm < 1) per_sm = 1;
     const long long cap = static_cast<long long>(sms) * per_sm;
     const unsigned grid = static_cast<unsigned>(ctas_needed < cap ? ctas_needed : cap);
     dcn_sample_kernel<BACKWARD, VEC><<<grid, kThreads, 0, stream>>>(p);

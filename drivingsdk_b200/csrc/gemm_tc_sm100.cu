@@ -36,6 +36,7 @@
 
 #include "gemm_sm100.h"
 #include "msda_common.cuh"
+#include "msda_launch.h"
 
 namespace msda {
 namespace {
@@ -538,10 +539,9 @@ bool mn_major_ok(const GemmArgs& g) {
 
 template <int BN, int PASSES>
 cudaError_t launch(const GemmArgs& g, int splits, int* status, cudaStream_t stream) {
-    // per device and cheap, so set on every launch (a process may drive several devices)
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, PASSES>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Tile<BN, PASSES>::kSmemBytes);
+    int resident = 0;   // one CTA per SM; the call sets the shared-memory limit
+    cudaError_t e = resident_ctas(reinterpret_cast<const void*>(gemm_tc_kernel<BN, PASSES>), kGemmThreads,
+                                  Tile<BN, PASSES>::kSmemBytes, &resident);
     if (e != cudaSuccess) return e;
     CUtensorMap map_a, map_b;
     constexpr int BK = Tile<BN, PASSES>::BK;
@@ -571,11 +571,8 @@ cudaError_t launch(const GemmArgs& g, int splits, int* status, cudaStream_t stre
     const long long tiles = static_cast<long long>((g.M + BM - 1) / BM) * p.n_tiles;
     if (tiles * p.n_splits >= (1ll << 31)) return cudaErrorInvalidValue;
     p.total_tiles = static_cast<int>(tiles);
-    int dev = 0, sms = 0;
-    e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
+    int sms = 0;
+    if (device_facts(&sms, nullptr) != 0) return cudaErrorInvalidDevice;
     const long long items = tiles * p.n_splits;
     const dim3 grid(static_cast<unsigned>(items < sms ? items : sms));   // one CTA per SM
     gemm_tc_kernel<BN, PASSES><<<grid, kGemmThreads, Tile<BN, PASSES>::kSmemBytes, stream>>>(map_a, map_b, p);

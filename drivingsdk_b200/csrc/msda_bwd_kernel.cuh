@@ -499,11 +499,6 @@ template <typename T, typename TG, int LPR, int NV, bool SCALAR, int MODE>
 static cudaError_t launch_bwd_inst(const Params& p, const LaunchShape& ls, size_t smem,
                                    cudaStream_t stream) {
     auto kern = msda_bwd_kernel<T, TG, LPR, NV, SCALAR, MODE>;
-    if (smem > 48 * 1024) {
-        cudaError_t e =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
     int grid = 0;
     cudaError_t e = persistent_grid(reinterpret_cast<const void*>(kern), smem, ls, p, &grid);
     if (e != cudaSuccess) return e;

@@ -38,9 +38,9 @@ struct SortLevels {
 __device__ __forceinline__ bool load_sort_levels(const Params& p, SortLevels& lv) {
     if (!device_level_table_ok(p)) return false;
     for (int l = threadIdx.x; l < p.L; l += blockDim.x) {
-        const int h = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l];
-        const int w = p.use_table ? p.lv.w[l] : p.shapes_dev[2 * l + 1];
-        const int start = p.use_table ? p.lv.start[l] : p.start_dev[l];
+        const int h = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l * p.table_step];
+        const int w = p.use_table ? p.lv.w[l] : p.shapes_dev[(2 * l + 1) * p.table_step];
+        const int start = p.use_table ? p.lv.start[l] : p.start_dev[l * p.table_step];
         lv.geo[l] = make_float4(static_cast<float>(w), static_cast<float>(h), __int_as_float(w),
                                 __int_as_float(start));
     }
@@ -144,8 +144,8 @@ sort_cells_kernel(const __grid_constant__ Params p, const __grid_constant__ Sort
     const uint32_t l = unit % p.L;
     unit /= p.L;
     const uint32_t h = unit % p.H, b = unit / p.H;
-    const int H = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l];
-    const int W = p.use_table ? p.lv.w[l] : p.shapes_dev[2 * l + 1];
+    const int H = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l * p.table_step];
+    const int W = p.use_table ? p.lv.w[l] : p.shapes_dev[(2 * l + 1) * p.table_step];
     const uint32_t cells = (CPS == 4) ? static_cast<uint32_t>(H + 1) * static_cast<uint32_t>(W + 1)
                                       : static_cast<uint32_t>(H) * static_cast<uint32_t>(W);
     const uint32_t samples = static_cast<uint32_t>(p.Q) * p.P;
@@ -864,9 +864,9 @@ static cudaError_t launch_sorted_main(Kernel kern, int streams, const Params& p,
                                       const LaunchShape& ls, cudaStream_t stream) {
     int per_sm = ls.ctas_per_sm;
     if (per_sm <= 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreadsPerCta, 0);
+        const cudaError_t e =
+            resident_ctas(reinterpret_cast<const void*>(kern), kThreadsPerCta, 0, &per_sm);
         if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
     }
     const uint32_t cap = static_cast<uint32_t>(ls.sm_count) * per_sm;
     // Long streams enter fewer cells, short ones level the load: eight tickets per resident
@@ -888,10 +888,10 @@ static cudaError_t launch_sorted_main(Kernel kern, int streams, const Params& p,
 template <typename TL, int CPS>
 static cudaError_t launch_sort(const Params& p, SortParams& sp, const LaunchShape& ls,
                                cudaStream_t stream) {
-    cudaError_t e;
     auto kern = sort_cells_kernel<TL, CPS>;
-    const int smem = static_cast<int>(kSortCells * sizeof(uint32_t));
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const size_t smem = kSortCells * sizeof(uint32_t);
+    int resident = 0;   // (asked for the shared-memory limit that the call sets)
+    const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kSortThreads, smem, &resident);
     if (e != cudaSuccess) return e;
     // the smallest cluster that gives most SMs work
     const uint32_t levels = static_cast<uint32_t>(p.B) * p.H * p.L;

@@ -5,6 +5,9 @@
 // No allocation, no synchronisation (except msda_sm100_device_status).
 #include <atomic>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 #include "../../include/msda_sm100.h"
 #include "msda_launch.h"
@@ -88,6 +91,13 @@ int pointer_on_device(const void* p, bool* on_device) {
     }
     *on_device = (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
     return MSDA_OK;
+}
+
+// Separates the level-table flags from a dtype argument.
+int split_flags(int* dtype) {
+    const int flags = *dtype & (MSDA_TABLES_INT64 | MSDA_TABLES_DEVICE);
+    if (*dtype >= 0) *dtype &= ~(MSDA_TABLES_INT64 | MSDA_TABLES_DEVICE);
+    return flags;
 }
 
 int check_dims(int B, int K, int H, int D, int L, int Q, int P, int dtype) {
@@ -185,7 +195,7 @@ bool sort_pays(const SortPlan& s, int K, int H, int D, int dtype, int B, int mod
 // Fills the parts of Params common to both directions.
 int fill_common(Params& p, const DeviceInfo* dev, const void* value, const int32_t* shapes,
                 const int32_t* starts, const void* loc, const void* attn, int B, int K, int H,
-                int D, int L, int Q, int P, int dtype, bool backward) {
+                int D, int L, int Q, int P, int dtype, int table_flags, bool backward) {
     std::memset(&p, 0, sizeof(p));
     p.value = value;
     p.loc = loc;
@@ -197,9 +207,13 @@ int fill_common(Params& p, const DeviceInfo* dev, const void* value, const int32
     p.nitems = (p.ntasks + p.tasks_per_item - 1) / p.tasks_per_item;
     p.status = dev->status_ptr;
 
-    bool shapes_dev = false, starts_dev = false;
-    pointer_on_device(shapes, &shapes_dev);
-    pointer_on_device(starts, &starts_dev);
+    bool shapes_dev = true, starts_dev = true;
+    if (!(table_flags & MSDA_TABLES_DEVICE)) {
+        pointer_on_device(shapes, &shapes_dev);
+        pointer_on_device(starts, &starts_dev);
+    }
+    const int step = (table_flags & MSDA_TABLES_INT64) ? 2 : 1;
+    p.table_step = step;
     if (shapes_dev != starts_dev) return MSDA_ERR_ALIGN;  // both host or both device
     if (shapes_dev) {
         p.use_table = 0;
@@ -208,9 +222,9 @@ int fill_common(Params& p, const DeviceInfo* dev, const void* value, const int32
     } else {
         p.use_table = 1;
         for (int l = 0; l < L; ++l) {
-            p.lv.h[l] = shapes[2 * l];
-            p.lv.w[l] = shapes[2 * l + 1];
-            p.lv.start[l] = starts[l];
+            p.lv.h[l] = shapes[2 * l * step];
+            p.lv.w[l] = shapes[(2 * l + 1) * step];
+            p.lv.start[l] = starts[l * step];
             if (p.lv.h[l] <= 0 || p.lv.w[l] <= 0 || p.lv.start[l] < 0 ||
                 static_cast<long long>(p.lv.start[l]) + static_cast<long long>(p.lv.h[l]) * p.lv.w[l] > K)
                 return MSDA_ERR_DIMS;
@@ -260,6 +274,7 @@ int backward_impl(const void* value, const int32_t* shapes, const int32_t* start
     // per sample, no location gradient); kFused = MSDA fed by reference points, offsets (in
     // `loc`) and logits (in `attn`)
     const bool nearest = mode == kNearest;
+    const int table_flags = split_flags(&dtype);
     if (!value || !shapes || !starts || !loc || !attn || !grad_out || !grad_value || !grad_attn ||
         (!nearest && !grad_loc) || (mode == kFused && (!ref || !grad_ref)))
         return MSDA_ERR_NULL;
@@ -272,7 +287,8 @@ int backward_impl(const void* value, const int32_t* shapes, const int32_t* start
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 
     Params p;
-    rc = fill_common(p, dev, value, shapes, starts, loc, attn, B, K, H, D, L, Q, P, dtype, true);
+    rc = fill_common(p, dev, value, shapes, starts, loc, attn, B, K, H, D, L, Q, P, dtype,
+                     table_flags, true);
     if (rc != MSDA_OK) return rc;
     const size_t e = elem_size(dtype);
     if (!aligned_to(grad_out, e) || !aligned_to(grad_value, e) || !aligned_to(grad_attn, e) ||
@@ -372,6 +388,7 @@ int forward_impl(const void* value, const int32_t* spatial_shapes,
                  const int32_t* level_start_index, const void* sampling_locations,
                  const void* attention_weights, void* output, int mode, const void* ref, int B,
                  int K, int H, int D, int L, int Q, int P, int dtype, void* stream_v) {
+    const int table_flags = split_flags(&dtype);
     if (mode == kFused && (!ref || static_cast<long long>(L) * P > 32))
         return ref ? MSDA_ERR_LIMIT : MSDA_ERR_NULL;
     if (!value || !spatial_shapes || !level_start_index || !sampling_locations ||
@@ -385,7 +402,7 @@ int forward_impl(const void* value, const int32_t* spatial_shapes,
 
     Params p;
     rc = fill_common(p, dev, value, spatial_shapes, level_start_index, sampling_locations,
-                     attention_weights, B, K, H, D, L, Q, P, dtype, false);
+                     attention_weights, B, K, H, D, L, Q, P, dtype, table_flags, false);
     if (rc != MSDA_OK) return rc;
     if (!aligned_to(output, elem_size(dtype))) return MSDA_ERR_ALIGN;
     p.out = output;
@@ -411,6 +428,44 @@ int forward_impl(const void* value, const int32_t* spatial_shapes,
 namespace msda {
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 int note_cuda_error(cudaError_t e) { return fail_cuda(e); }
+cudaError_t resident_ctas(const void* kernel, int threads, size_t smem, int* per_sm) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    struct Key {
+        const void* kernel;
+        size_t smem;
+        int threads, dev;
+        bool operator<(const Key& o) const {
+            return std::tie(kernel, smem, threads, dev) < std::tie(o.kernel, o.smem, o.threads, o.dev);
+        }
+    };
+    static std::mutex lock;
+    static std::map<Key, int> known;   // a handful of entries: kernels x their shared-memory sizes
+    const Key key{kernel, smem, threads, dev};
+    {
+        std::lock_guard<std::mutex> hold(lock);
+        const auto it = known.find(key);
+        if (it != known.end()) {
+            *per_sm = it->second;
+            return cudaSuccess;
+        }
+    }
+    // the limit only ever grows: launches of the kernel with more shared memory may be under way
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, kernel);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> hold(lock);
+    if (smem > static_cast<size_t>(attr.maxDynamicSharedSizeBytes)) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+    }
+    int n = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    *per_sm = known[key] = n < 1 ? 1 : n;
+    return cudaSuccess;
+}
 int device_facts(int* sm_count, int** status_word) {
     const DeviceInfo* d = nullptr;
     const int rc = device_info(&d);

@@ -99,6 +99,7 @@ struct Params {
     // level geometry on the device (used when use_table == 0)
     const int* shapes_dev;  // [L, 2] (H, W)
     const int* start_dev;   // [L]
+    int table_step;         // 32-bit words per entry of the two: 1 (int32) or 2 (int64, low word first)
     int B, K, H, D, L, Q, P;
     int LP;             // L * P
     int tasks_per_item; // consecutive (b, q, h) tasks one warp pass covers

@@ -279,11 +279,6 @@ template <typename T, int LPR, int NV, bool SCALAR, int MODE, bool PACK>
 static cudaError_t launch_fwd_pack(const Params& p, const LaunchShape& ls, size_t smem,
                                    cudaStream_t stream) {
     auto kern = msda_fwd_kernel<T, LPR, NV, SCALAR, MODE, PACK>;
-    if (smem > 48 * 1024) {
-        cudaError_t e =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
     int grid = 0;
     cudaError_t e = persistent_grid(reinterpret_cast<const void*>(kern), smem, ls, p, &grid);
     if (e != cudaSuccess) return e;

@@ -17,6 +17,11 @@ struct RowPlan {
     int nv;
 };
 
+// CTAs of `threads` threads and `smem` bytes of dynamic shared memory that one SM of the current
+// device holds at once (at least 1); lets the kernel use that much shared memory. Asked of the
+// runtime once per kernel, size and device: the query costs more host time than a launch.
+cudaError_t resident_ctas(const void* kernel, int threads, size_t smem, int* per_sm);
+
 // Grid of a persistent launch: `ctas_per_sm` CTAs on each of `sm_count` SMs, or — when
 // ctas_per_sm <= 0 — as many as the occupancy calculator says are resident at once for this
 // kernel and shared-memory size (a CTA that is not resident from the start would run its
@@ -27,12 +32,15 @@ struct LaunchShape {
 };
 inline cudaError_t persistent_grid(const void* kernel, size_t smem, const LaunchShape& ls,
                                    const Params& p, int* grid) {
+    int resident = 0;
     int per_sm = ls.ctas_per_sm;
-    if (per_sm <= 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel,
-                                                                      kThreadsPerCta, smem);
+    if (per_sm > 0) {
+        // a tuned count still needs the shared-memory limit
+        const cudaError_t e = resident_ctas(kernel, kThreadsPerCta, smem, &resident);
         if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
+    } else {
+        const cudaError_t e = resident_ctas(kernel, kThreadsPerCta, smem, &per_sm);
+        if (e != cudaSuccess) return e;
     }
     const long long ctas_needed = (p.nitems + kWarpsPerCta - 1) / kWarpsPerCta;
     const long long cap = static_cast<long long>(ls.sm_count) * per_sm;

@@ -61,9 +61,9 @@ __device__ __forceinline__ LaneLevels load_lane_levels(const Params& p, int lane
             ww = p.lv.w[l];
             ss = p.lv.start[l];
         } else {
-            hh = p.shapes_dev[2 * l];
-            ww = p.shapes_dev[2 * l + 1];
-            ss = p.start_dev[l];
+            hh = p.shapes_dev[2 * l * p.table_step];
+            ww = p.shapes_dev[(2 * l + 1) * p.table_step];
+            ss = p.start_dev[l * p.table_step];
         }
         if (c == 0) {
             lv.h0 = hh; lv.w0 = ww; lv.start0 = ss;
@@ -83,7 +83,9 @@ __device__ __forceinline__ bool device_level_table_ok(const Params& p) {
     if (p.use_table) return true;   // host tables were validated by the entry point
     bool bad = false;
     for (int l = threadIdx.x; l < p.L; l += blockDim.x) {
-        const int hh = p.shapes_dev[2 * l], ww = p.shapes_dev[2 * l + 1], ss = p.start_dev[l];
+        const int hh = p.shapes_dev[2 * l * p.table_step];
+        const int ww = p.shapes_dev[(2 * l + 1) * p.table_step];
+        const int ss = p.start_dev[l * p.table_step];
         bad |= hh <= 0 || ww <= 0 || ss < 0 ||
                static_cast<long long>(ss) + static_cast<long long>(hh) * ww > p.K;
     }

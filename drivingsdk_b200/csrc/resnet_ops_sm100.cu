@@ -41,7 +41,7 @@ template <typename T> struct alignas(16) Vec16 {
     T v[kN];
 };
 
-// BACKWARD == false: a = relu(a + b) written to `dst` (== a)
+// BACKWARD == false: relu(a + b) written to `dst` (may be a)
 // BACKWARD == true : dst = a > 0 ? b : 0          (a = forward result, b = grad_out)
 template <typename T, bool BACKWARD>
 __device__ __forceinline__ T combine(T a, T b) {
@@ -93,19 +93,10 @@ pointwise_scalar_kernel(const T* a, const T* __restrict__ b, T* dst,
         dst[i] = combine<T, BACKWARD>(a[i], b[i]);
 }
 
-int sm_count_of_current_device(int* sms) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return msda::note_cuda_error(e);
-    e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return msda::note_cuda_error(e);
-    return MSDA_OK;
-}
-
 template <typename T, bool BACKWARD>
 int launch_pointwise(const void* a, const void* b, void* dst, size_t n, cudaStream_t stream) {
     int sms = 0;
-    const int rc = sm_count_of_current_device(&sms);
+    const int rc = msda::device_facts(&sms, nullptr);
     if (rc != MSDA_OK) return rc;
     const T* ap = static_cast<const T*>(a);
     const T* bp = static_cast<const T*>(b);
@@ -230,7 +221,7 @@ maxpool3s2_kernel(const T* __restrict__ x, T* __restrict__ y, int H, int W, int 
 template <typename T>
 int launch_maxpool(const void* x, void* y, int N, int C, int H, int W, cudaStream_t stream) {
     int sms = 0;
-    const int rc = sm_count_of_current_device(&sms);
+    const int rc = msda::device_facts(&sms, nullptr);
     if (rc != MSDA_OK) return rc;
     const int OH = (H + 1) / 2, OW = (W + 1) / 2;
     const int groups_per_row = (OW + 3) / 4;
@@ -257,6 +248,11 @@ extern "C" {
 
 int addrelu_sm100_forward(void* x, const void* y, size_t n, int dtype, void* stream) {
     return dispatch_pointwise<false>(x, y, x, n, dtype, stream);
+}
+
+int addrelu_sm100_forward_out(const void* x, const void* y, void* out, size_t n, int dtype,
+                              void* stream) {
+    return dispatch_pointwise<false>(x, y, out, n, dtype, stream);
 }
 
 int addrelu_sm100_backward(const void* out, const void* grad_out, void* grad_in, size_t n,

@@ -46,4 +46,4 @@ class GeometricKernelAttentionFunc(Function):
         return grad_value, None, None, None, grad_attn_weights
 
 
-geometric_kernel_attention = GeometricKernelAttentionFunc.apply
+geometric_kernel_attention = _C.gka_autograd   # the same function, natively

@@ -55,7 +55,7 @@ class MultiScaleDeformableAttnFusedFunction(Function):
         return grad_value, None, None, grad_ref, grad_off, grad_logits
 
 
-multi_scale_deformable_attn_fused = MultiScaleDeformableAttnFusedFunction.apply
+multi_scale_deformable_attn_fused = _C.msda_fused_autograd   # the same function, natively
 
 
 def compose_unfused(reference_points, sampling_offsets, attention_logits, value_spatial_shapes):

@@ -1,7 +1,7 @@
 """Fused add + ReLU: autograd wrapper over the sm_100a kernels.
 
 Mirrors the reference wrapper (mx_driving/ops/npu_add_relu.py:19-37): ``AddReluFunction``
-and ``npu_add_relu = AddReluFunction.apply``. As in the reference, an ``x`` of at least
+and ``npu_add_relu = _C.add_relu_autograd   # the same function, natively``. As in the reference, an ``x`` of at least
 2,000,000 elements is overwritten with ``relu(x + y)`` and returned, a smaller one is left
 untouched and the result is a new tensor (the reference computes ``F.relu(x + y)`` there);
 the result is what backward keeps, and both addends receive the same gradient
@@ -46,4 +46,4 @@ class AddReluFunction(Function):
         return result, result
 
 
-npu_add_relu = AddReluFunction.apply
+npu_add_relu = _C.add_relu_autograd   # the same function, natively

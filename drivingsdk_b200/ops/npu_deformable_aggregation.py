@@ -50,5 +50,6 @@ class AdsDeformableAggregation(Function):
         return grad_mc_ms_feat, None, None, grad_sampling_location, grad_weights
 
 
-npu_deformable_aggregation = AdsDeformableAggregation.apply
-deformable_aggregation = AdsDeformableAggregation.apply
+# the same function, natively
+npu_deformable_aggregation = _C.deformable_aggregation_autograd
+deformable_aggregation = _C.deformable_aggregation_autograd

@@ -1,7 +1,7 @@
 """3x3 / stride 2 / padding 1 max pooling for inference: wrapper over the sm_100a kernel.
 
 Mirrors the reference wrapper (mx_driving/ops/npu_max_pool2d.py:13-19): ``MaxPool2d`` (an
-autograd Function without backward) and ``npu_max_pool2d = MaxPool2d.apply``; any other
+autograd Function without backward) and ``npu_max_pool2d = _C.max_pool2d_autograd   # the same function, natively``; any other
 kernel size, stride or padding is an error, as in the reference binding
 (mx_driving/csrc/MaxPool2d.cpp:31-33). No CPU path.
 """
@@ -23,4 +23,4 @@ class MaxPool2d(Function):
         return _C.npu_max_pool2d(x, kernel_size, stride, padding)
 
 
-npu_max_pool2d = MaxPool2d.apply
+npu_max_pool2d = _C.max_pool2d_autograd   # the same function, natively

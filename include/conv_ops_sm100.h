@@ -28,6 +28,9 @@ extern "C" {
  * dtype: MSDA_F32, MSDA_F16 or MSDA_BF16.
  */
 int addrelu_sm100_forward(void* x, const void* y, size_t n, int dtype, void* stream);
+/* The same into `out` (which may be x). */
+int addrelu_sm100_forward_out(const void* x, const void* y, void* out, size_t n, int dtype,
+                              void* stream);
 
 /*
  * grad_in[i] = out[i] > 0 ? grad_out[i] : 0, where `out` is what the forward left in x.

@@ -57,6 +57,13 @@ typedef enum msda_status {
     MSDA_ERR_CUDA = -7         /* a CUDA runtime call failed; see msda_sm100_last_cuda_error */
 } msda_status;
 
+/* May be or-ed into the dtype argument of the msda and gka forward and backward entry points.
+ *   MSDA_TABLES_INT64   the two level arrays hold int64 (values are taken modulo 2^32)
+ *   MSDA_TABLES_DEVICE  the two level arrays are known to be in device memory: the call does not
+ *                       ask the runtime where they are */
+#define MSDA_TABLES_INT64 0x100
+#define MSDA_TABLES_DEVICE 0x200
+
 /* Forward. Replaces aclnnMultiScaleDeformableAttn
  * (mx_driving/csrc/MultiScaleDeformableAttn.cpp:63-64; device kernel
  * kernels/multi_scale_deformable_attn/op_kernel/multi_scale_deformable_attn.cpp:349-387).
