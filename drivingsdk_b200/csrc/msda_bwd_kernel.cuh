@@ -145,7 +145,17 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
 
     const LaneLevels lv = load_lane_levels(p, lane);
     const T* __restrict__ value = static_cast<const T*>(p.value);
-    const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + j * 16;
+    // this lane's pieces of a row; past the end of the row it reads the last one again, with a
+    // zero grad_out piece, and reduces nothing
+    int voff[NV];
+    bool on[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        on[k] = SCALAR || j + k * LPR < p.pieces;
+        voff[k] = SCALAR ? 0 : min(j + k * LPR, p.pieces - 1) * 16;
+    }
+    const bool red_on[2] = {j < 2 * p.pieces, LPR + j < 2 * p.pieces};   // SPLIT_RED's two pieces
+    const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + voff[0];
     const T* __restrict__ gout = static_cast<const T*>(p.grad_out);
     TG* __restrict__ gval = static_cast<TG*>(p.grad_value);
     unsigned char* glane = static_cast<unsigned char*>(p.grad_value) + j * 16;
@@ -238,8 +248,9 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
 #pragma unroll
                 for (int k = 0; k < NV; ++k) {
                     if constexpr (!SCALAR) {
-                        const uint4 raw =
-                            *reinterpret_cast<const uint4*>(gout + obase + (j + k * LPR) * VEC);
+                        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+                        if (on[k])
+                            raw = *reinterpret_cast<const uint4*>(gout + obase + (j + k * LPR) * VEC);
                         unpack16<T>(raw, go[k]);
                     } else {
                         const int c = j + k * 32;
@@ -251,7 +262,8 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
                         const T* src = gout + obase + (half * LPR + j) * 4;
-                        const uint2 raw = *reinterpret_cast<const uint2*>(src);
+                        uint2 raw = make_uint2(0u, 0u);
+                        if (red_on[half]) raw = *reinterpret_cast<const uint2*>(src);
                         const uint32_t wds[2] = {raw.x, raw.y};
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
@@ -297,7 +309,7 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
 #pragma unroll
                             for (int k = 0; k < NV; ++k)
                                 raw[u][k] =
-                                    ldg16(vlane + static_cast<size_t>(off) * 16 + k * (LPR * 16));
+                                    ldg16(vlane + static_cast<size_t>(off) * 16 + (voff[k] - voff[0]));
                         }
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
@@ -309,12 +321,12 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
                             if constexpr (SPLIT_RED) {
                                 float* row = reinterpret_cast<float*>(
                                     glane + static_cast<size_t>(rec[u].x) * 32);
-                                if (has_row) {
+                                if (has_row && red_on[0])
                                     red_add_f32x4(row, w * gred[0][0], w * gred[0][1],
                                                   w * gred[0][2], w * gred[0][3]);
+                                if (has_row && red_on[1])
                                     red_add_f32x4(row + LPR * 4, w * gred[1][0], w * gred[1][1],
                                                   w * gred[1][2], w * gred[1][3]);
-                                }
                             } else {
 #pragma unroll
                                 for (int k = 0; k < NV; ++k) {
@@ -326,7 +338,7 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
                                         contrib[e] = c2.x;
                                         contrib[e + 1] = c2.y;
                                     }
-                                    if (has_row)
+                                    if (has_row && on[k])
                                         red_add_vec<TG, VEC>(
                                             reinterpret_cast<TG*>(
                                                 glane + static_cast<size_t>(rec[u].x) * 16 +

@@ -114,11 +114,12 @@ RowPlan plan_rows(int D, int dtype, bool ptrs_16B_aligned) {
     RowPlan rp{true, 32, 8};
     const size_t row_bytes = static_cast<size_t>(D) * elem_size(dtype);
     if (!ptrs_16B_aligned || row_bytes % 16 != 0) return rp;
-    const size_t pieces = row_bytes / 16;
-    if ((pieces & (pieces - 1)) != 0 || pieces > 64) return rp;
+    const int pieces = static_cast<int>(row_bytes / 16);
+    if (pieces > 64) return rp;
     rp.scalar = false;
-    rp.lpr = pieces < 32 ? static_cast<int>(pieces) : 32;
-    rp.nv = static_cast<int>(pieces) / rp.lpr;
+    rp.lpr = 1;
+    while (rp.lpr < pieces && rp.lpr < 32) rp.lpr *= 2;
+    rp.nv = (pieces + rp.lpr - 1) / rp.lpr;
     return rp;
 }
 
@@ -142,6 +143,7 @@ int set_row_units(Params& p, const RowPlan& rp, int dtype) {
     if (rows * units >= 0xffffffffull) return MSDA_ERR_LIMIT;
     p.row_units = static_cast<uint32_t>(units);
     p.limit_units = debug_limit(rows, units);
+    p.pieces = static_cast<int>(units);
     return MSDA_OK;
 }
 

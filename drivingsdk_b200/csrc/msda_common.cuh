@@ -114,6 +114,7 @@ struct Params {
     long long ntasks;   // B * Q * H
     long long nitems;   // ceil(ntasks / tasks_per_item)
     int* status;        // device status word
+    int pieces;              // vector path: 16-byte pieces per row (not necessarily a power of two)
     uint32_t row_units;      // offset units per value row: 16-byte pieces, or elements (scalar path)
     uint32_t limit_units;    // B * K * H * row_units: one past the last valid row offset + row
     uint32_t warp_smem;      // bytes of dynamic shared memory per warp

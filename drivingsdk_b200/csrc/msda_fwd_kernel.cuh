@@ -52,7 +52,11 @@ msda_fwd_kernel(const __grid_constant__ Params p) {
 
     const LaneLevels lv = load_lane_levels(p, lane);
     const T* __restrict__ value = static_cast<const T*>(p.value);
-    const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + j * 16;
+    // this lane's pieces of a row; past the end of the row it reads the last one again
+    int voff[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) voff[k] = SCALAR ? 0 : min(j + k * LPR, p.pieces - 1) * 16;
+    const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + voff[0];
     T* __restrict__ out = static_cast<T*>(p.out);
 
     const int TPC = p.tasks_per_item;
@@ -165,13 +169,13 @@ msda_fwd_kernel(const __grid_constant__ Params p) {
                             for (int k = 0; k < NV; ++k) {
                                 if constexpr (PRESENT) {
                                     raw[u][k] = ldg16(vlane + static_cast<size_t>(rec[u].x) * 16 +
-                                                      k * (LPR * 16));
+                                                      (voff[k] - voff[0]));
                                 } else {
                                     raw[u][k] = make_uint4(0u, 0u, 0u, 0u);
                                     if (rec[u].x != kNoRow)
                                         raw[u][k] = ldg16(vlane +
                                                           static_cast<size_t>(rec[u].x) * 16 +
-                                                          k * (LPR * 16));
+                                                          (voff[k] - voff[0]));
                                 }
                             }
                         }
@@ -252,7 +256,7 @@ msda_fwd_kernel(const __grid_constant__ Params p) {
                             for (int e = 0; e < VEC; ++e)
                                 acc[k][e] += __shfl_xor_sync(0xffffffffu, acc[k][e], off);
                         }
-                        if (g == 0) {
+                        if (g == 0 && (SCALAR || j + k * LPR < p.pieces)) {
                             if constexpr (!SCALAR) {
                                 float f[VEC];
 #pragma unroll

@@ -15,7 +15,7 @@
 //            in fp32 registers.
 //   epilogue the row-slot groups are summed with xor shuffles and one group
 //            writes the D outputs as 16-byte stores.
-// Rows whose byte length is not 16 * 2^k take the SCALAR instantiation: lane =
+// Rows whose byte length is not a multiple of 16 take the SCALAR instantiation: lane =
 // channel (mod 32), one row per instruction.
 #include "msda_fwd_kernel.cuh"
 
