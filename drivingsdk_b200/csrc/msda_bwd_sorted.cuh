@@ -19,14 +19,10 @@
 
 #include <type_traits>
 
-#include "msda_launch.h"
+#include "cell_sort.cuh"
 #include "msda_tile.cuh"
 
 namespace msda {
-
-constexpr int kSortThreads = 1024;
-constexpr uint32_t kSortCells = 24 * 1024;   // counters of one CTA: 96 KB, two CTAs per SM
-constexpr uint32_t kMaxStream = 256;         // most consecutive sorted samples in one stream
 
 // Level table of one CTA.
 struct SortLevels {
@@ -62,296 +58,52 @@ __device__ __forceinline__ SampleId sample_id(const Params& p, const SortParams&
     return r;
 }
 
-template <typename TL>
-__device__ __forceinline__ float2 load_pair(const TL* p);
-template <>
-__device__ __forceinline__ float2 load_pair<float>(const float* p) {
-    return __ldg(reinterpret_cast<const float2*>(p));
-}
-template <>
-__device__ __forceinline__ float2 load_pair<__half>(const __half* p) {
-    return __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
-}
-template <>
-__device__ __forceinline__ float2 load_pair<__nv_bfloat16>(const __nv_bfloat16* p) {
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
-    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
-
-// The sample's cell in its level, or kNoRow for a sample that takes no part.
-template <int CPS>
-__device__ __forceinline__ uint32_t sample_cell(float2 xy, int W, int H) {
-    if constexpr (CPS == 4) {
-        const float wf = static_cast<float>(W), hf = static_cast<float>(H);
-        const float x = xy.x * wf - 0.5f;
-        const float y = xy.y * hf - 0.5f;
-        if (!((x > -1.f) && (y > -1.f) && (x < wf) && (y < hf))) return kNoRow;
-        return static_cast<uint32_t>(__float2int_rd(y) + 1) * static_cast<uint32_t>(W + 1) +
-               static_cast<uint32_t>(__float2int_rd(x) + 1);
-    } else {
-        const int x = min(max(__float2int_rz(xy.x), 0), W - 1);
-        const int y = min(max(__float2int_rz(xy.y), 0), H - 1);
-        return static_cast<uint32_t>(y * W + x);
-    }
-}
-
-// Counters in the shared memory of CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t cluster_address(const uint32_t* p, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_count(uint32_t addr) {
-    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], 1;" ::"r"(addr) : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_take(uint32_t addr) {
-    uint32_t r;
-    asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(r) : "r"(addr) : "memory");
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_read(uint32_t addr) {
-    uint32_t r;
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(r) : "r"(addr) : "memory");
-    return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Counting sort of one (batch, head, level)'s samples by cell, with the counters in the shared
-// memory of a cluster of CTAs: atomics there are faster than in L2 (a version with one L2 counter
-// per cell took 72 + 42 us at the encoder shape, bound by the rate of L2 atomics). The CTAs of a
-// cluster share the queries and the cells of a level: each counts and places its queries'
-// samples, whoever holds the counter. Where cells hold many samples each CTA keeps to itself:
-// it sorts its own queries (whose runs are then that much shorter). The CTAs' results follow
-// each other in the order in which they get there.
+// What the sort needs to know (cell_sort.cuh): a map is one (batch, head, level).
 template <typename TL, int CPS>
-__global__ void __launch_bounds__(kSortThreads, 2)
-sort_cells_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
-    extern __shared__ uint32_t s_count[];   // [kSortCells]
-    __shared__ uint32_t warp_sum[32];
-    __shared__ uint32_t block_sum;           // samples this CTA's counters hold
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (blockIdx.x == 0 && tid == 0) *sp.ticket = 0u;
-    if (!device_level_table_ok(p)) {         // the same answer in every CTA
-        if (tid == 0) sp.regions[blockIdx.x / sp.parts] = make_uint2(0u, 0u);
-        return;
-    }
+struct AttentionSamples {
+    Params p;
+    FastDiv fd_p;       // division by the points per level
+    uint32_t samples;   // of one map: Q * P
 
-    uint32_t unit = blockIdx.x;
-    const uint32_t part = unit % sp.parts;   // rank in the cluster
-    unit /= sp.parts;
-    const uint32_t l = unit % p.L;
-    unit /= p.L;
-    const uint32_t h = unit % p.H, b = unit / p.H;
-    const int H = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l * p.table_step];
-    const int W = p.use_table ? p.lv.w[l] : p.shapes_dev[(2 * l + 1) * p.table_step];
-    const uint32_t cells = (CPS == 4) ? static_cast<uint32_t>(H + 1) * static_cast<uint32_t>(W + 1)
-                                      : static_cast<uint32_t>(H) * static_cast<uint32_t>(W);
-    const uint32_t samples = static_cast<uint32_t>(p.Q) * p.P;
-    // on its own: at least sixteen samples per cell are left to each CTA, and the counters fit
-    const bool alone = sp.parts == 1 || (samples / sp.parts >= 16u * cells && cells <= kSortCells);
-    const uint32_t q0 = static_cast<uint32_t>(static_cast<uint64_t>(p.Q) * part / sp.parts);
-    const uint32_t q1 = static_cast<uint32_t>(static_cast<uint64_t>(p.Q) * (part + 1) / sp.parts);
-    const uint32_t n = (q1 - q0) * p.P;
-    // sample i of the range: point i % P of query q0 + i / P
-    const uint32_t first = ((b * p.Q + q0) * p.H + h) * p.LP + l * p.P;
-    const uint32_t stride = static_cast<uint32_t>(p.H) * p.LP;
-    const TL* loc = static_cast<const TL*>(p.loc);
-    auto id_of = [&](uint32_t i) {
-        const uint32_t q = fd_div(i, sp.fd_p);
-        return first + q * stride + (i - q * p.P);
+    struct Map {
+        uint32_t cells, first;   // first: number of the map's first sample
+        int W, H;
     };
-
-    // cells held by one CTA at a time, by all of the cluster (or by this CTA alone) in a pass
-    const uint32_t holders = alone ? 1u : sp.parts;
-    const uint32_t held = min(kSortCells, (cells + holders - 1) / holders);
-    const uint32_t pass_cells = held * holders;
-    const FastDiv by_held = sp.parts == 1 ? FastDiv{0u, 0u} : device_fastdiv(held);
-    auto sync = [&]() {
-        if (alone) __syncthreads();
-        else cluster_barrier();
-    };
-    const uint32_t region = (blockIdx.x / sp.parts) * samples;
-    uint32_t placed = 0;         // samples of the region placed by earlier passes
-    constexpr uint32_t kU = 4;   // samples in flight per thread
-    for (uint32_t lo = 0; lo < cells; lo += pass_cells) {
-        for (uint32_t i = tid; i < held; i += kSortThreads) s_count[i] = 0u;
-        sync();
-        for (uint32_t i0 = tid; i0 < n; i0 += kU * kSortThreads) {
-            float2 xy[kU];
-            uint32_t id[kU];
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                const uint32_t i = i0 + u * kSortThreads;
-                id[u] = id_of(i < n ? i : 0u);
-                xy[u] = load_pair(loc + 2ull * id[u]);
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                if (i0 + u * kSortThreads >= n) break;
-                const uint32_t c = sample_cell<CPS>(xy[u], W, H);
-                if (c - lo < pass_cells) {
-                    if (alone) {
-                        atomicAdd(s_count + (c - lo), 1u);
-                    } else {
-                        const uint32_t rank = fd_div(c - lo, by_held);
-                        cluster_count(cluster_address(s_count + (c - lo - rank * held), rank));
-                    }
-                } else if (CPS == 4 && c == kNoRow && lo == 0) {
-                    store_pair(static_cast<TL*>(p.grad_loc) + 2ull * id[u], 0.f, 0.f);
-                    static_cast<TL*>(p.grad_attn)[id[u]] = Elem<TL>::from_f(0.f);
-                }
-            }
-        }
-        sync();
-        // counts -> first positions: a thread takes an odd number of neighbours (no bank conflicts)
-        const uint32_t per = ((held + kSortThreads - 1) / kSortThreads) | 1u;
-        const uint32_t begin = min(held, tid * per), stop = min(held, begin + per);
-        uint32_t sum = 0;
-        for (uint32_t i = begin; i < stop; ++i) sum += s_count[i];
-        uint32_t incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) warp_sum[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t mine = warp_sum[lane];
-            uint32_t w = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += v;
-            }
-            warp_sum[lane] = w - mine;
-            if (lane == 31) block_sum = w;
-        }
-        if (sp.parts == 1) __syncthreads();
-        else cluster_barrier();
-        // the samples of lower ranks come first
-        uint32_t at = region + placed + warp_sum[warp] + incl - sum;
-        for (uint32_t r = 0; r < sp.parts; ++r) {
-            const uint32_t m = sp.parts == 1 ? block_sum : cluster_read(cluster_address(&block_sum, r));
-            if (r < part) at += m;
-            placed += m;
-        }
-        for (uint32_t i = begin; i < stop; ++i) {
-            const uint32_t m = s_count[i];
-            s_count[i] = at;
-            at += m;
-        }
-        sync();
-        for (uint32_t i0 = tid; i0 < n; i0 += kU * kSortThreads) {
-            float2 xy[kU];
-            uint32_t id[kU], pos[kU];
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                const uint32_t i = i0 + u * kSortThreads;
-                id[u] = id_of(i < n ? i : 0u);
-                xy[u] = load_pair(loc + 2ull * id[u]);
-                pos[u] = kNoRow;
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                if (i0 + u * kSortThreads >= n) break;
-                const uint32_t c = sample_cell<CPS>(xy[u], W, H);
-                if (c - lo < pass_cells) {
-                    if (alone) {
-                        pos[u] = atomicAdd(s_count + (c - lo), 1u);
-                    } else {
-                        const uint32_t rank = fd_div(c - lo, by_held);
-                        pos[u] = cluster_take(cluster_address(s_count + (c - lo - rank * held), rank));
-                    }
-                }
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u)
-                if (pos[u] != kNoRow) sp.sorted[pos[u]] = id[u];
-        }
-        // nobody leaves, or clears the counters, while others still use them
-        if (sp.parts == 1) __syncthreads();
-        else cluster_barrier();
+    __device__ __forceinline__ bool ok() const { return device_level_table_ok(p); }
+    __device__ __forceinline__ Map map(uint32_t m) const {
+        const uint32_t l = m % p.L, bh = m / p.L;
+        const uint32_t h = bh % p.H, b = bh / p.H;
+        Map r;
+        r.H = p.use_table ? p.lv.h[l] : p.shapes_dev[2 * l * p.table_step];
+        r.W = p.use_table ? p.lv.w[l] : p.shapes_dev[(2 * l + 1) * p.table_step];
+        r.cells = (CPS == 4) ? static_cast<uint32_t>(r.H + 1) * static_cast<uint32_t>(r.W + 1)
+                             : static_cast<uint32_t>(r.H) * static_cast<uint32_t>(r.W);
+        r.first = (b * p.Q * p.H + h) * p.LP + l * p.P;
+        return r;
     }
-    if (tid == 0 && part == 0) sp.regions[blockIdx.x / sp.parts] = make_uint2(region, placed);
-}
+    // sample i of the map: point i % P of query i / P
+    __device__ __forceinline__ uint32_t id(const Map& m, uint32_t i) const {
+        const uint32_t q = fd_div(i, fd_p);
+        return m.first + q * (static_cast<uint32_t>(p.H) * p.LP) + (i - q * p.P);
+    }
+    __device__ __forceinline__ float2 position(uint32_t id) const {
+        return load_pair(static_cast<const TL*>(p.loc) + 2ull * id);
+    }
+    __device__ __forceinline__ uint32_t cell(const Map& m, float2 xy) const {
+        return sample_cell<CPS>(xy, m.W, m.H);
+    }
+    // a sample that takes no part has zero gradients
+    __device__ __forceinline__ void drop(uint32_t id) const {
+        if constexpr (CPS == 4) {
+            store_pair(static_cast<TL*>(p.grad_loc) + 2ull * id, 0.f, 0.f);
+            static_cast<TL*>(p.grad_attn)[id] = Elem<TL>::from_f(0.f);
+        }
+    }
+};
 
 // ---------------------------------------------------------------------------
 // main kernels
 // ---------------------------------------------------------------------------
-// Two fp32 values in one 64-bit register pair, the operand form of the packed multiply-add: kept
-// in this form throughout, so that no moves are needed to assemble operands.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float x, float y) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// Four channels of a row, as two fp32 pairs.
-template <typename T>
-__device__ __forceinline__ void load_quad(const T* p, f32x2 (&q)[2]) {
-    if constexpr (sizeof(T) == 4) {
-        const ulonglong2 r = __ldg(reinterpret_cast<const ulonglong2*>(p));
-        q[0] = r.x;
-        q[1] = r.y;
-    } else {
-        const uint2 r = __ldg(reinterpret_cast<const uint2*>(p));
-        const uint32_t w[2] = {r.x, r.y};
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if constexpr (std::is_same<T, __half>::value) {
-                const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-                q[i] = pack2(v.x, v.y);
-            } else {
-                q[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-            }
-        }
-    }
-}
-__device__ __forceinline__ void red_quad(float* p, const f32x2 (&q)[2]) {
-    const float2 a = unpack2(q[0]), b = unpack2(q[1]);
-    red_add_f32x4(p, a.x, a.y, b.x, b.y);
-}
-
-// Sums each of N per-lane values over groups of LPR lanes (N a power of two <= LPR): halving
-// steps in which a lane gives half of its values away and keeps the other half, then plain
-// steps. Lane j of a group ends up with the sum of value j / (LPR / N).
-template <int N, int LPR, typename V>
-__device__ __forceinline__ V reduce_values(V (&d)[N], int j) {
-    if constexpr (N == 1) {
-#pragma unroll
-        for (int o = LPR / 2; o >= 1; o >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], o);
-        return d[0];
-    } else {
-        const bool up = (j & (LPR / 2)) != 0;
-        V half[N / 2];
-#pragma unroll
-        for (int i = 0; i < N / 2; ++i) {
-            half[i] = up ? d[N / 2 + i] : d[i];
-            half[i] += __shfl_xor_sync(0xffffffffu, up ? d[i] : d[N / 2 + i], LPR / 2);
-        }
-        return reduce_values<N / 2, LPR / 2>(half, j);
-    }
-}
-
 // One sorted sample, on its lane.
 struct SortedSample {
     uint32_t row;    // row offset of the cell's top-left corner (wraps where that does not exist)
@@ -443,22 +195,6 @@ __device__ __forceinline__ SortedSample set_up_sample(const Params& p, const Sor
     debug_check_cell(p, r);
     return r;
 }
-// Warps draw tickets in order; a ticket is up to `len` consecutive sorted samples of one region.
-struct Ticket {
-    uint32_t begin, end;   // positions; begin >= end: nothing
-};
-__device__ __forceinline__ bool next_ticket(const SortParams& sp, uint32_t len, int lane, Ticket& t) {
-    uint32_t n = 0;
-    if (lane == 0) n = atomicAdd(sp.ticket, 1u);
-    n = __shfl_sync(0xffffffffu, n, 0);
-    if (n >= sp.tickets) return false;
-    const uint32_t region = fd_div(n, sp.fd_tickets);
-    const uint2 r = __ldg(sp.regions + region);
-    t.begin = r.x + (n - region * sp.tickets_per_region) * len;
-    t.end = min(r.x + r.y, t.begin + len);
-    return true;
-}
-
 // Flags of a sorted sample in its stream (low bits; level width << 8 and existing corners << 4
 // above them).
 constexpr uint32_t kEnters = 1;      // its cell is not the previous sample's
@@ -858,82 +594,44 @@ gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 // ---------------------------------------------------------------------------
 // launch
 // ---------------------------------------------------------------------------
-// `streams` per warp, a round of 32 samples being 32 / streams steps of each.
 template <typename Kernel>
 static cudaError_t launch_sorted_main(Kernel kern, int streams, const Params& p, SortParams sp,
-                                      const LaunchShape& ls, cudaStream_t stream) {
-    int per_sm = ls.ctas_per_sm;
-    if (per_sm <= 0) {
-        const cudaError_t e =
-            resident_ctas(reinterpret_cast<const void*>(kern), kThreadsPerCta, 0, &per_sm);
-        if (e != cudaSuccess) return e;
-    }
-    const uint32_t cap = static_cast<uint32_t>(ls.sm_count) * per_sm;
-    // Long streams enter fewer cells, short ones level the load: eight tickets per resident
-    // warp, as long as a stream keeps one round.
-    const uint32_t want = sp.nsamples / (cap * kWarpsPerCta * 8u * streams);
-    const uint32_t round = 32u / streams;
-    sp.stream = want / round * round;
-    if (sp.stream < round) sp.stream = round;
-    if (sp.stream > kMaxStream) sp.stream = kMaxStream;
-    const uint32_t len = sp.stream * streams;
-    sp.tickets_per_region = (static_cast<uint32_t>(p.Q) * p.P + len - 1) / len;
-    sp.fd_tickets = make_fastdiv(sp.tickets_per_region);
-    sp.tickets = sp.nregions * sp.tickets_per_region;
-    const uint32_t need = (sp.tickets + kWarpsPerCta - 1) / kWarpsPerCta;
-    kern<<<need < cap ? need : cap, kThreadsPerCta, 0, stream>>>(p, sp);
-    return cudaGetLastError();
-}
-
-template <typename TL, int CPS>
-static cudaError_t launch_sort(const Params& p, SortParams& sp, const LaunchShape& ls,
-                               cudaStream_t stream) {
-    auto kern = sort_cells_kernel<TL, CPS>;
-    const size_t smem = kSortCells * sizeof(uint32_t);
-    int resident = 0;   // (asked for the shared-memory limit that the call sets)
-    const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kSortThreads, smem, &resident);
+                                      uint32_t samples_per_map, const LaunchShape& ls,
+                                      cudaStream_t stream) {
+    uint32_t grid = 0;
+    const cudaError_t e = plan_tickets(reinterpret_cast<const void*>(kern), streams, sp,
+                                       samples_per_map, ls, &grid);
     if (e != cudaSuccess) return e;
-    // the smallest cluster that gives most SMs work
-    const uint32_t levels = static_cast<uint32_t>(p.B) * p.H * p.L;
-    sp.parts = 1;
-    while (sp.parts < kMaxSortParts && levels * sp.parts < 3u * ls.sm_count / 2u) sp.parts *= 2;
-    sp.nregions = levels;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(levels * sp.parts);
-    cfg.blockDim = dim3(kSortThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = sp.parts;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p, sp);
+    kern<<<grid, kThreadsPerCta, 0, stream>>>(p, sp);
+    return cudaGetLastError();
 }
 
 template <typename T, typename TL>
 static cudaError_t launch_sorted_bilinear(const Params& p, SortParams sp,
                                           const LaunchShape& ls, cudaStream_t stream) {
-    cudaError_t e = launch_sort<TL, 4>(p, sp, ls, stream);
+    const uint32_t n = static_cast<uint32_t>(p.Q) * p.P;
+    cudaError_t e = launch_sort(AttentionSamples<TL, 4>{p, sp.fd_p, n},
+                                static_cast<uint32_t>(p.B) * p.H * p.L, sp, ls.sm_count, stream);
     if (e != cudaSuccess) return e;
-    if (p.D <= 16) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 4>, 8, p, sp, ls, stream);
-    if (p.D <= 32) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 8>, 4, p, sp, ls, stream);
-    if (p.D <= 64) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 16>, 2, p, sp, ls, stream);
-    if (p.D <= 128) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 32>, 1, p, sp, ls, stream);
-    return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 2, 32>, 1, p, sp, ls, stream);
+    if (p.D <= 16) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 4>, 8, p, sp, n, ls, stream);
+    if (p.D <= 32) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 8>, 4, p, sp, n, ls, stream);
+    if (p.D <= 64) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 16>, 2, p, sp, n, ls, stream);
+    if (p.D <= 128) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 32>, 1, p, sp, n, ls, stream);
+    return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 2, 32>, 1, p, sp, n, ls, stream);
 }
 
 template <typename T>
 static cudaError_t launch_sorted_nearest(const Params& p, SortParams sp,
                                          const LaunchShape& ls, cudaStream_t stream) {
-    cudaError_t e = launch_sort<T, 1>(p, sp, ls, stream);
+    const uint32_t n = static_cast<uint32_t>(p.Q) * p.P;
+    cudaError_t e = launch_sort(AttentionSamples<T, 1>{p, sp.fd_p, n},
+                                static_cast<uint32_t>(p.B) * p.H * p.L, sp, ls.sm_count, stream);
     if (e != cudaSuccess) return e;
-    if (p.D <= 16) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 4>, 1, p, sp, ls, stream);
-    if (p.D <= 32) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 8>, 1, p, sp, ls, stream);
-    if (p.D <= 64) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 16>, 1, p, sp, ls, stream);
-    if (p.D <= 128) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 32>, 1, p, sp, ls, stream);
-    return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 2, 32>, 1, p, sp, ls, stream);
+    if (p.D <= 16) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 4>, 1, p, sp, n, ls, stream);
+    if (p.D <= 32) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 8>, 1, p, sp, n, ls, stream);
+    if (p.D <= 64) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 16>, 1, p, sp, n, ls, stream);
+    if (p.D <= 128) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 32>, 1, p, sp, n, ls, stream);
+    return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 2, 32>, 1, p, sp, n, ls, stream);
 }
 
 }  // namespace msda

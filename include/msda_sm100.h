@@ -207,10 +207,29 @@ int gka_sm100_backward_ws(const void* value, const int32_t* spatial_shapes,
 int da_sm100_forward(const void* feat, const int32_t* spatial_shape, const int32_t* scale_start,
                      const void* sampling_location, const void* weights, void* out, int B, int F,
                      int C, int A, int Pts, int cams, int scales, int G, void* stream);
+/* The same with feat, sampling_location and weights in `dtype`; out stays float32. 16-bit tensors
+ * need whole vector rows (C a power-of-two multiple of 4, groups of 2^k quads), else
+ * MSDA_ERR_ALIGN. */
+int da_sm100_forward_typed(const void* feat, const int32_t* spatial_shape, const int32_t* scale_start,
+                           const void* sampling_location, const void* weights, float* out, int B, int F,
+                           int C, int A, int Pts, int cams, int scales, int G, int dtype, void* stream);
 int da_sm100_backward(const void* feat, const int32_t* spatial_shape, const int32_t* scale_start,
                       const void* sampling_location, const void* weights, const void* grad_out,
                       void* grad_feat, void* grad_sampling_location, void* grad_weights, int B,
                       int F, int C, int A, int Pts, int cams, int scales, int G, void* stream);
+/* Backward over samples sorted by the cell they fall into, whose feature rows are loaded and
+ * reduced once per run of samples in a cell. feat, sampling_location, weights and grad_out in
+ * `dtype`, the three gradients in float32 (zero-filled by the call; grad_sampling_location is
+ * summed over the scales with atomics). `workspace`: at least
+ * da_sm100_backward_workspace_bytes() bytes of device memory, 16-byte aligned; 0 means that this
+ * form does not apply to the shape. */
+size_t da_sm100_backward_workspace_bytes(int B, int F, int C, int A, int Pts, int cams, int scales,
+                                         int G);
+int da_sm100_backward_ws(const void* feat, const int32_t* spatial_shape, const int32_t* scale_start,
+                         const void* sampling_location, const void* weights, const void* grad_out,
+                         float* grad_feat, float* grad_sampling_location, float* grad_weights,
+                         void* workspace, size_t workspace_bytes, int B, int F, int C, int A, int Pts,
+                         int cams, int scales, int G, int dtype, void* stream);
 int da_sm100_last_cuda_error(void);
 
 /* Algorithmic (compulsory) bytes one call moves: every operand read once and
