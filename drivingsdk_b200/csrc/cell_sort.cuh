@@ -229,30 +229,6 @@ __device__ __forceinline__ bool next_ticket(const SortParams& sp, uint32_t len, 
     return true;
 }
 
-// Two fp32 values in one 64-bit register pair, the operand form of the packed multiply-add: kept
-// in this form throughout, so that no moves are needed to assemble operands.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float x, float y) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // Four channels of a row, as two fp32 pairs.
 template <typename T>
 __device__ __forceinline__ void load_quad(const T* p, f32x2 (&q)[2]) {

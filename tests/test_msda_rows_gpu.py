@@ -23,3 +23,15 @@ def test_rows_that_leave_lanes_idle(D, dtype):
     finally:
         capi.load().msda_sm100_tune(capi.TUNE_SORT, old)
     assert capi.load().msda_sm100_device_status(1) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D,L,P", [(32, 1, 1), (32, 1, 3), (32, 1, 4), (16, 2, 4), (8, 3, 5), (64, 1, 2),
+                                   (128, 1, 1), (24, 1, 4)])
+def test_tasks_of_few_rows(D, L, P, dtype):
+    """Several tasks per warp, one per group of lanes: task counts that leave groups without one,
+    tasks that share several groups, a last item that is not full."""
+    levels = ((7, 9), (4, 5), (2, 2))[:L]
+    w = workloads.Workload("few", 1, 37, 3, D, levels, P, (-0.2, 1.2), seed=D + P)
+    inp = workloads.make_inputs(w, dtype)
+    parity.compare_all(inp, parity.run_python_api(parity.to_device(inp, dtype)), dtype)
