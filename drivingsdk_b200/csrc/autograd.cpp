@@ -170,6 +170,80 @@ struct AddRelu : Function<AddRelu> {
     }
 };
 
+// Deformable convolution, modulated where `mask` is given (then `bias` may be). Keeps copies, so
+// that the operands may be overwritten: the pair form its block and the weights, the fp32 form
+// (other channel counts, mixed types) the channels-last tensors and the columns.
+struct DeformConv : Function<DeformConv> {
+    static Tensor forward(AutogradContext* ctx, Tensor x, Tensor offset, std::optional<Tensor> mask_opt,
+                          Tensor weight, std::optional<Tensor> bias_opt, std::vector<int64_t> stride, std::vector<int64_t> padding,
+                          std::vector<int64_t> dilation, int64_t groups, int64_t deformable_groups,
+                          bool keep) {
+        const Tensor mask = mask_opt.value_or(Tensor()), bias = bias_opt.value_or(Tensor());
+        const bool modulated = mask.defined();
+        const Conv conv{stride, padding, dilation, groups, deformable_groups};
+        const auto kind = x.scalar_type();
+        const bool alike = (kind == at::kFloat || kind == at::kHalf || kind == at::kBFloat16) &&
+                           offset.scalar_type() == kind && weight.scalar_type() == kind &&
+                           (!modulated || mask.scalar_type() == kind);
+        ctx->saved_data["modulated"] = modulated;
+        Tensor out, saved;
+        std::vector<int64_t> shape;
+        if (alike) std::tie(out, saved) = conv_forward(x, offset, mask, weight, bias, conv, &shape);
+        ctx->saved_data["shape"] = shape;   // empty: the fp32 form
+        if (out.defined()) {
+            if (keep) {
+                ctx->save_for_backward({weight.clone(at::MemoryFormat::Contiguous), saved, bias});
+            }
+            return out;
+        }
+        ctx->saved_data["conv"] = std::vector<int64_t>{stride[0], stride[1], padding[0], padding[1], dilation[0],
+                                                       dilation[1], groups, deformable_groups};
+        const std::vector<int64_t> kernel{weight.size(2), weight.size(3)};
+        auto nhwc = [](const Tensor& t) { return t.permute({0, 2, 3, 1}).contiguous(); };
+        const Tensor nx = nhwc(x), noff = nhwc(offset), nw = nhwc(weight);
+        const Tensor nmask = modulated ? nhwc(mask) : mask;
+        Tensor columns;
+        if (modulated) {
+            std::tie(out, columns) = modulated_deformable_conv2d(
+                nx, noff, nmask, nw, bias.defined() ? c10::optional<Tensor>(bias) : c10::nullopt, kernel, stride,
+                padding, dilation, groups, deformable_groups, bias.defined() ? 1 : 0);
+        } else {
+            std::tie(out, columns) =
+                deformable_conv2d(nx, noff, nw, kernel, stride, padding, dilation, groups, deformable_groups);
+        }
+        ctx->save_for_backward({nw, columns, bias, nx, noff, nmask});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        const auto shape = ctx->saved_data["shape"].toIntVector();
+        const bool modulated = ctx->saved_data["modulated"].toBool(), with_bias = s[2].defined();
+        ConvGrads r;
+        {
+            const at::NoGradGuard no_grad;
+            if (!shape.empty()) {
+                r = conv_backward(s[0], modulated, with_bias, s[1], g[0], shape);
+                if (with_bias) r.bias = r.bias.to(s[2].scalar_type());
+            } else {
+                const auto c = ctx->saved_data["conv"].toIntVector();
+                const std::vector<int64_t> kernel{s[0].size(1), s[0].size(2)}, stride{c[0], c[1]},
+                    padding{c[2], c[3]}, dilation{c[4], c[5]};
+                const Tensor go = g[0].permute({0, 2, 3, 1}).contiguous();
+                if (modulated) {
+                    std::tie(r.x, r.weight, r.bias, r.offset, r.mask) = modulated_deformable_conv2d_backward(
+                        s[3], s[4], s[5], s[0], with_bias ? c10::optional<Tensor>(s[2]) : c10::nullopt, s[1], go,
+                        kernel, stride, padding, dilation, c[6], c[7], with_bias ? 1 : 0);
+                } else {
+                    std::tie(r.x, r.weight, r.offset) = deformable_conv2d_backward(
+                        s[3], s[0], s[4], s[1], go, kernel, stride, padding, dilation, c[6], c[7]);
+                }
+            }
+        }
+        return once({r.x, r.offset, r.mask, r.weight, r.bias, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()},
+                    g[0]);
+    }
+};
+
 // inference only, as in the reference: the result knows its input, but has no derivative
 struct MaxPool : Function<MaxPool> {
     static Tensor forward(AutogradContext*, const Tensor& x, int64_t kernel, int64_t stride,
@@ -204,6 +278,30 @@ Tensor add_relu(const Tensor& x, const Tensor& y) {
     return AddRelu::apply(x, y, in_place);
 }
 
+using Pair = std::vector<int64_t>;
+bool any_requires_grad(at::TensorList ts) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor& t : ts)
+        if (t.defined() && t.requires_grad()) return true;
+    return false;
+}
+Tensor deform_conv(const Tensor& x, const Tensor& offset, const Tensor& weight, const Pair& stride,
+                   const Pair& padding, const Pair& dilation, int64_t groups, int64_t deformable_groups) {
+    return DeformConv::apply(x, offset, std::optional<Tensor>(), weight, std::optional<Tensor>(), stride, padding, dilation, groups,
+                             deformable_groups, any_requires_grad({x, offset, weight}));
+}
+Tensor modulated_deform_conv(const Tensor& x, const Tensor& offset, const Tensor& mask, const Tensor& weight,
+                             const c10::optional<Tensor>& bias, const Pair& stride, const Pair& padding,
+                             const Pair& dilation, int64_t groups, int64_t deformable_groups) {
+    // custom_fwd(cast_inputs=torch.float32), the casts outside the function so that gradients
+    // return through them
+    const bool cast = at::autocast::is_autocast_enabled(at::kCUDA);
+    const Tensor b = bias.has_value() ? *bias : Tensor();
+    return DeformConv::apply(autocast_f32(x, cast), autocast_f32(offset, cast),
+                             std::optional<Tensor>(autocast_f32(mask, cast)), autocast_f32(weight, cast),
+                             b.defined() ? std::optional<Tensor>(autocast_f32(b, cast)) : std::nullopt, stride, padding,
+                             dilation, groups, deformable_groups, any_requires_grad({x, offset, mask, weight, b}));
+}
 Tensor max_pool2d(const Tensor& x, int64_t kernel, int64_t stride, int64_t padding) {
     return MaxPool::apply(x, kernel, stride, padding);
 }
@@ -216,6 +314,9 @@ void register_autograd(pybind11::module& m) {
     m.def("msda_fused_autograd", &fused, release(), "differentiable multi_scale_deformable_attn_fused");
     m.def("gka_autograd", &gka, release(), "differentiable geometric_kernel_attention");
     m.def("deformable_aggregation_autograd", &aggregation, release(), "differentiable deformable_aggregation");
+    m.def("deform_conv2d_autograd", &deform_conv, release(), "differentiable deform_conv2d");
+    m.def("modulated_deform_conv2d_autograd", &modulated_deform_conv, release(),
+          "differentiable modulated_deform_conv2d");
     m.def("max_pool2d_autograd", &max_pool2d, release(), "npu_max_pool2d, known to autograd");
     m.def("add_relu_autograd", &add_relu, release(), "differentiable npu_add_relu");
 }

@@ -698,10 +698,10 @@ struct DcnCall {
     at::Tensor x, offset, mask, weight;
 };
 
-DcnCall check_dcn(const at::Tensor& input, const at::Tensor& offset, const at::Tensor& mask,
-                  const at::Tensor& weight, at::IntArrayRef kernel_size, at::IntArrayRef stride,
-                  at::IntArrayRef padding, at::IntArrayRef dilation, int64_t groups,
-                  int64_t deformable_groups) {
+dcn_shape check_dcn_shape(const at::Tensor& input, const at::Tensor& offset, const at::Tensor& mask,
+                          const at::Tensor& weight, at::IntArrayRef kernel_size, at::IntArrayRef stride,
+                          at::IntArrayRef padding, at::IntArrayRef dilation, int64_t groups,
+                          int64_t deformable_groups) {
     TORCH_CHECK(input.is_cuda() && offset.is_cuda() && weight.is_cuda(),
                 "deformable_conv2d: CUDA tensors expected (this build has no CPU path)");
     TORCH_CHECK(input.dim() == 4, "input must to be a 4D Tensor, but got: ", input.dim());
@@ -730,24 +730,34 @@ DcnCall check_dcn(const at::Tensor& input, const at::Tensor& offset, const at::T
                         mask.size(2) == offset.size(2) && mask.size(3) == deformable_groups * taps,
                     "The shape of the mask is invalid");
     }
+    dcn_shape s;
+    s.N = static_cast<int>(input.size(0));
+    s.H = static_cast<int>(input.size(1));
+    s.W = static_cast<int>(input.size(2));
+    s.C = static_cast<int>(input.size(3));
+    s.Ho = static_cast<int>(offset.size(1));
+    s.Wo = static_cast<int>(offset.size(2));
+    s.Co = static_cast<int>(weight.size(0));
+    s.kh = static_cast<int>(kernel_size[0]);
+    s.kw = static_cast<int>(kernel_size[1]);
+    s.stride_h = static_cast<int>(stride[0]);
+    s.stride_w = static_cast<int>(stride[1]);
+    s.pad_h = static_cast<int>(padding[0]);
+    s.pad_w = static_cast<int>(padding[1]);
+    s.dil_h = static_cast<int>(dilation[0]);
+    s.dil_w = static_cast<int>(dilation[1]);
+    s.groups = static_cast<int>(groups);
+    s.deform_groups = static_cast<int>(deformable_groups);
+    return s;
+}
+
+DcnCall check_dcn(const at::Tensor& input, const at::Tensor& offset, const at::Tensor& mask,
+                  const at::Tensor& weight, at::IntArrayRef kernel_size, at::IntArrayRef stride,
+                  at::IntArrayRef padding, at::IntArrayRef dilation, int64_t groups,
+                  int64_t deformable_groups) {
     DcnCall c;
-    c.s.N = static_cast<int>(input.size(0));
-    c.s.H = static_cast<int>(input.size(1));
-    c.s.W = static_cast<int>(input.size(2));
-    c.s.C = static_cast<int>(input.size(3));
-    c.s.Ho = static_cast<int>(offset.size(1));
-    c.s.Wo = static_cast<int>(offset.size(2));
-    c.s.Co = static_cast<int>(weight.size(0));
-    c.s.kh = static_cast<int>(kernel_size[0]);
-    c.s.kw = static_cast<int>(kernel_size[1]);
-    c.s.stride_h = static_cast<int>(stride[0]);
-    c.s.stride_w = static_cast<int>(stride[1]);
-    c.s.pad_h = static_cast<int>(padding[0]);
-    c.s.pad_w = static_cast<int>(padding[1]);
-    c.s.dil_h = static_cast<int>(dilation[0]);
-    c.s.dil_w = static_cast<int>(dilation[1]);
-    c.s.groups = static_cast<int>(groups);
-    c.s.deform_groups = static_cast<int>(deformable_groups);
+    c.s = check_dcn_shape(input, offset, mask, weight, kernel_size, stride, padding, dilation, groups,
+                          deformable_groups);
     c.x = input.to(at::kFloat).contiguous();
     c.offset = offset.to(at::kFloat).contiguous();
     c.weight = weight.to(at::kFloat).contiguous();
@@ -833,6 +843,90 @@ DcnGrads dcn_backward(const char* what, const at::Tensor& input, const at::Tenso
 }
 
 }  // namespace
+
+namespace sdk {
+namespace {
+// NCHW-style tensors as the channels-last views that the checks are written for
+dcn_shape conv_shape(const at::Tensor& x, const at::Tensor& offset, const at::Tensor& mask,
+                     const at::Tensor& weight, const Conv& conv) {
+    TORCH_CHECK(x.dim() == 4 && offset.dim() == 4 && weight.dim() == 4 && (!mask.defined() || mask.dim() == 4),
+                "deformable_conv2d: 4D tensors expected");
+    auto nhwc = [](const at::Tensor& t) { return t.defined() ? t.permute({0, 2, 3, 1}) : t; };
+    return check_dcn_shape(nhwc(x), nhwc(offset), nhwc(mask), nhwc(weight), {weight.size(2), weight.size(3)},
+                           conv.stride, conv.padding, conv.dilation, conv.groups, conv.deformable_groups);
+}
+bool is_nhwc(const at::Tensor& t) { return !t.is_contiguous() && t.permute({0, 2, 3, 1}).is_contiguous(); }
+void* pointer(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+}  // namespace
+
+std::tuple<at::Tensor, at::Tensor> conv_forward(const at::Tensor& x_in, const at::Tensor& offset_in,
+                                                const at::Tensor& mask_in, const at::Tensor& weight_in,
+                                                const at::Tensor& bias_in, const Conv& conv,
+                                                std::vector<int64_t>* shape) {
+    const dcn_shape s = conv_shape(x_in, offset_in, mask_in, weight_in, conv);
+    const size_t saved_bytes = dcn_sm100_saved_bytes(&s);
+    if (saved_bytes == 0 || x_in.numel() == 0 || offset_in.numel() == 0) return {};
+    const int* fields = reinterpret_cast<const int*>(&s);
+    shape->assign(fields, fields + sizeof(s) / sizeof(int));
+    const c10::cuda::CUDAGuard guard(x_in.device());
+    const auto kind = x_in.scalar_type();
+    const at::Tensor x = is_nhwc(x_in) ? x_in : x_in.contiguous();
+    const at::Tensor offset = offset_in.contiguous();
+    const at::Tensor mask = mask_in.defined() ? mask_in.contiguous() : mask_in;
+    const at::Tensor weight = weight_in.contiguous();
+    at::Tensor bias;
+    if (bias_in.defined()) {
+        TORCH_CHECK(bias_in.is_cuda() && bias_in.numel() == s.Co, "bias must be a CUDA tensor [c_out]");
+        bias = bias_in.to(at::kFloat).contiguous();
+    }
+    const auto bytes = x.options().dtype(at::kByte);
+    at::Tensor saved = at::empty({static_cast<int64_t>(saved_bytes)}, bytes);
+    const size_t ws_bytes = dcn_sm100_nchw_workspace_bytes(&s, 0);
+    at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)}, bytes);
+    at::Tensor out = at::empty({s.N, s.Ho, s.Wo, s.Co}, x.options().dtype(at::kFloat));
+    const int rc = dcn_sm100_forward_nchw(
+        x.data_ptr(), is_nhwc(x_in) ? 1 : 0, offset.data_ptr(), pointer(mask), weight.data_ptr(),
+        bias.defined() ? bias.data_ptr<float>() : nullptr, out.data_ptr<float>(), saved.data_ptr(), saved_bytes,
+        ws.data_ptr(), ws_bytes, &s, dtype_code(kind), at::cuda::getCurrentCUDAStream().stream());
+    raise_on_error(rc, "deformable_conv2d");
+    return std::make_tuple(out.permute({0, 3, 1, 2}).to(kind), saved);
+}
+
+ConvGrads conv_backward(const at::Tensor& weight, bool modulated, bool with_bias, const at::Tensor& saved,
+                        const at::Tensor& grad_in, const std::vector<int64_t>& shape) {
+    dcn_shape s;
+    static_assert(sizeof(s) % sizeof(int) == 0, "dcn_shape holds ints");
+    int* fields = reinterpret_cast<int*>(&s);
+    for (size_t i = 0; i < sizeof(s) / sizeof(int); ++i) fields[i] = static_cast<int>(shape[i]);
+    TORCH_CHECK(grad_in.is_cuda() && grad_in.dim() == 4 && grad_in.size(0) == s.N && grad_in.size(1) == s.Co &&
+                    grad_in.size(2) == s.Ho && grad_in.size(3) == s.Wo,
+                "grad_output must be a CUDA tensor [n, c_out, h_out, w_out]");
+    const c10::cuda::CUDAGuard guard(weight.device());
+    const auto kind = weight.scalar_type();
+    at::Tensor grad = grad_in.to(kind);
+    const bool nhwc = is_nhwc(grad);
+    if (!nhwc) grad = grad.contiguous();
+    const auto f32 = weight.options().dtype(at::kFloat);
+    const int64_t taps = static_cast<int64_t>(s.deform_groups) * s.kh * s.kw;
+    at::Tensor gx = at::empty({s.N, s.H, s.W, s.C}, f32);
+    at::Tensor goff = at::empty({s.N, s.Ho, s.Wo, 2 * taps}, f32);
+    at::Tensor gmask = modulated ? at::empty({s.N, s.Ho, s.Wo, taps}, f32) : at::Tensor();
+    at::Tensor gw = at::empty({s.Co, s.kh, s.kw, s.C / s.groups}, f32);
+    at::Tensor gb = with_bias ? at::empty({s.Co}, f32) : at::Tensor();
+    const size_t ws_bytes = dcn_sm100_nchw_workspace_bytes(&s, 1);
+    at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)}, f32.dtype(at::kByte));
+    const int rc = dcn_sm100_backward_nchw(
+        weight.data_ptr(), grad.data_ptr(), nhwc ? 1 : 0, saved.data_ptr(), gx.data_ptr<float>(),
+        goff.data_ptr<float>(), static_cast<float*>(pointer(gmask)), gw.data_ptr<float>(),
+        static_cast<float*>(pointer(gb)), ws.data_ptr(), ws_bytes, &s, dtype_code(kind),
+        at::cuda::getCurrentCUDAStream().stream());
+    raise_on_error(rc, "deformable_conv2d_backward");
+    auto nchw = [](const at::Tensor& t, at::ScalarType k) {
+        return t.defined() ? t.permute({0, 3, 1, 2}).to(k) : t;
+    };
+    return {nchw(gx, kind), nchw(goff, kind), nchw(gmask, kind), nchw(gw, kind), gb};
+}
+}  // namespace sdk
 
 std::tuple<at::Tensor, at::Tensor> deformable_conv2d(
     const at::Tensor& input, const at::Tensor& offset, const at::Tensor& weight,

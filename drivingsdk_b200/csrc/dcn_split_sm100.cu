@@ -1,0 +1,560 @@
+// Deformable / modulated deformable convolution from NCHW tensors for sm_100a, products over fp16
+// pairs (gemm_split.h). Same decomposition as dcn_sm100.cu (gather, products, scatter), with every
+// operand of a product written as pairs by the kernel that produces it:
+//   forward   to_nhwc x / offset / mask (and the bounds of x and mask, which bound the columns);
+//             weight pairs; gather -> column pairs; out = columns x weight^T
+//   backward  bounds and pairs of grad_out, once scaled by pixel (its rows in the product that
+//             gives grad_columns) and once by channel (its rows in grad_weight); transposed weight
+//             pairs; grad_columns; scatter; grad_weight = grad_out^T x columns
+// The column pairs take the bytes that the fp32 columns would.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "../../include/conv_ops_sm100.h"
+#include "dcn_common.cuh"
+#include "dcn_split.h"
+#include "gemm_split.h"
+#include "msda_common.cuh"
+#include "split_scale.cuh"
+
+namespace {
+
+using namespace dcn;
+using msda::SplitOperand;
+using msda::SplitScale;
+using msda::Elem;
+
+// A tile of a [n][channels][pixels] tensor (or [n][pixels][channels]: channels_last) in shared
+// memory as [channel][pixel]; zero outside.
+template <typename T, int CH>
+__device__ __forceinline__ void load_tile(const T* src, int channels_last, int n, int c0, int p0, int C,
+                                          int P, float (&tile)[CH][33]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!channels_last) {
+#pragma unroll
+        for (int r = warp; r < CH; r += kThreads / 32) {
+            const int c = c0 + r, p = p0 + lane;
+            tile[r][lane] = (c < C && p < P) ? Elem<T>::to_f(src[(static_cast<size_t>(n) * C + c) * P + p]) : 0.f;
+        }
+    } else {
+#pragma unroll
+        for (int i = warp; i < CH; i += kThreads / 32) {
+            const int r = (i % (CH / 32)) * 32 + lane, q = i / (CH / 32);
+            const int c = c0 + r, p = p0 + q;
+            tile[r][q] = (c < C && p < P) ? Elem<T>::to_f(src[(static_cast<size_t>(n) * P + p) * C + c]) : 0.f;
+        }
+    }
+    __syncthreads();
+}
+
+// Raises *at to v; most callers find it high enough already and skip the atomic.
+__device__ __forceinline__ void raise_max(uint32_t* at, uint32_t v) {
+    if (v > *reinterpret_cast<volatile uint32_t*>(at)) atomicMax(at, v);
+}
+
+// [n][C][P] (or channels last) in T -> [n][P][C] in fp32; optionally the largest magnitude.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+to_nhwc_kernel(const T* __restrict__ src, int channels_last, float* __restrict__ dst, int C, int P,
+               uint32_t* magnitude) {
+    __shared__ float tile[32][33];
+    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32, n = blockIdx.z;
+    load_tile<T, 32>(src, channels_last, n, c0, p0, C, P, tile);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t most = 0;
+#pragma unroll
+    for (int r = warp; r < 32; r += kThreads / 32) {
+        const int p = p0 + r, c = c0 + lane;
+        const float v = tile[lane][r];
+        most = max(most, msda::finite_magnitude(v));
+        if (p < P && c < C) dst[(static_cast<size_t>(n) * P + p) * C + c] = v;
+    }
+    if (magnitude != nullptr) {
+        __shared__ uint32_t warp_most[kThreads / 32];
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) warp_most[warp] = most;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kThreads / 32; ++w) most = max(most, warp_most[w]);
+            raise_max(magnitude, most);
+        }
+    }
+}
+
+// Rows of a product's operand come from pixel p of image n: n * P + p, or, for weights seen as
+// [group][output channel][c * K + k], the column order k * Cg + c.
+struct RowOrder {
+    int P, K, Cg;   // K == 0: plain
+    __device__ __forceinline__ size_t row(int n, int p) const {
+        const int q = K == 0 ? p : (p % K) * Cg + p / K;
+        return static_cast<size_t>(n) * P + q;
+    }
+};
+
+// Largest magnitudes of a [n][C][P] tensor per row (pixel) and per channel, and the channel sums.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
+              uint32_t* row_most, uint32_t* channel_most, float* channel_sum) {
+    __shared__ float tile[64][33];
+    __shared__ uint32_t part[kThreads / 32][32];
+    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
+    load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int r = warp; r < 64; r += kThreads / 32) {
+        const float v = tile[r][lane];
+        const uint32_t a = msda::finite_magnitude(v);
+        mine = max(mine, a);
+        if (channel_most != nullptr) {
+            const uint32_t most = __reduce_max_sync(0xffffffffu, a);
+            if (lane == 0 && c0 + r < C) raise_max(channel_most + c0 + r, most);
+        }
+        if (channel_sum != nullptr) {
+            float s = v;
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0 && c0 + r < C) atomicAdd(channel_sum + c0 + r, s);
+        }
+    }
+    part[warp][lane] = mine;
+    __syncthreads();
+    if (warp == 0 && p0 + lane < order.P) {
+        for (int w = 1; w < kThreads / 32; ++w) mine = max(mine, part[w][lane]);
+        raise_max(row_most + order.row(n, p0 + lane), mine);
+    }
+}
+
+// [n][C][P] -> pairs [rows][C]: scaled by row, and (optional) by channel.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+pairs_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
+             const uint32_t* row_most, const uint32_t* channel_most, uint16_t* __restrict__ by_row,
+             uint16_t* __restrict__ by_channel, size_t plane) {
+    __shared__ float tile[64][33];
+    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
+    load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = c0 + 2 * lane;
+    if (c >= C) return;   // C is even
+    float sc[2] = {1.f, 1.f};
+    if (by_channel != nullptr) {
+        sc[0] = msda::exp2_int(msda::split_exponent(SplitScale{channel_most, 1, nullptr}, c));
+        sc[1] = msda::exp2_int(msda::split_exponent(SplitScale{channel_most, 1, nullptr}, c + 1));
+    }
+#pragma unroll
+    for (int q = warp; q < 32; q += kThreads / 32) {
+        if (p0 + q >= order.P) break;
+        const size_t row = order.row(n, p0 + q);
+        const float x = tile[2 * lane][q], y = tile[2 * lane + 1][q];
+        const float sr = msda::exp2_int(msda::split_exponent(SplitScale{row_most, 1, nullptr}, row));
+        const uint2 r = msda::split_pair(x, y, sr);
+        uint16_t* at = by_row + row * C + c;
+        *reinterpret_cast<uint32_t*>(at) = r.x;
+        *reinterpret_cast<uint32_t*>(at + plane) = r.y;
+        if (by_channel != nullptr) {
+            const uint2 h = msda::split_pair(x * sc[0], y * sc[1], 1.f);
+            uint16_t* to = by_channel + row * C + c;
+            *reinterpret_cast<uint32_t*>(to) = h.x;
+            *reinterpret_cast<uint32_t*>(to + plane) = h.y;
+        }
+    }
+}
+
+// weight [Co][Cg][K] -> pairs [Co][K * Cg], one CTA per output channel, scaled by it.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+weight_pairs_kernel(const T* __restrict__ w, int Cg, int K, uint32_t* most, uint16_t* __restrict__ pairs,
+                    size_t plane) {
+    __shared__ uint32_t warp_most[kThreads / 32];
+    const int co = blockIdx.x, Kd = Cg * K;
+    const T* src = w + static_cast<size_t>(co) * Kd;
+    uint32_t m = 0;
+    for (int i = threadIdx.x; i < Kd; i += kThreads) m = max(m, msda::finite_magnitude(Elem<T>::to_f(src[i])));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) warp_most[threadIdx.x >> 5] = m;
+    __syncthreads();
+    for (int i = 0; i < kThreads / 32; ++i) m = max(m, warp_most[i]);
+    if (threadIdx.x == 0) most[co] = m;
+    const uint32_t bound = m;
+    const float s = msda::exp2_int(msda::split_exponent(SplitScale{&bound, 0, nullptr}, 0));
+    for (int i = threadIdx.x; i < Kd / 2; i += kThreads) {
+        const int at = 2 * i, k = at / Cg, c = at - k * Cg;   // Cg is even
+        const uint2 r = msda::split_pair(Elem<T>::to_f(src[c * K + k]), Elem<T>::to_f(src[(c + 1) * K + k]), s);
+        uint16_t* to = pairs + static_cast<size_t>(co) * Kd + at;
+        *reinterpret_cast<uint32_t*>(to) = r.x;
+        *reinterpret_cast<uint32_t*>(to + plane) = r.y;
+    }
+}
+
+// Column pairs: mask * bilinear(x). A group of lanes per (pixel, deformable group, tap) moves
+// pieces of eight channels. A CTA walks a contiguous run of items, a slice of the channels at a
+// time: neighbouring taps and pixels read mostly the same rows.
+constexpr uint32_t kRunItems = 144;   // per slice: 16 pixels of a 3 x 3 kernel
+__global__ void __launch_bounds__(kThreads, 3)
+gather_pairs_kernel(const __grid_constant__ DcnParams p, uint16_t* __restrict__ columns, size_t plane,
+                    const SplitScale bound) {
+    const int lane = threadIdx.x & 31;
+    const int lpi = 1 << p.lpi_log2;
+    const int sub = lane & (lpi - 1);
+    const uint32_t slot = (threadIdx.x >> p.lpi_log2);             // item within the CTA's step
+    const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
+    const uint32_t begin = static_cast<uint32_t>(static_cast<uint64_t>(p.items) * blockIdx.x / gridDim.x);
+    const uint32_t end = static_cast<uint32_t>(static_cast<uint64_t>(p.items) * (blockIdx.x + 1) / gridDim.x);
+    const float scale = msda::exp2_int(msda::split_exponent(bound, 0));
+    for (uint32_t run = begin; run < end; run += kRunItems) {
+        const uint32_t stop = min(end, run + kRunItems);
+        for (int piece = sub; piece < p.pieces; piece += lpi) {
+#pragma unroll 1
+            for (uint32_t item = run + slot; item < stop; item += per_step) {
+                uint32_t m, dg, k;
+                float mk;
+                Sample s;
+                item_setup(p, item, &m, &dg, &k, &mk, &s);
+                float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+                if (s.valid) {
+                    float4 v[4][2];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        v[c][0] = load_piece<4>(s.row[c], 2 * piece);
+                        v[c][1] = load_piece<4>(s.row[c], 2 * piece + 1);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float w = s.w[c] * mk;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            acc[h].x = fmaf(w, v[c][h].x, acc[h].x);
+                            acc[h].y = fmaf(w, v[c][h].y, acc[h].y);
+                            acc[h].z = fmaf(w, v[c][h].z, acc[h].z);
+                            acc[h].w = fmaf(w, v[c][h].w, acc[h].w);
+                        }
+                    }
+                }
+                const uint2 r0 = msda::split_pair(acc[0].x, acc[0].y, scale);
+                const uint2 r1 = msda::split_pair(acc[0].z, acc[0].w, scale);
+                const uint2 r2 = msda::split_pair(acc[1].x, acc[1].y, scale);
+                const uint2 r3 = msda::split_pair(acc[1].z, acc[1].w, scale);
+                uint16_t* to = columns + column_index(p, m, k, dg * p.Cd + 8 * piece);
+                *reinterpret_cast<uint4*>(to) = make_uint4(r0.x, r1.x, r2.x, r3.x);
+                *reinterpret_cast<uint4*>(to + plane) = make_uint4(r0.y, r1.y, r2.y, r3.y);
+            }
+        }
+    }
+}
+
+size_t up(size_t v) { return (v + 255) / 256 * 256; }
+
+// What the forward leaves for the backward: bounds, x, offset and mask as [n][pixel][channel] fp32,
+// column pairs.
+struct Saved {
+    size_t bounds, x, offset, mask, columns, total;
+    size_t plane;   // halves per plane of the columns
+};
+Saved plan_saved(const dcn_shape* s, const Derived& d) {
+    Saved r;
+    r.bounds = 0;
+    r.x = 256;
+    r.offset = r.x + up(static_cast<size_t>(s->N) * s->H * s->W * s->C * 4);
+    const size_t taps = static_cast<size_t>(d.M) * s->deform_groups * d.K;
+    r.mask = r.offset + up(taps * 8);
+    r.columns = r.mask + up(taps * 4);
+    r.plane = static_cast<size_t>(d.M) * s->groups * d.Kd;
+    r.total = r.columns + up(r.plane * 4) + 256;   // row blocks of 64 may be read past the end
+    return r;
+}
+
+struct BackwardSpace {
+    size_t grad_columns, go_rows, go_channels, weight_t, row_most, channel_most, weight_most, total;
+};
+BackwardSpace plan_backward(const dcn_shape* s, const Derived& d) {
+    BackwardSpace r;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t here = at;
+        at += up(bytes);
+        return here;
+    };
+    const size_t go = static_cast<size_t>(d.M) * s->Co;
+    const size_t rows = static_cast<size_t>(s->groups) * d.Kd;
+    r.row_most = take(static_cast<size_t>(d.M) * 4);       // the three bounds: cleared together
+    r.channel_most = take(static_cast<size_t>(s->Co) * 4);
+    r.weight_most = take(rows * 4);
+    r.grad_columns = take(static_cast<size_t>(d.M) * rows * 4);
+    r.go_rows = take(go * 4);
+    r.go_channels = take(go * 4 + 256);
+    r.weight_t = take(rows * d.Cog * 4);
+    r.total = at;
+    return r;
+}
+
+struct ForwardSpace {
+    size_t weight_most, weight, total;
+};
+ForwardSpace plan_forward(const dcn_shape* s, const Derived& d) {
+    ForwardSpace r;
+    r.weight_most = 0;
+    r.weight = up(static_cast<size_t>(s->Co) * 4);
+    r.total = r.weight + up(static_cast<size_t>(s->Co) * d.Kd * 4);
+    return r;
+}
+
+#define RETURN_ON_CUDA(expr)                                          \
+    do {                                                              \
+        const cudaError_t err_ = (expr);                              \
+        if (err_ != cudaSuccess) return msda::note_cuda_error(err_);  \
+    } while (0)
+
+template <typename T>
+int to_nhwc(const void* src, int channels_last, float* dst, int N, int C, int P, uint32_t* magnitude,
+            cudaStream_t stream) {
+    const dim3 grid((P + 31) / 32, (C + 31) / 32, N);
+    to_nhwc_kernel<T><<<grid, kThreads, 0, stream>>>(static_cast<const T*>(src), channels_last, dst, C, P,
+                                                     magnitude);
+    RETURN_ON_CUDA(cudaGetLastError());
+    msda::count_launches(1);
+    return MSDA_OK;
+}
+
+void sample_params(const dcn_shape* s, const Derived& d, char* saved, const Saved& at, bool masked,
+                   DcnParams* p) {
+    fill_params(s, d, p);
+    p->x = reinterpret_cast<const float*>(saved + at.x);
+    p->offset = reinterpret_cast<const float*>(saved + at.offset);
+    p->mask = masked ? reinterpret_cast<const float*>(saved + at.mask) : nullptr;
+}
+
+template <typename T>
+int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mask, const void* weight,
+                  const float* bias, float* out, char* saved, char* ws, const dcn_shape* s, const Derived& d,
+                  cudaStream_t stream) {
+    int sms = 0;
+    int* status = nullptr;
+    int rc = msda::device_facts(&sms, &status);
+    if (rc != MSDA_OK) return rc;
+    const Saved at = plan_saved(s, d);
+    const ForwardSpace sp = plan_forward(s, d);
+    uint32_t* bounds = reinterpret_cast<uint32_t*>(saved + at.bounds);
+    RETURN_ON_CUDA(cudaMemsetAsync(bounds, 0, 16, stream));
+    const int HoWo = s->Ho * s->Wo, taps = s->deform_groups * d.K;
+    rc = to_nhwc<T>(x, x_nhwc, reinterpret_cast<float*>(saved + at.x), s->N, s->C, s->H * s->W, bounds, stream);
+    if (rc != MSDA_OK) return rc;
+    rc = to_nhwc<T>(offset, 0, reinterpret_cast<float*>(saved + at.offset), s->N, 2 * taps, HoWo, nullptr, stream);
+    if (rc != MSDA_OK) return rc;
+    if (mask != nullptr) {
+        rc = to_nhwc<T>(mask, 0, reinterpret_cast<float*>(saved + at.mask), s->N, taps, HoWo, bounds + 1, stream);
+        if (rc != MSDA_OK) return rc;
+    }
+    const size_t wplane = static_cast<size_t>(s->Co) * d.Kd;
+    uint16_t* wpairs = reinterpret_cast<uint16_t*>(ws + sp.weight);
+    uint32_t* wmost = reinterpret_cast<uint32_t*>(ws + sp.weight_most);
+    weight_pairs_kernel<T><<<s->Co, kThreads, 0, stream>>>(static_cast<const T*>(weight), d.Cg, d.K, wmost,
+                                                          wpairs, wplane);
+    RETURN_ON_CUDA(cudaGetLastError());
+
+    DcnParams p{};
+    sample_params(s, d, saved, at, mask != nullptr, &p);
+    p.pieces = d.Cd / 8;
+    int l = 0;
+    while ((1 << l) < p.pieces && l < 5) ++l;
+    p.lpi_log2 = l;
+    uint16_t* columns = reinterpret_cast<uint16_t*>(saved + at.columns);
+    const SplitScale col_scale{bounds, 0, mask != nullptr ? bounds + 1 : nullptr};
+    int per_sm = 0;
+    RETURN_ON_CUDA(msda::resident_ctas(reinterpret_cast<const void*>(gather_pairs_kernel), kThreads, 0, &per_sm));
+    const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
+    const uint32_t want = (p.items + per_step - 1) / per_step, cap = static_cast<uint32_t>(sms) * per_sm;
+    gather_pairs_kernel<<<want < cap ? want : cap, kThreads, 0, stream>>>(p, columns, at.plane, col_scale);
+    RETURN_ON_CUDA(cudaGetLastError());
+    msda::count_launches(2);
+
+    bool zeroed = false;
+    for (int g = 0; g < s->groups; ++g) {
+        const SplitOperand A{columns + static_cast<size_t>(g) * d.Kd, static_cast<long long>(s->groups) * d.Kd, 1,
+                             static_cast<long long>(at.plane), col_scale};
+        const SplitOperand B{wpairs + static_cast<size_t>(g) * d.Cog * d.Kd, d.Kd, 1,
+                             static_cast<long long>(wplane), SplitScale{wmost + g * d.Cog, 1, nullptr}};
+        const long long tiles = ((d.M + 127) / 128) * static_cast<long long>((d.Cog + 255) / 256);
+        const int splits = 2 * tiles <= sms ? balanced_splits(tiles, sms, (d.Kd + 255) / 256) : 1;
+        if (splits > 1 && !zeroed) {
+            RETURN_ON_CUDA(cudaMemsetAsync(out, 0, static_cast<size_t>(d.M) * s->Co * 4, stream));
+            zeroed = true;
+        }
+        RETURN_ON_CUDA(msda::gemm_split(A, B, out + static_cast<size_t>(g) * d.Cog, s->Co,
+                                        bias != nullptr ? bias + g * d.Cog : nullptr, static_cast<int>(d.M),
+                                        d.Cog, d.Kd, splits, status, stream));
+        msda::count_launches(1);
+    }
+    return MSDA_OK;
+}
+
+template <typename T>
+int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* saved, bool masked,
+                   float* grad_x, float* grad_offset, float* grad_mask, float* grad_weight, float* grad_bias,
+                   char* ws, const dcn_shape* s, const Derived& d, cudaStream_t stream) {
+    int sms = 0;
+    int* status = nullptr;
+    int rc = msda::device_facts(&sms, &status);
+    if (rc != MSDA_OK) return rc;
+    const Saved at = plan_saved(s, d);
+    const BackwardSpace sp = plan_backward(s, d);
+    const int M = static_cast<int>(d.M), HoWo = s->Ho * s->Wo;
+    uint32_t* bounds = reinterpret_cast<uint32_t*>(saved + at.bounds);
+    uint32_t* row_most = reinterpret_cast<uint32_t*>(ws + sp.row_most);
+    uint32_t* channel_most = reinterpret_cast<uint32_t*>(ws + sp.channel_most);
+    uint32_t* weight_most = reinterpret_cast<uint32_t*>(ws + sp.weight_most);
+    uint16_t* go_rows = reinterpret_cast<uint16_t*>(ws + sp.go_rows);
+    uint16_t* go_channels = reinterpret_cast<uint16_t*>(ws + sp.go_channels);
+    uint16_t* weight_t = reinterpret_cast<uint16_t*>(ws + sp.weight_t);
+    float* grad_columns = reinterpret_cast<float*>(ws + sp.grad_columns);
+    RETURN_ON_CUDA(cudaMemsetAsync(row_most, 0, sp.grad_columns - sp.row_most, stream));
+    if (grad_bias != nullptr) RETURN_ON_CUDA(cudaMemsetAsync(grad_bias, 0, static_cast<size_t>(s->Co) * 4, stream));
+    RETURN_ON_CUDA(cudaMemsetAsync(grad_x, 0, static_cast<size_t>(s->N) * s->H * s->W * s->C * 4, stream));
+
+    // grad_out: bounds, then pairs (the second reading mostly comes from L2)
+    const size_t go_plane = static_cast<size_t>(M) * s->Co;
+    {
+        const T* go = static_cast<const T*>(grad_out);
+        const dim3 grid((HoWo + 31) / 32, (s->Co + 63) / 64, s->N);
+        const RowOrder order{HoWo, 0, 0};
+        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, grad_bias);
+        pairs_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, go_rows,
+                                                       go_channels, go_plane);
+    }
+    // weights as [group][kd][output channel]
+    const size_t wt_plane = static_cast<size_t>(s->groups) * d.Kd * d.Cog;
+    {
+        const T* w = static_cast<const T*>(weight);
+        const dim3 grid((d.Kd + 31) / 32, (d.Cog + 63) / 64, s->groups);
+        const RowOrder order{d.Kd, d.K, d.Cg};
+        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, nullptr);
+        pairs_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, weight_t, nullptr,
+                                                       wt_plane);
+    }
+    RETURN_ON_CUDA(cudaGetLastError());
+    msda::count_launches(4);
+
+    const long long ld_cols = static_cast<long long>(s->groups) * d.Kd;
+    for (int g = 0; g < s->groups; ++g) {
+        const SplitOperand A{go_rows + static_cast<size_t>(g) * d.Cog, s->Co, 1, static_cast<long long>(go_plane),
+                             SplitScale{row_most, 1, nullptr}};
+        const SplitOperand B{weight_t + static_cast<size_t>(g) * d.Kd * d.Cog, d.Cog, 1,
+                             static_cast<long long>(wt_plane),
+                             SplitScale{weight_most + static_cast<size_t>(g) * d.Kd, 1, nullptr}};
+        RETURN_ON_CUDA(msda::gemm_split(A, B, grad_columns + static_cast<size_t>(g) * d.Kd, ld_cols, nullptr, M,
+                                        d.Kd, d.Cog, 1, status, stream));
+        msda::count_launches(1);
+    }
+
+    DcnParams p{};
+    sample_params(s, d, saved, at, masked, &p);
+    p.columns = grad_columns;
+    p.grad_x = grad_x;
+    p.grad_offset = grad_offset;
+    p.grad_mask = grad_mask;
+    rc = launch_scatter(p, sms, stream);
+    if (rc != MSDA_OK) return rc;
+
+    const uint16_t* columns = reinterpret_cast<const uint16_t*>(saved + at.columns);
+    const SplitScale col_scale{bounds, 0, masked ? bounds + 1 : nullptr};
+    bool zeroed = false;
+    for (int g = 0; g < s->groups; ++g) {
+        const SplitOperand A{go_channels + static_cast<size_t>(g) * d.Cog, 1, s->Co, static_cast<long long>(go_plane),
+                             SplitScale{channel_most + static_cast<size_t>(g) * d.Cog, 1, nullptr}};
+        const SplitOperand B{columns + static_cast<size_t>(g) * d.Kd, 1, ld_cols, static_cast<long long>(at.plane),
+                             col_scale};
+        const long long tiles = ((d.Cog + 127) / 128) * static_cast<long long>((d.Kd + 255) / 256);
+        const int splits = balanced_splits(tiles, sms, (M + 1023) / 1024);
+        if (splits > 1 && !zeroed) {
+            RETURN_ON_CUDA(cudaMemsetAsync(grad_weight, 0, static_cast<size_t>(s->Co) * d.Kd * 4, stream));
+            zeroed = true;
+        }
+        RETURN_ON_CUDA(msda::gemm_split(A, B, grad_weight + static_cast<size_t>(g) * d.Cog * d.Kd, d.Kd, nullptr,
+                                        d.Cog, d.Kd, M, splits, status, stream));
+        msda::count_launches(1);
+    }
+    return MSDA_OK;
+}
+
+int split_shape(const dcn_shape* s, Derived* d) {
+    const int rc = check_shape(s, d);
+    if (rc != MSDA_OK) return rc;
+    // 16-byte pieces of halves in every row
+    if (d->Cg % 8 != 0 || d->Cd % 8 != 0 || d->Cog % 8 != 0) return MSDA_ERR_ALIGN;
+    return dcn_sm100_use_tensor_cores(-1) == 1 ? MSDA_OK : MSDA_ERR_LIMIT;
+}
+
+}  // namespace
+
+extern "C" {
+
+size_t dcn_sm100_saved_bytes(const dcn_shape* s) {
+    Derived d;
+    return split_shape(s, &d) == MSDA_OK ? plan_saved(s, d).total : 0;
+}
+
+size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int backward) {
+    Derived d;
+    if (check_shape(s, &d) != MSDA_OK) return 0;
+    return backward ? plan_backward(s, d).total : plan_forward(s, d).total;
+}
+
+int dcn_sm100_forward_nchw(const void* x, int x_nhwc, const void* offset, const void* mask, const void* weight,
+                           const float* bias, float* out, void* saved, size_t saved_bytes, void* workspace,
+                           size_t workspace_bytes, const dcn_shape* s, int dtype, void* stream_v) {
+    if (x == nullptr || offset == nullptr || weight == nullptr || out == nullptr || saved == nullptr ||
+        workspace == nullptr)
+        return MSDA_ERR_NULL;
+    Derived d;
+    const int rc = split_shape(s, &d);
+    if (rc != MSDA_OK) return rc;
+    if (saved_bytes < plan_saved(s, d).total || workspace_bytes < plan_forward(s, d).total)
+        return MSDA_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(saved) | reinterpret_cast<uintptr_t>(workspace)) % 16 != 0) return MSDA_ERR_ALIGN;
+    char* sv = static_cast<char*>(saved);
+    char* ws = static_cast<char*>(workspace);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    switch (dtype) {
+        case MSDA_F32: return forward_typed<float>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, stream);
+        case MSDA_F16: return forward_typed<__half>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, stream);
+        case MSDA_BF16:
+            return forward_typed<__nv_bfloat16>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, stream);
+        default: return MSDA_ERR_DTYPE;
+    }
+}
+
+int dcn_sm100_backward_nchw(const void* weight, const void* grad_out, int grad_out_nhwc, const void* saved,
+                            float* grad_x, float* grad_offset, float* grad_mask, float* grad_weight,
+                            float* grad_bias, void* workspace, size_t workspace_bytes, const dcn_shape* s,
+                            int dtype, void* stream_v) {
+    if (weight == nullptr || grad_out == nullptr || saved == nullptr || grad_x == nullptr ||
+        grad_offset == nullptr || grad_weight == nullptr || workspace == nullptr)
+        return MSDA_ERR_NULL;
+    Derived d;
+    int rc = check_shape(s, &d);
+    if (rc != MSDA_OK) return rc;
+    if (d.Cg % 8 != 0 || d.Cd % 8 != 0 || d.Cog % 8 != 0) return MSDA_ERR_ALIGN;
+    if (workspace_bytes < plan_backward(s, d).total) return MSDA_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(saved) | reinterpret_cast<uintptr_t>(workspace) |
+         reinterpret_cast<uintptr_t>(grad_x)) % 16 != 0 || reinterpret_cast<uintptr_t>(grad_offset) % 8 != 0)
+        return MSDA_ERR_ALIGN;
+    char* sv = const_cast<char*>(static_cast<const char*>(saved));
+    char* ws = static_cast<char*>(workspace);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    const bool masked = grad_mask != nullptr;
+    switch (dtype) {
+        case MSDA_F32:
+            return backward_typed<float>(weight, grad_out, grad_out_nhwc, sv, masked, grad_x, grad_offset,
+                                         grad_mask, grad_weight, grad_bias, ws, s, d, stream);
+        case MSDA_F16:
+            return backward_typed<__half>(weight, grad_out, grad_out_nhwc, sv, masked, grad_x, grad_offset,
+                                          grad_mask, grad_weight, grad_bias, ws, s, d, stream);
+        case MSDA_BF16:
+            return backward_typed<__nv_bfloat16>(weight, grad_out, grad_out_nhwc, sv, masked, grad_x,
+                                                 grad_offset, grad_mask, grad_weight, grad_bias, ws, s, d, stream);
+        default: return MSDA_ERR_DTYPE;
+    }
+}
+
+}  // extern "C"

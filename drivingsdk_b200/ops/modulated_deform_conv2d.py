@@ -76,5 +76,6 @@ def modulated_deform_conv2d(x: torch.Tensor, offset: torch.Tensor, mask: torch.T
                             padding: Union[int, Tuple[int, ...]] = 0,
                             dilation: Union[int, Tuple[int, ...]] = 1, groups: int = 1,
                             deformable_groups: int = 1):
-    return ModulatedDeformConv2dFunction.apply(x, offset, mask, weight, bias, stride, padding,
-                                               dilation, groups, deformable_groups)
+    # the same function natively, its products over fp16 pairs where the channels allow it
+    return _C.modulated_deform_conv2d_autograd(x, offset, mask, weight, bias, _pair(stride),
+                                               _pair(padding), _pair(dilation), groups, deformable_groups)

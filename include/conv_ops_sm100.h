@@ -106,6 +106,28 @@ int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
                        const dcn_shape* s, void* stream);
 
 /*
+ * The same operator from NCHW tensors of `dtype` (x and grad_out may also be channels-last:
+ * x_nhwc / grad_out_nhwc = 1), its products over fp16 pairs of every operand: fp32-class accuracy
+ * at twice the rate of the TF32 pairs above. For C / groups, C / deform_groups and Co / groups that
+ * are multiples of 8 and dcn_sm100_use_tensor_cores() == 1; elsewhere dcn_sm100_saved_bytes() is 0.
+ *   weight [Co, C / groups, kh, kw]; offset [N, deform_groups * 2 * kh * kw, Ho, Wo]; mask likewise
+ *   saved: device memory of dcn_sm100_saved_bytes(), written by the forward, read by the backward
+ *          (16-byte aligned, like the workspaces)
+ *   out [N, Ho, Wo, Co] and the gradients are float32 in the layouts of the calls above
+ *          (grad_weight [Co, kh, kw, C / groups]); mask and grad_mask both or neither.
+ */
+size_t dcn_sm100_saved_bytes(const dcn_shape* s);
+size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int backward);
+int dcn_sm100_forward_nchw(const void* x, int x_nhwc, const void* offset, const void* mask,
+                           const void* weight, const float* bias, float* out, void* saved,
+                           size_t saved_bytes, void* workspace, size_t workspace_bytes,
+                           const dcn_shape* s, int dtype, void* stream);
+int dcn_sm100_backward_nchw(const void* weight, const void* grad_out, int grad_out_nhwc,
+                            const void* saved, float* grad_x, float* grad_offset, float* grad_mask,
+                            float* grad_weight, float* grad_bias, void* workspace,
+                            size_t workspace_bytes, const dcn_shape* s, int dtype, void* stream);
+
+/*
  * Which matrix-product kernels the two calls above use: 1 (default) = the tcgen05 kernel
  * (fp32 operands split into two TF32 parts, three tensor-core products per tile, fp32
  * accumulation in tensor memory; fp32-class accuracy) where the shape allows it; 2 = the same
