@@ -52,9 +52,9 @@ SIGNATURES = {
     "dcn_sm100_backward_workspace_bytes": (_sz, [_vp]),
     "dcn_sm100_forward": (_i, [_vp] * 7 + [_vp, _vp]),
     "dcn_sm100_backward": (_i, [_vp] * 11 + [_vp, _sz, _vp, _vp]),
-    "dcn_sm100_saved_bytes": (_sz, [_vp]),
-    "dcn_sm100_nchw_workspace_bytes": (_sz, [_vp, _i]),
-    "dcn_sm100_forward_nchw": (_i, [_vp, _i] + [_vp] * 6 + [_sz, _vp, _sz, _vp, _i, _vp]),
+    "dcn_sm100_saved_bytes": (_sz, [_vp, _i, _i]),
+    "dcn_sm100_nchw_workspace_bytes": (_sz, [_vp, _i, _i, _i]),
+    "dcn_sm100_forward_nchw": (_i, [_vp, _i] + [_vp] * 6 + [_sz, _vp, _sz, _vp, _i, _i, _vp]),
     "dcn_sm100_backward_nchw": (_i, [_vp, _vp, _i] + [_vp] * 7 + [_sz, _vp, _i, _vp]),
     "dcn_sm100_use_tensor_cores": (_i, [_i]),
     "gemm_tn_sm100_f32": (_i, [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp,

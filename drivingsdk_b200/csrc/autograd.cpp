@@ -188,7 +188,7 @@ struct DeformConv : Function<DeformConv> {
         ctx->saved_data["modulated"] = modulated;
         Tensor out, saved;
         std::vector<int64_t> shape;
-        if (alike) std::tie(out, saved) = conv_forward(x, offset, mask, weight, bias, conv, &shape);
+        if (alike) std::tie(out, saved) = conv_forward(x, offset, mask, weight, bias, conv, keep, &shape);
         ctx->saved_data["shape"] = shape;   // empty: the fp32 form
         if (out.defined()) {
             if (keep) {

@@ -861,10 +861,11 @@ void* pointer(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr
 
 std::tuple<at::Tensor, at::Tensor> conv_forward(const at::Tensor& x_in, const at::Tensor& offset_in,
                                                 const at::Tensor& mask_in, const at::Tensor& weight_in,
-                                                const at::Tensor& bias_in, const Conv& conv,
+                                                const at::Tensor& bias_in, const Conv& conv, bool keep,
                                                 std::vector<int64_t>* shape) {
     const dcn_shape s = conv_shape(x_in, offset_in, mask_in, weight_in, conv);
-    const size_t saved_bytes = dcn_sm100_saved_bytes(&s);
+    const int dtype = dtype_code(x_in.scalar_type());
+    const size_t saved_bytes = dcn_sm100_saved_bytes(&s, dtype, keep);
     if (saved_bytes == 0 || x_in.numel() == 0 || offset_in.numel() == 0) return {};
     const int* fields = reinterpret_cast<const int*>(&s);
     shape->assign(fields, fields + sizeof(s) / sizeof(int));
@@ -881,13 +882,13 @@ std::tuple<at::Tensor, at::Tensor> conv_forward(const at::Tensor& x_in, const at
     }
     const auto bytes = x.options().dtype(at::kByte);
     at::Tensor saved = at::empty({static_cast<int64_t>(saved_bytes)}, bytes);
-    const size_t ws_bytes = dcn_sm100_nchw_workspace_bytes(&s, 0);
+    const size_t ws_bytes = dcn_sm100_nchw_workspace_bytes(&s, dtype, keep, 0);
     at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)}, bytes);
     at::Tensor out = at::empty({s.N, s.Ho, s.Wo, s.Co}, x.options().dtype(at::kFloat));
     const int rc = dcn_sm100_forward_nchw(
         x.data_ptr(), is_nhwc(x_in) ? 1 : 0, offset.data_ptr(), pointer(mask), weight.data_ptr(),
         bias.defined() ? bias.data_ptr<float>() : nullptr, out.data_ptr<float>(), saved.data_ptr(), saved_bytes,
-        ws.data_ptr(), ws_bytes, &s, dtype_code(kind), at::cuda::getCurrentCUDAStream().stream());
+        ws.data_ptr(), ws_bytes, &s, dtype, keep, at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "deformable_conv2d");
     return std::make_tuple(out.permute({0, 3, 1, 2}).to(kind), saved);
 }
@@ -913,7 +914,7 @@ ConvGrads conv_backward(const at::Tensor& weight, bool modulated, bool with_bias
     at::Tensor gmask = modulated ? at::empty({s.N, s.Ho, s.Wo, taps}, f32) : at::Tensor();
     at::Tensor gw = at::empty({s.Co, s.kh, s.kw, s.C / s.groups}, f32);
     at::Tensor gb = with_bias ? at::empty({s.Co}, f32) : at::Tensor();
-    const size_t ws_bytes = dcn_sm100_nchw_workspace_bytes(&s, 1);
+    const size_t ws_bytes = dcn_sm100_nchw_workspace_bytes(&s, dtype_code(kind), 1, 1);
     at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)}, f32.dtype(at::kByte));
     const int rc = dcn_sm100_backward_nchw(
         weight.data_ptr(), grad.data_ptr(), nhwc ? 1 : 0, saved.data_ptr(), gx.data_ptr<float>(),

@@ -15,7 +15,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> msda_backward(
     const at::Tensor& loc, const at::Tensor& attn, const at::Tensor& grad_out);
 // Deformable convolution over fp16 pairs, from NCHW tensors of one type. conv_forward returns the
 // output and the block that conv_backward needs, or undefined tensors where the form does not
-// apply; `shape` receives the sizes for conv_backward. Nothing of x, offset and mask is needed
+// apply; `keep`: a backward may follow; `shape` receives the sizes for conv_backward. Nothing of x, offset and mask is needed
 // later, so callers may overwrite them.
 struct Conv {
     std::vector<int64_t> stride, padding, dilation;
@@ -26,7 +26,7 @@ struct ConvGrads {
 };
 std::tuple<at::Tensor, at::Tensor> conv_forward(const at::Tensor& x, const at::Tensor& offset,
                                                 const at::Tensor& mask, const at::Tensor& weight,
-                                                const at::Tensor& bias, const Conv& conv,
+                                                const at::Tensor& bias, const Conv& conv, bool keep,
                                                 std::vector<int64_t>* shape);
 ConvGrads conv_backward(const at::Tensor& weight, bool modulated, bool with_bias, const at::Tensor& saved,
                         const at::Tensor& grad_out, const std::vector<int64_t>& shape);

@@ -209,4 +209,10 @@ inline int balanced_splits(long long tiles, int sms, int max_splits) {
     return best;
 }
 
+// Parts into which the pixels are cut for the grad_weight product.
+inline int weight_splits(const Derived& d, int sms) {
+    const long long tiles = ((d.Cog + 127) / 128) * static_cast<long long>((d.Kd + 255) / 256);
+    return balanced_splits(tiles, sms, static_cast<int>((d.M + 1023) / 1024));
+}
+
 }  // namespace dcn

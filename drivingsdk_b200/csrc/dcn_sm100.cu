@@ -236,6 +236,44 @@ int public_product(const float* A, long long a_row, long long a_k, const float* 
 }  // namespace
 
 namespace dcn {
+// grad_weight[co, kd] = sum over m of grad_out[m, co] * columns[m, g, kd]: both operands are stored
+// pixel row by pixel row, i.e. with the row index (co, kd) contiguous and k = m strided. The
+// tensor-core kernel takes that form directly (K cut over CTAs so that every SM has work);
+// operands that miss its alignment rules go to the FMA kernel.
+int launch_weight_product(const float* grad_out, const float* columns, float* grad_weight, const dcn_shape* s,
+                          const Derived& d, int sms, int* status_word, cudaStream_t stream) {
+    const long long ld_cols = static_cast<long long>(s->groups) * d.Kd;
+    const int M = static_cast<int>(d.M);
+    const bool tc = g_use_tc.load(std::memory_order_relaxed) != 0;
+    bool zeroed = false;
+    for (int g = 0; g < s->groups; ++g) {
+        msda::GemmArgs a{};
+        a.A = grad_out + static_cast<size_t>(g) * d.Cog;
+        a.a_row = 1;
+        a.a_k = s->Co;
+        a.B = columns + static_cast<size_t>(g) * d.Kd;
+        a.b_row = 1;
+        a.b_k = ld_cols;
+        a.C = grad_weight + static_cast<size_t>(g) * d.Cog * d.Kd;
+        a.ldc = d.Kd;
+        a.M = d.Cog;
+        a.N = d.Kd;
+        a.K = M;
+        int splits = 1;
+        if (tc && msda::gemm_tc_supported(a)) {
+            splits = weight_splits(d, sms);
+            if (splits > 1 && !zeroed) {
+                const cudaError_t e = cudaMemsetAsync(grad_weight, 0, static_cast<size_t>(s->Co) * d.Kd * 4, stream);
+                if (e != cudaSuccess) return msda::note_cuda_error(e);
+                zeroed = true;
+            }
+        }
+        const int rc = product(a, splits, status_word, stream);
+        if (rc != MSDA_OK) return rc;
+    }
+    return MSDA_OK;
+}
+
 int launch_scatter(const DcnParams& p, int sm_count, cudaStream_t stream) {
     return launch_sample_vec<true, 4>(p, sm_count, stream);
 }
@@ -411,39 +449,9 @@ int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
     rc = launch_sample<true>(p, piece_width(s, d), sms, stream);
     if (rc != MSDA_OK) return rc;
 
-    // 3. grad_weight[co, kd] = sum over m of grad_out[m, co] * columns[m, g, kd]: both operands
-    //    are stored pixel row by pixel row, i.e. with the row index (co, kd) contiguous and
-    //    k = m strided. The tensor-core kernel takes that form directly (K cut over CTAs so
-    //    that every SM has work); operands that miss its alignment rules go to the FMA kernel.
-    {
-        bool zeroed = false;
-        for (int g = 0; g < s->groups; ++g) {
-            msda::GemmArgs a{};
-            a.A = grad_out + static_cast<size_t>(g) * d.Cog;
-            a.a_row = 1;
-            a.a_k = s->Co;
-            a.B = columns + static_cast<size_t>(g) * d.Kd;
-            a.b_row = 1;
-            a.b_k = ld_cols;
-            a.C = grad_weight + static_cast<size_t>(g) * d.Cog * d.Kd;
-            a.ldc = d.Kd;
-            a.M = d.Cog;
-            a.N = d.Kd;
-            a.K = M;
-            int splits = 1;
-            if (tc && msda::gemm_tc_supported(a)) {
-                const long long tiles = ((d.Cog + 127) / 128) * static_cast<long long>((d.Kd + 255) / 256);
-                splits = balanced_splits(tiles, sms, (M + 1023) / 1024);
-                if (splits > 1 && !zeroed) {
-                    e = cudaMemsetAsync(grad_weight, 0, static_cast<size_t>(s->Co) * d.Kd * 4, stream);
-                    if (e != cudaSuccess) return msda::note_cuda_error(e);
-                    zeroed = true;
-                }
-            }
-            rc = product(a, splits, status_word, stream);
-            if (rc != MSDA_OK) return rc;
-        }
-    }
+    // 3. grad_weight
+    rc = launch_weight_product(grad_out, columns, grad_weight, s, d, sms, status_word, stream);
+    if (rc != MSDA_OK) return rc;
 
     // 4. grad_bias
     if (grad_bias != nullptr) {

@@ -32,13 +32,15 @@ __device__ __forceinline__ void load_tile(const T* src, int channels_last, int n
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (!channels_last) {
 #pragma unroll
-        for (int r = warp; r < CH; r += kThreads / 32) {
+        for (int u = 0; u < CH * 32 / kThreads; ++u) {
+            const int r = warp + u * (kThreads / 32);
             const int c = c0 + r, p = p0 + lane;
             tile[r][lane] = (c < C && p < P) ? Elem<T>::to_f(src[(static_cast<size_t>(n) * C + c) * P + p]) : 0.f;
         }
     } else {
 #pragma unroll
-        for (int i = warp; i < CH; i += kThreads / 32) {
+        for (int u = 0; u < CH * 32 / kThreads; ++u) {
+            const int i = warp + u * (kThreads / 32);
             const int r = (i % (CH / 32)) * 32 + lane, q = i / (CH / 32);
             const int c = c0 + r, p = p0 + q;
             tile[r][q] = (c < C && p < P) ? Elem<T>::to_f(src[(static_cast<size_t>(n) * P + p) * C + c]) : 0.f;
@@ -63,7 +65,8 @@ to_nhwc_kernel(const T* __restrict__ src, int channels_last, float* __restrict__
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t most = 0;
 #pragma unroll
-    for (int r = warp; r < 32; r += kThreads / 32) {
+    for (int u = 0; u < 1024 / kThreads; ++u) {
+        const int r = warp + u * (kThreads / 32);
         const int p = p0 + r, c = c0 + lane;
         const float v = tile[lane][r];
         most = max(most, msda::finite_magnitude(v));
@@ -101,22 +104,29 @@ bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder orde
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
     load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t mine = 0;
+    constexpr int kRows = 64 * 32 / kThreads;    // channels of this warp; lane u keeps the u-th
+    uint32_t mine = 0, most = 0;
+    float sum = 0.f;
 #pragma unroll
-    for (int r = warp; r < 64; r += kThreads / 32) {
-        const float v = tile[r][lane];
+    for (int u = 0; u < kRows; ++u) {
+        const float v = tile[warp + u * (kThreads / 32)][lane];
         const uint32_t a = msda::finite_magnitude(v);
         mine = max(mine, a);
         if (channel_most != nullptr) {
-            const uint32_t most = __reduce_max_sync(0xffffffffu, a);
-            if (lane == 0 && c0 + r < C) raise_max(channel_most + c0 + r, most);
+            const uint32_t m = __reduce_max_sync(0xffffffffu, a);
+            if (lane == u) most = m;
         }
         if (channel_sum != nullptr) {
             float s = v;
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0 && c0 + r < C) atomicAdd(channel_sum + c0 + r, s);
+            if (lane == u) sum = s;
         }
+    }
+    const int channel = c0 + warp + lane * (kThreads / 32);
+    if (lane < kRows && channel < C) {
+        if (channel_most != nullptr) raise_max(channel_most + channel, most);
+        if (channel_sum != nullptr) atomicAdd(channel_sum + channel, sum);
     }
     part[warp][lane] = mine;
     __syncthreads();
@@ -126,12 +136,12 @@ bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder orde
     }
 }
 
-// [n][C][P] -> pairs [rows][C]: scaled by row, and (optional) by channel.
+// [n][C][P] -> pairs [rows][C] scaled by row, and (optional) the same scaled by channel or in fp32.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 pairs_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
              const uint32_t* row_most, const uint32_t* channel_most, uint16_t* __restrict__ by_row,
-             uint16_t* __restrict__ by_channel, size_t plane) {
+             uint16_t* __restrict__ by_channel, float* __restrict__ plain, size_t plane) {
     __shared__ float tile[64][33];
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
     load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
@@ -153,6 +163,7 @@ pairs_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order
         uint16_t* at = by_row + row * C + c;
         *reinterpret_cast<uint32_t*>(at) = r.x;
         *reinterpret_cast<uint32_t*>(at + plane) = r.y;
+        if (plain != nullptr) *reinterpret_cast<float2*>(plain + row * C + c) = make_float2(x, y);
         if (by_channel != nullptr) {
             const uint2 h = msda::split_pair(x * sc[0], y * sc[1], 1.f);
             uint16_t* to = by_channel + row * C + c;
@@ -188,80 +199,103 @@ weight_pairs_kernel(const T* __restrict__ w, int Cg, int K, uint32_t* most, uint
     }
 }
 
-// Column pairs: mask * bilinear(x). A group of lanes per (pixel, deformable group, tap) moves
-// pieces of eight channels. A CTA walks a contiguous run of items, a slice of the channels at a
-// time: neighbouring taps and pixels read mostly the same rows.
-constexpr uint32_t kRunItems = 144;   // per slice: 16 pixels of a 3 x 3 kernel
-__global__ void __launch_bounds__(kThreads, 3)
+// Column pairs: mask * bilinear(x), pixel by pixel. A group of lanes per (pixel, deformable group, tap)
+// moves pieces of eight channels.
+__global__ void __launch_bounds__(kThreads, 4)
 gather_pairs_kernel(const __grid_constant__ DcnParams p, uint16_t* __restrict__ columns, size_t plane,
-                    const SplitScale bound) {
-    const int lane = threadIdx.x & 31;
+                    const SplitScale bound, float* __restrict__ columns_f32) {
     const int lpi = 1 << p.lpi_log2;
-    const int sub = lane & (lpi - 1);
-    const uint32_t slot = (threadIdx.x >> p.lpi_log2);             // item within the CTA's step
+    const int sub = threadIdx.x & (lpi - 1);
+    const uint32_t slot = threadIdx.x >> p.lpi_log2;             // item within the CTA's step
     const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
-    const uint32_t begin = static_cast<uint32_t>(static_cast<uint64_t>(p.items) * blockIdx.x / gridDim.x);
-    const uint32_t end = static_cast<uint32_t>(static_cast<uint64_t>(p.items) * (blockIdx.x + 1) / gridDim.x);
     const float scale = msda::exp2_int(msda::split_exponent(bound, 0));
-    for (uint32_t run = begin; run < end; run += kRunItems) {
-        const uint32_t stop = min(end, run + kRunItems);
-        for (int piece = sub; piece < p.pieces; piece += lpi) {
 #pragma unroll 1
-            for (uint32_t item = run + slot; item < stop; item += per_step) {
-                uint32_t m, dg, k;
-                float mk;
-                Sample s;
-                item_setup(p, item, &m, &dg, &k, &mk, &s);
-                float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-                if (s.valid) {
-                    float4 v[4][2];
+    for (uint32_t item = blockIdx.x * per_step + slot; item < p.items; item += gridDim.x * per_step) {
+        uint32_t m, dg, k;
+        float mk;
+        Sample s;
+        item_setup(p, item, &m, &dg, &k, &mk, &s);
+        for (int piece = sub; piece < p.pieces; piece += lpi) {
+            float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+            if (s.valid) {
+                float4 v[4][2];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        v[c][0] = load_piece<4>(s.row[c], 2 * piece);
-                        v[c][1] = load_piece<4>(s.row[c], 2 * piece + 1);
-                    }
+                for (int c = 0; c < 4; ++c) {
+                    v[c][0] = load_piece<4>(s.row[c], 2 * piece);
+                    v[c][1] = load_piece<4>(s.row[c], 2 * piece + 1);
+                }
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float w = s.w[c] * mk;
+                for (int c = 0; c < 4; ++c) {
+                    const float w = s.w[c] * mk;
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            acc[h].x = fmaf(w, v[c][h].x, acc[h].x);
-                            acc[h].y = fmaf(w, v[c][h].y, acc[h].y);
-                            acc[h].z = fmaf(w, v[c][h].z, acc[h].z);
-                            acc[h].w = fmaf(w, v[c][h].w, acc[h].w);
-                        }
+                    for (int h = 0; h < 2; ++h) {
+                        acc[h].x = fmaf(w, v[c][h].x, acc[h].x);
+                        acc[h].y = fmaf(w, v[c][h].y, acc[h].y);
+                        acc[h].z = fmaf(w, v[c][h].z, acc[h].z);
+                        acc[h].w = fmaf(w, v[c][h].w, acc[h].w);
                     }
                 }
-                const uint2 r0 = msda::split_pair(acc[0].x, acc[0].y, scale);
-                const uint2 r1 = msda::split_pair(acc[0].z, acc[0].w, scale);
-                const uint2 r2 = msda::split_pair(acc[1].x, acc[1].y, scale);
-                const uint2 r3 = msda::split_pair(acc[1].z, acc[1].w, scale);
-                uint16_t* to = columns + column_index(p, m, k, dg * p.Cd + 8 * piece);
-                *reinterpret_cast<uint4*>(to) = make_uint4(r0.x, r1.x, r2.x, r3.x);
-                *reinterpret_cast<uint4*>(to + plane) = make_uint4(r0.y, r1.y, r2.y, r3.y);
             }
+            const uint2 r0 = msda::split_pair(acc[0].x, acc[0].y, scale);
+            const uint2 r1 = msda::split_pair(acc[0].z, acc[0].w, scale);
+            const uint2 r2 = msda::split_pair(acc[1].x, acc[1].y, scale);
+            const uint2 r3 = msda::split_pair(acc[1].z, acc[1].w, scale);
+            const size_t to_at = column_index(p, m, k, dg * p.Cd + 8 * piece);
+            uint16_t* to = columns + to_at;
+            if (columns_f32 != nullptr) {
+                *reinterpret_cast<float4*>(columns_f32 + to_at) = acc[0];
+                *reinterpret_cast<float4*>(columns_f32 + to_at + 4) = acc[1];
+            }
+            *reinterpret_cast<uint4*>(to) = make_uint4(r0.x, r1.x, r2.x, r3.x);
+            *reinterpret_cast<uint4*>(to + plane) = make_uint4(r0.y, r1.y, r2.y, r3.y);
         }
     }
 }
 
 size_t up(size_t v) { return (v + 255) / 256 * 256; }
 
+// Sampling over cell-sorted samples instead of pixel by pixel: pays where rows are long enough to
+// occupy a warp and the sort (some 15 us at least) is small against the sampling. Forward and backward,
+// pixel by pixel / sorted, in us: Cd = 512, 235 k samples 1510 / 1265; Cd = 128, 0.69 M 1445 / 1055,
+// 0.17 M 369 / 290, 43 k 170 / 174; Cd = 64, 0.17 M 241 / 233 but 67 / 79 for the forward alone,
+// Cd = 16, 0.69 M 251 / 356.
+bool sort_pays(const dcn_shape* s, const Derived& d) {
+    return d.Cd >= 96 && d.M * s->deform_groups * d.K >= 100000 && dcn::sorted_bytes(s, d) != 0;
+}
+
+// Whether grad_weight is formed from fp32 operands by the TF32 kernel. The tensor core truncates as it
+// accumulates, so a sum's error grows with its chain of products: at 13050 pixels a chain both kernels
+// are 9e-5 of the result off, in different ways (fp16 pairs half of that at the same cut). A caller
+// may get the same gradient from either form (the extension's own entry points use the other), so
+// they are held to agree to 2e-5 for fp32 tensors: past 4000 pixels a chain (4.7e-5 at 13050) this
+// one uses the other's kernel.
+bool weight_in_f32(const dcn_shape* s, const Derived& d, int dtype) {
+    (void)s;
+    int sms = 148;
+    msda::device_facts(&sms, nullptr);
+    return dtype == MSDA_F32 && d.M > 4000ll * weight_splits(d, sms);
+}
+
 // What the forward leaves for the backward: bounds, x, offset and mask as [n][pixel][channel] fp32,
-// column pairs.
+// the samples in cell order, and the columns as grad_weight wants them. `keep` == 0: no backward
+// will follow. The pairs of the columns are there too, or in the forward's workspace.
 struct Saved {
-    size_t bounds, x, offset, mask, columns, total;
+    size_t bounds, x, offset, mask, sorted, columns, total;
     size_t plane;   // halves per plane of the columns
+    bool f32;       // columns in fp32 (else pairs)
 };
-Saved plan_saved(const dcn_shape* s, const Derived& d) {
+Saved plan_saved(const dcn_shape* s, const Derived& d, int dtype, bool keep) {
     Saved r;
     r.bounds = 0;
     r.x = 256;
     r.offset = r.x + up(static_cast<size_t>(s->N) * s->H * s->W * s->C * 4);
     const size_t taps = static_cast<size_t>(d.M) * s->deform_groups * d.K;
     r.mask = r.offset + up(taps * 8);
-    r.columns = r.mask + up(taps * 4);
+    r.sorted = r.mask + up(taps * 4);
+    r.columns = r.sorted + up(sort_pays(s, d) ? dcn::sorted_bytes(s, d) : 0);
     r.plane = static_cast<size_t>(d.M) * s->groups * d.Kd;
     r.total = r.columns + up(r.plane * 4) + 256;   // row blocks of 64 may be read past the end
+    r.f32 = keep && weight_in_f32(s, d, dtype);
     return r;
 }
 
@@ -290,13 +324,14 @@ BackwardSpace plan_backward(const dcn_shape* s, const Derived& d) {
 }
 
 struct ForwardSpace {
-    size_t weight_most, weight, total;
+    size_t weight_most, weight, columns, total;
 };
-ForwardSpace plan_forward(const dcn_shape* s, const Derived& d) {
+ForwardSpace plan_forward(const dcn_shape* s, const Derived& d, const Saved& at) {
     ForwardSpace r;
     r.weight_most = 0;
     r.weight = up(static_cast<size_t>(s->Co) * 4);
-    r.total = r.weight + up(static_cast<size_t>(s->Co) * d.Kd * 4);
+    r.columns = r.weight + up(static_cast<size_t>(s->Co) * d.Kd * 4);
+    r.total = r.columns + (at.f32 ? up(at.plane * 4) : 0);
     return r;
 }
 
@@ -328,13 +363,12 @@ void sample_params(const dcn_shape* s, const Derived& d, char* saved, const Save
 template <typename T>
 int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mask, const void* weight,
                   const float* bias, float* out, char* saved, char* ws, const dcn_shape* s, const Derived& d,
-                  cudaStream_t stream) {
+                  const Saved& at, cudaStream_t stream) {
     int sms = 0;
     int* status = nullptr;
     int rc = msda::device_facts(&sms, &status);
     if (rc != MSDA_OK) return rc;
-    const Saved at = plan_saved(s, d);
-    const ForwardSpace sp = plan_forward(s, d);
+    const ForwardSpace sp = plan_forward(s, d, at);
     uint32_t* bounds = reinterpret_cast<uint32_t*>(saved + at.bounds);
     RETURN_ON_CUDA(cudaMemsetAsync(bounds, 0, 16, stream));
     const int HoWo = s->Ho * s->Wo, taps = s->deform_groups * d.K;
@@ -355,19 +389,28 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
 
     DcnParams p{};
     sample_params(s, d, saved, at, mask != nullptr, &p);
-    p.pieces = d.Cd / 8;
-    int l = 0;
-    while ((1 << l) < p.pieces && l < 5) ++l;
-    p.lpi_log2 = l;
-    uint16_t* columns = reinterpret_cast<uint16_t*>(saved + at.columns);
+    uint16_t* columns = reinterpret_cast<uint16_t*>(at.f32 ? ws + sp.columns : saved + at.columns);
+    float* columns_f32 = at.f32 ? reinterpret_cast<float*>(saved + at.columns) : nullptr;
     const SplitScale col_scale{bounds, 0, mask != nullptr ? bounds + 1 : nullptr};
-    int per_sm = 0;
-    RETURN_ON_CUDA(msda::resident_ctas(reinterpret_cast<const void*>(gather_pairs_kernel), kThreads, 0, &per_sm));
-    const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
-    const uint32_t want = (p.items + per_step - 1) / per_step, cap = static_cast<uint32_t>(sms) * per_sm;
-    gather_pairs_kernel<<<want < cap ? want : cap, kThreads, 0, stream>>>(p, columns, at.plane, col_scale);
-    RETURN_ON_CUDA(cudaGetLastError());
-    msda::count_launches(2);
+    msda::count_launches(1);
+    if (sort_pays(s, d)) {
+        rc = launch_gather_sorted(p, saved + at.sorted, d.M, s->N, columns, at.plane, col_scale, columns_f32, sms,
+                                  stream);
+        if (rc != MSDA_OK) return rc;
+    } else {
+        p.pieces = d.Cd / 8;
+        int l = 0;
+        while ((1 << l) < p.pieces && l < 5) ++l;
+        p.lpi_log2 = l;
+        int per_sm = 0;
+        RETURN_ON_CUDA(msda::resident_ctas(reinterpret_cast<const void*>(gather_pairs_kernel), kThreads, 0, &per_sm));
+        const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
+        const uint32_t want = (p.items + per_step - 1) / per_step, cap = static_cast<uint32_t>(sms) * per_sm;
+        gather_pairs_kernel<<<want < cap ? want : cap, kThreads, 0, stream>>>(p, columns, at.plane, col_scale,
+                                                                                       columns_f32);
+        RETURN_ON_CUDA(cudaGetLastError());
+        msda::count_launches(1);
+    }
 
     bool zeroed = false;
     for (int g = 0; g < s->groups; ++g) {
@@ -392,12 +435,12 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
 template <typename T>
 int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* saved, bool masked,
                    float* grad_x, float* grad_offset, float* grad_mask, float* grad_weight, float* grad_bias,
-                   char* ws, const dcn_shape* s, const Derived& d, cudaStream_t stream) {
+                   char* ws, const dcn_shape* s, const Derived& d, const Saved& at, cudaStream_t stream) {
     int sms = 0;
     int* status = nullptr;
     int rc = msda::device_facts(&sms, &status);
     if (rc != MSDA_OK) return rc;
-    const Saved at = plan_saved(s, d);
+    const bool weight_f32 = at.f32;
     const BackwardSpace sp = plan_backward(s, d);
     const int M = static_cast<int>(d.M), HoWo = s->Ho * s->Wo;
     uint32_t* bounds = reinterpret_cast<uint32_t*>(saved + at.bounds);
@@ -420,7 +463,9 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* 
         const RowOrder order{HoWo, 0, 0};
         bounds_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, grad_bias);
         pairs_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, go_rows,
-                                                       go_channels, go_plane);
+                                                       weight_f32 ? nullptr : go_channels,
+                                                       weight_f32 ? reinterpret_cast<float*>(go_channels) : nullptr,
+                                                       go_plane);
     }
     // weights as [group][kd][output channel]
     const size_t wt_plane = static_cast<size_t>(s->groups) * d.Kd * d.Cog;
@@ -430,7 +475,7 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* 
         const RowOrder order{d.Kd, d.K, d.Cg};
         bounds_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, nullptr);
         pairs_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, weight_t, nullptr,
-                                                       wt_plane);
+                                                       nullptr, wt_plane);
     }
     RETURN_ON_CUDA(cudaGetLastError());
     msda::count_launches(4);
@@ -453,23 +498,24 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* 
     p.grad_x = grad_x;
     p.grad_offset = grad_offset;
     p.grad_mask = grad_mask;
-    rc = launch_scatter(p, sms, stream);
+    if (sort_pays(s, d)) rc = launch_scatter_sorted(p, saved + at.sorted, d.M, s->N, sms, stream);
+    else rc = launch_scatter(p, sms, stream);
     if (rc != MSDA_OK) return rc;
 
+    if (weight_f32)
+        return launch_weight_product(reinterpret_cast<const float*>(go_channels),
+                                     reinterpret_cast<const float*>(saved + at.columns), grad_weight, s, d, sms,
+                                     status, stream);
     const uint16_t* columns = reinterpret_cast<const uint16_t*>(saved + at.columns);
     const SplitScale col_scale{bounds, 0, masked ? bounds + 1 : nullptr};
-    bool zeroed = false;
+    const int splits = weight_splits(d, sms);
+    if (splits > 1)
+        RETURN_ON_CUDA(cudaMemsetAsync(grad_weight, 0, static_cast<size_t>(s->Co) * d.Kd * 4, stream));
     for (int g = 0; g < s->groups; ++g) {
         const SplitOperand A{go_channels + static_cast<size_t>(g) * d.Cog, 1, s->Co, static_cast<long long>(go_plane),
                              SplitScale{channel_most + static_cast<size_t>(g) * d.Cog, 1, nullptr}};
         const SplitOperand B{columns + static_cast<size_t>(g) * d.Kd, 1, ld_cols, static_cast<long long>(at.plane),
                              col_scale};
-        const long long tiles = ((d.Cog + 127) / 128) * static_cast<long long>((d.Kd + 255) / 256);
-        const int splits = balanced_splits(tiles, sms, (M + 1023) / 1024);
-        if (splits > 1 && !zeroed) {
-            RETURN_ON_CUDA(cudaMemsetAsync(grad_weight, 0, static_cast<size_t>(s->Co) * d.Kd * 4, stream));
-            zeroed = true;
-        }
         RETURN_ON_CUDA(msda::gemm_split(A, B, grad_weight + static_cast<size_t>(g) * d.Cog * d.Kd, d.Kd, nullptr,
                                         d.Cog, d.Kd, M, splits, status, stream));
         msda::count_launches(1);
@@ -489,37 +535,38 @@ int split_shape(const dcn_shape* s, Derived* d) {
 
 extern "C" {
 
-size_t dcn_sm100_saved_bytes(const dcn_shape* s) {
+size_t dcn_sm100_saved_bytes(const dcn_shape* s, int dtype, int keep) {
     Derived d;
-    return split_shape(s, &d) == MSDA_OK ? plan_saved(s, d).total : 0;
+    return split_shape(s, &d) == MSDA_OK ? plan_saved(s, d, dtype, keep != 0).total : 0;
 }
 
-size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int backward) {
+size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int dtype, int keep, int backward) {
     Derived d;
     if (check_shape(s, &d) != MSDA_OK) return 0;
-    return backward ? plan_backward(s, d).total : plan_forward(s, d).total;
+    return backward ? plan_backward(s, d).total : plan_forward(s, d, plan_saved(s, d, dtype, keep != 0)).total;
 }
 
 int dcn_sm100_forward_nchw(const void* x, int x_nhwc, const void* offset, const void* mask, const void* weight,
                            const float* bias, float* out, void* saved, size_t saved_bytes, void* workspace,
-                           size_t workspace_bytes, const dcn_shape* s, int dtype, void* stream_v) {
+                           size_t workspace_bytes, const dcn_shape* s, int dtype, int keep, void* stream_v) {
     if (x == nullptr || offset == nullptr || weight == nullptr || out == nullptr || saved == nullptr ||
         workspace == nullptr)
         return MSDA_ERR_NULL;
     Derived d;
     const int rc = split_shape(s, &d);
     if (rc != MSDA_OK) return rc;
-    if (saved_bytes < plan_saved(s, d).total || workspace_bytes < plan_forward(s, d).total)
+    const Saved at = plan_saved(s, d, dtype, keep != 0);
+    if (saved_bytes < at.total || workspace_bytes < plan_forward(s, d, at).total)
         return MSDA_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(saved) | reinterpret_cast<uintptr_t>(workspace)) % 16 != 0) return MSDA_ERR_ALIGN;
     char* sv = static_cast<char*>(saved);
     char* ws = static_cast<char*>(workspace);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     switch (dtype) {
-        case MSDA_F32: return forward_typed<float>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, stream);
-        case MSDA_F16: return forward_typed<__half>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, stream);
+        case MSDA_F32: return forward_typed<float>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, at, stream);
+        case MSDA_F16: return forward_typed<__half>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, at, stream);
         case MSDA_BF16:
-            return forward_typed<__nv_bfloat16>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, stream);
+            return forward_typed<__nv_bfloat16>(x, x_nhwc, offset, mask, weight, bias, out, sv, ws, s, d, at, stream);
         default: return MSDA_ERR_DTYPE;
     }
 }
@@ -543,16 +590,17 @@ int dcn_sm100_backward_nchw(const void* weight, const void* grad_out, int grad_o
     char* ws = static_cast<char*>(workspace);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const bool masked = grad_mask != nullptr;
+    const Saved at = plan_saved(s, d, dtype, true);
     switch (dtype) {
         case MSDA_F32:
             return backward_typed<float>(weight, grad_out, grad_out_nhwc, sv, masked, grad_x, grad_offset,
-                                         grad_mask, grad_weight, grad_bias, ws, s, d, stream);
+                                         grad_mask, grad_weight, grad_bias, ws, s, d, at, stream);
         case MSDA_F16:
             return backward_typed<__half>(weight, grad_out, grad_out_nhwc, sv, masked, grad_x, grad_offset,
-                                          grad_mask, grad_weight, grad_bias, ws, s, d, stream);
+                                          grad_mask, grad_weight, grad_bias, ws, s, d, at, stream);
         case MSDA_BF16:
             return backward_typed<__nv_bfloat16>(weight, grad_out, grad_out_nhwc, sv, masked, grad_x,
-                                                 grad_offset, grad_mask, grad_weight, grad_bias, ws, s, d, stream);
+                                                 grad_offset, grad_mask, grad_weight, grad_bias, ws, s, d, at, stream);
         default: return MSDA_ERR_DTYPE;
     }
 }

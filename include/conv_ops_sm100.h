@@ -112,16 +112,16 @@ int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
  * are multiples of 8 and dcn_sm100_use_tensor_cores() == 1; elsewhere dcn_sm100_saved_bytes() is 0.
  *   weight [Co, C / groups, kh, kw]; offset [N, deform_groups * 2 * kh * kw, Ho, Wo]; mask likewise
  *   saved: device memory of dcn_sm100_saved_bytes(), written by the forward, read by the backward
- *          (16-byte aligned, like the workspaces)
+ *          (16-byte aligned, like the workspaces); keep = 0 where no backward will follow
  *   out [N, Ho, Wo, Co] and the gradients are float32 in the layouts of the calls above
  *          (grad_weight [Co, kh, kw, C / groups]); mask and grad_mask both or neither.
  */
-size_t dcn_sm100_saved_bytes(const dcn_shape* s);
-size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int backward);
+size_t dcn_sm100_saved_bytes(const dcn_shape* s, int dtype, int keep);
+size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int dtype, int keep, int backward);
 int dcn_sm100_forward_nchw(const void* x, int x_nhwc, const void* offset, const void* mask,
                            const void* weight, const float* bias, float* out, void* saved,
                            size_t saved_bytes, void* workspace, size_t workspace_bytes,
-                           const dcn_shape* s, int dtype, void* stream);
+                           const dcn_shape* s, int dtype, int keep, void* stream);
 int dcn_sm100_backward_nchw(const void* weight, const void* grad_out, int grad_out_nhwc,
                             const void* saved, float* grad_x, float* grad_offset, float* grad_mask,
                             float* grad_weight, float* grad_bias, void* workspace,

@@ -33,6 +33,12 @@ CASES = [
     (1, 128, 264, 12, 12, 1, 1, 2, True),
     (2, 64, 80, 10, 9, 1, 2, 1, True),
     (1, 512, 256, 13, 21, 1, 4, 1, False),
+    # enough samples for the cell-sorted sampling: one and two passes of the lanes, slices, idle
+    # lanes, several deformable groups
+    (3, 104, 48, 62, 63, 1, 1, 1, True),
+    (1, 264, 16, 111, 103, 1, 1, 1, True),
+    (2, 320, 32, 41, 70, 1, 1, 2, False),
+    (4, 256, 64, 55, 54, 1, 2, 2, True),
 ]
 
 
