@@ -127,7 +127,6 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
     // channels — it only needs grad_out for those channels (gred below).
     constexpr bool SPLIT_RED = !SCALAR && sizeof(T) == 2 && sizeof(TG) == 4;
 
-    if (!device_level_table_ok(p)) return;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -143,7 +142,9 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
     init_unused_slots<CPS>(s_slot, lane);
     WarpStage<T> st = warp_stage_init<T>(p, wb + kSlotBytes + kPartBytes, lane);
 
-    const LaneLevels lv = load_lane_levels(p, lane);
+    bool levels_ok;
+    const LaneLevels lv = load_lane_levels(p, lane, levels_ok);
+    if (!levels_ok) return;
     const T* __restrict__ value = static_cast<const T*>(p.value);
     // this lane's pieces of a row; past the end of the row it reads the last one again, with a
     // zero grad_out piece, and reduces nothing

@@ -194,6 +194,17 @@ bool sort_pays(const SortPlan& s, int K, int H, int D, int dtype, int B, int mod
     return per_cell >= (dtype == MSDA_F32 ? 50.0 : 25.0);
 }
 
+// Tasks that one warp pass takes together: as many as fill its lanes with samples, but fewer where
+// there are so few tasks that `warps` take all of them in one round with fewer each (300 queries
+// x 8 heads x 16 samples: forward 5.6 -> 4.5 us; with more rounds the fuller passes are faster).
+int tasks_per_item(int LP, long long tasks, int warps) {
+    if (LP >= msda::kChunk) return 1;
+    const int most = msda::kChunk / LP;
+    int t = 1;
+    while (t < most && (tasks + t - 1) / t > warps) t *= 2;
+    return t < most ? t : most;
+}
+
 // Fills the parts of Params common to both directions.
 int fill_common(Params& p, const DeviceInfo* dev, const void* value, const int32_t* shapes,
                 const int32_t* starts, const void* loc, const void* attn, int B, int K, int H,
@@ -204,7 +215,7 @@ int fill_common(Params& p, const DeviceInfo* dev, const void* value, const int32
     p.attn = attn;
     p.B = B; p.K = K; p.H = H; p.D = D; p.L = L; p.Q = Q; p.P = P;
     p.LP = L * P;
-    p.tasks_per_item = (p.LP >= msda::kChunk) ? 1 : (msda::kChunk / p.LP);
+    p.tasks_per_item = tasks_per_item(p.LP, static_cast<long long>(B) * Q * H, dev->sm_count * (backward ? 24 : 32));
     p.ntasks = static_cast<long long>(B) * Q * H;
     p.nitems = (p.ntasks + p.tasks_per_item - 1) / p.tasks_per_item;
     p.status = dev->status_ptr;

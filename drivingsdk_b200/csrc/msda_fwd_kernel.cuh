@@ -47,7 +47,6 @@ msda_fwd_kernel(const __grid_constant__ Params p) {
     constexpr int STEP = RPI * UNROLL;             // slots per trip of the gather loop
     static_assert(kSlots % STEP == 0 && STEP <= kSlotPad, "slot loop must tile the slots");
 
-    if (!device_level_table_ok(p)) return;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -59,7 +58,9 @@ msda_fwd_kernel(const __grid_constant__ Params p) {
     init_unused_slots<CPS>(s_slot, lane);
     WarpStage<T> st = warp_stage_init<T>(p, wb + kSlotBytes, lane);
 
-    const LaneLevels lv = load_lane_levels(p, lane);
+    bool levels_ok;
+    const LaneLevels lv = load_lane_levels(p, lane, levels_ok);
+    if (!levels_ok) return;
     const T* __restrict__ value = static_cast<const T*>(p.value);
     // this lane's pieces of a row; past the end of the row it reads the last one again
     int voff[NV];

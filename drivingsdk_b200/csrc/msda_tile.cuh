@@ -47,8 +47,12 @@ __device__ __forceinline__ void lane_sample_index(const Params& p, int chunk, in
     }
 }
 
-__device__ __forceinline__ LaneLevels load_lane_levels(const Params& p, int lane) {
+// `ok`: false when a table in device memory is inconsistent (device_level_table_ok's rule; the
+// lanes of a warp cover all levels, so each warp decides for itself, with the loads it needs
+// anyway and no barrier: a small launch is mostly the latency of its first loads).
+__device__ __forceinline__ LaneLevels load_lane_levels(const Params& p, int lane, bool& ok) {
     LaneLevels lv;
+    bool bad = false;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         int tl, s;
@@ -71,7 +75,11 @@ __device__ __forceinline__ LaneLevels load_lane_levels(const Params& p, int lane
         } else {
             lv.h1 = hh; lv.w1 = ww; lv.start1 = ss;
         }
+        bad |= hh <= 0 || ww <= 0 || ss < 0 ||
+               static_cast<long long>(ss) + static_cast<long long>(hh) * ww > p.K;
     }
+    ok = p.use_table || !__any_sync(0xffffffffu, bad);
+    if (!ok && lane == 0) atomicOr(p.status, kStatusBadLevels);
     return lv;
 }
 
