@@ -97,7 +97,9 @@ __device__ __forceinline__ SampleGrad sample_grad(const float* part, const Sampl
     return r;
 }
 
-template <typename T, typename TG, int LPR, int NV, bool SCALAR, int MODE>
+// RAGGED: rows of fewer pieces than the lanes hold (24 or 48 channels). A form of its own because its
+// checks cost the others 2 to 7 % (fused operator, fp16, 128 channels: 825 -> 887 us).
+template <typename T, typename TG, int LPR, int NV, bool SCALAR, int MODE, bool RAGGED>
 __global__ void __launch_bounds__(kThreadsPerCta, (SCALAR || NV > 1) ? 2 : MSDA_BWD_MIN_CTAS)
 msda_bwd_kernel(const __grid_constant__ Params p) {
     constexpr int CPS = (MODE == kModeFused) ? 4 : MODE;   // rows (corners) per sample
@@ -152,10 +154,11 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
     bool on[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        on[k] = SCALAR || j + k * LPR < p.pieces;
-        voff[k] = SCALAR ? 0 : min(j + k * LPR, p.pieces - 1) * 16;
+        on[k] = !RAGGED || j + k * LPR < p.pieces;
+        voff[k] = SCALAR ? 0 : (RAGGED ? min(j + k * LPR, p.pieces - 1) : j + k * LPR) * 16;
     }
-    const bool red_on[2] = {j < 2 * p.pieces, LPR + j < 2 * p.pieces};   // SPLIT_RED's two pieces
+    // SPLIT_RED's two pieces
+    const bool red_on[2] = {!RAGGED || j < 2 * p.pieces, !RAGGED || LPR + j < 2 * p.pieces};
     const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + voff[0];
     const T* __restrict__ gout = static_cast<const T*>(p.grad_out);
     TG* __restrict__ gval = static_cast<TG*>(p.grad_value);
@@ -310,7 +313,7 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
 #pragma unroll
                             for (int k = 0; k < NV; ++k)
                                 raw[u][k] =
-                                    ldg16(vlane + static_cast<size_t>(off) * 16 + (voff[k] - voff[0]));
+                                    ldg16(vlane + static_cast<size_t>(off) * 16 + (RAGGED ? voff[k] - voff[0] : k * (LPR * 16)));
                         }
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
@@ -508,10 +511,14 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
 // ---------------------------------------------------------------------------
 // launch table
 // ---------------------------------------------------------------------------
-template <typename T, typename TG, int LPR, int NV, bool SCALAR, int MODE>
+template <typename T, typename TG, int LPR, int NV, bool SCALAR, int MODE, bool RAGGED = false>
 static cudaError_t launch_bwd_inst(const Params& p, const LaunchShape& ls, size_t smem,
                                    cudaStream_t stream) {
-    auto kern = msda_bwd_kernel<T, TG, LPR, NV, SCALAR, MODE>;
+    if constexpr (!SCALAR && !RAGGED && LPR * NV > 2) {   // (one or two pieces fill their lanes)
+        if (p.pieces != LPR * NV)
+            return launch_bwd_inst<T, TG, LPR, NV, SCALAR, MODE, true>(p, ls, smem, stream);
+    }
+    auto kern = msda_bwd_kernel<T, TG, LPR, NV, SCALAR, MODE, RAGGED>;
     int grid = 0;
     cudaError_t e = persistent_grid(reinterpret_cast<const void*>(kern), smem, ls, p, &grid);
     if (e != cudaSuccess) return e;
