@@ -129,13 +129,15 @@ static cudaError_t launch_map_fwd(const Params& p, const LaunchShape& ls, cudaSt
     const int threads = (two || map + 32 * record > kMapSmem) ? 512 : 1024;
     const size_t smem = map + threads / 32 * record;
     if (smem > kMapSmem) return cudaSuccess;
-    // Every CTA and every map has its rows loaded once more: that pays from some four samples per
-    // row on (8 x 1000 x 4 tasks of 15 samples, 1500 pixels: 1.8 per row and 14.6 against 14.3 us;
-    // with 4000 queries 7.1 and 24.7 against 41.4 us).
+    // Every CTA and every map has its rows loaded once more. That pays from some three samples per
+    // loaded row on, two in 16 bits (24 x 204 x 4 tasks of 15 samples, 375 pixels of 256 bytes: 3.2 and
+    // 10.8 against 11.7 us, 2.2 and 9.8 against 9.6; bf16 2.2 and 10.0 against 11.3, 1.2 and 8.3
+    // against 8.1).
+    constexpr int kLeast = sizeof(T) == 4 ? 3 : 2;
     const long long grid = static_cast<long long>(ls.sm_count) *
                            (ls.ctas_per_sm > 0 ? ls.ctas_per_sm : two ? 2 : 1);
     const long long maps = static_cast<long long>(p.B) * p.H * slices;
-    if (p.ntasks * slices * p.LP < 4 * (grid + maps) * p.K) return cudaSuccess;
+    if (p.ntasks * slices * p.LP < kLeast * (grid + maps) * p.K) return cudaSuccess;
     int resident = 0;   // (asked for the shared-memory limit that the call sets)
     const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), threads, smem, &resident);
     if (e != cudaSuccess) return e;
