@@ -206,8 +206,9 @@ constexpr uint32_t kAmplified = 4;   // wants its dot products in double
 // be a power of two) and hold all four corners of a cell: value rows and gradient sums. A warp
 // walks 32 / LPR streams of sp.stream consecutive sorted samples side by side, in rounds of 32
 // samples whose set-up and final gradients are done lane = sample. The accumulation rows are
-// fp32.
-template <typename T, typename TL, int NV, int LPR>
+// fp32. RAGGED: some of those lanes are past D; without their checks the rest is 1 to 4 % faster
+// (encoder shape, fp32, 32 channels: 284 -> 274 us; 128 channels, bf16: 1894 -> 1867 us).
+template <typename T, typename TL, int NV, int LPR, bool RAGGED>
 __global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 3)
 msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
     constexpr int S = 32 / LPR;       // streams
@@ -232,7 +233,7 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
     const uint32_t step_x = static_cast<uint32_t>(p.H) * p.row_units;
     bool on[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) on[k] = (j + k * LPR) * 4 < p.D;
+    for (int k = 0; k < NV; ++k) on[k] = !RAGGED || (j + k * LPR) * 4 < p.D;
     const T* vlane = static_cast<const T*>(p.value) + j * 4;
     const T* glane = static_cast<const T*>(p.grad_out) + j * 4;
     float* alane = static_cast<float*>(p.grad_value) + j * 4;
@@ -463,7 +464,7 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
 
 // Nearest-pixel main kernel: one row per sample. LPR lanes cover a row (four channels each, NV
 // times), 32 / LPR samples of one pixel are worked on at a time and share its row.
-template <typename T, typename TL, int NV, int LPR>
+template <typename T, typename TL, int NV, int LPR, bool RAGGED>
 __global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 4)
 gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
     constexpr int U = 4;            // rows of grad_out in flight per lane
@@ -476,7 +477,7 @@ gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     float* dot = s_dot[warp];
     bool on[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) on[k] = (j + k * LPR) * 4 < p.D;
+    for (int k = 0; k < NV; ++k) on[k] = !RAGGED || (j + k * LPR) * 4 < p.D;
     const T* vlane = static_cast<const T*>(p.value) + j * 4;
     const T* glane = static_cast<const T*>(p.grad_out) + j * 4;
     float* alane = static_cast<float*>(p.grad_value) + j * 4;
@@ -606,6 +607,17 @@ static cudaError_t launch_sorted_main(Kernel kern, int streams, const Params& p,
     return cudaGetLastError();
 }
 
+// The lanes of a row of D channels: launch(pieces per lane, lanes).
+template <typename Launch>
+static cudaError_t for_row_width(int D, const Launch& launch) {
+    const std::integral_constant<int, 1> one;
+    if (D <= 16) return launch(one, std::integral_constant<int, 4>());
+    if (D <= 32) return launch(one, std::integral_constant<int, 8>());
+    if (D <= 64) return launch(one, std::integral_constant<int, 16>());
+    if (D <= 128) return launch(one, std::integral_constant<int, 32>());
+    return launch(std::integral_constant<int, 2>(), std::integral_constant<int, 32>());
+}
+
 template <typename T, typename TL>
 static cudaError_t launch_sorted_bilinear(const Params& p, SortParams sp,
                                           const LaunchShape& ls, cudaStream_t stream) {
@@ -613,11 +625,13 @@ static cudaError_t launch_sorted_bilinear(const Params& p, SortParams sp,
     cudaError_t e = launch_sort(AttentionSamples<TL, 4>{p, sp.fd_p, n},
                                 static_cast<uint32_t>(p.B) * p.H * p.L, sp, ls.sm_count, stream);
     if (e != cudaSuccess) return e;
-    if (p.D <= 16) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 4>, 8, p, sp, n, ls, stream);
-    if (p.D <= 32) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 8>, 4, p, sp, n, ls, stream);
-    if (p.D <= 64) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 16>, 2, p, sp, n, ls, stream);
-    if (p.D <= 128) return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 1, 32>, 1, p, sp, n, ls, stream);
-    return launch_sorted_main(msda_bwd_sorted_kernel<T, TL, 2, 32>, 1, p, sp, n, ls, stream);
+    auto main = [&](auto nv, auto lpr) {
+        constexpr int NV = decltype(nv)::value, LPR = decltype(lpr)::value;
+        return p.D == 4 * NV * LPR
+                   ? launch_sorted_main(msda_bwd_sorted_kernel<T, TL, NV, LPR, false>, 32 / LPR, p, sp, n, ls, stream)
+                   : launch_sorted_main(msda_bwd_sorted_kernel<T, TL, NV, LPR, true>, 32 / LPR, p, sp, n, ls, stream);
+    };
+    return for_row_width(p.D, main);
 }
 
 template <typename T>
@@ -627,11 +641,13 @@ static cudaError_t launch_sorted_nearest(const Params& p, SortParams sp,
     cudaError_t e = launch_sort(AttentionSamples<T, 1>{p, sp.fd_p, n},
                                 static_cast<uint32_t>(p.B) * p.H * p.L, sp, ls.sm_count, stream);
     if (e != cudaSuccess) return e;
-    if (p.D <= 16) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 4>, 1, p, sp, n, ls, stream);
-    if (p.D <= 32) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 8>, 1, p, sp, n, ls, stream);
-    if (p.D <= 64) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 16>, 1, p, sp, n, ls, stream);
-    if (p.D <= 128) return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 1, 32>, 1, p, sp, n, ls, stream);
-    return launch_sorted_main(gka_bwd_sorted_kernel<T, T, 2, 32>, 1, p, sp, n, ls, stream);
+    auto main = [&](auto nv, auto lpr) {
+        constexpr int NV = decltype(nv)::value, LPR = decltype(lpr)::value;
+        return p.D == 4 * NV * LPR
+                   ? launch_sorted_main(gka_bwd_sorted_kernel<T, T, NV, LPR, false>, 1, p, sp, n, ls, stream)
+                   : launch_sorted_main(gka_bwd_sorted_kernel<T, T, NV, LPR, true>, 1, p, sp, n, ls, stream);
+    };
+    return for_row_width(p.D, main);
 }
 
 }  // namespace msda
