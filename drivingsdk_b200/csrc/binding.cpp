@@ -416,6 +416,10 @@ bool vector_rows(const DaDims& d) {
            d.C / d.G <= 128;
 }
 
+bool same_type(const at::Tensor& feat, const at::Tensor& loc, const at::Tensor& wts) {
+    return loc.scalar_type() == feat.scalar_type() && wts.scalar_type() == feat.scalar_type();
+}
+
 // Sorting the samples by cell (two more launches) pays from about one sample per feature row on
 // (0.3 per row: 95 / 110 us unsorted / sorted, 1.0: 182 / 145, 3.1: 1774 / 951; forward and
 // backward), earlier for 16-bit tensors, which the unsorted kernel needs converted.
@@ -441,8 +445,9 @@ at::Tensor deformable_aggregation(const at::Tensor& feat_in, const at::Tensor& s
                                   const at::Tensor& wts_in) {
     const DaDims d = check_da_inputs(feat_in, shape_in, start_in, loc_in, wts_in);
     const c10::cuda::CUDAGuard guard(feat_in.device());
-    // vector rows are read in their own type, others as fp32
-    const auto kind = vector_rows(d) ? feat_in.scalar_type() : at::kFloat;
+    // vector rows of operands that share a type are read in it, all others as fp32: a location in
+    // a 16-bit type would be off by a third of a pixel on a map 176 pixels wide
+    const auto kind = vector_rows(d) && same_type(feat_in, loc_in, wts_in) ? feat_in.scalar_type() : at::kFloat;
     const at::Tensor feat = feat_in.to(kind).contiguous();
     const at::Tensor loc = loc_in.to(kind).contiguous();
     const at::Tensor wts = wts_in.to(kind).contiguous();
@@ -477,10 +482,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> deformable_aggregation_backward(
     const c10::cuda::CUDAGuard guard(feat_in.device());
     const size_t ws_bytes =
         da_sm100_backward_workspace_bytes(d.B, d.F, d.C, d.A, d.Pts, d.cams, d.scales, d.G);
-    if (ws_bytes > 0 && sort_da(d, feat_in.scalar_type())) {
-        // operands as they are, when they share a type; fp32 gradients
-        const auto kind = feat_in.scalar_type();
-        const at::Tensor feat = feat_in.contiguous();
+    // operands as they are, when they share a type, else as fp32; fp32 gradients
+    const auto kind = same_type(feat_in, loc_in, wts_in) && grad_out_in.scalar_type() == feat_in.scalar_type()
+                          ? feat_in.scalar_type() : at::kFloat;
+    if (ws_bytes > 0 && sort_da(d, kind)) {
+        const at::Tensor feat = feat_in.to(kind).contiguous();
         const at::Tensor loc = loc_in.to(kind).contiguous();
         const at::Tensor wts = wts_in.to(kind).contiguous();
         const at::Tensor shape = shape_in.contiguous();
@@ -498,7 +504,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> deformable_aggregation_backward(
             d.C, d.A, d.Pts, d.cams, d.scales, d.G, dtype_code(kind),
             at::cuda::getCurrentCUDAStream().stream());
         raise_on_da_error(rc, "npu_deformable_aggregation_backward");
-        return std::make_tuple(grad_feat.to(kind), grad_loc.to(loc_in.scalar_type()),
+        return std::make_tuple(grad_feat.to(feat_in.scalar_type()), grad_loc.to(loc_in.scalar_type()),
                                grad_wts.to(wts_in.scalar_type()));
     }
     const at::Tensor feat = feat_in.to(at::kFloat).contiguous();
