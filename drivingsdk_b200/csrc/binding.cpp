@@ -503,9 +503,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> deformable_aggregation_backward(
             grad_loc.data_ptr<float>(), grad_wts.data_ptr<float>(), ws.data_ptr(), ws_bytes, d.B, d.F,
             d.C, d.A, d.Pts, d.cams, d.scales, d.G, dtype_code(kind),
             at::cuda::getCurrentCUDAStream().stream());
-        raise_on_da_error(rc, "npu_deformable_aggregation_backward");
-        return std::make_tuple(grad_feat.to(feat_in.scalar_type()), grad_loc.to(loc_in.scalar_type()),
-                               grad_wts.to(wts_in.scalar_type()));
+        if (rc != MSDA_ERR_ALIGN) {   // (operands off the sorted form's alignment: below)
+            raise_on_da_error(rc, "npu_deformable_aggregation_backward");
+            return std::make_tuple(grad_feat.to(feat_in.scalar_type()), grad_loc.to(loc_in.scalar_type()),
+                                   grad_wts.to(wts_in.scalar_type()));
+        }
     }
     const at::Tensor feat = feat_in.to(at::kFloat).contiguous();
     const at::Tensor loc = loc_in.to(at::kFloat).contiguous();

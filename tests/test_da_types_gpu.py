@@ -63,3 +63,19 @@ def test_gradient_of_another_type(case):
     got = call(t["feat"], t["loc"], t["wts"])
     want = call(t["feat"].float(), t["loc"].float(), t["wts"].float())
     _agree([got[0], *got], [want[0], *want])
+
+
+def _off_by_one_element(t):
+    return torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("case", CASES, ids=["few", "sorted"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", NAMES)
+def test_contiguous_operands_at_odd_addresses(case, dtype, name):
+    tables, t = _operands(case)
+    t = {k: v.to(dtype) for k, v in t.items()}
+    want = _run(tables, t)
+    t[name] = _off_by_one_element(t[name])
+    assert t[name].is_contiguous() and t[name].data_ptr() % (2 * t[name].element_size()) != 0
+    _agree(_run(tables, t), want)
