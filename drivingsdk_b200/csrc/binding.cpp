@@ -291,6 +291,13 @@ Dims check_gka_inputs(const at::Tensor& value, const at::Tensor& shapes, const a
                 "sampling_locations / attention_weights shapes do not match value");
     TORCH_CHECK(shapes.numel() == 2 * d.L && starts.numel() == d.L,
                 "spatial_shapes must have one (H, W) row and level_start_index one entry per level");
+    // the call below does not ask the runtime where device tables are (dtype_and_tables)
+    TORCH_CHECK(shapes.device() == starts.device(),
+                "spatial_shapes and level_start_index must live on the same device");
+    TORCH_CHECK(!shapes.is_cuda() || shapes.device() == value.device(),
+                "spatial_shapes / level_start_index must be CPU tensors or live on value's device");
+    TORCH_CHECK(loc.device() == value.device() && attn.device() == value.device(),
+                "sampling_locations and attention_weights must live on value's device");
     return d;
 }
 

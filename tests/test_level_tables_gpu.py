@@ -1,0 +1,25 @@
+"""Level tables that the operators refuse, on the host before anything is launched."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _tables(kind):
+    cuda32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    shapes, starts = cuda32([[2, 3], [1, 2]]), cuda32([0, 6])
+    return {"starts on the host": (shapes, starts.cpu()), "shapes on the host": (shapes.cpu(), starts),
+            "int32 and int64": (shapes, starts.long()), "int64 and int32": (shapes.long(), starts),
+            "int16": (shapes.short(), starts.short())}[kind]
+
+
+@pytest.mark.parametrize("kind", ["starts on the host", "shapes on the host"])
+def test_kernel_attention_wants_its_tables_together(kind):
+    import drivingsdk_b200 as sdk
+    from drivingsdk_b200 import _C
+    value, attn = torch.zeros(1, 8, 1, 8, device="cuda"), torch.zeros(1, 3, 1, 2, 2, device="cuda")
+    loc, go = torch.zeros(1, 3, 1, 2, 2, 2, device="cuda"), torch.zeros(1, 3, 8, device="cuda")
+    with pytest.raises(RuntimeError, match="same device"):
+        sdk.geometric_kernel_attention(value, *_tables(kind), loc, attn)
+    with pytest.raises(RuntimeError, match="same device"):
+        _C.geometric_kernel_attention_backward(value, *_tables(kind), loc, attn, go)
