@@ -56,13 +56,17 @@ struct Dims {
     int B, K, H, D, L, Q, P;
 };
 
-// The tables may be int32 or int64, both alike; the exported functions of the reference's
-// extension take int32 only (check_int32_tables).
+// The tables may be int32 or int64, both alike: the kernels read both with one step. The exported
+// functions take int32 only (check_int32_tables).
 Dims check_inputs(const at::Tensor& value, const at::Tensor& shapes, const at::Tensor& starts,
                   const at::Tensor& loc, const at::Tensor& attn) {
     TORCH_CHECK(is_float_kind(value.scalar_type()),
                 "value: float16, bfloat16 or float32 tensor expected but got a tensor with dtype: ",
                 value.scalar_type());
+    TORCH_CHECK((shapes.scalar_type() == at::kInt || shapes.scalar_type() == at::kLong) &&
+                    starts.scalar_type() == shapes.scalar_type(),
+                "value_spatial_shapes and value_level_start_index: int32 tensors, or both int64, expected "
+                "but got tensors with dtypes: ", shapes.scalar_type(), " and ", starts.scalar_type());
     TORCH_CHECK(is_float_kind(loc.scalar_type()),
                 "sampling_locations: float16, bfloat16 or float32 tensor expected but got a tensor "
                 "with dtype: ", loc.scalar_type());
@@ -1016,10 +1020,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("geometric_kernel_attention_backward", &geometric_kernel_attention_backward,
           "GKA backward: (value, spatial_shapes, level_start_index, sampling_locations, "
           "attention_weights, grad_output) -> (grad_value, grad_attn_weights)");
-    m.def("msda_fused_forward", &msda_fused_forward,
+    m.def("msda_fused_forward",
+          [](const at::Tensor& value, const at::Tensor& shapes, const at::Tensor& starts, const at::Tensor& ref,
+             const at::Tensor& off, const at::Tensor& logits) {
+              check_int32_tables(shapes, starts);
+              return msda_fused_forward(value, shapes, starts, ref, off, logits);
+          },
           "fused MSDA forward: (value, spatial_shapes, level_start_index, reference_points, "
           "sampling_offsets, attention_logits) -> output");
-    m.def("msda_fused_backward", &msda_fused_backward,
+    m.def("msda_fused_backward",
+          [](const at::Tensor& value, const at::Tensor& shapes, const at::Tensor& starts, const at::Tensor& ref,
+             const at::Tensor& off, const at::Tensor& logits, const at::Tensor& grad_out) {
+              check_int32_tables(shapes, starts);
+              return msda_fused_backward(value, shapes, starts, ref, off, logits, grad_out);
+          },
           "fused MSDA backward -> (grad_value, grad_reference_points, grad_sampling_offsets, "
           "grad_attention_logits)");
     m.def("npu_deformable_aggregation", &deformable_aggregation,

@@ -23,3 +23,18 @@ def test_kernel_attention_wants_its_tables_together(kind):
         sdk.geometric_kernel_attention(value, *_tables(kind), loc, attn)
     with pytest.raises(RuntimeError, match="same device"):
         _C.geometric_kernel_attention_backward(value, *_tables(kind), loc, attn, go)
+
+
+@pytest.mark.parametrize("kind", ["int32 and int64", "int64 and int32", "int16"])
+def test_exported_functions_take_int32_tables(kind):
+    from drivingsdk_b200 import _C
+    value, logits = torch.zeros(1, 8, 1, 8, device="cuda"), torch.zeros(1, 3, 1, 2, 2, device="cuda")
+    loc, ref = torch.zeros(1, 3, 1, 2, 2, 2, device="cuda"), torch.zeros(1, 3, 2, 2, device="cuda")
+    go = torch.zeros(1, 3, 8, device="cuda")
+    for call in (lambda s, t: _C.msda_fused_forward(value, s, t, ref, loc, logits),
+                 lambda s, t: _C.msda_fused_backward(value, s, t, ref, loc, logits, go),
+                 lambda s, t: _C.multi_scale_deformable_attn(value, s, t, loc, logits),
+                 lambda s, t: _C.multi_scale_deformable_attn_backward(value, s, t, loc, logits, go)):
+        for place in ("cuda", "cpu"):
+            with pytest.raises(RuntimeError, match="int32 tensor expected"):
+                call(*(t.to(place) for t in _tables(kind)))
