@@ -23,13 +23,14 @@ LIB = os.path.join(PKG, "libmsda_sm100.so")
 DEBUG_LIB = os.path.join(PKG, "libmsda_sm100_dbg.so")
 EXT = os.path.join(PKG, "_C.so")
 
-CUDA_SOURCES = ["msda_capi.cu", "msda_fwd_sm100.cu", "msda_bwd_sm100.cu", "gka_fwd_sm100.cu",
-                "gka_bwd_sm100.cu", "msda_bwd_sorted_sm100.cu", "gka_bwd_sorted_sm100.cu", "msda_fused_fwd_sm100.cu", "msda_fused_bwd_sm100.cu", "da_sm100.cu", "da_sorted_sm100.cu",
-                "msda_static_scratch.cu", "hw_probe_sm100.cu", "resnet_ops_sm100.cu", "dcn_sm100.cu", "dcn_split_sm100.cu", "dcn_sorted_sm100.cu",
-                "gemm_split_sm100.cu",
-                "gemm_simt_sm100.cu", "gemm_tc_sm100.cu"]
+CUDA_SOURCES = ["msda_capi.cu", "resident_ctas.cu", "msda_fwd_sm100.cu", "msda_bwd_sm100.cu",
+                "gka_fwd_sm100.cu", "gka_bwd_sm100.cu", "msda_bwd_sorted_sm100.cu", "gka_bwd_sorted_sm100.cu",
+                "msda_fused_fwd_sm100.cu", "msda_fused_bwd_sm100.cu", "da_sm100.cu", "da_sorted_sm100.cu",
+                "msda_static_scratch.cu", "hw_probe_sm100.cu", "resnet_ops_sm100.cu", "dcn_sm100.cu",
+                "dcn_split_sm100.cu", "dcn_sorted_sm100.cu", "gemm_split_sm100.cu", "gemm_simt_sm100.cu",
+                "gemm_tc_sm100.cu"]
 EXT_SOURCES = ["binding.cpp", "autograd.cpp"]
-CUDA_HEADERS = ["msda_common.cuh", "msda_tile.cuh", "msda_launch.h", "msda_fwd_kernel.cuh",
+CUDA_HEADERS = ["msda_common.cuh", "msda_tile.cuh", "msda_launch.h", "resident_ctas.h", "msda_fwd_kernel.cuh",
                 "msda_bwd_kernel.cuh", "msda_bwd_sorted.cuh", "cell_sort.cuh", "da_params.h", "gemm_sm100.h",
                 "gemm_common.cuh", "gemm_split.h", "split_scale.cuh", "dcn_common.cuh", "dcn_split.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

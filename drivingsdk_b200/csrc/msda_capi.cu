@@ -5,9 +5,6 @@
 // No allocation, no synchronisation (except msda_sm100_device_status).
 #include <atomic>
 #include <cstring>
-#include <map>
-#include <mutex>
-#include <tuple>
 
 #include "../../include/msda_sm100.h"
 #include "msda_launch.h"
@@ -441,44 +438,6 @@ int forward_impl(const void* value, const int32_t* spatial_shapes,
 namespace msda {
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 int note_cuda_error(cudaError_t e) { return fail_cuda(e); }
-cudaError_t resident_ctas(const void* kernel, int threads, size_t smem, int* per_sm) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    struct Key {
-        const void* kernel;
-        size_t smem;
-        int threads, dev;
-        bool operator<(const Key& o) const {
-            return std::tie(kernel, smem, threads, dev) < std::tie(o.kernel, o.smem, o.threads, o.dev);
-        }
-    };
-    static std::mutex lock;
-    static std::map<Key, int> known;   // a handful of entries: kernels x their shared-memory sizes
-    const Key key{kernel, smem, threads, dev};
-    {
-        std::lock_guard<std::mutex> hold(lock);
-        const auto it = known.find(key);
-        if (it != known.end()) {
-            *per_sm = it->second;
-            return cudaSuccess;
-        }
-    }
-    // the limit only ever grows: launches of the kernel with more shared memory may be under way
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, kernel);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> hold(lock);
-    if (smem > static_cast<size_t>(attr.maxDynamicSharedSizeBytes)) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
-    int n = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
-    if (e != cudaSuccess) return e;
-    *per_sm = known[key] = n < 1 ? 1 : n;
-    return cudaSuccess;
-}
 int device_facts(int* sm_count, int** status_word) {
     const DeviceInfo* d = nullptr;
     const int rc = device_info(&d);

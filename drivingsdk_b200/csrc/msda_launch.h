@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "msda_common.cuh"
+#include "resident_ctas.h"
 
 namespace msda {
 
@@ -18,11 +19,6 @@ struct RowPlan {
     int lpr;
     int nv;
 };
-
-// CTAs of `threads` threads and `smem` bytes of dynamic shared memory that one SM of the current
-// device holds at once (at least 1); lets the kernel use that much shared memory. Asked of the
-// runtime once per kernel, size and device: the query costs more host time than a launch.
-cudaError_t resident_ctas(const void* kernel, int threads, size_t smem, int* per_sm);
 
 // Grid of a persistent launch: `ctas_per_sm` CTAs on each of `sm_count` SMs, or — when
 // ctas_per_sm <= 0 — as many as the occupancy calculator says are resident at once for this
