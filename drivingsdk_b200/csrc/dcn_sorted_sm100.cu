@@ -459,12 +459,11 @@ int launch_gather_sorted(const DcnParams& p, void* workspace, long long M, int N
     return MSDA_OK;
 }
 
-int launch_scatter_sorted(const DcnParams& p, void* workspace, long long M, int N, int sm_count,
-                          cudaStream_t stream) {
+int launch_scatter_sorted(const DcnParams& p, const void* sorted, uint32_t* ticket, long long M, int N,
+                          int sm_count, cudaStream_t stream) {
     const size_t items = static_cast<size_t>(M) * p.DG * p.K;
-    SortParams sp = sorted_params(workspace, items, static_cast<uint32_t>(N) * p.DG);
-    cudaError_t e = cudaMemsetAsync(sp.ticket, 0, sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return note_cuda_error(e);
+    SortParams sp = sorted_params(const_cast<void*>(sorted), items, static_cast<uint32_t>(N) * p.DG);
+    sp.ticket = ticket;   // the regions and sample numbers are only read
     auto launch = [&](auto kern, int channels) -> cudaError_t {
         uint32_t slices = 1, grid = 0;
         cudaError_t err = plan_slices(kern, channels, p, sm_count, sp, &slices, &grid);
@@ -477,7 +476,8 @@ int launch_scatter_sorted(const DcnParams& p, void* workspace, long long M, int 
         kern<<<grid, kThreadsPerCta, 0, stream>>>(p, sp, slices);
         return cudaGetLastError();
     };
-    e = p.Cd > 128 ? launch(scatter_sorted_kernel<2>, 256) : launch(scatter_sorted_kernel<1>, 128);
+    const cudaError_t e =
+        p.Cd > 128 ? launch(scatter_sorted_kernel<2>, 256) : launch(scatter_sorted_kernel<1>, 128);
     if (e != cudaSuccess) return note_cuda_error(e);
     count_launches(1);
     return MSDA_OK;

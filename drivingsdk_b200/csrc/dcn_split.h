@@ -17,12 +17,14 @@ int launch_weight_product(const float* grad_out, const float* columns, float* gr
                           const Derived& d, int sms, int* status_word, cudaStream_t stream);
 
 // Over cell-sorted samples (dcn_sorted_sm100.cu), in a workspace of sorted_bytes() (0 where the form
-// does not apply). The gather sorts, and writes the columns as fp16 pairs; the scatter works on
-// what a gather of the same samples left in the workspace. columns_f32 may be null.
+// does not apply). The gather sorts, and writes the columns as fp16 pairs; the scatter reads what a
+// gather of the same samples left in the workspace, and counts in *ticket, which must be zero (a
+// counter of its own: backward passes over one forward may run at the same time). columns_f32 may
+// be null.
 size_t sorted_bytes(const dcn_shape* s, const Derived& d);
 int launch_gather_sorted(const DcnParams& p, void* workspace, long long M, int N, uint16_t* columns,
                          size_t plane, const msda::SplitScale& bound, float* columns_f32, int sm_count,
                          cudaStream_t stream);
-int launch_scatter_sorted(const DcnParams& p, void* workspace, long long M, int N, int sm_count,
-                          cudaStream_t stream);
+int launch_scatter_sorted(const DcnParams& p, const void* sorted, uint32_t* ticket, long long M, int N,
+                          int sm_count, cudaStream_t stream);
 }  // namespace dcn

@@ -300,7 +300,7 @@ Saved plan_saved(const dcn_shape* s, const Derived& d, int dtype, bool keep) {
 }
 
 struct BackwardSpace {
-    size_t grad_columns, go_rows, go_channels, weight_t, row_most, channel_most, weight_most, total;
+    size_t ticket, grad_columns, go_rows, go_channels, weight_t, row_most, channel_most, weight_most, total;
 };
 BackwardSpace plan_backward(const dcn_shape* s, const Derived& d) {
     BackwardSpace r;
@@ -312,7 +312,8 @@ BackwardSpace plan_backward(const dcn_shape* s, const Derived& d) {
     };
     const size_t go = static_cast<size_t>(d.M) * s->Co;
     const size_t rows = static_cast<size_t>(s->groups) * d.Kd;
-    r.row_most = take(static_cast<size_t>(d.M) * 4);       // the three bounds: cleared together
+    r.ticket = take(sizeof(uint32_t));                     // with the three bounds: cleared together
+    r.row_most = take(static_cast<size_t>(d.M) * 4);
     r.channel_most = take(static_cast<size_t>(s->Co) * 4);
     r.weight_most = take(rows * 4);
     r.grad_columns = take(static_cast<size_t>(d.M) * rows * 4);
@@ -352,7 +353,7 @@ int to_nhwc(const void* src, int channels_last, float* dst, int N, int C, int P,
     return MSDA_OK;
 }
 
-void sample_params(const dcn_shape* s, const Derived& d, char* saved, const Saved& at, bool masked,
+void sample_params(const dcn_shape* s, const Derived& d, const char* saved, const Saved& at, bool masked,
                    DcnParams* p) {
     fill_params(s, d, p);
     p->x = reinterpret_cast<const float*>(saved + at.x);
@@ -433,7 +434,7 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
 }
 
 template <typename T>
-int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* saved, bool masked,
+int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const char* saved, bool masked,
                    float* grad_x, float* grad_offset, float* grad_mask, float* grad_weight, float* grad_bias,
                    char* ws, const dcn_shape* s, const Derived& d, const Saved& at, cudaStream_t stream) {
     int sms = 0;
@@ -443,7 +444,7 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* 
     const bool weight_f32 = at.f32;
     const BackwardSpace sp = plan_backward(s, d);
     const int M = static_cast<int>(d.M), HoWo = s->Ho * s->Wo;
-    uint32_t* bounds = reinterpret_cast<uint32_t*>(saved + at.bounds);
+    const uint32_t* bounds = reinterpret_cast<const uint32_t*>(saved + at.bounds);
     uint32_t* row_most = reinterpret_cast<uint32_t*>(ws + sp.row_most);
     uint32_t* channel_most = reinterpret_cast<uint32_t*>(ws + sp.channel_most);
     uint32_t* weight_most = reinterpret_cast<uint32_t*>(ws + sp.weight_most);
@@ -451,7 +452,7 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* 
     uint16_t* go_channels = reinterpret_cast<uint16_t*>(ws + sp.go_channels);
     uint16_t* weight_t = reinterpret_cast<uint16_t*>(ws + sp.weight_t);
     float* grad_columns = reinterpret_cast<float*>(ws + sp.grad_columns);
-    RETURN_ON_CUDA(cudaMemsetAsync(row_most, 0, sp.grad_columns - sp.row_most, stream));
+    RETURN_ON_CUDA(cudaMemsetAsync(ws + sp.ticket, 0, sp.grad_columns - sp.ticket, stream));
     if (grad_bias != nullptr) RETURN_ON_CUDA(cudaMemsetAsync(grad_bias, 0, static_cast<size_t>(s->Co) * 4, stream));
     RETURN_ON_CUDA(cudaMemsetAsync(grad_x, 0, static_cast<size_t>(s->N) * s->H * s->W * s->C * 4, stream));
 
@@ -498,7 +499,9 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, char* 
     p.grad_x = grad_x;
     p.grad_offset = grad_offset;
     p.grad_mask = grad_mask;
-    if (sort_pays(s, d)) rc = launch_scatter_sorted(p, saved + at.sorted, d.M, s->N, sms, stream);
+    if (sort_pays(s, d))
+        rc = launch_scatter_sorted(p, saved + at.sorted, reinterpret_cast<uint32_t*>(ws + sp.ticket), d.M, s->N, sms,
+                                   stream);
     else rc = launch_scatter(p, sms, stream);
     if (rc != MSDA_OK) return rc;
 
@@ -586,7 +589,7 @@ int dcn_sm100_backward_nchw(const void* weight, const void* grad_out, int grad_o
     if ((reinterpret_cast<uintptr_t>(saved) | reinterpret_cast<uintptr_t>(workspace) |
          reinterpret_cast<uintptr_t>(grad_x)) % 16 != 0 || reinterpret_cast<uintptr_t>(grad_offset) % 8 != 0)
         return MSDA_ERR_ALIGN;
-    char* sv = const_cast<char*>(static_cast<const char*>(saved));
+    const char* sv = static_cast<const char*>(saved);
     char* ws = static_cast<char*>(workspace);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const bool masked = grad_mask != nullptr;
