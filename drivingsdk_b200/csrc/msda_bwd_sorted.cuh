@@ -446,6 +446,11 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
                         for (int c = 0; c < 4; ++c) S4[c] = s_wide[warp][lane][c];
                     }
                 }
+                // a corner outside the map counts as zero whatever grad_out holds: its product of zeros
+                // with an infinity is not a number
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (((s.cell >> c) & 1u) == 0u) S4[c] = Acc(0);
                 const Acc lw = s.lw, lh = s.lh, wf = s.wf, hf = s.hf, a = s.a;
                 const Acc hw = Acc(1) - lw, hh = Acc(1) - lh;
                 const float ga = static_cast<float>(hh * hw * S4[0] + hh * lw * S4[1] +

@@ -1,12 +1,10 @@
-"""Infinities reach what they contribute to and nothing else: corners outside the map, and the lanes
-of a row that is narrower than they are, take no part in a gradient."""
+"""Infinities reach what they contribute to and nothing else: corners outside the map take no part in
+a gradient."""
 import pytest
 import torch
 
 from drivingsdk_b200 import capi, workloads
-from oracle import msda_oracle
 from tests import parity
-from tests.test_da_gpu import _random_case
 
 pytestmark = pytest.mark.gpu
 
