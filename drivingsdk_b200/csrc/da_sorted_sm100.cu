@@ -240,8 +240,10 @@ da_bwd_sorted_kernel(const __grid_constant__ DaParams p, const __grid_constant__
                     float tc[4];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
+                        // (a corner outside the map: zeros, whose product with an infinite grad_out
+                        // is not a number)
                         const float2 h = unpack2(t[c]);
-                        tc[c] = h.x + h.y;
+                        tc[c] = ((cell >> c) & 1u) ? h.x + h.y : 0.f;
                     }
                     d_loc[u][0] = q.wf * ((1.f - q.lh) * (tc[1] - tc[0]) + q.lh * (tc[3] - tc[2]));
                     d_loc[u][1] = q.hf * ((1.f - q.lw) * (tc[2] - tc[0]) + q.lw * (tc[3] - tc[1]));

@@ -5,6 +5,7 @@ import torch
 
 from drivingsdk_b200 import capi, workloads
 from tests import parity
+from tests.test_da_gpu import _random_case
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +37,28 @@ def test_sorted_backward_with_an_infinite_gradient(D, dtype):
     assert any(torch.isinf(g).any() for g in grads[0][1:])
     for name, want, got in zip(("value", "loc", "attn"), *grads):
         _same(name, got.float(), want.float())
+
+
+def test_sorted_aggregation_with_an_infinite_gradient():
+    c = _random_case(5, 1, 128, 9, 7, 4, [[(3, 4), (1, 2)]])
+    c["feat"], c["grad_out"] = abs(c["feat"]) + 0.1, abs(c["grad_out"]) + 0.1
+    c["wts"] = abs(c["wts"]) + 0.1
+    c["grad_out"][0, ::2, 7] = float("inf")
+    dev = {k: torch.from_numpy(c[k]).cuda() for k in c if k in ("feat", "shapes", "starts", "loc", "wts", "grad_out")}
+    lib, stream = capi.load(), torch.cuda.current_stream().cuda_stream
+    B, F, C = dev["feat"].shape
+    dims = (B, F, C, *dev["wts"].shape[1:])
+    ins = [dev[k].data_ptr() for k in ("feat", "shapes", "starts", "loc", "wts", "grad_out")]
+    results = []
+    for form in ("tasks", "sorted"):
+        grads = [torch.empty_like(dev[k]) for k in ("feat", "loc", "wts")]
+        outs = [g.data_ptr() for g in grads]
+        if form == "tasks":
+            capi.check(lib.da_sm100_backward(*ins, *outs, *dims, stream), form)
+        else:
+            ws = torch.empty(lib.da_sm100_backward_workspace_bytes(*dims), dtype=torch.uint8, device="cuda")
+            capi.check(lib.da_sm100_backward_ws(*ins, *outs, ws.data_ptr(), ws.numel(), *dims, capi.F32, stream), form)
+        results.append(grads)
+    assert torch.isinf(results[0][1]).any()
+    for name, want, got in zip(("feat", "loc", "wts"), *results):
+        _same(name, got, want)
