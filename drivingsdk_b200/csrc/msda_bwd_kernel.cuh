@@ -148,18 +148,14 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
     const LaneLevels lv = load_lane_levels(p, lane, levels_ok);
     if (!levels_ok) return;
     const T* __restrict__ value = static_cast<const T*>(p.value);
-    // this lane's pieces of a row; past the end of the row it reads the last one again, with a
-    // zero grad_out piece, and reduces nothing
-    int voff[NV];
+    // which of this lane's pieces the row has; the others are zero in both factors of a product (a
+    // piece of another lane in their place could hold an infinity) and reduce nothing
     bool on[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        on[k] = !RAGGED || j + k * LPR < p.pieces;
-        voff[k] = SCALAR ? 0 : (RAGGED ? min(j + k * LPR, p.pieces - 1) : j + k * LPR) * 16;
-    }
+    for (int k = 0; k < NV; ++k) on[k] = !RAGGED || j + k * LPR < p.pieces;
     // SPLIT_RED's two pieces
     const bool red_on[2] = {!RAGGED || j < 2 * p.pieces, !RAGGED || LPR + j < 2 * p.pieces};
-    const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + voff[0];
+    const unsigned char* vlane = static_cast<const unsigned char*>(p.value) + j * 16;
     const T* __restrict__ gout = static_cast<const T*>(p.grad_out);
     TG* __restrict__ gval = static_cast<TG*>(p.grad_value);
     unsigned char* glane = static_cast<unsigned char*>(p.grad_value) + j * 16;
@@ -311,9 +307,11 @@ msda_bwd_kernel(const __grid_constant__ Params p) {
                         for (int u = 0; u < U; ++u) {
                             const uint32_t off = (rec[u].x != kNoRow) ? rec[u].x : 0u;
 #pragma unroll
-                            for (int k = 0; k < NV; ++k)
-                                raw[u][k] =
-                                    ldg16(vlane + static_cast<size_t>(off) * 16 + (RAGGED ? voff[k] - voff[0] : k * (LPR * 16)));
+                            for (int k = 0; k < NV; ++k) {
+                                raw[u][k] = make_uint4(0u, 0u, 0u, 0u);
+                                if (on[k])
+                                    raw[u][k] = ldg16(vlane + static_cast<size_t>(off) * 16 + k * (LPR * 16));
+                            }
                         }
 #pragma unroll
                         for (int u = 0; u < U; ++u) {

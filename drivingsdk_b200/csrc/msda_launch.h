@@ -11,8 +11,8 @@ namespace msda {
 // How one value row (D elements) is spread over the lanes of a warp.
 //   scalar == false: the row is up to `lpr * nv` pieces of 16 bytes; `lpr` lanes hold
 //                    one piece each, `nv` times (nv == 2 only for rows above 512 bytes). Lanes
-//                    past the last piece (rows of 6 or 12 pieces: 24 or 48 channels) read the
-//                    last one again and write nothing.
+//                    past the last piece (rows of 6 or 12 pieces: 24 or 48 channels) write
+//                    nothing; the forward's read the last one again, the backward's nothing.
 //   scalar == true : lane = channel mod 32, any D up to 256, no alignment need.
 struct RowPlan {
     bool scalar;

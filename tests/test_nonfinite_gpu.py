@@ -1,5 +1,5 @@
-"""Infinities reach what they contribute to and nothing else: corners outside the map take no part in
-a gradient."""
+"""Infinities reach what they contribute to and nothing else: corners outside the map, and the lanes
+of a row that is narrower than they are, take no part in a gradient."""
 import pytest
 import torch
 
@@ -62,3 +62,37 @@ def test_sorted_aggregation_with_an_infinite_gradient():
     assert torch.isinf(results[0][1]).any()
     for name, want, got in zip(("feat", "loc", "wts"), *results):
         _same(name, got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("fused", [False, True])
+def test_rows_that_leave_lanes_idle_with_an_infinite_value(dtype, fused):
+    """An infinity in the last piece of a row: the row's own product with grad_out decides."""
+    import drivingsdk_b200 as sdk
+    D = 24
+    w = workloads.Workload("inf", 1, 40, 2, D, ((3, 4), (2, 2)), 4, (0.2, 0.8), seed=3)
+    dev = parity.to_device(workloads.make_inputs(w, dtype), dtype)
+    value = dev["value"].abs() + 0.1
+    value[0, 5, 0, D - 1] = float("inf")
+    go = torch.ones(1, 40, 2 * D, dtype=dtype, device="cuda")
+    call = sdk.multi_scale_deformable_attn
+    rest = [dev["loc"], dev["attn"]]
+    if fused:
+        call = sdk.multi_scale_deformable_attn_fused
+        rest = [torch.full((1, 40, 2, 2), 0.5, dtype=dtype, device="cuda"),
+                ((dev["loc"].float() - 0.5) * 3).to(dtype), dev["attn"]]
+    grads = []
+    for odd in (True, False):   # at an odd address: channel by channel, no idle lanes
+        v = value
+        if odd:
+            v = torch.empty(value.numel() + 1, dtype=dtype, device="cuda")[1:].view(value.shape).copy_(value)
+        old = capi.load().msda_sm100_tune(capi.TUNE_SORT, 0)
+        try:
+            ts = [t.detach().requires_grad_() for t in (v, *rest)]
+            out = call(ts[0], dev["shapes"], dev["starts"], *ts[1:])
+            grads.append([g.float() for g in torch.autograd.grad(out, ts, go)])
+        finally:
+            capi.load().msda_sm100_tune(capi.TUNE_SORT, old)
+    assert not torch.isfinite(grads[0][-1]).all()
+    for i, (want, got) in enumerate(zip(*grads)):
+        _same(i, got, want)
