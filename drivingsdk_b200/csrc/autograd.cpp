@@ -111,7 +111,7 @@ struct Gka : Function<Gka> {
     static Tensor forward(AutogradContext* ctx, Tensor value, Tensor shapes, Tensor starts,
                           Tensor loc, Tensor attn) {
         TORCH_CHECK(value.dim() == 4, "geometric_kernel_attention: value [bs, keys, heads, dims] expected");
-        // written in full by the kernel
+        // written in full by the kernel, with zeros if it refuses a level table
         Tensor out = at::empty({value.size(0), attn.size(1), value.size(2) * value.size(3)}, value.options());
         geometric_kernel_attention_forward(value, shapes, starts, loc, attn, out);
         ctx->save_for_backward({value, shapes, starts, loc, attn});

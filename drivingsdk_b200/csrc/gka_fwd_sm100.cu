@@ -27,7 +27,10 @@ gka_map_fwd_kernel(const __grid_constant__ Params p, const uint32_t slices, cons
     constexpr uint32_t TASKS = 32 / LPR;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ SortLevels lv;
-    if (!load_sort_levels(p, lv)) return;
+    if (!load_sort_levels(p, lv)) {
+        clear_output<T>(p);
+        return;
+    }
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const uint32_t g = lane / LPR, j = lane % LPR;
     const uint32_t Q = p.Q, H = p.H, LP = p.LP;

@@ -60,7 +60,10 @@ msda_fwd_kernel(const __grid_constant__ Params p) {
 
     bool levels_ok;
     const LaneLevels lv = load_lane_levels(p, lane, levels_ok);
-    if (!levels_ok) return;
+    if (!levels_ok) {
+        if constexpr (MODE == kModeNearest) clear_output<T>(p);
+        return;
+    }
     const T* __restrict__ value = static_cast<const T*>(p.value);
     // this lane's pieces of a row; past the end of the row it reads the last one again
     int voff[NV];

@@ -102,6 +102,16 @@ __device__ __forceinline__ bool device_level_table_ok(const Params& p) {
     return !any;
 }
 
+// Zeros for all of the output, by all threads of the grid: what the nearest-pixel operator returns for
+// a refused table (its memory would otherwise show what an earlier tensor left there).
+template <typename T>
+__device__ __forceinline__ void clear_output(const Params& p) {
+    T* out = static_cast<T*>(p.out);
+    const long long n = p.ntasks * p.D, step = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += step)
+        out[i] = Elem<T>::from_f(0.f);
+}
+
 // The sequence of items one warp walks through: warp w of CTA c takes items c*8 + w, then
 // + gridDim*8, ... (a CTA's eight warps hold eight consecutive tasks, i.e. with eight heads all
 // heads of one query).

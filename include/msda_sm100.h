@@ -175,7 +175,8 @@ int msda_sm100_fused_backward_ws(const void* value, const int32_t* spatial_shape
  * device kernel kernels/geometric_kernel_attention/op_kernel/geometric_kernel_attention.cpp).
  * Same layouts as above, but sampling_locations holds PIXEL coordinates (x, y) of each
  * level (in `dtype`), which are truncated to integers and clamped into the level:
- *   output[b,q,h,:] = sum_{l,p} attention[b,q,h,l,p] * value[b, start_l + y*W_l + x, h, :]. */
+ *   output[b,q,h,:] = sum_{l,p} attention[b,q,h,l,p] * value[b, start_l + y*W_l + x, h, :].
+ * All of output is zero where a level table in device memory is refused. */
 int gka_sm100_forward(const void* value, const int32_t* spatial_shapes,
                       const int32_t* level_start_index, const void* sampling_locations,
                       const void* attention_weights, void* output, int B, int K, int H, int D,

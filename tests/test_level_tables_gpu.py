@@ -1,6 +1,9 @@
-"""Level tables that the operators refuse, on the host before anything is launched."""
+"""Level tables that the operators refuse: on the host before anything is launched, or in the kernel
+where the host cannot read them."""
 import pytest
 import torch
+
+from drivingsdk_b200 import capi
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +41,22 @@ def test_exported_functions_take_int32_tables(kind):
         for place in ("cuda", "cpu"):
             with pytest.raises(RuntimeError, match="int32 tensor expected"):
                 call(*(t.to(place) for t in _tables(kind)))
+
+
+@pytest.mark.parametrize("Q", [5, 4000], ids=["gather", "map"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_refused_table_leaves_zeros(Q, dtype):
+    """geometric_kernel_attention's output is zero where the kernel refuses the table (its memory
+    is not what an earlier tensor left there)."""
+    import drivingsdk_b200 as sdk
+    value = torch.ones(2, 12, 4, 64, device="cuda", dtype=dtype)
+    attn = torch.ones(2, Q, 4, 1, 15, device="cuda", dtype=dtype)
+    loc = torch.zeros(2, Q, 4, 1, 15, 2, device="cuda", dtype=dtype)
+    shapes = torch.tensor([[100, 100]], device="cuda")   # more pixels than there are keys
+    starts = torch.zeros(1, dtype=torch.int64, device="cuda")
+    assert capi.load().msda_sm100_device_status(1) == 0
+    stale = torch.full((2, Q, 256), 7.0, device="cuda", dtype=dtype)
+    del stale
+    out = sdk.geometric_kernel_attention(value, shapes, starts, loc, attn)
+    assert capi.load().msda_sm100_device_status(1) == 4
+    assert not out.any()
