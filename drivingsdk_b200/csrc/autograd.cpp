@@ -5,9 +5,12 @@
 // to them in drivingsdk_b200/ops (which callers may still subclass, patch or apply):
 //   * under autocast the attention operators run in float32 on cast inputs;
 //   * an empty operand raises the reference's Exception;
-//   * gradients are once-differentiable: using them in a graph raises.
+//   * gradients are once-differentiable: using them in a graph raises;
+//   * while torch.jit.trace records, the calls go through those classes, which the tracer sees (a
+//     call that it does not see becomes a constant: the result for the example input).
 #include <ATen/autocast_mode.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include "bindings.h"
@@ -256,23 +259,44 @@ struct MaxPool : Function<MaxPool> {
     }
 };
 
+// `apply` of a Python class in drivingsdk_b200/ops.
+template <typename... Args>
+Tensor apply_class(const char* module, const char* name, const Args&... args) {
+    pybind11::gil_scoped_acquire gil;
+    const std::string path = std::string("drivingsdk_b200.ops.") + module;
+    return pybind11::module_::import(path.c_str()).attr(name).attr("apply")(args...).template cast<Tensor>();
+}
+using torch::jit::tracer::isTracing;
+
 Tensor msda(const Tensor& value, const Tensor& shapes, const Tensor& starts, const Tensor& loc,
             const Tensor& attn) {
+    if (isTracing())
+        return apply_class("multi_scale_deformable_attn", "MultiScaleDeformableAttnFunction", value, shapes,
+                           starts, loc, attn);
     return Msda::apply(value, shapes, starts, loc, attn);
 }
 Tensor fused(const Tensor& value, const Tensor& shapes, const Tensor& starts, const Tensor& ref,
              const Tensor& off, const Tensor& logits) {
+    if (isTracing())
+        return apply_class("msda_fused", "MultiScaleDeformableAttnFusedFunction", value, shapes, starts, ref, off,
+                           logits);
     return Fused::apply(value, shapes, starts, ref, off, logits);
 }
 Tensor gka(const Tensor& value, const Tensor& shapes, const Tensor& starts, const Tensor& loc,
            const Tensor& attn) {
+    if (isTracing())
+        return apply_class("geometric_kernel_attention", "GeometricKernelAttentionFunc", value, shapes, starts,
+                           loc, attn);
     return Gka::apply(value, shapes, starts, loc, attn);
 }
 Tensor aggregation(const Tensor& feat, const Tensor& shape, const Tensor& start, const Tensor& loc,
                    const Tensor& wts) {
+    if (isTracing())
+        return apply_class("npu_deformable_aggregation", "AdsDeformableAggregation", feat, shape, start, loc, wts);
     return Aggregation::apply(feat, shape, start, loc, wts);
 }
 Tensor add_relu(const Tensor& x, const Tensor& y) {
+    if (isTracing()) return apply_class("npu_add_relu", "AddReluFunction", x, y);
     const bool in_place = x.numel() >= kInPlaceMinNumel && x.is_contiguous() &&
                           !(x.is_leaf() && x.requires_grad());
     return AddRelu::apply(x, y, in_place);
@@ -287,12 +311,18 @@ bool any_requires_grad(at::TensorList ts) {
 }
 Tensor deform_conv(const Tensor& x, const Tensor& offset, const Tensor& weight, const Pair& stride,
                    const Pair& padding, const Pair& dilation, int64_t groups, int64_t deformable_groups) {
+    if (isTracing())
+        return apply_class("deform_conv2d", "DeformConv2dFunction", x, offset, weight, stride, padding, dilation,
+                           groups, deformable_groups);
     return DeformConv::apply(x, offset, std::optional<Tensor>(), weight, std::optional<Tensor>(), stride, padding, dilation, groups,
                              deformable_groups, any_requires_grad({x, offset, weight}));
 }
 Tensor modulated_deform_conv(const Tensor& x, const Tensor& offset, const Tensor& mask, const Tensor& weight,
                              const c10::optional<Tensor>& bias, const Pair& stride, const Pair& padding,
                              const Pair& dilation, int64_t groups, int64_t deformable_groups) {
+    if (isTracing())
+        return apply_class("modulated_deform_conv2d", "ModulatedDeformConv2dFunction", x, offset, mask, weight, bias,
+                           stride, padding, dilation, groups, deformable_groups);
     // custom_fwd(cast_inputs=torch.float32), the casts outside the function so that gradients
     // return through them
     const bool cast = at::autocast::is_autocast_enabled(at::kCUDA);
@@ -303,6 +333,7 @@ Tensor modulated_deform_conv(const Tensor& x, const Tensor& offset, const Tensor
                              dilation, groups, deformable_groups, any_requires_grad({x, offset, mask, weight, b}));
 }
 Tensor max_pool2d(const Tensor& x, int64_t kernel, int64_t stride, int64_t padding) {
+    if (isTracing()) return apply_class("npu_max_pool2d", "MaxPool2d", x, kernel, stride, padding);
     return MaxPool::apply(x, kernel, stride, padding);
 }
 

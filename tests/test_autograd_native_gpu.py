@@ -65,3 +65,34 @@ def test_add_relu_in_place_under_autograd():
     assert out.data_ptr() == x.data_ptr()
     gx, gy = torch.autograd.grad(out.sum(), (base, y))
     assert torch.equal(gx, (out > 0).float()) and torch.equal(gx, gy)
+
+
+def _traced_calls():
+    import drivingsdk_b200 as sdk
+    shapes, starts, (v, l, a) = _leaves()
+    r = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    yield "msda", lambda v, l, a: sdk.multi_scale_deformable_attn(v, shapes, starts, l, a), (v, l, a)
+    off, ref = r(*l.shape), torch.rand(l.shape[0], l.shape[1], l.shape[3], 2, device="cuda")
+    yield "fused", lambda v, f, o, a: sdk.multi_scale_deformable_attn_fused(v, shapes, starts, f, o, a), \
+        (v, ref, off, a)
+    tables = torch.tensor([[4, 5]], device="cuda"), torch.tensor([0], device="cuda")
+    loc = torch.randint(0, 4, (1, 6, 2, 1, 3, 2), device="cuda").float()
+    yield "gka", lambda v, a: sdk.geometric_kernel_attention(v, *tables, loc, a), (r(1, 20, 2, 8), r(1, 6, 2, 1, 3))
+    maps = torch.tensor([[[4, 5]]], device="cuda"), torch.tensor([[0]], device="cuda")
+    yield "da", lambda f, l, w: sdk.deformable_aggregation(f, *maps, l, w), \
+        (r(1, 20, 32), torch.rand(1, 3, 2, 1, 2, device="cuda"), r(1, 3, 2, 1, 1, 8))
+    conv = r(1, 8, 5, 5), r(1, 18, 5, 5), r(8, 8, 3, 3)
+    yield "dcn", lambda x, o, w: sdk.deform_conv2d(x, o, w, 1, 1), conv
+    yield "mdcn", lambda x, o, m, w, b: sdk.modulated_deform_conv2d(x, o, m, w, b, 1, 1), \
+        (conv[0], conv[1], r(1, 9, 5, 5), conv[2], r(8))
+    yield "add_relu", sdk.npu_add_relu, (r(3, 7), r(3, 7))
+    yield "max_pool", lambda x: sdk.npu_max_pool2d(x, 3, 2, 1), (r(1, 2, 9, 9),)
+
+
+def test_traced_operators_follow_their_inputs():
+    """torch.jit.trace: the operators are in the graph, and not their results for the example."""
+    for name, fn, args in _traced_calls():
+        args = tuple(t.detach() for t in args)
+        traced = torch.jit.trace(fn, args, check_trace=False)
+        others = tuple(t.roll(1, 0) * 0.9 for t in args)
+        torch.testing.assert_close(traced(*others), fn(*others), msg=lambda m, n=name: f"{n}: {m}")
