@@ -531,7 +531,11 @@ int split_shape(const dcn_shape* s, Derived* d) {
     if (rc != MSDA_OK) return rc;
     // 16-byte pieces of halves in every row
     if (d->Cg % 8 != 0 || d->Cd % 8 != 0 || d->Cog % 8 != 0) return MSDA_ERR_ALIGN;
-    return dcn_sm100_use_tensor_cores(-1) == 1 ? MSDA_OK : MSDA_ERR_LIMIT;
+    // images (or groups) and blocks of channels are the y and z of the layout kernels' grids
+    constexpr int kGrid = 65535;
+    const long long taps = static_cast<long long>(s->deform_groups) * d->K;
+    return s->N <= kGrid && s->groups <= kGrid && s->C / 32 < kGrid && s->Co / 64 < kGrid && 2 * taps / 32 < kGrid
+               ? MSDA_OK : MSDA_ERR_LIMIT;
 }
 
 }  // namespace
@@ -540,7 +544,8 @@ extern "C" {
 
 size_t dcn_sm100_saved_bytes(const dcn_shape* s, int dtype, int keep) {
     Derived d;
-    return split_shape(s, &d) == MSDA_OK ? plan_saved(s, d, dtype, keep != 0).total : 0;
+    return split_shape(s, &d) == MSDA_OK && dcn_sm100_use_tensor_cores(-1) == 1
+               ? plan_saved(s, d, dtype, keep != 0).total : 0;
 }
 
 size_t dcn_sm100_nchw_workspace_bytes(const dcn_shape* s, int dtype, int keep, int backward) {
@@ -558,6 +563,7 @@ int dcn_sm100_forward_nchw(const void* x, int x_nhwc, const void* offset, const 
     Derived d;
     const int rc = split_shape(s, &d);
     if (rc != MSDA_OK) return rc;
+    if (dcn_sm100_use_tensor_cores(-1) != 1) return MSDA_ERR_LIMIT;
     const Saved at = plan_saved(s, d, dtype, keep != 0);
     if (saved_bytes < at.total || workspace_bytes < plan_forward(s, d, at).total)
         return MSDA_ERR_WORKSPACE;
@@ -582,9 +588,8 @@ int dcn_sm100_backward_nchw(const void* weight, const void* grad_out, int grad_o
         grad_offset == nullptr || grad_weight == nullptr || workspace == nullptr)
         return MSDA_ERR_NULL;
     Derived d;
-    int rc = check_shape(s, &d);
+    const int rc = split_shape(s, &d);
     if (rc != MSDA_OK) return rc;
-    if (d.Cg % 8 != 0 || d.Cd % 8 != 0 || d.Cog % 8 != 0) return MSDA_ERR_ALIGN;
     if (workspace_bytes < plan_backward(s, d).total) return MSDA_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(saved) | reinterpret_cast<uintptr_t>(workspace) |
          reinterpret_cast<uintptr_t>(grad_x)) % 16 != 0 || reinterpret_cast<uintptr_t>(grad_offset) % 8 != 0)

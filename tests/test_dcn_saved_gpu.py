@@ -32,3 +32,22 @@ def test_backward_only_reads_what_the_forward_saved():
     capi.check(lib.dcn_sm100_backward_nchw(w.data_ptr(), go.data_ptr(), 0, *ptr(saved, gx, goff, gmask, gw), None,
                                            ws.data_ptr(), ws.numel(), ref, 0, stream), "backward")
     assert torch.equal(saved, before)
+
+
+def test_more_images_than_a_grid_has_planes():
+    import drivingsdk_b200 as sdk
+    N = 65537
+    x, off = torch.randn(N, 8, 2, 2, device="cuda"), torch.randn(N, 18, 2, 2, device="cuda")
+    w = torch.randn(8, 8, 3, 3, device="cuda")
+    ts = [t.requires_grad_() for t in (x, off, w)]
+    out = sdk.deform_conv2d(*ts, 1, 1)
+    go = torch.randn_like(out)
+    got = torch.autograd.grad(out, ts, go)
+    parts = []
+    for half in (slice(0, 30000), slice(30000, N)):
+        p = [x.detach()[half].requires_grad_(), off.detach()[half].requires_grad_(), w.detach().requires_grad_()]
+        o = sdk.deform_conv2d(*p, 1, 1)
+        parts.append((o.detach(), *torch.autograd.grad(o, p, go[half])))
+    want = [torch.cat([a[i] for a in parts]) for i in range(3)] + [parts[0][3] + parts[1][3]]
+    for a, b in zip((out, *got), want):
+        assert (a - b).norm() <= 1e-5 * b.norm()
