@@ -209,6 +209,13 @@ inline int balanced_splits(long long tiles, int sms, int max_splits) {
     return best;
 }
 
+// Parts into which the columns are cut for the forward product: more than one where there are few
+// output tiles (small batches), so that every SM has work.
+inline int forward_splits(const Derived& d, int sms) {
+    const long long tiles = ((d.M + 127) / 128) * static_cast<long long>((d.Cog + 255) / 256);
+    return 2 * tiles <= sms ? balanced_splits(tiles, sms, (d.Kd + 255) / 256) : 1;
+}
+
 // Parts into which the pixels are cut for the grad_weight product.
 inline int weight_splits(const Derived& d, int sms) {
     const long long tiles = ((d.Cog + 127) / 128) * static_cast<long long>((d.Kd + 255) / 256);

@@ -236,16 +236,53 @@ int public_product(const float* A, long long a_row, long long a_k, const float* 
 }  // namespace
 
 namespace dcn {
+// out[m, co] = sum over kd of columns[m, g, kd] * weight[co, kd] (+ bias[co])
+int launch_forward_product(const float* columns, const float* weight, const float* bias, float* out,
+                           const dcn_shape* s, const Derived& d, int sms, const msda::RangeGate& gate,
+                           int* status_word, cudaStream_t stream) {
+    const long long ld_cols = static_cast<long long>(s->groups) * d.Kd;
+    bool zeroed = gate.range[0] != nullptr;
+    for (int g = 0; g < s->groups; ++g) {
+        msda::GemmArgs a{};
+        a.A = columns + static_cast<size_t>(g) * d.Kd;
+        a.a_row = ld_cols;
+        a.a_k = 1;
+        a.B = weight + static_cast<size_t>(g) * d.Cog * d.Kd;
+        a.b_row = d.Kd;
+        a.b_k = 1;
+        a.C = out + static_cast<size_t>(g) * d.Cog;
+        a.ldc = s->Co;
+        a.bias = bias ? bias + static_cast<size_t>(g) * d.Cog : nullptr;
+        a.M = static_cast<int>(d.M);
+        a.N = d.Cog;
+        a.K = d.Kd;
+        a.gate = gate;
+        int splits = 1;
+        if (g_use_tc.load(std::memory_order_relaxed) != 0 && msda::gemm_tc_supported(a)) {
+            splits = forward_splits(d, sms);
+            if (splits > 1 && !zeroed) {
+                const cudaError_t e = cudaMemsetAsync(out, 0, static_cast<size_t>(d.M) * s->Co * 4, stream);
+                if (e != cudaSuccess) return msda::note_cuda_error(e);
+                zeroed = true;
+            }
+        }
+        const int rc = product(a, splits, status_word, stream);
+        if (rc != MSDA_OK) return rc;
+    }
+    return MSDA_OK;
+}
+
 // grad_weight[co, kd] = sum over m of grad_out[m, co] * columns[m, g, kd]: both operands are stored
 // pixel row by pixel row, i.e. with the row index (co, kd) contiguous and k = m strided. The
 // tensor-core kernel takes that form directly (K cut over CTAs so that every SM has work);
 // operands that miss its alignment rules go to the FMA kernel.
 int launch_weight_product(const float* grad_out, const float* columns, float* grad_weight, const dcn_shape* s,
-                          const Derived& d, int sms, int* status_word, cudaStream_t stream) {
+                          const Derived& d, int sms, const msda::RangeGate& gate, int* status_word,
+                          cudaStream_t stream) {
     const long long ld_cols = static_cast<long long>(s->groups) * d.Kd;
     const int M = static_cast<int>(d.M);
     const bool tc = g_use_tc.load(std::memory_order_relaxed) != 0;
-    bool zeroed = false;
+    bool zeroed = gate.range[0] != nullptr;
     for (int g = 0; g < s->groups; ++g) {
         msda::GemmArgs a{};
         a.A = grad_out + static_cast<size_t>(g) * d.Cog;
@@ -259,6 +296,7 @@ int launch_weight_product(const float* grad_out, const float* columns, float* gr
         a.M = d.Cog;
         a.N = d.Kd;
         a.K = M;
+        a.gate = gate;
         int splits = 1;
         if (tc && msda::gemm_tc_supported(a)) {
             splits = weight_splits(d, sms);
@@ -336,37 +374,7 @@ int dcn_sm100_forward(const float* x, const float* offset, const float* mask, co
     rc = launch_sample<false>(p, piece_width(s, d), sms, stream);
     if (rc != MSDA_OK) return rc;
 
-    const long long ld_cols = static_cast<long long>(s->groups) * d.Kd;
-    bool zeroed = false;
-    for (int g = 0; g < s->groups; ++g) {
-        msda::GemmArgs a{};
-        a.A = columns + static_cast<size_t>(g) * d.Kd;
-        a.a_row = ld_cols;
-        a.a_k = 1;
-        a.B = weight + static_cast<size_t>(g) * d.Cog * d.Kd;
-        a.b_row = d.Kd;
-        a.b_k = 1;
-        a.C = out + static_cast<size_t>(g) * d.Cog;
-        a.ldc = s->Co;
-        a.bias = bias ? bias + static_cast<size_t>(g) * d.Cog : nullptr;
-        a.M = static_cast<int>(d.M);
-        a.N = d.Cog;
-        a.K = d.Kd;
-        // few output tiles (small batches): cut K so that every SM has work
-        int splits = 1;
-        if (g_use_tc.load(std::memory_order_relaxed) != 0 && msda::gemm_tc_supported(a)) {
-            const long long tiles = ((d.M + 127) / 128) * static_cast<long long>((d.Cog + 255) / 256);
-            if (2 * tiles <= sms) splits = balanced_splits(tiles, sms, (d.Kd + 255) / 256);
-            if (splits > 1 && !zeroed) {
-                const cudaError_t e = cudaMemsetAsync(out, 0, static_cast<size_t>(d.M) * s->Co * 4, stream);
-                if (e != cudaSuccess) return msda::note_cuda_error(e);
-                zeroed = true;
-            }
-        }
-        rc = product(a, splits, status_word, stream);
-        if (rc != MSDA_OK) return rc;
-    }
-    return MSDA_OK;
+    return launch_forward_product(columns, weight, bias, out, s, d, sms, msda::RangeGate{}, status_word, stream);
 }
 
 int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
@@ -450,7 +458,7 @@ int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
     if (rc != MSDA_OK) return rc;
 
     // 3. grad_weight
-    rc = launch_weight_product(grad_out, columns, grad_weight, s, d, sms, status_word, stream);
+    rc = launch_weight_product(grad_out, columns, grad_weight, s, d, sms, msda::RangeGate{}, status_word, stream);
     if (rc != MSDA_OK) return rc;
 
     // 4. grad_bias

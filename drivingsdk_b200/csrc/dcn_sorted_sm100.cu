@@ -143,16 +143,16 @@ struct LaneSlice {
     }
 };
 
-// Forward. The bound of the columns gives the scale of the pairs.
+// Forward. The bound of the columns gives the scale of the pairs, their range the form.
 template <int NV>
 __global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 3 : 4)
 gather_sorted_kernel(const __grid_constant__ DcnParams p, const __grid_constant__ SortParams sp,
-                     uint32_t slices, uint16_t* __restrict__ columns, size_t plane, const SplitScale bound,
-                     float* __restrict__ columns_f32) {
+                     uint32_t slices, const __grid_constant__ ColumnsOut out) {
     __shared__ __align__(16) Record s_rec[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t units = static_cast<uint32_t>(p.C) / 4, step_y = static_cast<uint32_t>(p.W) * units;
-    const float scale = exp2_int(split_exponent(bound, 0));
+    const float scale = exp2_int(split_exponent(out.bound, 0));
+    const bool pairs = !range_is_wide(out.range), plain = !pairs || out.keep_f32;
 
     Ticket ticket;
     uint32_t region, slice;
@@ -227,11 +227,13 @@ gather_sorted_kernel(const __grid_constant__ DcnParams p, const __grid_constant_
                     }
                     if (ls.on[k]) {
                         const size_t to_at = (static_cast<size_t>(q.columns) + ls.column_at[k]) * 4;
-                        uint16_t* to = columns + to_at;
-                        *reinterpret_cast<uint2*>(to) = make_uint2(part[0].x, part[1].x);
-                        *reinterpret_cast<uint2*>(to + plane) = make_uint2(part[0].y, part[1].y);
-                        if (columns_f32 != nullptr)
-                            *reinterpret_cast<float4*>(columns_f32 + to_at) =
+                        if (pairs) {
+                            uint16_t* to = out.pairs + to_at;
+                            *reinterpret_cast<uint2*>(to) = make_uint2(part[0].x, part[1].x);
+                            *reinterpret_cast<uint2*>(to + out.plane) = make_uint2(part[0].y, part[1].y);
+                        }
+                        if (plain)
+                            *reinterpret_cast<float4*>(out.f32 + to_at) =
                                 make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
                     }
                 }
@@ -439,9 +441,8 @@ cudaError_t plan_slices(Kernel kern, int channels, const DcnParams& p, int sm_co
     return e;
 }
 
-int launch_gather_sorted(const DcnParams& p, void* workspace, long long M, int N, uint16_t* columns,
-                         size_t plane, const SplitScale& bound, float* columns_f32, int sm_count,
-                         cudaStream_t stream) {
+int launch_gather_sorted(const DcnParams& p, void* workspace, long long M, int N, const ColumnsOut& to,
+                         int sm_count, cudaStream_t stream) {
     const uint32_t maps = static_cast<uint32_t>(N) * p.DG;
     SortParams sp = sorted_params(workspace, static_cast<size_t>(M) * p.DG * p.K, maps);
     cudaError_t e = launch_sort(ConvSamples{p, static_cast<uint32_t>(p.HoWo) * p.K}, maps, sp, sm_count, stream);
@@ -450,7 +451,7 @@ int launch_gather_sorted(const DcnParams& p, void* workspace, long long M, int N
         uint32_t slices = 1, grid = 0;
         const cudaError_t err = plan_slices(kern, channels, p, sm_count, sp, &slices, &grid);
         if (err != cudaSuccess) return err;
-        kern<<<grid, kThreadsPerCta, 0, stream>>>(p, sp, slices, columns, plane, bound, columns_f32);
+        kern<<<grid, kThreadsPerCta, 0, stream>>>(p, sp, slices, to);
         return cudaGetLastError();
     };
     e = p.Cd > 128 ? launch(gather_sorted_kernel<2>, 256) : launch(gather_sorted_kernel<1>, 128);

@@ -6,7 +6,10 @@
 //   backward  bounds and pairs of grad_out, once scaled by pixel (its rows in the product that
 //             gives grad_columns) and once by channel (its rows in grad_weight); transposed weight
 //             pairs; grad_columns; scatter; grad_weight = grad_out^T x columns
-// The column pairs take the bytes that the fp32 columns would.
+// The column pairs take the bytes that the fp32 columns would. Where x and the mask, or grad_out, spread
+// too wide for pairs (range_gate.h) the columns, weights and grad_out are written in fp32 instead, into
+// the same memory, and the products over TF32 pairs of dcn_sm100.cu take over; otherwise those return at
+// once (some 2 us each).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -22,6 +25,8 @@ namespace {
 using namespace dcn;
 using msda::SplitOperand;
 using msda::SplitScale;
+using msda::RangeGate;
+using msda::gate_open;
 using msda::Elem;
 
 // A tile of a [n][channels][pixels] tensor (or [n][pixels][channels]: channels_last) in shared
@@ -54,32 +59,49 @@ __device__ __forceinline__ void raise_max(uint32_t* at, uint32_t v) {
     if (v > *reinterpret_cast<volatile uint32_t*>(at)) atomicMax(at, v);
 }
 
-// [n][C][P] (or channels last) in T -> [n][P][C] in fp32; optionally the largest magnitude.
+// kLeastFrom minus a block's maximum: the larger, the smaller the maximum; 0 for a block of zeros.
+__device__ __forceinline__ uint32_t smallness(uint32_t most) { return most == 0u ? 0u : msda::kLeastFrom - most; }
+
+// [n][C][P] (or channels last) in T -> [n][P][C] in fp32; optionally its range (range_gate.h): the
+// largest magnitude into range[0], the smallness of the block maxima into range[2].
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 to_nhwc_kernel(const T* __restrict__ src, int channels_last, float* __restrict__ dst, int C, int P,
-               uint32_t* magnitude) {
+               uint32_t* range) {
     __shared__ float tile[32][33];
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32, n = blockIdx.z;
     load_tile<T, 32>(src, channels_last, n, c0, p0, C, P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t most = 0;
+    uint32_t most = 0, small = 0;   // of this lane's channel; of this warp's pixels
 #pragma unroll
     for (int u = 0; u < 1024 / kThreads; ++u) {
         const int r = warp + u * (kThreads / 32);
         const int p = p0 + r, c = c0 + lane;
         const float v = tile[lane][r];
-        most = max(most, msda::finite_magnitude(v));
         if (p < P && c < C) dst[(static_cast<size_t>(n) * P + p) * C + c] = v;
+        if (range != nullptr) {
+            const uint32_t a = msda::finite_magnitude(v);
+            most = max(most, a);
+            small = max(small, smallness(__reduce_max_sync(0xffffffffu, a)));
+        }
     }
-    if (magnitude != nullptr) {
-        __shared__ uint32_t warp_most[kThreads / 32];
-        most = __reduce_max_sync(0xffffffffu, most);
-        if (lane == 0) warp_most[warp] = most;
+    if (range != nullptr) {
+        __shared__ uint32_t warp_most[kThreads / 32][32], warp_small[kThreads / 32];
+        warp_most[warp][lane] = most;
+        if (lane == 0) warp_small[warp] = small;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < kThreads / 32; ++w) most = max(most, warp_most[w]);
-            raise_max(magnitude, most);
+        if (warp == 0) {
+            for (int w = 1; w < kThreads / 32; ++w) {
+                most = max(most, warp_most[w][lane]);
+                small = max(small, warp_small[w]);
+            }
+            // single elements are often small: a channel counts with eight pixels or more
+            if (P - p0 >= 8) small = max(small, __reduce_max_sync(0xffffffffu, smallness(most)));
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (lane == 0) {
+                raise_max(range, most);
+                raise_max(range + 2, small);
+            }
         }
     }
 }
@@ -94,11 +116,12 @@ struct RowOrder {
     }
 };
 
-// Largest magnitudes of a [n][C][P] tensor per row (pixel) and per channel, and the channel sums.
+// Largest magnitudes of a [n][C][P] tensor per row (pixel) and per channel, and the channel sums;
+// optionally its range, over blocks of 64 channels of a pixel.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
-              uint32_t* row_most, uint32_t* channel_most, float* channel_sum) {
+              uint32_t* row_most, uint32_t* channel_most, float* channel_sum, uint32_t* range) {
     __shared__ float tile[64][33];
     __shared__ uint32_t part[kThreads / 32][32];
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
@@ -130,19 +153,32 @@ bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder orde
     }
     part[warp][lane] = mine;
     __syncthreads();
-    if (warp == 0 && p0 + lane < order.P) {
+    if (warp == 0) {
         for (int w = 1; w < kThreads / 32; ++w) mine = max(mine, part[w][lane]);
-        raise_max(row_most + order.row(n, p0 + lane), mine);
+        if (p0 + lane < order.P) raise_max(row_most + order.row(n, p0 + lane), mine);
+        if (range != nullptr) {
+            const uint32_t small = __reduce_max_sync(0xffffffffu, smallness(mine));
+            const uint32_t tile_most = __reduce_max_sync(0xffffffffu, mine);
+            if (lane == 0) {
+                raise_max(range, tile_most);
+                raise_max(range + 2, small);
+            }
+        }
     }
 }
 
-// [n][C][P] -> pairs [rows][C] scaled by row, and (optional) the same scaled by channel or in fp32.
+// [n][C][P] -> pairs [rows][C] scaled by row, and (optional) the same scaled by channel or in fp32:
+// where both are given, in fp32 if the gate is open.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 pairs_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
              const uint32_t* row_most, const uint32_t* channel_most, uint16_t* __restrict__ by_row,
-             uint16_t* __restrict__ by_channel, float* __restrict__ plain, size_t plane) {
+             uint16_t* by_channel, float* plain, size_t plane, const RangeGate if_plain) {
     __shared__ float tile[64][33];
+    if (by_channel != nullptr && plain != nullptr) {
+        if (gate_open(if_plain)) by_channel = nullptr;
+        else plain = nullptr;
+    }
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
     load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -173,14 +209,23 @@ pairs_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order
     }
 }
 
-// weight [Co][Cg][K] -> pairs [Co][K * Cg], one CTA per output channel, scaled by it.
+// weight [Co][Cg][K] -> pairs [Co][K * Cg], one CTA per output channel, scaled by it; or in fp32, into
+// the same memory, where the columns' range is wide.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 weight_pairs_kernel(const T* __restrict__ w, int Cg, int K, uint32_t* most, uint16_t* __restrict__ pairs,
-                    size_t plane) {
+                    size_t plane, const uint32_t* columns_range) {
     __shared__ uint32_t warp_most[kThreads / 32];
     const int co = blockIdx.x, Kd = Cg * K;
     const T* src = w + static_cast<size_t>(co) * Kd;
+    if (msda::range_is_wide(columns_range)) {
+        float* to = reinterpret_cast<float*>(pairs) + static_cast<size_t>(co) * Kd;
+        for (int i = threadIdx.x; i < Kd; i += kThreads) {
+            const int k = i / Cg, c = i - k * Cg;
+            to[i] = Elem<T>::to_f(src[c * K + k]);
+        }
+        return;
+    }
     uint32_t m = 0;
     for (int i = threadIdx.x; i < Kd; i += kThreads) m = max(m, msda::finite_magnitude(Elem<T>::to_f(src[i])));
     m = __reduce_max_sync(0xffffffffu, m);
@@ -202,13 +247,13 @@ weight_pairs_kernel(const T* __restrict__ w, int Cg, int K, uint32_t* most, uint
 // Column pairs: mask * bilinear(x), pixel by pixel. A group of lanes per (pixel, deformable group, tap)
 // moves pieces of eight channels.
 __global__ void __launch_bounds__(kThreads, 4)
-gather_pairs_kernel(const __grid_constant__ DcnParams p, uint16_t* __restrict__ columns, size_t plane,
-                    const SplitScale bound, float* __restrict__ columns_f32) {
+gather_pairs_kernel(const __grid_constant__ DcnParams p, const __grid_constant__ ColumnsOut out) {
     const int lpi = 1 << p.lpi_log2;
     const int sub = threadIdx.x & (lpi - 1);
     const uint32_t slot = threadIdx.x >> p.lpi_log2;             // item within the CTA's step
     const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
-    const float scale = msda::exp2_int(msda::split_exponent(bound, 0));
+    const float scale = msda::exp2_int(msda::split_exponent(out.bound, 0));
+    const bool pairs = !msda::range_is_wide(out.range), plain = !pairs || out.keep_f32;
 #pragma unroll 1
     for (uint32_t item = blockIdx.x * per_step + slot; item < p.items; item += gridDim.x * per_step) {
         uint32_t m, dg, k;
@@ -236,19 +281,44 @@ gather_pairs_kernel(const __grid_constant__ DcnParams p, uint16_t* __restrict__ 
                     }
                 }
             }
-            const uint2 r0 = msda::split_pair(acc[0].x, acc[0].y, scale);
-            const uint2 r1 = msda::split_pair(acc[0].z, acc[0].w, scale);
-            const uint2 r2 = msda::split_pair(acc[1].x, acc[1].y, scale);
-            const uint2 r3 = msda::split_pair(acc[1].z, acc[1].w, scale);
             const size_t to_at = column_index(p, m, k, dg * p.Cd + 8 * piece);
-            uint16_t* to = columns + to_at;
-            if (columns_f32 != nullptr) {
-                *reinterpret_cast<float4*>(columns_f32 + to_at) = acc[0];
-                *reinterpret_cast<float4*>(columns_f32 + to_at + 4) = acc[1];
+            if (plain) {
+                *reinterpret_cast<float4*>(out.f32 + to_at) = acc[0];
+                *reinterpret_cast<float4*>(out.f32 + to_at + 4) = acc[1];
             }
-            *reinterpret_cast<uint4*>(to) = make_uint4(r0.x, r1.x, r2.x, r3.x);
-            *reinterpret_cast<uint4*>(to + plane) = make_uint4(r0.y, r1.y, r2.y, r3.y);
+            if (pairs) {
+                const uint2 r0 = msda::split_pair(acc[0].x, acc[0].y, scale);
+                const uint2 r1 = msda::split_pair(acc[0].z, acc[0].w, scale);
+                const uint2 r2 = msda::split_pair(acc[1].x, acc[1].y, scale);
+                const uint2 r3 = msda::split_pair(acc[1].z, acc[1].w, scale);
+                uint16_t* to = out.pairs + to_at;
+                *reinterpret_cast<uint4*>(to) = make_uint4(r0.x, r1.x, r2.x, r3.x);
+                *reinterpret_cast<uint4*>(to + out.plane) = make_uint4(r0.y, r1.y, r2.y, r3.y);
+            }
         }
+    }
+}
+
+// The columns as grad_weight's fp32 product wants them, from what the forward saved: pairs put together
+// again (22 bits, and narrow, or they would be fp32), or the fp32 columns.
+__global__ void __launch_bounds__(kThreads)
+join_columns_kernel(const void* __restrict__ saved, const uint32_t* columns_range, SplitScale bound, size_t plane,
+                    float* __restrict__ out, const RangeGate gate) {
+    if (!gate_open(gate)) return;
+    const bool f32 = msda::range_is_wide(columns_range);
+    const float back = msda::exp2_int(-msda::split_exponent(bound, 0));
+    const size_t step = static_cast<size_t>(gridDim.x) * kThreads * 4;
+    for (size_t i = (static_cast<size_t>(blockIdx.x) * kThreads + threadIdx.x) * 4; i < plane; i += step) {
+        float4 v;
+        if (f32) {
+            v = *reinterpret_cast<const float4*>(static_cast<const float*>(saved) + i);
+        } else {
+            const __half* hi = static_cast<const __half*>(saved) + i;
+            float sum[4];
+            for (int e = 0; e < 4; ++e) sum[e] = (__half2float(hi[e]) + __half2float(hi[plane + e])) * back;
+            v = make_float4(sum[0], sum[1], sum[2], sum[3]);
+        }
+        *reinterpret_cast<float4*>(out + i) = v;
     }
 }
 
@@ -282,7 +352,7 @@ bool weight_in_f32(const dcn_shape* s, const Derived& d, int dtype) {
 struct Saved {
     size_t bounds, x, offset, mask, sorted, columns, total;
     size_t plane;   // halves per plane of the columns
-    bool f32;       // columns in fp32 (else pairs)
+    bool f32;       // columns in fp32 (else pairs, or fp32 where their range is wide)
 };
 Saved plan_saved(const dcn_shape* s, const Derived& d, int dtype, bool keep) {
     Saved r;
@@ -300,7 +370,7 @@ Saved plan_saved(const dcn_shape* s, const Derived& d, int dtype, bool keep) {
 }
 
 struct BackwardSpace {
-    size_t ticket, grad_columns, go_rows, go_channels, weight_t, row_most, channel_most, weight_most, total;
+    size_t ticket, go_range, grad_columns, go_rows, go_channels, weight_t, row_most, channel_most, weight_most, total;
 };
 BackwardSpace plan_backward(const dcn_shape* s, const Derived& d) {
     BackwardSpace r;
@@ -312,7 +382,8 @@ BackwardSpace plan_backward(const dcn_shape* s, const Derived& d) {
     };
     const size_t go = static_cast<size_t>(d.M) * s->Co;
     const size_t rows = static_cast<size_t>(s->groups) * d.Kd;
-    r.ticket = take(sizeof(uint32_t));                     // with the three bounds: cleared together
+    r.ticket = take(sizeof(uint32_t));                     // these five: cleared together
+    r.go_range = take(4 * sizeof(uint32_t));
     r.row_most = take(static_cast<size_t>(d.M) * 4);
     r.channel_most = take(static_cast<size_t>(s->Co) * 4);
     r.weight_most = take(rows * 4);
@@ -343,11 +414,10 @@ ForwardSpace plan_forward(const dcn_shape* s, const Derived& d, const Saved& at)
     } while (0)
 
 template <typename T>
-int to_nhwc(const void* src, int channels_last, float* dst, int N, int C, int P, uint32_t* magnitude,
+int to_nhwc(const void* src, int channels_last, float* dst, int N, int C, int P, uint32_t* range,
             cudaStream_t stream) {
     const dim3 grid((P + 31) / 32, (C + 31) / 32, N);
-    to_nhwc_kernel<T><<<grid, kThreads, 0, stream>>>(static_cast<const T*>(src), channels_last, dst, C, P,
-                                                     magnitude);
+    to_nhwc_kernel<T><<<grid, kThreads, 0, stream>>>(static_cast<const T*>(src), channels_last, dst, C, P, range);
     RETURN_ON_CUDA(cudaGetLastError());
     msda::count_launches(1);
     return MSDA_OK;
@@ -385,18 +455,18 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
     uint16_t* wpairs = reinterpret_cast<uint16_t*>(ws + sp.weight);
     uint32_t* wmost = reinterpret_cast<uint32_t*>(ws + sp.weight_most);
     weight_pairs_kernel<T><<<s->Co, kThreads, 0, stream>>>(static_cast<const T*>(weight), d.Cg, d.K, wmost,
-                                                          wpairs, wplane);
+                                                          wpairs, wplane, bounds);
     RETURN_ON_CUDA(cudaGetLastError());
 
     DcnParams p{};
     sample_params(s, d, saved, at, mask != nullptr, &p);
     uint16_t* columns = reinterpret_cast<uint16_t*>(at.f32 ? ws + sp.columns : saved + at.columns);
-    float* columns_f32 = at.f32 ? reinterpret_cast<float*>(saved + at.columns) : nullptr;
+    float* columns_f32 = reinterpret_cast<float*>(saved + at.columns);
     const SplitScale col_scale{bounds, 0, mask != nullptr ? bounds + 1 : nullptr};
+    const ColumnsOut to{columns, at.plane, columns_f32, at.f32 ? 1 : 0, col_scale, bounds};
     msda::count_launches(1);
     if (sort_pays(s, d)) {
-        rc = launch_gather_sorted(p, saved + at.sorted, d.M, s->N, columns, at.plane, col_scale, columns_f32, sms,
-                                  stream);
+        rc = launch_gather_sorted(p, saved + at.sorted, d.M, s->N, to, sms, stream);
         if (rc != MSDA_OK) return rc;
     } else {
         p.pieces = d.Cd / 8;
@@ -407,30 +477,25 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
         RETURN_ON_CUDA(msda::resident_ctas(reinterpret_cast<const void*>(gather_pairs_kernel), kThreads, 0, &per_sm));
         const uint32_t per_step = static_cast<uint32_t>(kThreads) >> p.lpi_log2;
         const uint32_t want = (p.items + per_step - 1) / per_step, cap = static_cast<uint32_t>(sms) * per_sm;
-        gather_pairs_kernel<<<want < cap ? want : cap, kThreads, 0, stream>>>(p, columns, at.plane, col_scale,
-                                                                                       columns_f32);
+        gather_pairs_kernel<<<want < cap ? want : cap, kThreads, 0, stream>>>(p, to);
         RETURN_ON_CUDA(cudaGetLastError());
         msda::count_launches(1);
     }
 
-    bool zeroed = false;
+    const int splits = forward_splits(d, sms);
+    if (splits > 1) RETURN_ON_CUDA(cudaMemsetAsync(out, 0, static_cast<size_t>(d.M) * s->Co * 4, stream));
     for (int g = 0; g < s->groups; ++g) {
         const SplitOperand A{columns + static_cast<size_t>(g) * d.Kd, static_cast<long long>(s->groups) * d.Kd, 1,
                              static_cast<long long>(at.plane), col_scale};
         const SplitOperand B{wpairs + static_cast<size_t>(g) * d.Cog * d.Kd, d.Kd, 1,
                              static_cast<long long>(wplane), SplitScale{wmost + g * d.Cog, 1, nullptr}};
-        const long long tiles = ((d.M + 127) / 128) * static_cast<long long>((d.Cog + 255) / 256);
-        const int splits = 2 * tiles <= sms ? balanced_splits(tiles, sms, (d.Kd + 255) / 256) : 1;
-        if (splits > 1 && !zeroed) {
-            RETURN_ON_CUDA(cudaMemsetAsync(out, 0, static_cast<size_t>(d.M) * s->Co * 4, stream));
-            zeroed = true;
-        }
         RETURN_ON_CUDA(msda::gemm_split(A, B, out + static_cast<size_t>(g) * d.Cog, s->Co,
                                         bias != nullptr ? bias + g * d.Cog : nullptr, static_cast<int>(d.M),
-                                        d.Cog, d.Kd, splits, status, stream));
+                                        d.Cog, d.Kd, splits, RangeGate{{bounds, nullptr}, 0}, status, stream));
         msda::count_launches(1);
     }
-    return MSDA_OK;
+    return launch_forward_product(columns_f32, reinterpret_cast<const float*>(wpairs), bias, out, s, d, sms,
+                                  RangeGate{{bounds, nullptr}, 1}, status, stream);
 }
 
 template <typename T>
@@ -452,6 +517,8 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
     uint16_t* go_channels = reinterpret_cast<uint16_t*>(ws + sp.go_channels);
     uint16_t* weight_t = reinterpret_cast<uint16_t*>(ws + sp.weight_t);
     float* grad_columns = reinterpret_cast<float*>(ws + sp.grad_columns);
+    uint32_t* go_range = reinterpret_cast<uint32_t*>(ws + sp.go_range);
+    const RangeGate narrow{{bounds, go_range}, 0}, wide{{bounds, go_range}, 1};
     RETURN_ON_CUDA(cudaMemsetAsync(ws + sp.ticket, 0, sp.grad_columns - sp.ticket, stream));
     if (grad_bias != nullptr) RETURN_ON_CUDA(cudaMemsetAsync(grad_bias, 0, static_cast<size_t>(s->Co) * 4, stream));
     RETURN_ON_CUDA(cudaMemsetAsync(grad_x, 0, static_cast<size_t>(s->N) * s->H * s->W * s->C * 4, stream));
@@ -462,11 +529,11 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
         const T* go = static_cast<const T*>(grad_out);
         const dim3 grid((HoWo + 31) / 32, (s->Co + 63) / 64, s->N);
         const RowOrder order{HoWo, 0, 0};
-        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, grad_bias);
+        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, grad_bias,
+                                                        go_range);
         pairs_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, go_rows,
                                                        weight_f32 ? nullptr : go_channels,
-                                                       weight_f32 ? reinterpret_cast<float*>(go_channels) : nullptr,
-                                                       go_plane);
+                                                       reinterpret_cast<float*>(go_channels), go_plane, wide);
     }
     // weights as [group][kd][output channel]
     const size_t wt_plane = static_cast<size_t>(s->groups) * d.Kd * d.Cog;
@@ -474,9 +541,9 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
         const T* w = static_cast<const T*>(weight);
         const dim3 grid((d.Kd + 31) / 32, (d.Cog + 63) / 64, s->groups);
         const RowOrder order{d.Kd, d.K, d.Cg};
-        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, nullptr);
+        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, nullptr, nullptr);
         pairs_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, weight_t, nullptr,
-                                                       nullptr, wt_plane);
+                                                       nullptr, wt_plane, RangeGate{});
     }
     RETURN_ON_CUDA(cudaGetLastError());
     msda::count_launches(4);
@@ -489,7 +556,7 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
                              static_cast<long long>(wt_plane),
                              SplitScale{weight_most + static_cast<size_t>(g) * d.Kd, 1, nullptr}};
         RETURN_ON_CUDA(msda::gemm_split(A, B, grad_columns + static_cast<size_t>(g) * d.Kd, ld_cols, nullptr, M,
-                                        d.Kd, d.Cog, 1, status, stream));
+                                        d.Kd, d.Cog, 1, RangeGate{}, status, stream));
         msda::count_launches(1);
     }
 
@@ -508,7 +575,7 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
     if (weight_f32)
         return launch_weight_product(reinterpret_cast<const float*>(go_channels),
                                      reinterpret_cast<const float*>(saved + at.columns), grad_weight, s, d, sms,
-                                     status, stream);
+                                     RangeGate{}, status, stream);
     const uint16_t* columns = reinterpret_cast<const uint16_t*>(saved + at.columns);
     const SplitScale col_scale{bounds, 0, masked ? bounds + 1 : nullptr};
     const int splits = weight_splits(d, sms);
@@ -520,10 +587,15 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
         const SplitOperand B{columns + static_cast<size_t>(g) * d.Kd, 1, ld_cols, static_cast<long long>(at.plane),
                              col_scale};
         RETURN_ON_CUDA(msda::gemm_split(A, B, grad_weight + static_cast<size_t>(g) * d.Cog * d.Kd, d.Kd, nullptr,
-                                        d.Cog, d.Kd, M, splits, status, stream));
+                                        d.Cog, d.Kd, M, splits, narrow, status, stream));
         msda::count_launches(1);
     }
-    return MSDA_OK;
+    // or, where a range is wide, over the fp32 columns (the gradient of the columns is used up)
+    join_columns_kernel<<<2 * sms, kThreads, 0, stream>>>(columns, bounds, col_scale, at.plane, grad_columns, wide);
+    RETURN_ON_CUDA(cudaGetLastError());
+    msda::count_launches(1);
+    return launch_weight_product(reinterpret_cast<const float*>(go_channels), grad_columns, grad_weight, s, d, sms,
+                                 wide, status, stream);
 }
 
 int split_shape(const dcn_shape* s, Derived* d) {

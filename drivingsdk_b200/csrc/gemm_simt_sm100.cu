@@ -44,6 +44,7 @@ __device__ __forceinline__ void stage_tile(const float* __restrict__ base, long 
 template <bool A_KMAJOR, bool B_KMAJOR>
 __global__ void __launch_bounds__(kThreads)
 gemm_simt_kernel(GemmArgs g) {
+    if (!gate_open(g.gate)) return;
     __shared__ __align__(16) float sA[BK][BM + kPad];
     __shared__ __align__(16) float sB[BK][BN + kPad];
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;

@@ -6,6 +6,8 @@
 
 #include <cuda_runtime.h>
 
+#include "range_gate.h"
+
 namespace msda {
 
 struct GemmArgs {
@@ -17,6 +19,7 @@ struct GemmArgs {
     long long ldc;
     const float* bias;   // added per column n when not null
     int M, N, K;
+    RangeGate gate;      // left zero: always
 };
 
 // Plain fp32 FMA kernel: any strides, any sizes. Overwrites C.

@@ -6,11 +6,15 @@
 // of that bound and 2^-40 of it in absolute terms below (a TF32 pair keeps 21). Three products
 // (lo*hi + hi*lo + hi*hi) at the fp16 rate give fp32-class accuracy at twice the rate of the
 // three TF32 products of gemm_tc_sm100.cu, whose shared-memory traffic also includes splitting
-// every tile.
+// every tile. That accuracy is relative to the scale: a row (or, under one scale, a pixel) all of whose
+// values lie far below it loses it, at 2^-30 all but 10 bits. Callers whose operands may spread that
+// wide choose by range_gate.h.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "range_gate.h"
 
 namespace msda {
 
@@ -34,7 +38,7 @@ struct SplitOperand {
 // parts that are added into C (which must be zero before). Row-contiguous operands are read in
 // blocks of 64 rows: up to 126 bytes past the last row of the last k must be readable.
 cudaError_t gemm_split(const SplitOperand& A, const SplitOperand& B, float* C, long long ldc,
-                       const float* bias, int M, int N, int K, int splits, int* status_word,
-                       cudaStream_t stream);
+                       const float* bias, int M, int N, int K, int splits, const RangeGate& gate,
+                       int* status_word, cudaStream_t stream);
 
 }  // namespace msda

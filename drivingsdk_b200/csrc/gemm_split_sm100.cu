@@ -79,6 +79,7 @@ struct SplitParams {
     int row_major;      // operands have the row index contiguous
     int reduce;
     int vec;            // 32-byte stores / 16-byte reductions are aligned
+    RangeGate gate;
     int* status;
 };
 
@@ -101,6 +102,7 @@ template <int BN>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ SplitParams p) {
+    if (!gate_open(p.gate)) return;
     using T = SplitTile<BN>;
     constexpr int kStages = T::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -369,8 +371,8 @@ cudaError_t launch_split(const SplitOperand& A, const SplitOperand& B, SplitPara
 }  // namespace
 
 cudaError_t gemm_split(const SplitOperand& A, const SplitOperand& B, float* C, long long ldc,
-                       const float* bias, int M, int N, int K, int splits, int* status_word,
-                       cudaStream_t stream) {
+                       const float* bias, int M, int N, int K, int splits, const RangeGate& gate,
+                       int* status_word, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0 || status_word == nullptr) return cudaErrorInvalidValue;
     const bool rows = A.k_stride != 1;
     for (const SplitOperand* o : {&A, &B}) {
@@ -390,6 +392,7 @@ cudaError_t gemm_split(const SplitOperand& A, const SplitOperand& B, float* C, l
     p.K = K;
     p.row_major = rows ? 1 : 0;
     p.vec = (ldc % 8 == 0 && reinterpret_cast<uintptr_t>(C) % 32 == 0) ? 1 : 0;
+    p.gate = gate;
     p.status = status_word;
     if (N > 192) return launch_split<256>(A, B, p, splits, stream);
     if (N > 96) return launch_split<128>(A, B, p, splits, stream);

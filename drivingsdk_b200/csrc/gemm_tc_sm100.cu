@@ -108,6 +108,7 @@ struct TcParams {
     int total_tiles;    // tiles of C; work item w = split * total_tiles + tile, tile = m_tile * n_tiles + n_tile
     int mn_major;       // operands are row-contiguous (A[k][m], B[k][n]) instead of k-contiguous
     int reduce;         // add into C with reductions (K is cut across work items)
+    RangeGate gate;
     int* status;
 };
 
@@ -137,6 +138,7 @@ template <int BN, int PASSES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const TcParams p) {
+    if (!gate_open(p.gate)) return;
     using T = Tile<BN, PASSES>;
     constexpr int kStages = T::kStages;
     constexpr int BK = T::BK;
@@ -466,6 +468,7 @@ cudaError_t launch(const GemmArgs& g, int splits, int* status, cudaStream_t stre
     p.kb_per_split = (kb_total + splits - 1) / splits;
     p.n_splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;   // no part is empty
     p.reduce = p.n_splits > 1 ? 1 : 0;
+    p.gate = g.gate;
     p.status = status;
     p.n_tiles = (g.N + BN - 1) / BN;
     p.mn_major = mn_major ? 1 : 0;

@@ -108,7 +108,10 @@ int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
 /*
  * The same operator from NCHW tensors of `dtype` (x and grad_out may also be channels-last:
  * x_nhwc / grad_out_nhwc = 1), its products over fp16 pairs of every operand: fp32-class accuracy
- * at twice the rate of the TF32 pairs above. For C / groups, C / deform_groups and Co / groups that
+ * at twice the rate of the TF32 pairs above. Where the magnitudes of x times the mask, or of grad_out
+ * for grad_weight, spread over more than 2^16 between pixels or channels, the TF32 pairs take over,
+ * which do not depend on the range (decided on the device). The error is relative to the largest
+ * value of a pixel's row of columns or of grad_out, and of an output channel's weights. For C / groups, C / deform_groups and Co / groups that
  * are multiples of 8, up to 65535 images and groups, and dcn_sm100_use_tensor_cores() == 1; elsewhere
  * dcn_sm100_saved_bytes() is 0.
  *   weight [Co, C / groups, kh, kw]; offset [N, deform_groups * 2 * kh * kw, Ho, Wo]; mask likewise
