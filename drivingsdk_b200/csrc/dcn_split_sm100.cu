@@ -54,6 +54,35 @@ __device__ __forceinline__ void load_tile(const T* src, int channels_last, int n
     __syncthreads();
 }
 
+// Tiles of 32 pixels and some channels of up to three tensors, one CTA each, in one launch: a launch
+// costs a small call as much as its work (4 x 128 x 30 x 40 forward and backward: 186 -> 171 us
+// for four launches fewer).
+struct Tiles {
+    uint32_t pixels, channels, count;   // tiles along each, and of the tensor; count 0: no tensor
+};
+struct Tile {
+    int n, c0, p0;
+};
+Tiles tiles_of(int N, int C, int P, int channels) {
+    Tiles t;
+    t.pixels = static_cast<uint32_t>((P + 31) / 32);
+    t.channels = static_cast<uint32_t>((C + channels - 1) / channels);
+    t.count = static_cast<uint32_t>(N) * t.pixels * t.channels;
+    return t;
+}
+// The tensor and tile of CTA `b`.
+template <typename Jobs>
+__device__ __forceinline__ int find_tile(const Jobs& jobs, uint32_t b, int channels, Tile& at) {
+    int k = 0;
+    while (b >= jobs.job[k].tiles.count) b -= jobs.job[k++].tiles.count;
+    const Tiles& t = jobs.job[k].tiles;
+    const uint32_t row = b / t.pixels, n = row / t.channels;
+    at.p0 = static_cast<int>(b - row * t.pixels) * 32;
+    at.c0 = static_cast<int>(row - n * t.channels) * channels;
+    at.n = static_cast<int>(n);
+    return k;
+}
+
 // Raises *at to v; most callers find it high enough already and skip the atomic.
 __device__ __forceinline__ void raise_max(uint32_t* at, uint32_t v) {
     if (v > *reinterpret_cast<volatile uint32_t*>(at)) atomicMax(at, v);
@@ -64,13 +93,26 @@ __device__ __forceinline__ uint32_t smallness(uint32_t most) { return most == 0u
 
 // [n][C][P] (or channels last) in T -> [n][P][C] in fp32; optionally its range (range_gate.h): the
 // largest magnitude into range[0], the smallness of the block maxima into range[2].
+struct LayoutJob {
+    Tiles tiles;
+    const void* src;
+    float* dst;
+    int channels_last, C, P;
+    uint32_t* range;
+};
+struct LayoutJobs {
+    LayoutJob job[3];
+};
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-to_nhwc_kernel(const T* __restrict__ src, int channels_last, float* __restrict__ dst, int C, int P,
-               uint32_t* range) {
+to_nhwc_kernel(const __grid_constant__ LayoutJobs jobs) {
     __shared__ float tile[32][33];
-    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32, n = blockIdx.z;
-    load_tile<T, 32>(src, channels_last, n, c0, p0, C, P, tile);
+    Tile at;
+    const LayoutJob& job = jobs.job[find_tile(jobs, blockIdx.x, 32, at)];
+    const int p0 = at.p0, c0 = at.c0, n = at.n, C = job.C, P = job.P;
+    float* __restrict__ dst = job.dst;
+    uint32_t* range = job.range;
+    load_tile<T, 32>(static_cast<const T*>(job.src), job.channels_last, n, c0, p0, C, P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t most = 0, small = 0;   // of this lane's channel; of this warp's pixels
 #pragma unroll
@@ -118,14 +160,35 @@ struct RowOrder {
 
 // Largest magnitudes of a [n][C][P] tensor per row (pixel) and per channel, and the channel sums;
 // optionally its range, over blocks of 64 channels of a pixel.
+struct OperandJob {
+    Tiles tiles;
+    const void* src;
+    int channels_last, C;
+    RowOrder order;
+    uint32_t *row_most, *channel_most;   // channel_most, channel_sum, range: optional
+    float* channel_sum;
+    uint32_t* range;
+    // pairs_kernel: pairs scaled by row, and (optional) scaled by channel or in fp32
+    uint16_t *by_row, *by_channel;
+    float* plain;
+    size_t plane;
+    RangeGate if_plain;
+};
+struct OperandJobs {
+    OperandJob job[2];
+};
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
-              uint32_t* row_most, uint32_t* channel_most, float* channel_sum, uint32_t* range) {
+bounds_kernel(const __grid_constant__ OperandJobs jobs) {
     __shared__ float tile[64][33];
     __shared__ uint32_t part[kThreads / 32][32];
-    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
-    load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
+    Tile at;
+    const OperandJob& job = jobs.job[find_tile(jobs, blockIdx.x, 64, at)];
+    const int p0 = at.p0, c0 = at.c0, n = at.n, C = job.C;
+    const RowOrder order = job.order;
+    uint32_t *row_most = job.row_most, *channel_most = job.channel_most, *range = job.range;
+    float* channel_sum = job.channel_sum;
+    load_tile<T, 64>(static_cast<const T*>(job.src), job.channels_last, n, c0, p0, C, order.P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kRows = 64 * 32 / kThreads;    // channels of this warp; lane u keeps the u-th
     uint32_t mine = 0, most = 0;
@@ -171,16 +234,21 @@ bounds_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder orde
 // where both are given, in fp32 if the gate is open.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-pairs_kernel(const T* __restrict__ src, int channels_last, int C, RowOrder order,
-             const uint32_t* row_most, const uint32_t* channel_most, uint16_t* __restrict__ by_row,
-             uint16_t* by_channel, float* plain, size_t plane, const RangeGate if_plain) {
+pairs_kernel(const __grid_constant__ OperandJobs jobs) {
     __shared__ float tile[64][33];
+    Tile tile_at;
+    const OperandJob& job = jobs.job[find_tile(jobs, blockIdx.x, 64, tile_at)];
+    const int p0 = tile_at.p0, c0 = tile_at.c0, n = tile_at.n, C = job.C;
+    const RowOrder order = job.order;
+    const uint32_t *row_most = job.row_most, *channel_most = job.channel_most;
+    uint16_t *by_row = job.by_row, *by_channel = job.by_channel;
+    float* plain = job.plain;
+    const size_t plane = job.plane;
     if (by_channel != nullptr && plain != nullptr) {
-        if (gate_open(if_plain)) by_channel = nullptr;
+        if (gate_open(job.if_plain)) by_channel = nullptr;
         else plain = nullptr;
     }
-    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64, n = blockIdx.z;
-    load_tile<T, 64>(src, channels_last, n, c0, p0, C, order.P, tile);
+    load_tile<T, 64>(static_cast<const T*>(job.src), job.channels_last, n, c0, p0, C, order.P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = c0 + 2 * lane;
     if (c >= C) return;   // C is even
@@ -413,16 +481,6 @@ ForwardSpace plan_forward(const dcn_shape* s, const Derived& d, const Saved& at)
         if (err_ != cudaSuccess) return msda::note_cuda_error(err_);  \
     } while (0)
 
-template <typename T>
-int to_nhwc(const void* src, int channels_last, float* dst, int N, int C, int P, uint32_t* range,
-            cudaStream_t stream) {
-    const dim3 grid((P + 31) / 32, (C + 31) / 32, N);
-    to_nhwc_kernel<T><<<grid, kThreads, 0, stream>>>(static_cast<const T*>(src), channels_last, dst, C, P, range);
-    RETURN_ON_CUDA(cudaGetLastError());
-    msda::count_launches(1);
-    return MSDA_OK;
-}
-
 void sample_params(const dcn_shape* s, const Derived& d, const char* saved, const Saved& at, bool masked,
                    DcnParams* p) {
     fill_params(s, d, p);
@@ -443,14 +501,15 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
     uint32_t* bounds = reinterpret_cast<uint32_t*>(saved + at.bounds);
     RETURN_ON_CUDA(cudaMemsetAsync(bounds, 0, 16, stream));
     const int HoWo = s->Ho * s->Wo, taps = s->deform_groups * d.K;
-    rc = to_nhwc<T>(x, x_nhwc, reinterpret_cast<float*>(saved + at.x), s->N, s->C, s->H * s->W, bounds, stream);
-    if (rc != MSDA_OK) return rc;
-    rc = to_nhwc<T>(offset, 0, reinterpret_cast<float*>(saved + at.offset), s->N, 2 * taps, HoWo, nullptr, stream);
-    if (rc != MSDA_OK) return rc;
-    if (mask != nullptr) {
-        rc = to_nhwc<T>(mask, 0, reinterpret_cast<float*>(saved + at.mask), s->N, taps, HoWo, bounds + 1, stream);
-        if (rc != MSDA_OK) return rc;
-    }
+    auto place = [&](size_t offset_in_saved) { return reinterpret_cast<float*>(saved + offset_in_saved); };
+    const LayoutJobs jobs{{{tiles_of(s->N, s->C, s->H * s->W, 32), x, place(at.x), x_nhwc, s->C, s->H * s->W, bounds},
+                           {tiles_of(s->N, 2 * taps, HoWo, 32), offset, place(at.offset), 0, 2 * taps, HoWo, nullptr},
+                           {tiles_of(mask != nullptr ? s->N : 0, taps, HoWo, 32), mask, place(at.mask), 0, taps, HoWo,
+                            bounds + 1}}};
+    to_nhwc_kernel<T><<<jobs.job[0].tiles.count + jobs.job[1].tiles.count + jobs.job[2].tiles.count, kThreads, 0,
+                        stream>>>(jobs);
+    RETURN_ON_CUDA(cudaGetLastError());
+    msda::count_launches(1);
     const size_t wplane = static_cast<size_t>(s->Co) * d.Kd;
     uint16_t* wpairs = reinterpret_cast<uint16_t*>(ws + sp.weight);
     uint32_t* wmost = reinterpret_cast<uint32_t*>(ws + sp.weight_most);
@@ -523,30 +582,40 @@ int backward_typed(const void* weight, const void* grad_out, int go_nhwc, const 
     if (grad_bias != nullptr) RETURN_ON_CUDA(cudaMemsetAsync(grad_bias, 0, static_cast<size_t>(s->Co) * 4, stream));
     RETURN_ON_CUDA(cudaMemsetAsync(grad_x, 0, static_cast<size_t>(s->N) * s->H * s->W * s->C * 4, stream));
 
-    // grad_out: bounds, then pairs (the second reading mostly comes from L2)
+    // grad_out, and the weights as [group][kd][output channel]: bounds, then pairs (the second reading
+    // mostly comes from L2)
     const size_t go_plane = static_cast<size_t>(M) * s->Co;
-    {
-        const T* go = static_cast<const T*>(grad_out);
-        const dim3 grid((HoWo + 31) / 32, (s->Co + 63) / 64, s->N);
-        const RowOrder order{HoWo, 0, 0};
-        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, grad_bias,
-                                                        go_range);
-        pairs_kernel<T><<<grid, kThreads, 0, stream>>>(go, go_nhwc, s->Co, order, row_most, channel_most, go_rows,
-                                                       weight_f32 ? nullptr : go_channels,
-                                                       reinterpret_cast<float*>(go_channels), go_plane, wide);
-    }
-    // weights as [group][kd][output channel]
     const size_t wt_plane = static_cast<size_t>(s->groups) * d.Kd * d.Cog;
     {
-        const T* w = static_cast<const T*>(weight);
-        const dim3 grid((d.Kd + 31) / 32, (d.Cog + 63) / 64, s->groups);
-        const RowOrder order{d.Kd, d.K, d.Cg};
-        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, nullptr, nullptr);
-        pairs_kernel<T><<<grid, kThreads, 0, stream>>>(w, 0, d.Cog, order, weight_most, nullptr, weight_t, nullptr,
-                                                       nullptr, wt_plane, RangeGate{});
+        OperandJobs jobs{};
+        OperandJob &go = jobs.job[0], &w = jobs.job[1];
+        go.tiles = tiles_of(s->N, s->Co, HoWo, 64);
+        go.src = grad_out;
+        go.channels_last = go_nhwc;
+        go.C = s->Co;
+        go.order = RowOrder{HoWo, 0, 0};
+        go.row_most = row_most;
+        go.channel_most = channel_most;
+        go.channel_sum = grad_bias;
+        go.range = go_range;
+        go.by_row = go_rows;
+        go.by_channel = weight_f32 ? nullptr : go_channels;
+        go.plain = reinterpret_cast<float*>(go_channels);
+        go.plane = go_plane;
+        go.if_plain = wide;
+        w.tiles = tiles_of(s->groups, d.Cog, d.Kd, 64);
+        w.src = weight;
+        w.C = d.Cog;
+        w.order = RowOrder{d.Kd, d.K, d.Cg};
+        w.row_most = weight_most;
+        w.by_row = weight_t;
+        w.plane = wt_plane;
+        const uint32_t grid = go.tiles.count + w.tiles.count;
+        bounds_kernel<T><<<grid, kThreads, 0, stream>>>(jobs);
+        pairs_kernel<T><<<grid, kThreads, 0, stream>>>(jobs);
     }
     RETURN_ON_CUDA(cudaGetLastError());
-    msda::count_launches(4);
+    msda::count_launches(2);
 
     const long long ld_cols = static_cast<long long>(s->groups) * d.Kd;
     for (int g = 0; g < s->groups; ++g) {
@@ -603,11 +672,12 @@ int split_shape(const dcn_shape* s, Derived* d) {
     if (rc != MSDA_OK) return rc;
     // 16-byte pieces of halves in every row
     if (d->Cg % 8 != 0 || d->Cd % 8 != 0 || d->Cog % 8 != 0) return MSDA_ERR_ALIGN;
-    // images (or groups) and blocks of channels are the y and z of the layout kernels' grids
-    constexpr int kGrid = 65535;
-    const long long taps = static_cast<long long>(s->deform_groups) * d->K;
-    return s->N <= kGrid && s->groups <= kGrid && s->C / 32 < kGrid && s->Co / 64 < kGrid && 2 * taps / 32 < kGrid
-               ? MSDA_OK : MSDA_ERR_LIMIT;
+    // one CTA per tile in the layout kernels
+    const long long HoWo = static_cast<long long>(s->Ho) * s->Wo, taps = static_cast<long long>(s->deform_groups) * d->K;
+    auto tiles = [](long long n, long long C, long long P) { return n * ((C + 31) / 32) * ((P + 31) / 32); };
+    const long long most = tiles(s->N, s->C, static_cast<long long>(s->H) * s->W) + tiles(s->N, 3 * taps, HoWo) + s->N +
+                           tiles(s->N, s->Co, HoWo) + tiles(s->groups, d->Cog, d->Kd);
+    return most < (1ll << 31) ? MSDA_OK : MSDA_ERR_LIMIT;
 }
 
 }  // namespace

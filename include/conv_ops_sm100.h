@@ -111,8 +111,9 @@ int dcn_sm100_backward(const float* x, const float* offset, const float* mask,
  * at twice the rate of the TF32 pairs above. Where the magnitudes of x times the mask, or of grad_out
  * for grad_weight, spread over more than 2^16 between pixels or channels, the TF32 pairs take over,
  * which do not depend on the range (decided on the device). The error is relative to the largest
- * value of a pixel's row of columns or of grad_out, and of an output channel's weights. For C / groups, C / deform_groups and Co / groups that
- * are multiples of 8, up to 65535 images and groups, and dcn_sm100_use_tensor_cores() == 1; elsewhere
+ * value of a pixel's row of columns or of grad_out, and of an output channel's weights.
+ * For C / groups, C / deform_groups and Co / groups that are multiples of 8 and
+ * dcn_sm100_use_tensor_cores() == 1; elsewhere, and where a tensor has 2^31 tiles of 32 x 32 or more,
  * dcn_sm100_saved_bytes() is 0.
  *   weight [Co, C / groups, kh, kw]; offset [N, deform_groups * 2 * kh * kw, Ho, Wo]; mask likewise
  *   saved: device memory of dcn_sm100_saved_bytes(), written by the forward, read by the backward
