@@ -59,6 +59,7 @@ __device__ __forceinline__ void load_tile(const T* src, int channels_last, int n
 // for four launches fewer).
 struct Tiles {
     uint32_t pixels, channels, count;   // tiles along each, and of the tensor; count 0: no tensor
+    FastDiv by_pixels, by_channels;
 };
 struct Tile {
     int n, c0, p0;
@@ -68,6 +69,8 @@ Tiles tiles_of(int N, int C, int P, int channels) {
     t.pixels = static_cast<uint32_t>((P + 31) / 32);
     t.channels = static_cast<uint32_t>((C + channels - 1) / channels);
     t.count = static_cast<uint32_t>(N) * t.pixels * t.channels;
+    t.by_pixels = msda::make_fastdiv(t.pixels);
+    t.by_channels = msda::make_fastdiv(t.channels);
     return t;
 }
 // The tensor and tile of CTA `b`.
@@ -76,7 +79,7 @@ __device__ __forceinline__ int find_tile(const Jobs& jobs, uint32_t b, int chann
     int k = 0;
     while (b >= jobs.job[k].tiles.count) b -= jobs.job[k++].tiles.count;
     const Tiles& t = jobs.job[k].tiles;
-    const uint32_t row = b / t.pixels, n = row / t.channels;
+    const uint32_t row = fd_div(b, t.by_pixels), n = fd_div(row, t.by_channels);
     at.p0 = static_cast<int>(b - row * t.pixels) * 32;
     at.c0 = static_cast<int>(row - n * t.channels) * channels;
     at.n = static_cast<int>(n);
@@ -91,14 +94,24 @@ __device__ __forceinline__ void raise_max(uint32_t* at, uint32_t v) {
 // kLeastFrom minus a block's maximum: the larger, the smaller the maximum; 0 for a block of zeros.
 __device__ __forceinline__ uint32_t smallness(uint32_t most) { return most == 0u ? 0u : msda::kLeastFrom - most; }
 
-// [n][C][P] (or channels last) in T -> [n][P][C] in fp32; optionally its range (range_gate.h): the
-// largest magnitude into range[0], the smallness of the block maxima into range[2].
+// The same for a tensor's two words of a range (range_gate.h), `which` of two tensors, read together: all
+// CTAs of a launch read this one line, which serves about one of them a clock.
+__device__ __forceinline__ void raise_range(uint32_t* range, int which, uint32_t most, uint32_t small) {
+    uint32_t w[4];
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(range) : "memory");
+    if (most > (which == 0 ? w[0] : w[1])) atomicMax(range + which, most);
+    if (small > (which == 0 ? w[2] : w[3])) atomicMax(range + 2 + which, small);
+}
+
+// [n][C][P] (or channels last) in T -> [n][P][C] in fp32; optionally its range, as tensor `which`.
 struct LayoutJob {
     Tiles tiles;
     const void* src;
     float* dst;
     int channels_last, C, P;
     uint32_t* range;
+    int which;
 };
 struct LayoutJobs {
     LayoutJob job[3];
@@ -112,6 +125,7 @@ to_nhwc_kernel(const __grid_constant__ LayoutJobs jobs) {
     const int p0 = at.p0, c0 = at.c0, n = at.n, C = job.C, P = job.P;
     float* __restrict__ dst = job.dst;
     uint32_t* range = job.range;
+    const int which = job.which;
     load_tile<T, 32>(static_cast<const T*>(job.src), job.channels_last, n, c0, p0, C, P, tile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t most = 0, small = 0;   // of this lane's channel; of this warp's pixels
@@ -140,10 +154,7 @@ to_nhwc_kernel(const __grid_constant__ LayoutJobs jobs) {
             // single elements are often small: a channel counts with eight pixels or more
             if (P - p0 >= 8) small = max(small, __reduce_max_sync(0xffffffffu, smallness(most)));
             most = __reduce_max_sync(0xffffffffu, most);
-            if (lane == 0) {
-                raise_max(range, most);
-                raise_max(range + 2, small);
-            }
+            if (lane == 0) raise_range(range, which, most, small);
         }
     }
 }
@@ -222,10 +233,7 @@ bounds_kernel(const __grid_constant__ OperandJobs jobs) {
         if (range != nullptr) {
             const uint32_t small = __reduce_max_sync(0xffffffffu, smallness(mine));
             const uint32_t tile_most = __reduce_max_sync(0xffffffffu, mine);
-            if (lane == 0) {
-                raise_max(range, tile_most);
-                raise_max(range + 2, small);
-            }
+            if (lane == 0) raise_range(range, 0, tile_most, small);
         }
     }
 }
@@ -502,10 +510,12 @@ int forward_typed(const void* x, int x_nhwc, const void* offset, const void* mas
     RETURN_ON_CUDA(cudaMemsetAsync(bounds, 0, 16, stream));
     const int HoWo = s->Ho * s->Wo, taps = s->deform_groups * d.K;
     auto place = [&](size_t offset_in_saved) { return reinterpret_cast<float*>(saved + offset_in_saved); };
-    const LayoutJobs jobs{{{tiles_of(s->N, s->C, s->H * s->W, 32), x, place(at.x), x_nhwc, s->C, s->H * s->W, bounds},
-                           {tiles_of(s->N, 2 * taps, HoWo, 32), offset, place(at.offset), 0, 2 * taps, HoWo, nullptr},
+    const LayoutJobs jobs{{{tiles_of(s->N, s->C, s->H * s->W, 32), x, place(at.x), x_nhwc, s->C, s->H * s->W, bounds,
+                            0},
+                           {tiles_of(s->N, 2 * taps, HoWo, 32), offset, place(at.offset), 0, 2 * taps, HoWo, nullptr,
+                            0},
                            {tiles_of(mask != nullptr ? s->N : 0, taps, HoWo, 32), mask, place(at.mask), 0, taps, HoWo,
-                            bounds + 1}}};
+                            bounds, 1}}};
     to_nhwc_kernel<T><<<jobs.job[0].tiles.count + jobs.job[1].tiles.count + jobs.job[2].tiles.count, kThreads, 0,
                         stream>>>(jobs);
     RETURN_ON_CUDA(cudaGetLastError());
