@@ -37,6 +37,7 @@ def test_backward_only_reads_what_the_forward_saved():
 def test_more_images_than_a_grid_has_planes():
     import drivingsdk_b200 as sdk
     N = 65537
+    torch.manual_seed(5)
     x, off = torch.randn(N, 8, 2, 2, device="cuda"), torch.randn(N, 18, 2, 2, device="cuda")
     w = torch.randn(8, 8, 3, 3, device="cuda")
     ts = [t.requires_grad_() for t in (x, off, w)]
@@ -49,5 +50,7 @@ def test_more_images_than_a_grid_has_planes():
         o = sdk.deform_conv2d(*p, 1, 1)
         parts.append((o.detach(), *torch.autograd.grad(o, p, go[half])))
     want = [torch.cat([a[i] for a in parts]) for i in range(3)] + [parts[0][3] + parts[1][3]]
-    for a, b in zip((out, *got), want):
-        assert (a - b).norm() <= 1e-5 * b.norm()
+    for name, a, b in zip(("out", "grad_x", "grad_offset", "grad_weight"), (out, *got), want):
+        # grad_weight may be one serial fp32 sum over n = 262148 pixels, whose rounding is off by some
+        # 2^-24 * sqrt(n / 6) = 1.2e-5 of the result; four times that
+        assert (a - b).norm() <= (5e-5 if name == "grad_weight" else 1e-5) * b.norm(), name
