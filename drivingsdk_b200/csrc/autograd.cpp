@@ -199,8 +199,6 @@ struct DeformConv : Function<DeformConv> {
             }
             return out;
         }
-        ctx->saved_data["conv"] = std::vector<int64_t>{stride[0], stride[1], padding[0], padding[1], dilation[0],
-                                                       dilation[1], groups, deformable_groups};
         const std::vector<int64_t> kernel{weight.size(2), weight.size(3)};
         auto nhwc = [](const Tensor& t) { return t.permute({0, 2, 3, 1}).contiguous(); };
         const Tensor nx = nhwc(x), noff = nhwc(offset), nw = nhwc(weight);
@@ -214,6 +212,9 @@ struct DeformConv : Function<DeformConv> {
             std::tie(out, columns) =
                 deformable_conv2d(nx, noff, nw, kernel, stride, padding, dilation, groups, deformable_groups);
         }
+        // (two entries each: checked by the call)
+        ctx->saved_data["conv"] = std::vector<int64_t>{stride[0], stride[1], padding[0], padding[1], dilation[0],
+                                                       dilation[1], groups, deformable_groups};
         ctx->save_for_backward({nw, columns, bias, nx, noff, nmask});
         return out;
     }

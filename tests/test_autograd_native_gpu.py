@@ -67,6 +67,15 @@ def test_add_relu_in_place_under_autograd():
     assert torch.equal(gx, (out > 0).float()) and torch.equal(gx, gy)
 
 
+def test_convolution_wants_two_strides():
+    import drivingsdk_b200 as sdk
+    for channels in (8, 6):   # the native form, and the fp32 form
+        x, off, w = (torch.randn(*n, device="cuda") for n in ((1, channels, 5, 5), (1, 18, 5, 5), (8, channels, 3, 3)))
+        for stride in ((1,), (1, 1, 1)):
+            with pytest.raises(RuntimeError, match="two entries"):
+                sdk.deform_conv2d(x, off, w, stride, 1)
+
+
 def _traced_calls():
     import drivingsdk_b200 as sdk
     shapes, starts, (v, l, a) = _leaves()
