@@ -56,8 +56,8 @@ def parse_args():
                          "deformable convolution, add+ReLU, stem max pooling (the operators "
                          "behind the other default patches); all of these on one GPU")
     ap.add_argument("--tensor-cores", type=int, default=1, choices=[0, 1, 2],
-                    help="--op dcn: 1 = tcgen05 3xTF32 products (default), 2 = tcgen05 single "
-                         "TF32 product, 0 = fp32 FMA kernel")
+                    help="--op dcn: 1 = the form of the Python operators, tcgen05 products over fp16 "
+                         "and TF32 pairs (default), 2 = tcgen05 single TF32 product, 0 = fp32 FMA kernel")
     ap.add_argument("--workload", default="bevformer_sca")
     ap.add_argument("--dtype", default="float32", choices=["float32", "float16", "bfloat16"])
     ap.add_argument("--batch", type=int, default=None,
@@ -279,7 +279,7 @@ def run_native(args):
     gv = torch.empty(B, K, H, D, device=dev, dtype=dtype)
     gl = torch.empty(B, Q, H, L, P, 2, device=dev, dtype=dtype)
     ga = torch.empty(B, Q, H, L, P, device=dev, dtype=dtype)
-    ws_bytes = lib.msda_sm100_backward_workspace_bytes(B, K, H, D, code)
+    ws_bytes = lib.msda_sm100_backward_sorted_workspace_bytes(*dims, code)
     ws = torch.empty(max(ws_bytes, 16), device=dev, dtype=torch.uint8)
     stream = torch.cuda.current_stream()
 
@@ -385,7 +385,7 @@ def run_native(args):
     bwd_gbs = bb / (bwd_ms * 1e-3) / 1e9
     fwd_gbs = fb / (fwd_ms * 1e-3) / 1e9
     step_gbs = (fb + bb) / (ms_per_step * 1e-3) / 1e9
-    bwd_kernel = backward_kernel_name(lib, capi, w.D, esize)
+    bwd_kernel = backward_kernel_name(ws_bytes > lib.msda_sm100_backward_workspace_bytes(B, K, H, D, code))
     # what actually bounds the two kernels: rows moved between L2 and the SMs, against the
     # rates the library's probe measures on this device in this run
     rows = count_corner_rows(sets[0]["loc"], shapes_i32)
@@ -478,9 +478,10 @@ def measured_row_ceilings(lib, capi, dev, D, esize):
             "red_row_bytes": r_row, "red_rows_per_s": r.value}
 
 
-def backward_kernel_name(lib, capi, D, dtype_size):
-    """Name of the kernel msda_sm100_backward_ws launches (one template, msda_bwd_kernel)."""
-    return "msda_bwd_kernel"
+def backward_kernel_name(sorted_samples):
+    """Name of the kernels msda_sm100_backward_ws launches: the task-ordered one, or the two over
+    cell-sorted samples where the size makes the sort pay."""
+    return "sort_cells_kernel + msda_bwd_sorted_kernel" if sorted_samples else "msda_bwd_kernel"
 
 
 def run_planned_splits(lib, dist, dev, rank, world, w, dtype, replica_ms_per_step, barrier):
@@ -509,7 +510,7 @@ def run_planned_splits(lib, dist, dev, rank, world, w, dtype, replica_ms_per_ste
         d1 = (1, wl.K, wl.H, wl.D, wl.L, wl.Q, wl.P)
         o1 = torch.empty(1, wl.Q, wl.H * wl.D, device=dev, dtype=dt)
         g1 = [torch.empty_like(dv[k]) for k in ("value", "loc", "attn")]
-        wsb = lib.msda_sm100_backward_workspace_bytes(1, wl.K, wl.H, wl.D, code)
+        wsb = lib.msda_sm100_backward_sorted_workspace_bytes(*d1, code)
         ws1 = torch.empty(max(wsb, 16), device=dev, dtype=torch.uint8)
         ea, eb = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         single = []
@@ -559,7 +560,7 @@ def run_planned_splits(lib, dist, dev, rank, world, w, dtype, replica_ms_per_ste
             dims = (nb, wl.K, wl.H, wl.D, wl.L, nq, wl.P)
             out = torch.empty(nb, nq, wl.H * wl.D, device=dev, dtype=dt)
             gv, gl, ga = torch.empty_like(value), torch.empty_like(loc), torch.empty_like(attn)
-            ws_bytes = lib.msda_sm100_backward_workspace_bytes(nb, wl.K, wl.H, wl.D, code)
+            ws_bytes = lib.msda_sm100_backward_sorted_workspace_bytes(*dims, code)
             ws = torch.empty(max(ws_bytes, 16), device=dev, dtype=torch.uint8)
         e = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
 
@@ -731,6 +732,8 @@ def run_sibling(args):
         out = torch.empty(B, Q, H * D, device=dev)
         gv, ga = torch.empty_like(value), torch.empty_like(attn)
         dims = (B, K, H, D, L, Q, P)
+        ws_bytes = lib.gka_sm100_backward_sorted_workspace_bytes(*dims, capi.F32)
+        ws = torch.empty(max(ws_bytes, 16), device=dev, dtype=torch.uint8)
         samples = B
         nv, ns, no = value.numel(), attn.numel(), out.numel()
         fwd_bytes, bwd_bytes = 4 * (nv + 3 * ns + no), 4 * (2 * nv + 4 * ns + no)
@@ -743,8 +746,8 @@ def run_sibling(args):
         def bwd():
             capi.check(lib.gka_sm100_backward_ws(
                 value.data_ptr(), shapes.data_ptr(), starts.data_ptr(), loc.data_ptr(),
-                attn.data_ptr(), go.data_ptr(), gv.data_ptr(), ga.data_ptr(), None, 0, *dims,
-                capi.F32, stream.cuda_stream), "gka bwd")
+                attn.data_ptr(), go.data_ptr(), gv.data_ptr(), ga.data_ptr(), ws.data_ptr(),
+                ws_bytes, *dims, capi.F32, stream.cuda_stream), "gka bwd")
 
         def cpu_once(nb):
             n = lambda t: t[:nb].cpu().numpy()
@@ -815,6 +818,8 @@ def run_sibling(args):
         out = torch.empty(B, A, C, device=dev)
         gf, gl, gw = torch.empty_like(feat), torch.empty_like(loc), torch.empty_like(wts)
         dims = (B, F, C, A, Pts, cams, scales, G)
+        ws_bytes = lib.da_sm100_backward_workspace_bytes(*dims)
+        ws = torch.empty(ws_bytes, device=dev, dtype=torch.uint8)
         samples = B
         nf, nl, nw, no = feat.numel(), loc.numel(), wts.numel(), out.numel()
         fwd_bytes, bwd_bytes = 4 * (nf + nl + nw + no), 4 * (2 * nf + 2 * nl + 2 * nw + no)
@@ -825,10 +830,10 @@ def run_sibling(args):
                                             stream.cuda_stream), "da fwd")
 
         def bwd():
-            capi.check(lib.da_sm100_backward(feat.data_ptr(), shapes.data_ptr(), starts.data_ptr(),
-                                             loc.data_ptr(), wts.data_ptr(), go.data_ptr(),
-                                             gf.data_ptr(), gl.data_ptr(), gw.data_ptr(), *dims,
-                                             stream.cuda_stream), "da bwd")
+            capi.check(lib.da_sm100_backward_ws(
+                feat.data_ptr(), shapes.data_ptr(), starts.data_ptr(), loc.data_ptr(), wts.data_ptr(),
+                go.data_ptr(), gf.data_ptr(), gl.data_ptr(), gw.data_ptr(), ws.data_ptr(), ws_bytes,
+                *dims, capi.F32, stream.cuda_stream), "da bwd")
 
         def cpu_once(nb):
             n = lambda t: t[:nb].cpu().numpy()
@@ -936,12 +941,32 @@ def run_conv_side(args):
         gx, goff, gmask, gw = (torch.empty_like(t) for t in (x, off, mask, w))
         old_tc = lib.dcn_sm100_use_tensor_cores(args.tensor_cores)
 
+        if args.tensor_cores == 1:
+            # the form that the Python operators take: offset, mask and weight as NCHW
+            ref = ctypes.byref(shape)
+            nchw = lambda t: t.permute(0, 3, 1, 2).contiguous()  # noqa: E731
+            off_c, mask_c, w_c = nchw(off), nchw(mask), nchw(w)
+            block = lambda n: torch.empty(n, device=dev, dtype=torch.uint8)  # noqa: E731
+            saved = block(lib.dcn_sm100_saved_bytes(ref, capi.F32, 1))
+            ws_f = block(lib.dcn_sm100_nchw_workspace_bytes(ref, capi.F32, 1, 0))
+            ws_b = block(lib.dcn_sm100_nchw_workspace_bytes(ref, capi.F32, 1, 1))
+
         def fwd():
+            if args.tensor_cores == 1:
+                capi.check(lib.dcn_sm100_forward_nchw(
+                    x.data_ptr(), 1, off_c.data_ptr(), mask_c.data_ptr(), w_c.data_ptr(), None, out.data_ptr(),
+                    saved.data_ptr(), saved.numel(), ws_f.data_ptr(), ws_f.numel(), ref, capi.F32, 1, st), "dcn fwd")
+                return
             capi.check(lib.dcn_sm100_forward(x.data_ptr(), off.data_ptr(), mask.data_ptr(),
                                              w.data_ptr(), None, out.data_ptr(), cols.data_ptr(),
                                              ctypes.byref(shape), st), "dcn fwd")
 
         def bwd():
+            if args.tensor_cores == 1:
+                capi.check(lib.dcn_sm100_backward_nchw(
+                    w_c.data_ptr(), go.data_ptr(), 1, saved.data_ptr(), gx.data_ptr(), goff.data_ptr(),
+                    gmask.data_ptr(), gw.data_ptr(), None, ws_b.data_ptr(), ws_b.numel(), ref, capi.F32, st), "dcn bwd")
+                return
             capi.check(lib.dcn_sm100_backward(
                 x.data_ptr(), off.data_ptr(), mask.data_ptr(), w.data_ptr(), cols.data_ptr(),
                 go.data_ptr(), gx.data_ptr(), goff.data_ptr(), gmask.data_ptr(), gw.data_ptr(), None,
@@ -963,7 +988,8 @@ def run_conv_side(args):
                      "backward": 4 * (2 * nx + 2 * ns + 2 * nw + no + nc)}
         config = {"workload": "modulated_dcn_test_shape", "N": N, "C": C, "Co": Co, "H": H, "W": W,
                   "kernel": k, "groups": 1, "deform_groups": 1,
-                  "products": ["fp32 FMA", "tcgen05 3xTF32", "tcgen05 1xTF32"][args.tensor_cores]}
+                  "products": ["fp32 FMA", "tcgen05 over fp16 pairs, grad_weight over TF32 pairs",
+                               "tcgen05 1xTF32"][args.tensor_cores]}
         kernel_name = "three matrix products (forward, grad_columns, grad_weight)"
     elif args.op == "addrelu":
         shape_t = (18, 256, 232, 100)
@@ -1044,7 +1070,7 @@ def run_conv_side(args):
             "hbm_algorithmic_bytes": hbm_bytes}
     if args.op == "dcn":
         roof["note"] = ("achieved counts each fp32 product once (2*M*N*K); with --tensor-cores 1 "
-                        "the tensor cores execute three TF32 products for it")
+                        "the tensor cores execute three fp16 or TF32 products for it")
         lib.dcn_sm100_use_tensor_cores(old_tc)
     line = {
         "metric": f"{args.op}_samples_per_s", "value": samples / (ms * 1e-3), "unit": UNIT,
