@@ -1,9 +1,9 @@
 """Fused add + ReLU: autograd wrapper over the sm_100a kernels.
 
 Mirrors the reference wrapper (mx_driving/ops/npu_add_relu.py:19-37): ``AddReluFunction``
-and ``npu_add_relu = _C.add_relu_autograd   # the same function, natively``. As in the reference, an ``x`` of at least
-2,000,000 elements is overwritten with ``relu(x + y)`` and returned, a smaller one is left
-untouched and the result is a new tensor (the reference computes ``F.relu(x + y)`` there);
+and ``npu_add_relu = AddReluFunction.apply`` (here its native counterpart). As in the
+reference, an ``x`` of at least 2,000,000 elements is overwritten with ``relu(x + y)`` and
+returned, a smaller one is left untouched and the result is a new tensor (the reference computes ``F.relu(x + y)`` there);
 the result is what backward keeps, and both addends receive the same gradient
 ``grad_output * (result > 0)``. Differences: the kernel runs at every size (on a copy of
 ``x`` below the threshold), the overwrite is declared to autograd (``mark_dirty``), and an

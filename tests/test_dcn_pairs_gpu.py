@@ -1,7 +1,7 @@
 """The convolution's products over fp16 pairs, at the edges of their tiles and against the fp32 FMA
 products: channel counts that fill 64, 128 and 256 wide tiles or leave remainders, groups whose row
-blocks reach into the next group's, operands whose magnitudes differ by many orders between pixels,
-channels-last gradients, Inf."""
+blocks reach into the next group's, operands whose magnitudes differ by many orders between pixels (as
+one norm over each result; pixel by pixel in test_dcn_range_gpu.py), channels-last gradients, Inf."""
 import pytest
 import torch
 
