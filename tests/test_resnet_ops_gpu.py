@@ -116,3 +116,19 @@ def test_max_pool2d_nan_and_argument_checks():
             mx_driving.npu_max_pool2d(x, *bad)
     with pytest.raises(RuntimeError):
         mx_driving.npu_max_pool2d(x[0], 3, 2, 1)
+
+
+# strips of output rows, groups of output columns, lanes at the edge of a row, misaligned rows and tensors
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("W", [1, 2, 7, 8, 63, 64, 65, 66, 72, 129, 136])
+@pytest.mark.parametrize("H", [1, 2, 7, 8, 9, 15, 17])
+def test_max_pool2d_at_the_edges_of_its_tiles(H, W, dtype):
+    import mx_driving
+    g = torch.Generator().manual_seed(H * 1000 + W)
+    x = (torch.rand((2, 3, H, W), generator=g) - 0.5).to(dtype).cuda()
+    x.view(-1)[:: 37] = -float("inf")
+    x.view(-1)[5 :: 91] = float("nan")
+    skewed = torch.empty(x.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(x).copy_(x)
+    want = F.max_pool2d(x.float(), 3, 2, 1).to(dtype)
+    for given in (x, skewed):
+        assert torch.equal(mx_driving.npu_max_pool2d(given, 3, 2, 1).nan_to_num(9.0), want.nan_to_num(9.0))
