@@ -3,6 +3,7 @@
 // deformable aggregation (da_sorted_sm100.cu).
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "msda_common.cuh"
@@ -12,6 +13,7 @@ namespace msda {
 
 constexpr int kSortThreads = 1024;
 constexpr uint32_t kSortCells = 24 * 1024;   // counters of one CTA: 96 KB, two CTAs per SM
+constexpr uint32_t kSortRoom = 28 * 1024;    // ... and the most that two CTAs per SM may have
 constexpr uint32_t kMaxStream = 256;         // most consecutive sorted samples in one stream
 
 template <typename TL>
@@ -28,6 +30,19 @@ template <>
 __device__ __forceinline__ float2 load_pair<__nv_bfloat16>(const __nv_bfloat16* p) {
     const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
+// Zeros for `bytes` bytes from p on, by all threads of the grid.
+__device__ __forceinline__ void clear_bytes(void* p, size_t bytes) {
+    unsigned char* at = static_cast<unsigned char*>(p);
+    const size_t head = min(bytes, static_cast<size_t>((16u - (reinterpret_cast<uintptr_t>(at) & 15u)) & 15u));
+    uint4* body = reinterpret_cast<uint4*>(at + head);
+    const size_t pieces = (bytes - head) / 16, tail = head + pieces * 16;
+    const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
+    const size_t first = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (size_t i = first; i < pieces; i += step) body[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (first < head) at[first] = 0;
+    if (first < bytes - tail) at[tail + first] = 0;
 }
 
 // The sample's cell in its level, or kNoRow for a sample that takes no part.
@@ -66,92 +81,111 @@ __device__ __forceinline__ uint32_t cluster_read(uint32_t addr) {
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(r) : "r"(addr) : "memory");
     return r;
 }
+__device__ __forceinline__ void cluster_write(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Counting sort of the samples of one map (MSDA: a batch entry, head and level) by cell, with the counters in the shared
-// memory of a cluster of CTAs: atomics there are faster than in L2 (a version with one L2 counter
-// per cell took 72 + 42 us at the encoder shape, bound by the rate of L2 atomics). The CTAs of a
-// cluster share the samples and the cells of a map: each counts and places its samples,
-// whoever holds the counter. Where cells hold many samples each CTA keeps to itself:
-// it sorts its own queries (whose runs are then that much shorter). The CTAs' results follow
-// each other in the order in which they get there.
-template <typename Source>
-__global__ void __launch_bounds__(kSortThreads, 2)
-sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ SortParams sp) {
-    extern __shared__ uint32_t s_count[];   // [kSortCells]
-    __shared__ uint32_t warp_sum[32];
-    __shared__ uint32_t block_sum;           // samples this CTA's counters hold
+// Counting sort of the samples of one map (MSDA: a batch entry, head and level) by cell, by a cluster of
+// CTAs that share the map's samples, with the counters in their shared memory (one L2 counter per cell:
+// 114 us at the encoder shape). Bound by scattered accesses of 4 bytes: one store per sample in any
+// case, some 200 G per second through L2, and what passes between the CTAs of a cluster, a few bytes per
+// clock and SM. So the counters are kept in one of three ways, by samples per cell:
+//   split   every CTA holds a part of the cells, all count and place in them with remote atomics: two
+//           remote accesses per sample;
+//   merged  every CTA counts its samples on its own, then the CTAs turn a slice of the cells each into
+//           first positions for all (cell by cell, a cell's parts by CTA): three remote accesses, side
+//           by side, per cell and CTA;
+//   alone   many samples per cell: every CTA sorts its samples on its own, the results follow each other.
+enum class Counters { kSplit, kMerged, kAlone };
+
+// One CTA's part of the sort of a map; returns how many of the map's samples have a place.
+template <Counters KEPT, typename Source>
+__device__ __forceinline__ uint32_t sort_map(const Source& src, const SortParams& sp,
+                                             const typename Source::Map& map, uint32_t* s_count,
+                                             uint32_t* warp_sum, uint32_t* block_sum) {
+    constexpr bool kSplit = KEPT == Counters::kSplit, kMerged = KEPT == Counters::kMerged;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (blockIdx.x == 0 && tid == 0) *sp.ticket = 0u;
-    if (!src.ok()) {         // the same answer in every CTA
-        if (tid == 0) sp.regions[blockIdx.x / sp.parts] = make_uint2(0u, 0u);
-        return;
-    }
-
-    const uint32_t part = blockIdx.x % sp.parts;   // rank in the cluster
-    const typename Source::Map map = src.map(blockIdx.x / sp.parts);
-    const uint32_t cells = map.cells, samples = src.samples;
-    // on its own: at least sixteen samples per cell are left to each CTA, and the counters fit
-    const bool alone = sp.parts == 1 || (samples / sp.parts >= 16u * cells && cells <= kSortCells);
-    const uint32_t begin_sample = static_cast<uint32_t>(static_cast<uint64_t>(samples) * part / sp.parts);
+    const uint32_t parts = sp.parts, part = blockIdx.x % parts;   // rank in the cluster
+    const uint32_t samples = src.samples, cells = map.cells;
+    const uint32_t begin_sample = static_cast<uint32_t>(static_cast<uint64_t>(samples) * part / parts);
     const uint32_t n =
-        static_cast<uint32_t>(static_cast<uint64_t>(samples) * (part + 1) / sp.parts) - begin_sample;
-
-    // cells held by one CTA at a time, by all of the cluster (or by this CTA alone) in a pass
-    const uint32_t holders = alone ? 1u : sp.parts;
-    const uint32_t held = min(kSortCells, (cells + holders - 1) / holders);
-    const uint32_t pass_cells = held * holders;
-    const FastDiv by_held = sp.parts == 1 ? FastDiv{0u, 0u} : device_fastdiv(held);
+        static_cast<uint32_t>(static_cast<uint64_t>(samples) * (part + 1) / parts) - begin_sample;
     auto sync = [&]() {
-        if (alone) __syncthreads();
+        if (!kSplit && !kMerged) __syncthreads();
         else cluster_barrier();
     };
-    const uint32_t region = (blockIdx.x / sp.parts) * samples;
-    uint32_t placed = 0;         // samples of the region placed by earlier passes
+
+    // A thread's samples are a whole number of periods apart (a period: the points of a query), which
+    // makes their numbers an arithmetic sequence: no division per sample.
+    const uint32_t periods = kSortThreads / src.period, threads = periods * src.period;
+    const uint32_t first = tid < threads ? tid : n, id_step = periods * src.period_step;
+    const uint32_t first_id = src.id(map, begin_sample + (first < n ? first : 0u));
+
+    // cells held by a CTA at a time, and by all of the cluster in a pass
+    const uint32_t held = min(kSortCells, kSplit ? (cells + parts - 1) / parts : cells);
+    const uint32_t pass_cells = kSplit ? held * parts : held;
+    const FastDiv by_held = kSplit ? device_fastdiv(held) : FastDiv{0u, 0u};
+    auto remote = [&](uint32_t c) {   // the counter of cell c of the pass
+        const uint32_t rank = fd_div(c, by_held);
+        return cluster_address(s_count + (c - rank * held), rank);
+    };
+
+    // room for the sorted numbers, which then leave side by side (96 maps of 107 K samples on 375 cells:
+    // 97 us before, 81 now)
+    const bool staged = KEPT == Counters::kAlone && cells + n <= sp.room;
+    uint32_t placed = 0;         // samples of the map placed by earlier passes
     constexpr uint32_t kU = 4;   // samples in flight per thread
+    // each(cell of this pass, sample number)
+    auto for_each_sample = [&](uint32_t lo, auto&& each) {
+        uint32_t id = first_id;
+        for (uint32_t i0 = first; i0 < n; i0 += kU * threads) {
+            float2 xy[kU];
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u)
+                xy[u] = src.position(i0 + u * threads < n ? id + u * id_step : first_id);
+#pragma unroll
+            for (uint32_t u = 0; u < kU; ++u) {
+                if (i0 + u * threads >= n) break;
+                const uint32_t c = src.cell(map, xy[u]) - lo;   // (none: far beyond the pass)
+                if (c < pass_cells) each(c, id + u * id_step);
+            }
+            id += kU * id_step;
+        }
+    };
     for (uint32_t lo = 0; lo < cells; lo += pass_cells) {
         for (uint32_t i = tid; i < held; i += kSortThreads) s_count[i] = 0u;
         sync();
-        for (uint32_t i0 = tid; i0 < n; i0 += kU * kSortThreads) {
-            float2 xy[kU];
-            uint32_t id[kU];
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                const uint32_t i = i0 + u * kSortThreads;
-                id[u] = src.id(map, begin_sample + (i < n ? i : 0u));
-                xy[u] = src.position(id[u]);
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                if (i0 + u * kSortThreads >= n) break;
-                const uint32_t c = src.cell(map, xy[u]);
-                if (c - lo < pass_cells) {
-                    if (alone) {
-                        atomicAdd(s_count + (c - lo), 1u);
-                    } else {
-                        const uint32_t rank = fd_div(c - lo, by_held);
-                        cluster_count(cluster_address(s_count + (c - lo - rank * held), rank));
-                    }
-                } else if (c == kNoRow && lo == 0) {
-                    src.drop(id[u]);
-                }
-            }
-        }
+        for_each_sample(lo, [&](uint32_t c, uint32_t) {
+            if (kSplit) cluster_count(remote(c));
+            else atomicAdd(s_count + c, 1u);
+        });
         sync();
-        // counts -> first positions: a thread takes an odd number of neighbours (no bank conflicts)
-        const uint32_t per = ((held + kSortThreads - 1) / kSortThreads) | 1u;
-        const uint32_t begin = min(held, tid * per), stop = min(held, begin + per);
-        uint32_t sum = 0;
-        for (uint32_t i = begin; i < stop; ++i) sum += s_count[i];
-        uint32_t incl = sum;
+        // counts -> first positions: of this CTA's counters, or, merged, of a slice of everybody's. A
+        // warp takes a range of whole groups of 32 cells.
+        const uint32_t slice = kMerged ? (held + parts - 1) / parts : held;
+        const uint32_t slice_begin = kMerged ? part * slice : 0u, slice_end = min(held, slice_begin + slice);
+        const uint32_t range = ((slice + kSortThreads - 1) / kSortThreads) * 32u;
+        const uint32_t begin = slice_begin + warp * range, stop = min(slice_end, begin + range);
+        // a cell's counts; a CTA begins with its own counter and goes on to another one than the others
+        uint32_t m[kMaxSortParts];
+        auto count_of = [&](uint32_t i) {
+            uint32_t all = m[0] = s_count[i];
+            if (kMerged) {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) warp_sum[warp] = incl;
+                for (uint32_t r = 1; r < kMaxSortParts; ++r)
+                    m[r] = r < parts ? cluster_read(cluster_address(s_count + i, r ^ part)) : 0u;
+#pragma unroll
+                for (uint32_t r = 1; r < kMaxSortParts; ++r) all += m[r];
+            }
+            return all;
+        };
+        uint32_t sum = 0;
+        for (uint32_t i = begin + lane; i < stop; i += 32) sum += count_of(i);
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) warp_sum[warp] = sum;
         __syncthreads();
         if (warp == 0) {
             const uint32_t mine = warp_sum[lane];
@@ -162,55 +196,83 @@ sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ So
                 if (lane >= o) w += v;
             }
             warp_sum[lane] = w - mine;
-            if (lane == 31) block_sum = w;
+            if (lane == 31) *block_sum = w;
         }
-        if (sp.parts == 1) __syncthreads();
+        if (parts == 1) __syncthreads();
         else cluster_barrier();
-        // the samples of lower ranks come first
-        uint32_t at = region + placed + warp_sum[warp] + incl - sum;
-        for (uint32_t r = 0; r < sp.parts; ++r) {
-            const uint32_t m = sp.parts == 1 ? block_sum : cluster_read(cluster_address(&block_sum, r));
-            if (r < part) at += m;
-            placed += m;
+        // what lower ranks hold comes first
+        uint32_t base = blockIdx.x / parts * samples + placed;
+        for (uint32_t r = 0; r < parts; ++r) {
+            const uint32_t there = parts == 1 ? *block_sum : cluster_read(cluster_address(block_sum, r));
+            if (r < part) base += there;
+            placed += there;
         }
-        for (uint32_t i = begin; i < stop; ++i) {
-            const uint32_t m = s_count[i];
-            s_count[i] = at;
-            at += m;
-        }
-        sync();
-        for (uint32_t i0 = tid; i0 < n; i0 += kU * kSortThreads) {
-            float2 xy[kU];
-            uint32_t id[kU], pos[kU];
+        uint32_t at = warp_sum[warp] + (staged ? 0u : base);
+        for (uint32_t i0 = begin; i0 < stop; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const uint32_t count = i < stop ? count_of(i) : 0u;
+            uint32_t incl = count;
 #pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                const uint32_t i = i0 + u * kSortThreads;
-                id[u] = src.id(map, begin_sample + (i < n ? i : 0u));
-                xy[u] = src.position(id[u]);
-                pos[u] = kNoRow;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
             }
+            if (i < stop) {
+                uint32_t pos = at + incl - count;
+                s_count[i] = pos;
+                if (kMerged) {
 #pragma unroll
-            for (uint32_t u = 0; u < kU; ++u) {
-                if (i0 + u * kSortThreads >= n) break;
-                const uint32_t c = src.cell(map, xy[u]);
-                if (c - lo < pass_cells) {
-                    if (alone) {
-                        pos[u] = atomicAdd(s_count + (c - lo), 1u);
-                    } else {
-                        const uint32_t rank = fd_div(c - lo, by_held);
-                        pos[u] = cluster_take(cluster_address(s_count + (c - lo - rank * held), rank));
+                    for (uint32_t r = 1; r < kMaxSortParts; ++r) {
+                        pos += m[r - 1];
+                        if (r < parts) cluster_write(cluster_address(s_count + i, r ^ part), pos);
                     }
                 }
             }
-#pragma unroll
-            for (uint32_t u = 0; u < kU; ++u)
-                if (pos[u] != kNoRow) sp.sorted[pos[u]] = id[u];
+            at += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        sync();
+        if (!staged) {
+            for_each_sample(lo, [&](uint32_t c, uint32_t id) {
+                sp.sorted[kSplit ? cluster_take(remote(c)) : atomicAdd(s_count + c, 1u)] = id;
+            });
+        } else {
+            uint32_t* to = s_count + held;
+            for_each_sample(lo, [&](uint32_t c, uint32_t id) { to[atomicAdd(s_count + c, 1u)] = id; });
+            __syncthreads();
+            for (uint32_t i = tid; i < *block_sum; i += kSortThreads) sp.sorted[base + i] = to[i];
         }
         // nobody leaves, or clears the counters, while others still use them
-        if (sp.parts == 1) __syncthreads();
+        if (parts == 1) __syncthreads();
         else cluster_barrier();
     }
-    if (tid == 0 && part == 0) sp.regions[blockIdx.x / sp.parts] = make_uint2(region, placed);
+    return placed;
+}
+
+template <typename Source>
+__global__ void __launch_bounds__(kSortThreads, 2)
+sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ SortParams sp) {
+    extern __shared__ uint32_t s_count[];   // [kSortCells]
+    __shared__ uint32_t warp_sum[32];
+    __shared__ uint32_t block_sum;           // samples this CTA's counters, or slice of them, hold
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sp.ticket = 0u;
+    const uint32_t parts = sp.parts, region = blockIdx.x / parts;
+    if (!src.ok()) {         // the same answer in every CTA
+        if (threadIdx.x == 0) sp.regions[region] = make_uint2(0u, 0u);
+        return;
+    }
+    src.clear();
+    const typename Source::Map map = src.map(region);
+    // Two levels of 14 and 53 samples per cell in two parts took 80 us split, 32 merged; at 5 per cell
+    // the two are equal. Alone from 16 samples per cell and CTA on.
+    const bool fits = map.cells <= kSortCells;
+    uint32_t placed;
+    if (parts == 1 || (fits && src.samples / parts >= 16u * map.cells))
+        placed = sort_map<Counters::kAlone>(src, sp, map, s_count, warp_sum, &block_sum);
+    else if (fits && 2u * src.samples >= parts * map.cells)
+        placed = sort_map<Counters::kMerged>(src, sp, map, s_count, warp_sum, &block_sum);
+    else
+        placed = sort_map<Counters::kSplit>(src, sp, map, s_count, warp_sum, &block_sum);
+    if (threadIdx.x == 0 && blockIdx.x % parts == 0) sp.regions[region] = make_uint2(region * src.samples, placed);
 }
 
 // Warps draw tickets in order; a ticket is up to `len` consecutive sorted samples of one region.
@@ -306,14 +368,32 @@ template <typename Source>
 static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp, int sm_count,
                                cudaStream_t stream) {
     auto kern = sort_cells_kernel<Source>;
-    const size_t smem = kSortCells * sizeof(uint32_t);
+    // The cluster that is done first, by a model of the time in ns: an SM works on two CTAs at a time, 1.5
+    // per sample of both (one alone takes 0.65 of the time of two); a cluster costs 8 us, and 3.1 per
+    // cell and other CTA (merged) or 2.8 per sample (split). More parts have to gain a tenth: apart,
+    // they leave shorter runs. (Samples alone, us: 256 maps of 80 K 258 / 227 / 208 in 1 / 4 / 8 parts,
+    // 192 of 20 K 67 / 56 / 57 in 1 / 2 / 4, 96 of 107 K 111 / 127 / 95 / 84 in 1 / 2 / 4 / 8; 144 of
+    // 5 K, whole sort: 17 / 28 in 1 / 2.)
+    double least = 0.0;
+    for (uint32_t parts = 1; parts <= kMaxSortParts; parts *= 2) {
+        const uint32_t per_sm = (maps * parts + sm_count - 1) / sm_count;
+        const double share = (per_sm / 2 + 0.65 * (per_sm % 2)) / parts;
+        const double between = std::min(3.1 * src.mean_cells * (parts - 1), 2.8 * src.samples);
+        const double ns = share * (1.5 * src.samples + (parts > 1 ? between : 0.0)) + (parts > 1 ? 8000.0 : 0.0);
+        if (parts == 1 || ns < 0.9 * least) {
+            least = ns;
+            sp.parts = parts;
+        }
+    }
+    sp.nregions = maps;
+    // more room only where that lets every map's samples be staged (it costs L1: the encoder shape's
+    // sort takes 82 instead of 69 us)
+    const uint32_t part = (src.samples - 1) / sp.parts + 1;
+    sp.room = part + src.most_cells <= kSortRoom && part >= 16u * src.most_cells ? kSortRoom : kSortCells;
+    const size_t smem = sp.room * sizeof(uint32_t);
     int resident = 0;   // (asked for the shared-memory limit that the call sets)
     const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kSortThreads, smem, &resident);
     if (e != cudaSuccess) return e;
-    // the smallest cluster that gives most SMs work
-    sp.parts = 1;
-    while (sp.parts < kMaxSortParts && maps * sp.parts < 3u * sm_count / 2u) sp.parts *= 2;
-    sp.nregions = maps;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(maps * sp.parts);
     cfg.blockDim = dim3(kSortThreads);

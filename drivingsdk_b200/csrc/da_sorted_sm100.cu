@@ -26,6 +26,8 @@ struct AggregationSamples {
     DaParams p;
     DaDivs fd;
     uint32_t samples;   // of one map: A * Pts
+    uint32_t period, period_step;   // 1, cams * scales
+    uint32_t most_cells, mean_cells;   // of a map
 
     struct Map {
         uint32_t cells, first;
@@ -52,7 +54,7 @@ struct AggregationSamples {
         const bool inside = xy.x > 0.f && xy.x < 1.f && xy.y > 0.f && xy.y < 1.f;
         return inside ? sample_cell<4>(xy, m.W, m.H) : kNoRow;
     }
-    __device__ __forceinline__ void drop(uint32_t) const {}   // the gradients start from zero
+    __device__ __forceinline__ void clear() const {}   // the caller does it
 };
 
 template <typename T, int NV>
@@ -289,8 +291,9 @@ template <typename T>
 static cudaError_t launch_da_sorted(const DaParams& p, SortParams sp, int sm_count, cudaStream_t stream) {
     const uint32_t samples = static_cast<uint32_t>(p.A) * p.Pts;
     const DaDivs fd{make_fastdiv(p.scales), make_fastdiv(p.cams), make_fastdiv(p.Pts), make_fastdiv(p.A)};
-    cudaError_t e = launch_sort(AggregationSamples<T>{p, fd, samples},
-                                static_cast<uint32_t>(p.B) * p.cams * p.scales, sp, sm_count, stream);
+    const uint32_t maps = static_cast<uint32_t>(p.cams) * p.scales, F = static_cast<uint32_t>(p.F);
+    cudaError_t e = launch_sort(AggregationSamples<T>{p, fd, samples, 1u, maps, 2u * (F + 1u), F / maps},
+                                static_cast<uint32_t>(p.B) * maps, sp, sm_count, stream);
     if (e != cudaSuccess) return e;
     const LaunchShape ls{sm_count, 0};
     auto launch = [&](auto kern) -> cudaError_t {

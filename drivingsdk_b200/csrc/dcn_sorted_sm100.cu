@@ -25,6 +25,8 @@ using namespace msda;
 struct ConvSamples {
     DcnParams p;
     uint32_t samples;   // of one map: Ho * Wo * K
+    uint32_t period, period_step;   // K, DG * K
+    uint32_t most_cells, mean_cells;   // of a map
 
     struct Map {
         uint32_t cells, n, dg;
@@ -48,7 +50,7 @@ struct ConvSamples {
         return static_cast<uint32_t>(__float2int_rd(at.x) + 1) * static_cast<uint32_t>(p.W + 1) +
                static_cast<uint32_t>(__float2int_rd(at.y) + 1);
     }
-    __device__ __forceinline__ void drop(uint32_t) const {}   // none: every sample has a cell
+    __device__ __forceinline__ void clear() const {}   // every sample has a cell
     static __device__ __forceinline__ bool inside(const DcnParams& p, float2 at) {   // false for NaN
         return at.x > -1.f && at.y > -1.f && at.x < static_cast<float>(p.H) && at.y < static_cast<float>(p.W);
     }
@@ -407,8 +409,8 @@ size_t up(size_t v) { return (v + 255) / 256 * 256; }
 size_t sorted_bytes(const dcn_shape* s, const Derived& d) {
     const size_t items = static_cast<size_t>(d.M) * s->deform_groups * d.K;
     const size_t maps = static_cast<size_t>(s->N) * s->deform_groups;
-    // 32-bit offsets, in quads
-    if (d.M * s->groups * d.Kd / 4 >= (1ll << 32) ||
+    // 32-bit offsets, in quads; no more taps than the sort has threads (its Source::period)
+    if (d.K > static_cast<int>(kSortThreads) || d.M * s->groups * d.Kd / 4 >= (1ll << 32) ||
         static_cast<long long>(s->N) * s->H * s->W * (s->C / 4) >= (1ll << 32) || items + maps >= (1ull << 28))
         return 0;
     return 256 + up(maps * sizeof(uint2)) + up(items * 4);
@@ -445,7 +447,10 @@ int launch_gather_sorted(const DcnParams& p, void* workspace, long long M, int N
                          int sm_count, cudaStream_t stream) {
     const uint32_t maps = static_cast<uint32_t>(N) * p.DG;
     SortParams sp = sorted_params(workspace, static_cast<size_t>(M) * p.DG * p.K, maps);
-    cudaError_t e = launch_sort(ConvSamples{p, static_cast<uint32_t>(p.HoWo) * p.K}, maps, sp, sm_count, stream);
+    const uint32_t K = static_cast<uint32_t>(p.K);
+    const uint32_t cells = static_cast<uint32_t>(p.H + 1) * static_cast<uint32_t>(p.W + 1) + 1u;
+    const ConvSamples samples{p, static_cast<uint32_t>(p.HoWo) * K, K, static_cast<uint32_t>(p.DG) * K, cells, cells};
+    cudaError_t e = launch_sort(samples, maps, sp, sm_count, stream);
     if (e != cudaSuccess) return note_cuda_error(e);
     auto launch = [&](auto kern, int channels) -> cudaError_t {
         uint32_t slices = 1, grid = 0;

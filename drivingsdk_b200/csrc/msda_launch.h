@@ -74,6 +74,7 @@ struct SortParams {
     FastDiv fd_p;           // division by the points per level
     // set by the launch:
     uint32_t parts;         // CTAs per (batch, head, level) of the sort
+    uint32_t room;          // words of shared memory of each
     uint32_t nregions, tickets, tickets_per_region;
     FastDiv fd_tickets;     // division by tickets_per_region
     uint32_t stream;        // sorted samples per stream
