@@ -204,7 +204,21 @@ __device__ __forceinline__ SortedSample set_up_sample(const Params& p, const Sor
 // above them).
 constexpr uint32_t kEnters = 1;      // its cell is not the previous sample's
 constexpr uint32_t kJumps = 2;       // ... and not the next one to the right either
-constexpr uint32_t kAmplified = 4;   // wants its dot products in double
+
+// Rows of grad_out in flight per lane and CTAs per SM. The kernel waits for the latency of its own
+// instructions more than for memory (with grad_out from L1 it is no faster), so rows in flight count as
+// long as no register spills: at 80 registers two, more with one CTA less. Measured (us, main kernel):
+//   128 channels, 16 bit, 20.5 M samples   2 rows x 3 CTAs 1820   4 x 2 1772   8 x 2 1622
+//   128 channels, fp32, 4.6 M               630   617   1009 (spills)
+//    64 channels, fp32, 5.1 M               378   394    673
+//    32 channels, fp32, 4.6 M               265   267    358
+//    16 channels, fp32, 5.1 M               196   173      -
+template <typename T, int NV, int LPR>
+struct SortedTile {
+    static constexpr bool kMore = NV == 1 && (LPR == 32 || LPR == 4);
+    static constexpr int kRows = !kMore ? 2 : (LPR == 32 && sizeof(T) == 2) ? 8 : 4;
+    static constexpr int kCtas = (kMore || NV > 1) ? 2 : 3;
+};
 
 // Bilinear main kernel. T: type of value / grad_out; TL: type of locations, weights and their
 // gradients. LPR lanes cover a row (4 channels each, NV times; lanes past D are idle, D need not
@@ -214,10 +228,10 @@ constexpr uint32_t kAmplified = 4;   // wants its dot products in double
 // fp32. RAGGED: some of those lanes are past D; without their checks the rest is 1 to 4 % faster
 // (encoder shape, fp32, 32 channels: 284 -> 274 us; 128 channels, bf16: 1894 -> 1867 us).
 template <typename T, typename TL, int NV, int LPR, bool RAGGED>
-__global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 3)
+__global__ void __launch_bounds__(kThreadsPerCta, SortedTile<T, NV, LPR>::kCtas)
 msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
     constexpr int S = 32 / LPR;       // streams
-    constexpr int U = 2;              // rows of grad_out in flight per lane
+    constexpr int U = SortedTile<T, NV, LPR>::kRows;   // rows of grad_out in flight per lane
     // fp32 bilinear operator: some dot products need double precision (see sample_grad)
     constexpr bool WIDE = sizeof(TL) == 4 && sizeof(T) == 4;
     static_assert(LPR % U == 0, "a round is LPR steps");
@@ -230,6 +244,13 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
     __shared__ double s_wide[WIDE ? kWarpsPerCta : 1][WIDE ? 32 : 1][4];
     __shared__ uint2 s_rec[kWarpsPerCta][32];
     __shared__ uint32_t s_row[kWarpsPerCta][32];
+    // what a lane needs of its sample after the products, out of the way of their registers
+    struct Parked {
+        uint32_t id, cell;
+        float lw, lh, a, wf, hf;
+        uint32_t amplified;
+    };
+    __shared__ __align__(16) Parked s_park[kWarpsPerCta][32];
     if (!load_sort_levels(p, lv)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / LPR, j = lane % LPR;
@@ -308,9 +329,11 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
             next.id = next_id;
             load_raw<TL>(p, next, at + LPR < end);
             next_id = at + 2 * LPR < end ? __ldg(sp.sorted + at + 2 * LPR) : 0u;
-            const SortedSample s = set_up_sample<4>(p, sp, lv, raw, at < end);
-            raw = next;
+            uint32_t m_enter, m_jump, m_wide;   // bit = lane = (step, stream) of the round
             {
+                const SortedSample s = set_up_sample<4>(p, sp, lv, raw, at < end);
+                raw = next;
+                s_park[warp][lane] = Parked{s.id, s.cell, s.lw, s.lh, s.a, s.wf, s.hf, s.amplified ? 1u : 0u};
                 uint32_t prow = __shfl_up_sync(0xffffffffu, s.row, S);
                 uint32_t pcell = __shfl_up_sync(0xffffffffu, s.cell, S);
                 const uint32_t srow = __shfl_sync(0xffffffffu, cur, my_stream * LPR);
@@ -325,7 +348,9 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
                                        ((pcell >> 1) & 5u) == (s.cell & 5u);
                     flags |= right ? kEnters : (kEnters | kJumps);
                 }
-                if (WIDE && s.amplified) flags |= kAmplified;
+                m_enter = __ballot_sync(0xffffffffu, flags & kEnters);
+                m_jump = __ballot_sync(0xffffffffu, flags & kJumps);
+                m_wide = WIDE ? __ballot_sync(0xffffffffu, s.amplified) : 0u;
                 s_w[warp][lane][0] = make_ulonglong2(pack2(s.w[0], s.w[0]), pack2(s.w[1], s.w[1]));
                 s_w[warp][lane][1] = make_ulonglong2(pack2(s.w[2], s.w[2]), pack2(s.w[3], s.w[3]));
                 s_rec[warp][lane] = make_uint2(s.task * p.row_units, flags);
@@ -350,34 +375,9 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
                     }
                 }
                 float d[U * 4];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
+                constexpr uint32_t kStep = (S == 32) ? 0xffffffffu : (1u << S) - 1u;   // bits of a step
+                auto products = [&](int u) {
                     const int slot = (t0 + u) * S + g;
-                    const uint32_t any = (S == 1) ? flags[u] : __reduce_or_sync(0xffffffffu, flags[u] & 7u);
-                    if (any & kEnters) {
-                        const bool enters = flags[u] & kEnters, jumps = flags[u] & kJumps;
-                        flush(0, enters);
-                        flush(2, enters);
-                        if (any & kJumps) {
-                            flush(1, jumps);
-                            flush(3, jumps);
-                            clear(0, jumps);
-                            clear(2, jumps);
-                        }
-                        shift(0, enters && !jumps);
-                        shift(2, enters && !jumps);
-                        clear(1, enters);
-                        clear(3, enters);
-                        cur = s_row[warp][slot];      // the same for a stream that stays
-                        cell = flags[u] >> 4;
-                        below = (cell >> 4) * step_x;
-                        if (any & kJumps) {
-                            fetch(0, jumps);
-                            fetch(2, jumps);
-                        }
-                        fetch(1, enters);
-                        fetch(3, enters);
-                    }
                     f32x2 w[4];
                     {
                         const ulonglong2 w01 = s_w[warp][slot][0], w23 = s_w[warp][slot][1];
@@ -400,27 +400,64 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
                         const float2 h = unpack2(a2);
                         d[u * 4 + c] = h.x + h.y;
                     }
-                    if constexpr (WIDE) {
-                        // A step with an amplified sample forms its dot products in double as
-                        // well; each sample takes the kind it asked for, so its gradients do
-                        // not depend on which samples share the step.
-                        if (any & kAmplified) {
-                            double dd[4] = {0.0, 0.0, 0.0, 0.0};
+                };
+                // Most often nothing but products: without a branch between them the steps overlap.
+                const uint32_t here = (m_enter | m_wide) >> (t0 * S);
+                if (NV == 1 && (here & ((1u << (U * S - 1) << 1) - 1u)) == 0u) {
 #pragma unroll
-                            for (int k = 0; k < NV; ++k)
+                    for (int u = 0; u < U; ++u) products(u);
+                } else {
 #pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    const float2 gf = unpack2(go[u][k][e]);
-                                    const double gx = gf.x, gy = gf.y;
+                    for (int u = 0; u < U; ++u) {
+                        const int slot = (t0 + u) * S + g;
+                        if ((m_enter >> ((t0 + u) * S)) & kStep) {
+                            const bool enters = flags[u] & kEnters, jumps = flags[u] & kJumps;
+                            const bool any_jumps = ((m_jump >> ((t0 + u) * S)) & kStep) != 0u;
+                            flush(0, enters);
+                            flush(2, enters);
+                            if (any_jumps) {
+                                flush(1, jumps);
+                                flush(3, jumps);
+                                clear(0, jumps);
+                                clear(2, jumps);
+                            }
+                            shift(0, enters && !jumps);
+                            shift(2, enters && !jumps);
+                            clear(1, enters);
+                            clear(3, enters);
+                            cur = s_row[warp][slot];      // the same for a stream that stays
+                            cell = flags[u] >> 4;
+                            below = (cell >> 4) * step_x;
+                            if (any_jumps) {
+                                fetch(0, jumps);
+                                fetch(2, jumps);
+                            }
+                            fetch(1, enters);
+                            fetch(3, enters);
+                        }
+                        products(u);
+                        if constexpr (WIDE) {
+                            // A step with an amplified sample forms its dot products in double as
+                            // well; each sample takes the kind it asked for, so its gradients do
+                            // not depend on which samples share the step.
+                            if ((m_wide >> ((t0 + u) * S)) & kStep) {
+                                double dd[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-                                    for (int c = 0; c < 4; ++c) {
-                                        const float2 vf = unpack2(val[c][k][e]);
-                                        dd[c] = fma(static_cast<double>(vf.x), gx, dd[c]);
-                                        dd[c] = fma(static_cast<double>(vf.y), gy, dd[c]);
+                                for (int k = 0; k < NV; ++k)
+#pragma unroll
+                                    for (int e = 0; e < 2; ++e) {
+                                        const float2 gf = unpack2(go[u][k][e]);
+                                        const double gx = gf.x, gy = gf.y;
+#pragma unroll
+                                        for (int c = 0; c < 4; ++c) {
+                                            const float2 vf = unpack2(val[c][k][e]);
+                                            dd[c] = fma(static_cast<double>(vf.x), gx, dd[c]);
+                                            dd[c] = fma(static_cast<double>(vf.y), gy, dd[c]);
+                                        }
                                     }
-                                }
-                            const double r = reduce_values<4, LPR>(dd, j);
-                            if (j % (LPR / 4) == 0) s_wide[warp][slot][j / (LPR / 4)] = r;
+                                const double r = reduce_values<4, LPR>(dd, j);
+                                if (j % (LPR / 4) == 0) s_wide[warp][slot][j / (LPR / 4)] = r;
+                            }
                         }
                     }
                 }
@@ -443,6 +480,7 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
             // ---- lane = sample: gradients of location and weight ---------------------------
             if (at < end) {
                 using Acc = typename std::conditional<WIDE, double, float>::type;
+                const Parked s = s_park[warp][lane];
                 const float4 h4 = *reinterpret_cast<const float4*>(s_w[warp][lane]);
                 Acc S4[4] = {h4.x, h4.y, h4.z, h4.w};
                 if constexpr (WIDE) {
