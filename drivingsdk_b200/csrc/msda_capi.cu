@@ -169,26 +169,32 @@ bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, SortP
     return true;
 }
 
-// Where sorting pays: the gain is the rows that samples of one cell share, the cost a sort of
-// 15-25 ps per sample, so it takes enough samples per cell, fewer of them the longer the rows.
-// Measured on one level set from 64x100 down, uniform locations, old / sorted (us):
-//   D = 128  0.26 M samples, 1.9 per cell: 128 / 122   0.77 M, 5.6: 288 / 190   6.9 M, 51: 2412 / 1028
-//   D = 64   5.6 per cell: 154 / 145   17: 418 / 285   51: 1216 / 669
-//   D = 32   17 per cell: 204 / 233 (fp32), 233 / 209 (bf16)   51: 582 / 495, 654 / 411
-// (fp32 unless noted; with one query per pixel and samples around it, as in an encoder, 17 per cell
-// pays for fp32 at D = 32 too: 431 / 366). Below about 0.1 M samples two more launches cost more
-// than they save. The nearest-pixel operator has one row per sample and no double-precision
-// dot products: 519 / 397 at 24 x 107 k samples on 375 pixels.
+// Where sorting pays: the gain is the rows that samples of one cell share, the cost a sort of 9 to 25 ps
+// per sample, so it takes enough samples per cell, fewer of them the longer the rows, and enough samples
+// for two more launches and their tails. Measured, whole backward, unsorted / sorted (us):
+//   samples, per cell      D = 16 f32, bf16        32 f32, bf16            64 f32, bf16           128 f32, bf16
+//    0.64 M uniform   9.4   56/69     67/72         71/75     81/76        130/93    118/95       247/130   218/126
+//    0.64 M grid      4.0   83/85     77/85         89/112    93/97        159/165   142/136
+//    0.77 M uniform   2.8   65/79     71/83         87/114    97/101       159/167   155/165      300/222   298/245
+//    1.28 M           2.6   96/128   109/130       136/171   157/177       261/237   263/259
+//    1.28 M          18.8   87/87    118/87        118/106   134/101       235/132   208/130
+//    2.56 M grid      4.0  282/253   245/230       297/357   321/294       566/533   517/435
+//    3.84 M uniform   2.6  255/276   300/292       373/392   441/411       729/564   755/648
+//    3.07 M          11.3  192/167   216/165       272/220   307/208       544/292   484/296
+// The nearest-pixel operator has one row per sample and no double-precision dot products: 519 / 397 at
+// 24 x 107 k samples on 375 pixels.
 bool sort_pays(const SortPlan& s, int K, int H, int D, int dtype, int B, int mode) {
     if (mode == kFused || g_tune_sort.load() == 0) return false;
     if (g_tune_sort.load() == 2) return true;
-    if (s.nsamples < 100000u) return false;
-    const double per_cell = static_cast<double>(s.nsamples) / (static_cast<double>(B) * K * H);
+    const uint32_t n = s.nsamples;
+    if (n < 100000u) return false;
+    const double per_cell = static_cast<double>(n) / (static_cast<double>(B) * K * H);
     if (mode == kNearest) return per_cell >= 16.0;
-    if (D > 64) return per_cell >= 3.0;
-    if (D > 32) return per_cell >= 6.0;
-    if (D > 16) return per_cell >= (dtype == MSDA_F32 ? 15.0 : 12.0) && s.nsamples >= 1000000u;
-    return per_cell >= (dtype == MSDA_F32 ? 50.0 : 25.0);
+    if (D > 64) return per_cell >= 2.0;
+    if (D > 32) return per_cell >= (n >= 1200000u ? 2.5 : 6.0);
+    if (n < 1000000u) return false;
+    if (dtype == MSDA_F32) return per_cell >= 9.0 && (D > 16 || n >= 2000000u);
+    return per_cell >= (n >= 3500000u ? 2.5 : n >= 2500000u ? 3.5 : 9.0);
 }
 
 // Tasks that one warp pass takes together: as many as fill its lanes with samples, but fewer where
