@@ -519,6 +519,7 @@ gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     constexpr int SL = 32 / LPR;    // samples per step
     __shared__ SortLevels lv;
     __shared__ float s_dot[kWarpsPerCta][32];
+    __shared__ uint2 s_rec[kWarpsPerCta][32];   // offset of the sample's grad_out row, weight
     if (!load_sort_levels(p, lv)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = lane % LPR, g = lane / LPR;
@@ -577,6 +578,45 @@ gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             }
             const uint32_t m_other =
                 __ballot_sync(0xffffffffu, lane < n && (s.row != prow || s.cell != pcell));
+            s_rec[warp][lane] = make_uint2(s.task * p.row_units, __float_as_uint(s.a));
+            __syncwarp();
+            // U * SL samples of the pixel from i0 on; WHOLE: none of them lies past `last`
+            auto products = [&](int i0, int last, auto whole_tag) {
+                constexpr bool WHOLE = decltype(whole_tag)::value;
+                f32x2 go[U][NV][2];
+                float w[U], d[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int i = i0 + u * SL + g;
+                    const bool live = WHOLE || i < last;
+                    const uint2 rec = s_rec[warp][WHOLE ? i : min(i, 31)];
+                    w[u] = live ? __uint_as_float(rec.y) : 0.f;
+                    const T* row = glane + static_cast<size_t>(rec.x) * 4;
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        if (!WHOLE || RAGGED) go[u][k][0] = go[u][k][1] = 0ull;
+                        if (live && on[k]) load_quad<T>(row + k * (LPR * 4), go[u][k]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const f32x2 w2 = pack2(w[u], w[u]);
+                    f32x2 a2 = 0ull;
+#pragma unroll
+                    for (int k = 0; k < NV; ++k)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            acc[k][e] = fma2(w2, go[u][k][e], acc[k][e]);
+                            a2 = (k + e == 0) ? mul2(val[k][e], go[u][k][e])
+                                              : fma2(val[k][e], go[u][k][e], a2);
+                        }
+                    const float2 h = unpack2(a2);
+                    d[u] = h.x + h.y;
+                }
+                const float r = reduce_values<U, LPR>(d, j);
+                const int i = i0 + (j / (LPR / U)) * SL + g;
+                if (j % (LPR / U) == 0 && (WHOLE || i < last)) dot[i] = r;
+            };
 #pragma unroll 1
             for (int first = 0; first < n;) {
                 // samples [first, last) share a pixel
@@ -593,43 +633,10 @@ gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ 
                             load_quad<T>(vlane + (static_cast<size_t>(cur) + k * LPR) * 4, val[k]);
                     }
                 }
+                int i0 = first;
 #pragma unroll 1
-                for (int i0 = first; i0 < last; i0 += U * SL) {
-                    f32x2 go[U][NV][2];
-                    float w[U], d[U];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int i = i0 + u * SL + g;
-                        const uint32_t task = __shfl_sync(0xffffffffu, s.task, i);
-                        w[u] = __shfl_sync(0xffffffffu, s.a, i);
-                        const bool live = i < last;
-                        const T* row = glane + static_cast<size_t>(task) * p.D;
-#pragma unroll
-                        for (int k = 0; k < NV; ++k) {
-                            go[u][k][0] = go[u][k][1] = 0ull;
-                            if (live && on[k]) load_quad<T>(row + k * (LPR * 4), go[u][k]);
-                        }
-                        if (!live) w[u] = 0.f;
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const f32x2 w2 = pack2(w[u], w[u]);
-                        f32x2 a2 = 0ull;
-#pragma unroll
-                        for (int k = 0; k < NV; ++k)
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                acc[k][e] = fma2(w2, go[u][k][e], acc[k][e]);
-                                a2 = (k + e == 0) ? mul2(val[k][e], go[u][k][e])
-                                                  : fma2(val[k][e], go[u][k][e], a2);
-                            }
-                        const float2 h = unpack2(a2);
-                        d[u] = h.x + h.y;
-                    }
-                    const float r = reduce_values<U, LPR>(d, j);
-                    const int i = i0 + (j / (LPR / U)) * SL + g;
-                    if (j % (LPR / U) == 0 && i < last) dot[i] = r;
-                }
+                for (; i0 + U * SL <= last; i0 += U * SL) products(i0, last, std::true_type{});
+                if (i0 < last) products(i0, last, std::false_type{});
                 first = last;
             }
             __syncwarp();
