@@ -249,7 +249,7 @@ template <int NV>
 __global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 3)
 scatter_sorted_kernel(const __grid_constant__ DcnParams p, const __grid_constant__ SortParams sp,
                       uint32_t slices) {
-    constexpr int U = NV > 1 ? 2 : 4;    // samples in flight
+    constexpr int U = 4;    // samples in flight (512 channels: 181 us with two, 156 with four)
     __shared__ __align__(16) Record s_rec[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t units = static_cast<uint32_t>(p.C) / 4, step_y = static_cast<uint32_t>(p.W) * units;
