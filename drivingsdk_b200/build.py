@@ -25,7 +25,7 @@ EXT = os.path.join(PKG, "_C.so")
 
 CUDA_SOURCES = ["msda_capi.cu", "resident_ctas.cu", "msda_fwd_sm100.cu", "msda_bwd_sm100.cu",
                 "gka_fwd_sm100.cu", "gka_bwd_sm100.cu", "msda_bwd_sorted_sm100.cu", "gka_bwd_sorted_sm100.cu",
-                "msda_fused_fwd_sm100.cu", "msda_fused_bwd_sm100.cu", "da_sm100.cu", "da_sorted_sm100.cu",
+                "msda_fused_fwd_sm100.cu", "msda_fused_bwd_sm100.cu", "msda_fused_sorted_sm100.cu", "da_sm100.cu", "da_sorted_sm100.cu",
                 "msda_static_scratch.cu", "hw_probe_sm100.cu", "resnet_ops_sm100.cu", "dcn_sm100.cu",
                 "dcn_split_sm100.cu", "dcn_sorted_sm100.cu", "gemm_split_sm100.cu", "gemm_simt_sm100.cu",
                 "gemm_tc_sm100.cu"]

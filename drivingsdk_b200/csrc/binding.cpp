@@ -606,7 +606,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> msda_fused_backward(
     const int dt = dtype_code(value.scalar_type());
     at::Tensor workspace;
     void* ws_ptr = nullptr;
-    const size_t ws_bytes = msda_sm100_backward_workspace_bytes(d.B, d.K, d.H, d.D, dt);
+    const size_t ws_bytes =
+        msda_sm100_fused_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
     if (ws_bytes > 0) {
         workspace = at::empty({static_cast<int64_t>(ws_bytes / sizeof(float))},
                               value.options().dtype(at::kFloat));

@@ -145,15 +145,16 @@ int set_row_units(Params& p, const RowPlan& rp, int dtype) {
 }
 
 // Layout of the sorted backward's workspace: fp32 accumulation rows (16-bit tensors only),
-// ticket counter, regions, sorted sample numbers.
+// ticket counter, regions, sorted sample numbers; for the fused operator locations, weights and, 16-bit
+// tensors only, their gradients.
 struct SortPlan {
-    size_t ticket, regions, sorted, total;
+    size_t ticket, regions, sorted, loc, prob, grad_loc, grad_attn, total;
     uint32_t nsamples;
 };
 
 // False where the sorted backward does not apply: rows that are not whole groups of four
 // channels, more samples than 32-bit counters hold.
-bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, SortPlan* s) {
+bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, int mode, SortPlan* s) {
     if (D % 4 != 0) return false;
     const unsigned long long n = 1ull * B * Q * H * L * P;
     // ... nor as many tickets (regions of a few samples each get one)
@@ -165,7 +166,12 @@ bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, SortP
     s->ticket = dtype == MSDA_F32 ? 0 : up(static_cast<size_t>(B) * K * H * D * 4);
     s->regions = s->ticket + 256;
     s->sorted = s->regions + up(static_cast<size_t>(B) * H * L * sizeof(uint2));
-    s->total = s->sorted + up(n * 4);
+    s->loc = s->sorted + up(n * 4);
+    s->prob = s->loc + (mode == kFused ? up(n * 8) : 0);
+    s->grad_loc = s->prob + (mode == kFused ? up(n * 4) : 0);
+    const bool own = mode == kFused && dtype != MSDA_F32;
+    s->grad_attn = s->grad_loc + (own ? up(n * 8) : 0);
+    s->total = s->grad_attn + (own ? up(n * 4) : 0);
     return true;
 }
 
@@ -182,14 +188,24 @@ bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, SortP
 //    3.84 M uniform   2.6  255/276   300/292       373/392   441/411       729/564   755/648
 //    3.07 M          11.3  192/167   216/165       272/220   307/208       544/292   484/296
 // The nearest-pixel operator has one row per sample and no double-precision dot products: 519 / 397 at
-// 24 x 107 k samples on 375 pixels.
+// 24 x 107 k samples on 375 pixels. The fused operator pays for two more kernels:
+//    0.64 M           9.4   66/87     75/95         83/102    89/104       144/124   128/124      257/157   228/155
+//    1.28 M           2.6  110/160   130/171       156/200   179/218       298/263   294/296      612/374   593/441
+//    3.84 M           2.6  296/353   343/372       419/463   487/495       824/646   804/736     1798/1075 1872/1208
+//    3.07 M          11.3  239/251   243/247       317/310   320/292       585/378   488/373     1142/560   974/509
 bool sort_pays(const SortPlan& s, int K, int H, int D, int dtype, int B, int mode) {
-    if (mode == kFused || g_tune_sort.load() == 0) return false;
+    if (g_tune_sort.load() == 0) return false;
     if (g_tune_sort.load() == 2) return true;
     const uint32_t n = s.nsamples;
     if (n < 100000u) return false;
     const double per_cell = static_cast<double>(n) / (static_cast<double>(B) * K * H);
     if (mode == kNearest) return per_cell >= 16.0;
+    if (mode == kFused) {
+        if (n < 500000u || D <= 16) return false;
+        if (D > 64) return per_cell >= 2.0;
+        if (D > 32) return per_cell >= (n >= (dtype == MSDA_F32 ? 1200000u : 2500000u) ? 2.5 : 9.0);
+        return per_cell >= 9.0 && n >= 2000000u;
+    }
     if (D > 64) return per_cell >= 2.0;
     if (D > 32) return per_cell >= (n >= 1200000u ? 2.5 : 6.0);
     if (n < 1000000u) return false;
@@ -315,7 +331,7 @@ int backward_impl(const void* value, const int32_t* shapes, const int32_t* start
     const bool acc_f32 = use_ws && dtype != MSDA_F32;
     // the sorted form, where the caller brought the workspace for it
     SortPlan plan;
-    if (use_ws && plan_sort(B, K, H, D, L, Q, P, dtype, &plan) &&
+    if (use_ws && plan_sort(B, K, H, D, L, Q, P, dtype, mode, &plan) &&
         sort_pays(plan, K, H, D, dtype, B, mode) &&
         workspace && workspace_bytes >= plan.total && aligned_to(workspace, 16) &&
         aligned_to(value, 4 * e) && aligned_to(grad_out, 4 * e) &&
@@ -340,11 +356,24 @@ int backward_impl(const void* value, const int32_t* shapes, const int32_t* start
             cudaError_t ce = cudaMemsetAsync(acc, 0, static_cast<size_t>(nval) * sizeof(float), stream);
             if (ce != cudaSuccess) return fail_cuda(ce);
             prof_record(2, stream);
-            ce = nearest ? msda::launch_gka_backward_sorted(p, sp, dtype, shape, stream)
-                                     : msda::launch_backward_sorted(p, sp, dtype, shape, stream);
+            if (mode == kFused) {
+                p.ref = ref;
+                p.grad_ref = grad_ref;
+                msda::FusedSamples fs;
+                fs.loc = reinterpret_cast<float2*>(ws + plan.loc);
+                fs.prob = reinterpret_cast<float*>(ws + plan.prob);
+                fs.grad_loc = acc_f32 ? reinterpret_cast<float2*>(ws + plan.grad_loc) : static_cast<float2*>(grad_loc);
+                fs.grad_attn = acc_f32 ? reinterpret_cast<float*>(ws + plan.grad_attn) : static_cast<float*>(grad_attn);
+                ce = cudaMemsetAsync(grad_ref, 0, static_cast<size_t>(B) * Q * L * 2 * sizeof(float), stream);
+                if (ce == cudaSuccess)
+                    ce = msda::launch_fused_backward_sorted(p, sp, fs, dtype, shape, stream);
+            } else {
+                ce = nearest ? msda::launch_gka_backward_sorted(p, sp, dtype, shape, stream)
+                             : msda::launch_backward_sorted(p, sp, dtype, shape, stream);
+            }
             prof_record(3, stream);
             if (ce != cudaSuccess) return fail_cuda(ce);
-            g_launches.fetch_add(2, std::memory_order_relaxed);
+            g_launches.fetch_add(mode == kFused ? 4 : 2, std::memory_order_relaxed);
             if (acc_f32) {
                 ce = msda::launch_downcast(acc, grad_value, nval, dtype, stream);
                 if (ce != cudaSuccess) return fail_cuda(ce);
@@ -530,7 +559,7 @@ size_t msda_sm100_backward_workspace_bytes(int B, int K, int H, int D, int dtype
 static size_t sorted_workspace(int B, int K, int H, int D, int L, int Q, int P, int dtype, int mode) {
     SortPlan plan;
     if (check_dims(B, K, H, D, L, Q, P, dtype) != MSDA_OK ||
-        !plan_sort(B, K, H, D, L, Q, P, dtype, &plan) || !sort_pays(plan, K, H, D, dtype, B, mode))
+        !plan_sort(B, K, H, D, L, Q, P, dtype, mode, &plan) || !sort_pays(plan, K, H, D, dtype, B, mode))
         return msda_sm100_backward_workspace_bytes(B, K, H, D, dtype);
     return plan.total;
 }
@@ -538,6 +567,11 @@ static size_t sorted_workspace(int B, int K, int H, int D, int L, int Q, int P, 
 size_t msda_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
                                                   int dtype) {
     return sorted_workspace(B, K, H, D, L, Q, P, dtype, kBilinear);
+}
+
+size_t msda_sm100_fused_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
+                                                        int dtype) {
+    return sorted_workspace(B, K, H, D, L, Q, P, dtype, kFused);
 }
 
 size_t gka_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,

@@ -90,6 +90,17 @@ cudaError_t launch_fused_forward(const Params& p, int dtype, const RowPlan& rp,
 cudaError_t launch_fused_backward(const Params& p, int dtype, int acc_f32, const RowPlan& rp,
                                   const LaunchShape& ls, cudaStream_t stream);
 
+// ... its backward over cell-sorted samples. fp32, one entry per sample; device memory, part of the
+// caller's workspace (the gradients may be the result tensors if those are fp32).
+struct FusedSamples {
+    float2* loc;
+    float* prob;
+    float2* grad_loc;
+    float* grad_attn;
+};
+cudaError_t launch_fused_backward_sorted(const Params& p, const SortParams& sp, const FusedSamples& fs, int dtype,
+                                         const LaunchShape& ls, cudaStream_t stream);
+
 // Adds to the library-wide kernel launch counter (msda_sm100_launch_count).
 void count_launches(int n);
 

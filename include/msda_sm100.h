@@ -103,13 +103,15 @@ int msda_sm100_backward_ws(const void* value, const int32_t* spatial_shapes,
                            void* workspace, size_t workspace_bytes, int B, int K, int H, int D,
                            int L, int Q, int P, int dtype, void* stream);
 
-/* Workspace with which msda_sm100_backward_ws() and gka_sm100_backward_ws() take their form over
- * samples sorted by the cell they fall into, whose shared rows are loaded and reduced once. Any
+/* Workspace with which msda_sm100_backward_ws(), msda_sm100_fused_backward_ws() and
+ * gka_sm100_backward_ws() take their form over samples sorted by the cell they fall into, whose shared rows are loaded and reduced once. Any
  * smaller workspace that satisfies the rule above selects the form that needs no sort. Equals
  * msda_sm100_backward_workspace_bytes() where the sort would not apply (D not a multiple of
  * four) or not pay (few samples per cell). */
 size_t msda_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
                                                   int dtype);
+size_t msda_sm100_fused_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
+                                                        int dtype);
 size_t gka_sm100_backward_sorted_workspace_bytes(int B, int K, int H, int D, int L, int Q, int P,
                                                  int dtype);
 
