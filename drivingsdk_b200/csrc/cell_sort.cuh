@@ -32,14 +32,12 @@ __device__ __forceinline__ float2 load_pair<__nv_bfloat16>(const __nv_bfloat16* 
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
 
-// Zeros for `bytes` bytes from p on, by all threads of the grid.
-__device__ __forceinline__ void clear_bytes(void* p, size_t bytes) {
+// Zeros for `bytes` bytes from p on, by thread `first` of `step`.
+__device__ __forceinline__ void clear_bytes(void* p, size_t bytes, size_t first, size_t step) {
     unsigned char* at = static_cast<unsigned char*>(p);
     const size_t head = min(bytes, static_cast<size_t>((16u - (reinterpret_cast<uintptr_t>(at) & 15u)) & 15u));
     uint4* body = reinterpret_cast<uint4*>(at + head);
     const size_t pieces = (bytes - head) / 16, tail = head + pieces * 16;
-    const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
-    const size_t first = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     for (size_t i = first; i < pieces; i += step) body[i] = make_uint4(0u, 0u, 0u, 0u);
     if (first < head) at[first] = 0;
     if (first < bytes - tail) at[tail + first] = 0;
@@ -254,13 +252,25 @@ sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ So
     extern __shared__ uint32_t s_count[];   // [kSortCells]
     __shared__ uint32_t warp_sum[32];
     __shared__ uint32_t block_sum;           // samples this CTA's counters, or slice of them, hold
+    // CTAs past those that sort (whole clusters) fill with zeros what the main kernel adds to or may
+    // leave out: the sort leaves most of the memory's rate to them
+    const uint32_t sorting = sp.nregions * sp.parts;
+    if (blockIdx.x >= sorting) {
+        const size_t first = static_cast<size_t>(blockIdx.x - sorting) * kSortThreads + threadIdx.x;
+        const size_t step = static_cast<size_t>(gridDim.x - sorting) * kSortThreads;
+        if (sp.clear_sums) clear_bytes(src.sums(), src.sums_bytes(), first, step);
+        src.clear(first, step);
+        return;
+    }
+    if (gridDim.x == sorting)   // no room beside them
+        src.clear(static_cast<size_t>(blockIdx.x) * kSortThreads + threadIdx.x,
+                  static_cast<size_t>(sorting) * kSortThreads);
     if (blockIdx.x == 0 && threadIdx.x == 0) *sp.ticket = 0u;
     const uint32_t parts = sp.parts, region = blockIdx.x / parts;
     if (!src.ok()) {         // the same answer in every CTA
         if (threadIdx.x == 0) sp.regions[region] = make_uint2(0u, 0u);
         return;
     }
-    src.clear();
     const typename Source::Map map = src.map(region);
     // Two levels of 14 and 53 samples per cell in two parts took 80 us split, 32 merged; at 5 per cell
     // the two are equal. Alone from 16 samples per cell and CTA on.
@@ -395,8 +405,24 @@ static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp,
     int resident = 0;   // (asked for the shared-memory limit that the call sets)
     const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kSortThreads, smem, &resident);
     if (e != cudaSuccess) return e;
+    // The sums are filled with zeros beside the sort where that leaves CTAs room and takes about as
+    // long (192 maps of 20 K samples, 189 MB: 51 + 32 -> 61 us; 16 of 160 K, 82 MB: 59 + 15 -> 60), and
+    // by a memset otherwise (256 of 80 K, 490 MB: 194 + 79 -> 314; key points, 553 MB: 17 + 104 -> 123).
+    const bool room = maps * sp.parts <= 3u * sm_count / 2u;
+    const bool beside = room && src.sums_bytes() / 6e3 <= 1.5 * least;
+    sp.clear_sums = beside ? 1u : 0u;
+    if (!beside && src.sums_bytes() > 0) {
+        const cudaError_t err = cudaMemsetAsync(src.sums(), 0, src.sums_bytes(), stream);
+        if (err != cudaSuccess) return err;
+    }
+    // the zeros: 128 KB or more for a CTA, whole clusters, no more than fit at once; where there is no
+    // room the sorting CTAs see to them first (256 maps of 80 K: 194 us against 209 after the others)
+    size_t clearing = ((beside ? src.sums_bytes() : 0) + src.clear_size() + (128u << 10) - 1) >> 17;
+    if (!room) clearing = 0;
+    clearing = std::min<size_t>(clearing, 2u * sm_count);
+    clearing = (clearing + sp.parts - 1) / sp.parts * sp.parts;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(maps * sp.parts);
+    cfg.gridDim = dim3(static_cast<unsigned>(maps * sp.parts + clearing));
     cfg.blockDim = dim3(kSortThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

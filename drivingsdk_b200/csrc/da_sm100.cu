@@ -731,11 +731,7 @@ int da_sm100_backward_ws(const void* feat, const int32_t* spatial_shape, const i
     sp.sorted = reinterpret_cast<uint32_t*>(ws + plan.sorted);
     sp.nsamples = plan.nsamples;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    const size_t points = static_cast<size_t>(B) * A * Pts * cams;
-    cudaError_t e = cudaMemsetAsync(grad_feat, 0, static_cast<size_t>(B) * F * C * 4, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(grad_sampling_location, 0, points * 8, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(grad_weights, 0, points * scales * G * 4, stream);
-    if (e == cudaSuccess) e = msda::launch_da_backward_sorted(p, sp, dtype, sms, stream);
+    const cudaError_t e = msda::launch_da_backward_sorted(p, sp, dtype, sms, stream);   // fills with zeros, too
     if (e != cudaSuccess) {
         t_da_cuda_error = static_cast<int>(e);
         return MSDA_ERR_CUDA;

@@ -54,7 +54,16 @@ struct AggregationSamples {
         const bool inside = xy.x > 0.f && xy.x < 1.f && xy.y > 0.f && xy.y < 1.f;
         return inside ? sample_cell<4>(xy, m.W, m.H) : kNoRow;
     }
-    __device__ __forceinline__ void clear() const {}   // the caller does it
+    // all gradients start from zero
+    __host__ __device__ void* sums() const { return p.grad_feat; }
+    __host__ __device__ size_t sums_bytes() const { return static_cast<size_t>(p.B) * p.F * p.C * sizeof(float); }
+    __host__ __device__ size_t points() const { return static_cast<size_t>(p.B) * p.A * p.Pts * p.cams; }
+    __host__ __device__ size_t weight_bytes() const { return points() * p.scales * p.G * sizeof(float); }
+    size_t clear_size() const { return points() * 8 + weight_bytes(); }
+    __device__ __forceinline__ void clear(size_t first, size_t step) const {
+        clear_bytes(p.grad_loc, points() * 8, first, step);
+        clear_bytes(p.grad_wts, weight_bytes(), first, step);
+    }
 };
 
 template <typename T, int NV>

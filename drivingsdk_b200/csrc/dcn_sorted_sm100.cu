@@ -8,7 +8,7 @@
 // at the operator's test shape, and reduces as many: 168 and 385 us, bound by the return path of
 // 128-bit loads and by the reductions. With a 3 x 3 kernel some nine samples share a cell: sorted
 // by cell, corner rows and their sums stay in registers and what is left is to write or read the
-// columns once (481 MB): 98 and 169 us, plus 21 us for the sort, which both directions use.
+// columns once (481 MB): 98 and 156 us, plus 21 us for the sort, which both directions use.
 // One sample at a time per warp, lane = channel quads j and j + 32 of a slice of NV * 128 channels;
 // backward slices add their parts of the t_c up with atomics.
 #include "cell_sort.cuh"
@@ -50,7 +50,11 @@ struct ConvSamples {
         return static_cast<uint32_t>(__float2int_rd(at.x) + 1) * static_cast<uint32_t>(p.W + 1) +
                static_cast<uint32_t>(__float2int_rd(at.y) + 1);
     }
-    __device__ __forceinline__ void clear() const {}   // every sample has a cell
+    // nothing to clear: every sample has a cell, and the caller clears the gradients
+    __host__ __device__ void* sums() const { return nullptr; }
+    __host__ __device__ size_t sums_bytes() const { return 0; }
+    size_t clear_size() const { return 0; }
+    __device__ __forceinline__ void clear(size_t, size_t) const {}
     static __device__ __forceinline__ bool inside(const DcnParams& p, float2 at) {   // false for NaN
         return at.x > -1.f && at.y > -1.f && at.x < static_cast<float>(p.H) && at.y < static_cast<float>(p.W);
     }

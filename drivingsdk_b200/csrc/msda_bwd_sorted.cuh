@@ -9,7 +9,7 @@
 // samples in a cell (and only the new two when the walk moves one cell to the right).
 //
 //   1 sort     cluster of CTAs = (batch, head, level): counting sort by cell in shared memory;
-//              gradients of locations and weights start from zero.
+//              zeros for all that the main kernel adds to or may leave out.
 //   2 main     warp = a ticket of consecutive sorted samples, in 32 / LPR streams: a stream is
 //              LPR lanes, each lane four channels of all corners.
 // The main kernel compares the cells themselves, so the order is only a matter of speed.
@@ -94,14 +94,21 @@ struct AttentionSamples {
     __device__ __forceinline__ uint32_t cell(const Map& m, float2 xy) const {
         return sample_cell<CPS>(xy, m.W, m.H);
     }
-    // A sample that takes no part has zero gradients, so all gradients of locations and weights start
-    // from zero: zeros for the dropped samples alone, a few bytes each, cost 55 us where 28 % of
-    // 20 M are dropped, this 19 us or less.
-    __device__ __forceinline__ void clear() const {
+    // What starts from zero: the sums of value's gradient ...
+    __host__ __device__ void* sums() const { return p.grad_value; }
+    __host__ __device__ size_t sums_bytes() const {
+        return static_cast<size_t>(p.B) * p.K * p.H * p.D * sizeof(float);
+    }
+    // ... and the gradients of locations and weights, since a sample that takes no part has none (zeros
+    // for the dropped samples alone, a few bytes each, cost 55 us where 28 % of 20 M are dropped).
+    __host__ __device__ size_t samples_bytes() const {   // of one number per sample
+        return CPS == 4 ? static_cast<size_t>(p.ntasks) * p.LP * sizeof(TL) : 0;
+    }
+    size_t clear_size() const { return 3 * samples_bytes(); }
+    __device__ __forceinline__ void clear(size_t first, size_t step) const {
         if constexpr (CPS == 4) {
-            const size_t n = static_cast<size_t>(p.ntasks) * p.LP;
-            clear_bytes(p.grad_loc, 2 * n * sizeof(TL));
-            clear_bytes(p.grad_attn, n * sizeof(TL));
+            clear_bytes(p.grad_loc, 2 * samples_bytes(), first, step);
+            clear_bytes(p.grad_attn, samples_bytes(), first, step);
         }
     }
 };
@@ -511,7 +518,10 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
 }
 
 // Nearest-pixel main kernel: one row per sample. LPR lanes cover a row (four channels each, NV
-// times), 32 / LPR samples of one pixel are worked on at a time and share its row.
+// times), 32 / LPR samples of one pixel are worked on at a time and share its row. Bound by its
+// instructions and by shared memory and L1 together (with grad_out rows from L1 7 % faster): records
+// in shared memory instead of two shuffles per row, and no guards for groups within their pixel,
+// took 10.3 M samples on 375 pixels, 64 channels, from 317 to 287 us (bf16 327 to 260).
 template <typename T, typename TL, int NV, int LPR, bool RAGGED>
 __global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 4)
 gka_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {

@@ -75,6 +75,7 @@ struct SortParams {
     // set by the launch:
     uint32_t parts;         // CTAs per (batch, head, level) of the sort
     uint32_t room;          // words of shared memory of each
+    uint32_t clear_sums;    // 1: the sort fills the main kernel's sums with zeros
     uint32_t nregions, tickets, tickets_per_region;
     FastDiv fd_tickets;     // division by tickets_per_region
     uint32_t stream;        // sorted samples per stream
