@@ -772,6 +772,8 @@ def run_sibling(args):
         gv, goff, glog = torch.empty_like(value), torch.empty_like(off), torch.empty_like(logits)
         gref = torch.empty(B, Q, L, 2, device=dev)
         dims = (B, K, H, D, L, Q, P)
+        ws_bytes = lib.msda_sm100_fused_backward_sorted_workspace_bytes(*dims, capi.F32)
+        ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=dev)
         samples = B
         nv, ns, no, nr = value.numel(), logits.numel(), out.numel(), ref.numel()
         fwd_bytes = 4 * (nv + 3 * ns + nr + no)
@@ -787,7 +789,7 @@ def run_sibling(args):
             capi.check(lib.msda_sm100_fused_backward_ws(
                 value.data_ptr(), shapes.data_ptr(), starts.data_ptr(), ref.data_ptr(),
                 off.data_ptr(), logits.data_ptr(), go.data_ptr(), gv.data_ptr(), gref.data_ptr(),
-                goff.data_ptr(), glog.data_ptr(), None, 0, *dims, capi.F32, stream.cuda_stream),
+                goff.data_ptr(), glog.data_ptr(), ws.data_ptr(), ws_bytes, *dims, capi.F32, stream.cuda_stream),
                 "fused bwd")
 
         def cpu_once(nb):
