@@ -135,7 +135,7 @@ __device__ __forceinline__ uint32_t sort_map(const Source& src, const SortParams
     // 97 us before, 81 now)
     const bool staged = KEPT == Counters::kAlone && cells + n <= sp.room;
     uint32_t placed = 0;         // samples of the map placed by earlier passes
-    constexpr uint32_t kU = 4;   // samples in flight per thread
+    constexpr uint32_t kU = Source::kInFlight;   // samples in flight per thread
     // each(cell of this pass, sample number)
     auto for_each_sample = [&](uint32_t lo, auto&& each) {
         uint32_t id = first_id;
@@ -246,7 +246,17 @@ __device__ __forceinline__ uint32_t sort_map(const Source& src, const SortParams
     return placed;
 }
 
-template <typename Source>
+// How the counters of a map are kept. Two levels of 14 and 53 samples per cell in two parts took 80 us split,
+// 32 merged; at 5 per cell the two are equal. Alone from 16 samples per cell and CTA on.
+__host__ __device__ __forceinline__ Counters counters_of(uint32_t parts, uint32_t samples, uint32_t cells) {
+    const bool fits = cells <= kSortCells;
+    if (parts == 1 || (fits && samples / parts >= 16u * cells)) return Counters::kAlone;
+    return fits && 2u * samples >= parts * cells ? Counters::kMerged : Counters::kSplit;
+}
+
+// KEPT: the one way, for maps that are all alike (a kernel that holds all three spills more; 18 and 12
+// convolution maps of 13 K samples: 26.6 and 26.0 us, now 13.7 and 10.0); -1: chosen map by map.
+template <typename Source, int KEPT>
 __global__ void __launch_bounds__(kSortThreads, 2)
 sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ SortParams sp) {
     extern __shared__ uint32_t s_count[];   // [kSortCells]
@@ -272,13 +282,11 @@ sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ So
         return;
     }
     const typename Source::Map map = src.map(region);
-    // Two levels of 14 and 53 samples per cell in two parts took 80 us split, 32 merged; at 5 per cell
-    // the two are equal. Alone from 16 samples per cell and CTA on.
-    const bool fits = map.cells <= kSortCells;
+    const Counters kept = KEPT >= 0 ? static_cast<Counters>(KEPT) : counters_of(parts, src.samples, map.cells);
     uint32_t placed;
-    if (parts == 1 || (fits && src.samples / parts >= 16u * map.cells))
+    if (kept == Counters::kAlone)
         placed = sort_map<Counters::kAlone>(src, sp, map, s_count, warp_sum, &block_sum);
-    else if (fits && 2u * src.samples >= parts * map.cells)
+    else if (kept == Counters::kMerged)
         placed = sort_map<Counters::kMerged>(src, sp, map, s_count, warp_sum, &block_sum);
     else
         placed = sort_map<Counters::kSplit>(src, sp, map, s_count, warp_sum, &block_sum);
@@ -378,25 +386,35 @@ static cudaError_t plan_tickets(const void* kernel, int streams, SortParams& sp,
 template <typename Source>
 static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp, int sm_count,
                                cudaStream_t stream) {
-    auto kern = sort_cells_kernel<Source>;
     // The cluster that is done first, by a model of the time in ns: an SM works on two CTAs at a time, 1.5
     // per sample of both (one alone takes 0.65 of the time of two); a cluster costs 8 us, and 3.1 per
     // cell and other CTA (merged) or 2.8 per sample (split). More parts have to gain a tenth: apart,
     // they leave shorter runs. (Samples alone, us: 256 maps of 80 K 258 / 227 / 208 in 1 / 4 / 8 parts,
     // 192 of 20 K 67 / 56 / 57 in 1 / 2 / 4, 96 of 107 K 111 / 127 / 95 / 84 in 1 / 2 / 4 / 8; 144 of
-    // 5 K, whole sort: 17 / 28 in 1 / 2.)
+    // 5 K, whole sort: 17 / 28 in 1 / 2.) In a kernel that holds one way only a cluster costs 5 us (12 and 18
+    // maps of 13 K samples on 1.5 K cells: 15.6 and 15.5 us in 1 part, 11.5 and 11.6 in 4, 10.2 and 13.5 in 8).
+    const double cluster = Source::kMapsAlike ? 5000.0 : 8000.0;
     double least = 0.0;
     for (uint32_t parts = 1; parts <= kMaxSortParts; parts *= 2) {
         const uint32_t per_sm = (maps * parts + sm_count - 1) / sm_count;
         const double share = (per_sm / 2 + 0.65 * (per_sm % 2)) / parts;
         const double between = std::min(3.1 * src.mean_cells * (parts - 1), 2.8 * src.samples);
-        const double ns = share * (1.5 * src.samples + (parts > 1 ? between : 0.0)) + (parts > 1 ? 8000.0 : 0.0);
+        const double ns = share * (1.5 * src.samples + (parts > 1 ? between : 0.0)) + (parts > 1 ? cluster : 0.0);
         if (parts == 1 || ns < 0.9 * least) {
             least = ns;
             sp.parts = parts;
         }
     }
     sp.nregions = maps;
+    void (*kern)(const Source, const SortParams) = nullptr;
+    if constexpr (Source::kMapsAlike) {
+        const Counters kept = counters_of(sp.parts, src.samples, src.most_cells);
+        kern = kept == Counters::kAlone    ? sort_cells_kernel<Source, static_cast<int>(Counters::kAlone)>
+               : kept == Counters::kMerged ? sort_cells_kernel<Source, static_cast<int>(Counters::kMerged)>
+                                           : sort_cells_kernel<Source, static_cast<int>(Counters::kSplit)>;
+    } else {
+        kern = sort_cells_kernel<Source, -1>;
+    }
     // more room only where that lets every map's samples be staged (it costs L1: the encoder shape's
     // sort takes 82 instead of 69 us)
     const uint32_t part = (src.samples - 1) / sp.parts + 1;

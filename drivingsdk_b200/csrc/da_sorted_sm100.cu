@@ -23,6 +23,8 @@ struct DaDivs {
 // point) pairs.
 template <typename T>
 struct AggregationSamples {
+    static constexpr uint32_t kInFlight = 4;   // samples in flight per thread of the sort
+    static constexpr bool kMapsAlike = false;   // scales differ
     DaParams p;
     DaDivs fd;
     uint32_t samples;   // of one map: A * Pts

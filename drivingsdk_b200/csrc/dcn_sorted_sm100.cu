@@ -23,6 +23,10 @@ using namespace msda;
 
 // What the sort needs to know: a map is one (image, deformable group).
 struct ConvSamples {
+    // Samples in flight per thread of the sort: a position takes two loads and five divisions, so more
+    // than one spills (18 maps of 13 K samples, alone: 15.5 us with one, 19.6 with two, 26 with four).
+    static constexpr uint32_t kInFlight = 1;
+    static constexpr bool kMapsAlike = true;    // all have the same cells
     DcnParams p;
     uint32_t samples;   // of one map: Ho * Wo * K
     uint32_t period, period_step;   // K, DG * K

@@ -61,6 +61,8 @@ __device__ __forceinline__ SampleId sample_id(const Params& p, const SortParams&
 // What the sort needs to know (cell_sort.cuh): a map is one (batch, head, level).
 template <typename TL, int CPS>
 struct AttentionSamples {
+    static constexpr uint32_t kInFlight = 4;   // samples in flight per thread of the sort
+    static constexpr bool kMapsAlike = false;   // levels differ
     Params p;
     FastDiv fd_p;       // division by the points per level
     uint32_t samples;   // of one map: Q * P

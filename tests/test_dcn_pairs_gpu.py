@@ -39,6 +39,10 @@ CASES = [
     (1, 264, 16, 111, 103, 1, 1, 1, True),
     (2, 320, 32, 41, 70, 1, 1, 2, False),
     (4, 256, 64, 55, 54, 1, 2, 2, True),
+    # the sort's ways of keeping its counters that those do not take: split over a cluster (27226 cells),
+    # one CTA per map
+    (1, 104, 16, 164, 164, 1, 1, 1, True),
+    (40, 104, 24, 20, 20, 1, 1, 1, True),
 ]
 
 
