@@ -213,6 +213,7 @@ __device__ __forceinline__ SortedSample set_up_sample(const Params& p, const Sor
 // above them).
 constexpr uint32_t kEnters = 1;      // its cell is not the previous sample's
 constexpr uint32_t kJumps = 2;       // ... and not the next one to the right either
+constexpr uint32_t kAmplified = 4;   // its dot products are formed in double
 
 // Rows of grad_out in flight per lane and CTAs per SM. The kernel waits for the latency of its own
 // instructions more than for memory (with grad_out from L1 it is no faster), so rows in flight count as
@@ -338,7 +339,10 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
             next.id = next_id;
             load_raw<TL>(p, next, at + LPR < end);
             next_id = at + 2 * LPR < end ? __ldg(sp.sorted + at + 2 * LPR) : 0u;
-            uint32_t m_enter, m_jump, m_wide;   // bit = lane = (step, stream) of the round
+            // Bit = lane = (step, stream) of the round. Not with two quads per lane: there a warp is one stream,
+            // whose flags all lanes hold, and the masks cost spills (256 channels, fp32, 4.7 M samples:
+            // 1328 us with them, 1119 without).
+            uint32_t m_enter = 0u, m_jump = 0u, m_wide = 0u;
             {
                 const SortedSample s = set_up_sample<4>(p, sp, lv, raw, at < end);
                 raw = next;
@@ -352,14 +356,17 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
                     pcell = scell;
                 }
                 uint32_t flags = s.cell << 4;
+                if (WIDE && s.amplified) flags |= kAmplified;
                 if (s.row != prow || s.cell != pcell) {
                     const bool right = s.row == prow + step_x && (s.cell >> 4) == (pcell >> 4) &&
                                        ((pcell >> 1) & 5u) == (s.cell & 5u);
                     flags |= right ? kEnters : (kEnters | kJumps);
                 }
-                m_enter = __ballot_sync(0xffffffffu, flags & kEnters);
-                m_jump = __ballot_sync(0xffffffffu, flags & kJumps);
-                m_wide = WIDE ? __ballot_sync(0xffffffffu, s.amplified) : 0u;
+                if constexpr (NV == 1) {
+                    m_enter = __ballot_sync(0xffffffffu, flags & kEnters);
+                    m_jump = __ballot_sync(0xffffffffu, flags & kJumps);
+                    m_wide = WIDE ? __ballot_sync(0xffffffffu, s.amplified) : 0u;
+                }
                 s_w[warp][lane][0] = make_ulonglong2(pack2(s.w[0], s.w[0]), pack2(s.w[1], s.w[1]));
                 s_w[warp][lane][1] = make_ulonglong2(pack2(s.w[2], s.w[2]), pack2(s.w[3], s.w[3]));
                 s_rec[warp][lane] = make_uint2(s.task * p.row_units, flags);
@@ -419,9 +426,13 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const int slot = (t0 + u) * S + g;
-                        if ((m_enter >> ((t0 + u) * S)) & kStep) {
+                        static_assert(NV == 1 || S == 1, "flags speak for the whole step");
+                        auto any = [&](uint32_t mask, uint32_t flag) {   // of the streams in this step
+                            return (NV == 1 ? (mask >> ((t0 + u) * S)) & kStep : flags[u] & flag) != 0u;
+                        };
+                        if (any(m_enter, kEnters)) {
                             const bool enters = flags[u] & kEnters, jumps = flags[u] & kJumps;
-                            const bool any_jumps = ((m_jump >> ((t0 + u) * S)) & kStep) != 0u;
+                            const bool any_jumps = any(m_jump, kJumps);
                             flush(0, enters);
                             flush(2, enters);
                             if (any_jumps) {
@@ -449,7 +460,7 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
                             // A step with an amplified sample forms its dot products in double as
                             // well; each sample takes the kind it asked for, so its gradients do
                             // not depend on which samples share the step.
-                            if ((m_wide >> ((t0 + u) * S)) & kStep) {
+                            if (any(m_wide, kAmplified)) {
                                 double dd[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
                                 for (int k = 0; k < NV; ++k)
