@@ -216,16 +216,19 @@ constexpr uint32_t kJumps = 2;       // ... and not the next one to the right ei
 constexpr uint32_t kAmplified = 4;   // its dot products are formed in double
 
 // Rows of grad_out in flight per lane and CTAs per SM. The kernel waits for the latency of its own
-// instructions more than for memory (with grad_out from L1 it is no faster), so rows in flight count as
-// long as no register spills: at 80 registers two, more with one CTA less. Measured (us, main kernel):
+// instructions more than for memory (with grad_out from L1 it is no faster): at 80 registers and three CTAs
+// two rows, more where two CTAs are as fast. Measured (us, main kernel):
 //   128 channels, 16 bit, 20.5 M samples   2 rows x 3 CTAs 1820   4 x 2 1772   8 x 2 1622
 //   128 channels, fp32, 4.6 M               630   617   1009 (spills)
 //    64 channels, fp32, 5.1 M               378   394    673
 //    32 channels, fp32, 4.6 M               265   267    358
 //    16 channels, fp32, 5.1 M               196   173      -
-template <typename T, int NV, int LPR>
+// SPARSE: 16-bit rows that leave some of 32 lanes idle enter cells more slowly with eight rows than with two
+// (whole backward, 96 channels, bf16: 1.65 M samples, 4 per cell 450 / 376; 1.39 M, 13 per cell 238 / 222;
+// 5.1 M, 21 per cell 656 / 644; 2.56 M, 143 per cell 288 / 312).
+template <typename T, int NV, int LPR, bool SPARSE>
 struct SortedTile {
-    static constexpr bool kMore = NV == 1 && (LPR == 32 || LPR == 4);
+    static constexpr bool kMore = NV == 1 && (LPR == 32 || LPR == 4) && !SPARSE;
     static constexpr int kRows = !kMore ? 2 : (LPR == 32 && sizeof(T) == 2) ? 8 : 4;
     static constexpr int kCtas = (kMore || NV > 1) ? 2 : 3;
 };
@@ -237,11 +240,11 @@ struct SortedTile {
 // samples whose set-up and final gradients are done lane = sample. The accumulation rows are
 // fp32. RAGGED: some of those lanes are past D; without their checks the rest is 1 to 4 % faster
 // (encoder shape, fp32, 32 channels: 284 -> 274 us; 128 channels, bf16: 1894 -> 1867 us).
-template <typename T, typename TL, int NV, int LPR, bool RAGGED>
-__global__ void __launch_bounds__(kThreadsPerCta, SortedTile<T, NV, LPR>::kCtas)
+template <typename T, typename TL, int NV, int LPR, bool RAGGED, bool SPARSE>
+__global__ void __launch_bounds__(kThreadsPerCta, SortedTile<T, NV, LPR, SPARSE>::kCtas)
 msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__ SortParams sp) {
     constexpr int S = 32 / LPR;       // streams
-    constexpr int U = SortedTile<T, NV, LPR>::kRows;   // rows of grad_out in flight per lane
+    constexpr int U = SortedTile<T, NV, LPR, SPARSE>::kRows;   // rows of grad_out in flight per lane
     // fp32 bilinear operator: some dot products need double precision (see sample_grad)
     constexpr bool WIDE = sizeof(TL) == 4 && sizeof(T) == 4;
     static_assert(LPR % U == 0, "a round is LPR steps");
@@ -713,9 +716,13 @@ static cudaError_t launch_sorted_bilinear(const Params& p, SortParams sp,
     if (e != cudaSuccess) return e;
     auto main = [&](auto nv, auto lpr) {
         constexpr int NV = decltype(nv)::value, LPR = decltype(lpr)::value;
-        return p.D == 4 * NV * LPR
-                   ? launch_sorted_main(msda_bwd_sorted_kernel<T, TL, NV, LPR, false>, 32 / LPR, p, sp, n, ls, stream)
-                   : launch_sorted_main(msda_bwd_sorted_kernel<T, TL, NV, LPR, true>, 32 / LPR, p, sp, n, ls, stream);
+        auto launch = [&](auto kern) { return launch_sorted_main(kern, 32 / LPR, p, sp, n, ls, stream); };
+        if (p.D == 4 * NV * LPR) return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, false, false>);
+        if constexpr (NV == 1 && LPR == 32 && sizeof(T) == 2) {   // (see SortedTile)
+            const double cells = static_cast<double>(p.B) * p.K * p.H;
+            if (sp.nsamples < 20.0 * cells) return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, true, true>);
+        }
+        return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, true, false>);
     };
     return for_row_width(p.D, main);
 }
