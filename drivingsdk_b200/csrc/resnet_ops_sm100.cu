@@ -148,10 +148,9 @@ int dispatch_pointwise(const void* a, const void* b, void* dst, size_t n, int dt
 // neighbouring outputs of R output rows, which share all but the outermost of their 2 R + 1 input rows,
 // and asks for all of its inputs before it uses the first. The column to the left comes from the
 // neighbouring lane. COLS = 4 reads 16 bytes at a time and needs rows that start on 16 bytes
-// (6 x 64 x 464 x 800 fp32: 112 us, 0.98 of the copy rate; one output row per thread with 64-bit
-// divisions took 133); other widths and addresses take COLS = 1, whose loads of every other element
-// meet the same cache lines (9 x 32 x 199 x 149 fp32 17.4 -> 11.3 us, 9 x 32 x 133 x 290 fp16
-// 17.7 -> 11.5).
+// (6 x 64 x 464 x 800: fp32 111 us, 0.98 of the copy rate, fp16 64; one output row per thread with 64-bit
+// divisions and looser loads took 133 and 120); other widths and addresses take COLS = 1, whose loads of
+// every other element meet the same cache lines (6 x 64 x 464 x 799 fp32 235 -> 126 us, fp16 148 -> 112).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
     float r;
@@ -162,7 +161,7 @@ __device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either 
 struct PoolGrid {
     int H, W, OH, OW;
     uint32_t groups, strips, total;            // of COLS outputs in a row; of R output rows; threads
-    int first_row;                             // output row of the first strip
+    int first_row;                             // output row of the first thread
     msda::FastDiv by_groups, by_strips;
 };
 
@@ -247,39 +246,38 @@ int launch_maxpool(const T* x, T* y, size_t planes, int H, int W, cudaStream_t s
     // 16-byte loads need every row to start on a 16-byte boundary; vector stores likewise
     const int per_vec = 16 / static_cast<int>(sizeof(T));
     const bool vec_in = (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (W % per_vec == 0);
-    constexpr int kVecRows = sizeof(T) == 4 ? 2 : 4;         // as many as registers hold
-    const int cols = vec_in ? 4 : 1, rows = vec_in ? kVecRows : 4;
     PoolGrid p;
     p.H = H; p.W = W; p.OH = (H - 1) / 2 + 1; p.OW = (W - 1) / 2 + 1;
-    p.groups = static_cast<uint32_t>((p.OW - 1) / cols + 1);
-    p.strips = static_cast<uint32_t>((p.OH - 1) / rows + 1);
+    p.groups = static_cast<uint32_t>((p.OW - 1) / (vec_in ? 4 : 1) + 1);
     p.by_groups = msda::make_fastdiv(p.groups);
+    // Rows of a thread: two of fp32, or four single outputs, unless the plane has few rows or the threads
+    // would be few (32 x 104 x 104 fp32 3.7 us with two, 3.2 with one; 64000 x 8 x 8 9.3 and 7.2; 400 K x
+    // 3 x 3 9.6 with four, 7.5 with two). In 16 bits one row is never slower than two or four (6 x 64 x 464 x
+    // 800 67 us with four, 63 with one; 512 x 56 x 56 4.0 and 3.1).
+    int rows = !vec_in ? 4 : sizeof(T) == 4 ? 2 : 1;
+    auto strips = [&](int r) { return static_cast<uint32_t>((p.OH - 1) / r + 1); };
+    while (rows > 1 && ((vec_in ? 2 * rows : rows / 2) >= p.OH || planes * strips(rows) * p.groups < (1u << 16)))
+        rows /= 2;
+    p.strips = strips(rows);
     p.by_strips = msda::make_fastdiv(p.strips);
-    p.first_row = 0;
     const int vec_out = (reinterpret_cast<uintptr_t>(y) % 16 == 0) && (p.OW % 4 == 0);
+    auto kernel = vec_in ? (rows == 1 ? maxpool3s2_kernel<T, 4, 1> : maxpool3s2_kernel<T, 4, sizeof(T) == 4 ? 2 : 1>)
+                         : (rows == 1   ? maxpool3s2_kernel<T, 1, 1>
+                            : rows == 2 ? maxpool3s2_kernel<T, 1, 2>
+                                        : maxpool3s2_kernel<T, 1, 4>);
+    // FastDiv takes 2^31 - 1 threads: nearly always one launch, else some planes at a time, or some strips
+    // of one where a plane has more
+    const size_t most = (1u << 31) - 1, all = planes * p.strips, whole = most / p.groups / p.strips;
     int launches = 0;
-    auto launch = [&](size_t first, size_t count) {
-        p.total = static_cast<uint32_t>(count * p.groups * p.strips);
-        const unsigned grid = (p.total - 1) / kThreads + 1;
-        const T* from = x + first * H * W;
-        T* to = y + first * p.OH * p.OW;
-        if (vec_in) maxpool3s2_kernel<T, 4, kVecRows><<<grid, kThreads, 0, stream>>>(from, to, p, vec_out);
-        else maxpool3s2_kernel<T, 1, 4><<<grid, kThreads, 0, stream>>>(from, to, p, vec_out);
-        ++launches;
-    };
-    // FastDiv takes 2^31 - 1 threads: nearly always one launch, else some planes, or some strips of
-    // one plane, at a time
-    const unsigned long long most = (1ull << 31) - 1, all_strips = p.strips;
-    const unsigned long long at_once = most / (p.groups * all_strips);
-    for (size_t first = 0; first < planes && at_once > 0; first += at_once)
-        launch(first, std::min<unsigned long long>(planes - first, at_once));
-    for (size_t first = 0; first < planes && at_once == 0; ++first) {
-        for (unsigned long long strip = 0; strip < all_strips; strip += p.strips) {
-            p.strips = static_cast<uint32_t>(std::min(most / p.groups, all_strips - strip));
-            p.by_strips = msda::make_fastdiv(p.strips);
-            p.first_row = static_cast<int>(strip) * rows;
-            launch(first, 1);
-        }
+    for (size_t first = 0; first < all; ++launches) {
+        const size_t plane = first / p.strips, strip = first - plane * p.strips;
+        const size_t count = whole > 0 ? std::min(whole, planes - plane) * p.strips
+                                       : std::min(most / p.groups, p.strips - strip);
+        p.first_row = static_cast<int>(strip) * rows;
+        p.total = static_cast<uint32_t>(count * p.groups);
+        kernel<<<(p.total - 1) / kThreads + 1, kThreads, 0, stream>>>(x + plane * H * W, y + plane * p.OH * p.OW, p,
+                                                                      vec_out);
+        first += count;
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return msda::note_cuda_error(e);

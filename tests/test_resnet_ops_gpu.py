@@ -8,6 +8,8 @@ import pytest
 import torch
 import torch.nn.functional as F
 
+from drivingsdk_b200 import capi
+
 pytestmark = pytest.mark.gpu
 
 DTYPES = [torch.float32, torch.float16, torch.bfloat16]
@@ -132,3 +134,26 @@ def test_max_pool2d_at_the_edges_of_its_tiles(H, W, dtype):
     want = F.max_pool2d(x.float(), 3, 2, 1).to(dtype)
     for given in (x, skewed):
         assert torch.equal(mx_driving.npu_max_pool2d(given, 3, 2, 1).nan_to_num(9.0), want.nan_to_num(9.0))
+
+
+# calls large enough for several output rows per thread: whole strips, a last one that is not, rows of 16-byte
+# pieces, single columns, planes of two or three output rows
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [(3, 900, 17, 72), (2, 1500, 13, 40), (3, 500, 19, 65), (3, 900, 9, 33), (40, 1000, 3, 5),
+                                   (30, 1000, 5, 3)])
+def test_max_pool2d_over_several_rows(shape, dtype):
+    import mx_driving
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = (torch.rand(shape, generator=g, device="cuda") - 0.5).to(dtype)
+    x.view(-1)[:: 37] = -float("inf")
+    x.view(-1)[5 :: 191] = float("nan")
+    want = F.max_pool2d(x.float(), 3, 2, 1).to(dtype)
+    assert torch.equal(mx_driving.npu_max_pool2d(x, 3, 2, 1).nan_to_num(9.0), want.nan_to_num(9.0))
+
+
+def test_max_pool2d_of_more_planes_than_one_launch_takes():
+    import mx_driving
+    x = torch.rand(65537, 32768, 1, 1, dtype=torch.float16, device="cuda")   # 2^31 + 32768 planes of one pixel
+    before = capi.load().msda_sm100_launch_count()
+    assert torch.equal(mx_driving.npu_max_pool2d(x, 3, 2, 1), x)
+    assert capi.load().msda_sm100_launch_count() - before == 2
