@@ -56,6 +56,24 @@ struct Dims {
     int B, K, H, D, L, Q, P;
 };
 
+// Workspace of *bytes for an attention backward or, where there is no room for the samples that its sorted
+// form keeps there, of what its other form needs.
+at::Tensor backward_workspace(const at::Tensor& value, const Dims& d, int dtype, size_t* bytes) {
+    const size_t least = msda_sm100_backward_workspace_bytes(d.B, d.K, d.H, d.D, dtype);
+    auto make = [&](size_t n) {
+        return n > 0 ? at::empty({static_cast<int64_t>(n)}, value.options().dtype(at::kByte)) : at::Tensor();
+    };
+    if (*bytes > least) {
+        try {
+            return make(*bytes);
+        } catch (const c10::OutOfMemoryError&) {
+            *bytes = least;
+        }
+    }
+    return make(*bytes);
+}
+void* workspace_pointer(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
 // The tables may be int32 or int64, both alike: the kernels read both with one step. The exported
 // functions take int32 only (check_int32_tables).
 Dims check_inputs(const at::Tensor& value, const at::Tensor& shapes, const at::Tensor& starts,
@@ -212,18 +230,12 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> msda_backward(
         return std::make_tuple(grad_value, grad_loc, grad_attn);
     }
     const int dt = dtype_code(value.scalar_type());
-    at::Tensor workspace;
-    void* ws_ptr = nullptr;
     size_t ws_bytes = msda_sm100_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
-    if (ws_bytes > 0) {
-        workspace = at::empty({static_cast<int64_t>(ws_bytes / sizeof(float))},
-                              value.options().dtype(at::kFloat));
-        ws_ptr = workspace.data_ptr();
-    }
+    const at::Tensor workspace = backward_workspace(value, d, dt, &ws_bytes);
     const int rc = msda_sm100_backward_ws(
         value.data_ptr(), table(shapes), table(starts), loc.data_ptr(),
         attn.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(), grad_loc.data_ptr(),
-        grad_attn.data_ptr(), ws_ptr, ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
+        grad_attn.data_ptr(), workspace_pointer(workspace), ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
         dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "multi_scale_deformable_attn_backward");
     return std::make_tuple(grad_value, grad_loc, grad_attn);
@@ -356,18 +368,12 @@ std::tuple<at::Tensor, at::Tensor> geometric_kernel_attention_backward(
         return std::make_tuple(grad_value, grad_attn);
     }
     const int dt = dtype_code(value.scalar_type());
-    at::Tensor workspace;
-    void* ws_ptr = nullptr;
-    const size_t ws_bytes = gka_sm100_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
-    if (ws_bytes > 0) {
-        workspace = at::empty({static_cast<int64_t>(ws_bytes / sizeof(float))},
-                              value.options().dtype(at::kFloat));
-        ws_ptr = workspace.data_ptr();
-    }
+    size_t ws_bytes = gka_sm100_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
+    const at::Tensor workspace = backward_workspace(value, d, dt, &ws_bytes);
     const int rc = gka_sm100_backward_ws(
         value.data_ptr(), table(shapes), table(starts), loc.data_ptr(),
-        attn.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(), grad_attn.data_ptr(), ws_ptr,
-        ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
+        attn.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(), grad_attn.data_ptr(),
+        workspace_pointer(workspace), ws_bytes, d.B, d.K, d.H, d.D, d.L, d.Q, d.P,
         dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "geometric_kernel_attention_backward");
     return std::make_tuple(grad_value, grad_attn);
@@ -604,19 +610,13 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> msda_fused_backward(
     at::Tensor grad_logits = at::empty_like(logits);
     at::Tensor grad_ref = at::empty(ref.sizes(), ref.options().dtype(at::kFloat));
     const int dt = dtype_code(value.scalar_type());
-    at::Tensor workspace;
-    void* ws_ptr = nullptr;
-    const size_t ws_bytes =
+    size_t ws_bytes =
         msda_sm100_fused_backward_sorted_workspace_bytes(d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dt);
-    if (ws_bytes > 0) {
-        workspace = at::empty({static_cast<int64_t>(ws_bytes / sizeof(float))},
-                              value.options().dtype(at::kFloat));
-        ws_ptr = workspace.data_ptr();
-    }
+    const at::Tensor workspace = backward_workspace(value, d, dt, &ws_bytes);
     const int rc = msda_sm100_fused_backward_ws(
         value.data_ptr(), table(shapes), table(starts), ref.data_ptr(),
         off.data_ptr(), logits.data_ptr(), grad_out.data_ptr(), grad_value.data_ptr(),
-        grad_ref.data_ptr<float>(), grad_off.data_ptr(), grad_logits.data_ptr(), ws_ptr, ws_bytes,
+        grad_ref.data_ptr<float>(), grad_off.data_ptr(), grad_logits.data_ptr(), workspace_pointer(workspace), ws_bytes,
         d.B, d.K, d.H, d.D, d.L, d.Q, d.P, dtype_and_tables(value, shapes), at::cuda::getCurrentCUDAStream().stream());
     raise_on_error(rc, "msda_fused_backward");
     return std::make_tuple(grad_value, grad_ref.to(ref.scalar_type()), grad_off, grad_logits);
