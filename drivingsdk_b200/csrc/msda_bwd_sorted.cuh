@@ -225,7 +225,8 @@ constexpr uint32_t kAmplified = 4;   // its dot products are formed in double
 //    16 channels, fp32, 5.1 M               196   173      -
 // SPARSE: 16-bit rows that leave some of 32 lanes idle enter cells more slowly with eight rows than with two
 // (whole backward, 96 channels, bf16: 1.65 M samples, 4 per cell 450 / 376; 1.39 M, 13 per cell 238 / 222;
-// 5.1 M, 21 per cell 656 / 644; 2.56 M, 143 per cell 288 / 312).
+// 5.1 M, 21 per cell 656 / 644; 2.56 M, 143 per cell 288 / 312; where most samples fall outside their
+// map fewer share a cell than the number says: 80 channels, 4.9 M, 23 per cell 507 / 433).
 template <typename T, int NV, int LPR, bool SPARSE>
 struct SortedTile {
     static constexpr bool kMore = NV == 1 && (LPR == 32 || LPR == 4) && !SPARSE;
@@ -720,7 +721,7 @@ static cudaError_t launch_sorted_bilinear(const Params& p, SortParams sp,
         if (p.D == 4 * NV * LPR) return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, false, false>);
         if constexpr (NV == 1 && LPR == 32 && sizeof(T) == 2) {   // (see SortedTile)
             const double cells = static_cast<double>(p.B) * p.K * p.H;
-            if (sp.nsamples < 20.0 * cells) return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, true, true>);
+            if (sp.nsamples < 40.0 * cells) return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, true, true>);
         }
         return launch(msda_bwd_sorted_kernel<T, TL, NV, LPR, true, false>);
     };

@@ -4,6 +4,7 @@
 // and multi_scale_deformable_attn_grad.cpp:35-86), and kernel launches.
 // No allocation, no synchronisation (except msda_sm100_device_status).
 #include <atomic>
+#include <cmath>
 #include <cstring>
 
 #include "../../include/msda_sm100.h"
@@ -176,41 +177,60 @@ bool plan_sort(int B, int K, int H, int D, int L, int Q, int P, int dtype, int m
 }
 
 // Where sorting pays: the gain is the rows that samples of one cell share, the cost a sort of 9 to 25 ps
-// per sample, so it takes enough samples per cell, fewer of them the longer the rows, and enough samples
-// for two more launches and their tails. Measured, whole backward, unsorted / sorted (us):
-//   samples, per cell      D = 16 f32, bf16        32 f32, bf16            64 f32, bf16           128 f32, bf16
-//    0.64 M uniform   9.4   56/69     67/72         71/75     81/76        130/93    118/95       247/130   218/126
-//    0.64 M grid      4.0   83/85     77/85         89/112    93/97        159/165   142/136
-//    0.77 M uniform   2.8   65/79     71/83         87/114    97/101       159/167   155/165      300/222   298/245
-//    1.28 M           2.6   96/128   109/130       136/171   157/177       261/237   263/259
-//    1.28 M          18.8   87/87    118/87        118/106   134/101       235/132   208/130
-//    2.56 M grid      4.0  282/253   245/230       297/357   321/294       566/533   517/435
-//    3.84 M uniform   2.6  255/276   300/292       373/392   441/411       729/564   755/648
-//    3.07 M          11.3  192/167   216/165       272/220   307/208       544/292   484/296
-// The nearest-pixel operator has one row per sample and no double-precision dot products: 519 / 397 at
-// 24 x 107 k samples on 375 pixels. The fused operator pays for two more kernels:
-//    0.64 M           9.4   66/87     75/95         83/102    89/104       144/124   128/124      257/157   228/155
-//    1.28 M           2.6  110/160   130/171       156/200   179/218       298/263   294/296      612/374   593/441
-//    3.84 M           2.6  296/353   343/372       419/463   487/495       824/646   804/736     1798/1075 1872/1208
-//    3.07 M          11.3  239/251   243/247       317/310   320/292       585/378   488/373     1142/560   974/509
+// per sample, so it takes enough samples per cell, fewer of them the wider the rows, and enough samples for
+// the tails of two more launches (four for the fused operator). A line per width: `least` million samples,
+// `sparse` per cell and per_cell * millions^(3/4 or 3/2) >= `line`. The lines were drawn through 8000 calls
+// of 0.1 to 30 M samples, 1.5 to 3000 per cell, one to five levels, 1 to 64 heads times images, locations
+// uniform, around a grid or mostly outside: 1 to 4 % slower than the better form of each call (8 and 9 %
+// for up to 16 channels of fp32 and for few samples of the fused operator). Whole backward on both sides of
+// a line, millions of samples, per cell: unsorted / sorted (us); at 8 channels both occur beyond it, too
+// (fp32 9.43, 16 per cell: 439/548; 16 bits 0.92, 24: 48/83):
+//   width    fp32                                             16 bits
+//   <= 8     0.49  61: 26/38    3.88  2.4: 243/291            1.76  10: 91/181   7.14   11: 365/464
+//            0.40 168: 71/42    2.33   26: 294/163            0.81  26: 101/65   2.98   22: 183/138
+//   <= 16    0.48  34: 40/42    1.88  5.2: 132/135            0.62  17: 50/58    1.19  4.1: 105/99
+//            0.68  46: 99/56    2.42   10: 161/140            1.49  10: 118/97   2.50  6.0: 222/183
+//   <= 32    0.35  53: 38/42    3.25  2.5: 361/388            0.33  28: 50/48    1.45  5.4: 150/134
+//            0.60  35: 93/85    1.54  6.6: 323/214            0.53  58: 89/54    2.90  5.7: 306/275
+//   <= 64    0.11 5.3: 38/46    0.72  1.5: 216/218            0.17  11: 48/48    0.85  2.7: 177/169
+//            0.33 4.1: 79/60    1.66  1.9: 431/402            0.29  12: 73/56    2.49  2.9: 423/384
+//   <= 128   0.30 2.0: 116/116  2.47  2.9: 937/730            0.10 4.2: 54/54    0.73  1.7: 257/261
+//            0.26 2.0: 132/124  0.67  3.0: 274/230            0.18 3.5: 132/83   1.22  3.3: 519/374
+//   <= 256   0.24 2.1: 226/159  1.65  4.2: 1281/572           0.14 1.6: 140/132  0.66  2.4: 701/394
+//   fused    0.47  70: 60/68    2.13  2.0: 301/410  (<= 32)   0.56  75: 62/76    3.52  5.3: 405/388
+//            0.87  32: 157/128  3.70   19: 720/458            1.74  27: 228/187  3.96   13: 511/394
+//            0.11  34: 40/48    0.66  3.1: 151/153  (<= 64)   0.33  57: 62/70    2.68  2.6: 536/562
+//            0.35  15: 89/76    1.23  2.5: 374/347            0.70  18: 126/102  2.80  3.1: 593/505
+//            0.11  38: 60/75    0.21  2.1: 116/126  (<= 128)  0.33  2.7: 118/134 0.41  3.6: 140/142
+//            0.20 7.0: 91/73    0.80  1.7: 378/332            0.23   23: 77/68   1.25  6.6: 343/276
+// Up to 16 channels the two more kernels of the fused operator cost what the sort gains (1.28 M, 3.3 per
+// cell 265/179, but 1.36 M, 4.7: 122/171). 16-bit rows that are not whole 16-byte pieces go through the
+// unsorted kernel one channel at a time: sorted 2 to 16 times as fast from 1.5 per cell on. The
+// nearest-pixel operator has one row per sample and no double-precision dot products: 519 / 397 at
+// 24 x 107 k samples on 375 pixels.
+struct SortLine {
+    double least, sparse, line;
+};
 bool sort_pays(const SortPlan& s, int K, int H, int D, int dtype, int B, int mode) {
     if (g_tune_sort.load() == 0) return false;
     if (g_tune_sort.load() == 2) return true;
-    const uint32_t n = s.nsamples;
-    if (n < 100000u) return false;
-    const double per_cell = static_cast<double>(n) / (static_cast<double>(B) * K * H);
+    if (s.nsamples < 100000u) return false;
+    const double per_cell = static_cast<double>(s.nsamples) / (static_cast<double>(B) * K * H);
     if (mode == kNearest) return per_cell >= 16.0;
-    if (mode == kFused) {
-        if (n < 500000u || D <= 16) return false;
-        if (D > 64) return per_cell >= 2.0;
-        if (D > 32) return per_cell >= (n >= (dtype == MSDA_F32 ? 1200000u : 2500000u) ? 2.5 : 9.0);
-        return per_cell >= 9.0 && n >= 2000000u;
-    }
-    if (D > 64) return per_cell >= 2.0;
-    if (D > 32) return per_cell >= (n >= 1200000u ? 2.5 : 6.0);
-    if (n < 1000000u) return false;
-    if (dtype == MSDA_F32) return per_cell >= 9.0 && (D > 16 || n >= 2000000u);
-    return per_cell >= (n >= 3500000u ? 2.5 : n >= 2500000u ? 3.5 : 9.0);
+    const bool f32 = dtype == MSDA_F32;
+    if (!f32 && D % 8 != 0) return per_cell >= 1.5;
+    static const SortLine plain[2][6] = {
+        {{0.1, 12.0, 15.0}, {0.1, 6.0, 15.0}, {0.5, 2.5, 10.0}, {0.1, 2.5, 2.5}, {0.1, 2.0, 0.6}, {0.1, 1.5, 0.5}},
+        {{0.1, 12.0, 40.0}, {0.1, 6.0, 25.0}, {0.5, 6.0, 12.0}, {0.1, 1.5, 1.5}, {0.1, 1.5, 0.0}, {0.1, 1.5, 0.0}}};
+    static const SortLine fused[2][4] = {
+        {{0.8, 9.0, 30.0}, {0.5, 2.5, 9.0}, {0.2, 2.0, 1.3}, {0.1, 1.5, 0.15}},
+        {{0.8, 9.0, 25.0}, {0.3, 1.5, 2.0}, {0.2, 1.5, 0.5}, {0.1, 1.5, 0.0}}};
+    const int width = D <= 8 ? 0 : D <= 16 ? 1 : D <= 32 ? 2 : D <= 64 ? 3 : D <= 128 ? 4 : 5;
+    if (mode == kFused && width < 2) return false;
+    const SortLine& at = mode == kFused ? fused[f32][width - 2] : plain[f32][width];
+    const double millions = 1e-6 * s.nsamples;
+    return millions >= at.least && per_cell >= at.sparse &&
+           per_cell * std::pow(millions, mode == kFused || width < 3 ? 1.5 : 0.75) >= at.line;
 }
 
 // Tasks that one warp pass takes together: as many as fill its lanes with samples, but fewer where

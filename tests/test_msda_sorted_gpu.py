@@ -33,7 +33,7 @@ CASES = [
     (1, 90, 2, 256, ((7, 9),), 8, (-0.1, 1.1)),
     (1, 120, 2, 256, ((40, 60), (20, 30)), 4, (-0.1, 1.1)),   # some dot products in double
     (1, 100, 2, 192, ((40, 60),), 4, (-0.1, 1.1)),
-    (1, 150, 3, 96, ((10, 14), (5, 7)), 4, (-0.1, 1.1)),      # under 20 samples per pixel
+    (1, 150, 3, 96, ((10, 14), (5, 7)), 4, (-0.1, 1.1)),      # under 40 samples per pixel
     (1, 400, 2, 96, ((6, 7), (3, 4)), 4, (-0.1, 1.1)),        # more
     (1, 900, 1, 32, ((210, 240), (2, 2)), 2, (0.0, 1.0)),  # 50851 cells: more than one CTA holds
 ]
