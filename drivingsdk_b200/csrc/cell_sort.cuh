@@ -259,7 +259,7 @@ __host__ __device__ __forceinline__ Counters counters_of(uint32_t parts, uint32_
 template <typename Source, int KEPT>
 __global__ void __launch_bounds__(kSortThreads, 2)
 sort_cells_kernel(const __grid_constant__ Source src, const __grid_constant__ SortParams sp) {
-    extern __shared__ uint32_t s_count[];   // [kSortCells]
+    extern __shared__ uint32_t s_count[];   // [sp.room]: counters, then staged sample numbers
     __shared__ uint32_t warp_sum[32];
     __shared__ uint32_t block_sum;           // samples this CTA's counters, or slice of them, hold
     // CTAs past those that sort (whole clusters) fill with zeros what the main kernel adds to or may
@@ -416,9 +416,9 @@ static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp,
         kern = sort_cells_kernel<Source, -1>;
     }
     // more room only where that lets every map's samples be staged (it costs L1: the encoder shape's
-    // sort takes 82 instead of 69 us)
-    const uint32_t part = (src.samples - 1) / sp.parts + 1;
-    sp.room = part + src.most_cells <= kSortRoom && part >= 16u * src.most_cells ? kSortRoom : kSortCells;
+    // sort takes 82 instead of 69 us; one in a hundred of the whole backward where it is not needed)
+    const uint32_t part = (src.samples - 1) / sp.parts + 1, staged = part + src.most_cells;
+    sp.room = staged > kSortCells && staged <= kSortRoom && part >= 16u * src.most_cells ? kSortRoom : kSortCells;
     const size_t smem = sp.room * sizeof(uint32_t);
     int resident = 0;   // (asked for the shared-memory limit that the call sets)
     const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kSortThreads, smem, &resident);
@@ -433,8 +433,9 @@ static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp,
         const cudaError_t err = cudaMemsetAsync(src.sums(), 0, src.sums_bytes(), stream);
         if (err != cudaSuccess) return err;
     }
-    // the zeros: 128 KB or more for a CTA, whole clusters, no more than fit at once; where there is no
-    // room the sorting CTAs see to them first (256 maps of 80 K: 194 us against 209 after the others)
+    // the zeros: 128 KB or more for a CTA, whole clusters, at most two CTAs per SM (those that find no room
+    // beside the sorting ones follow them); where that is too few the sorting CTAs see to them first (256
+    // maps of 80 K: 194 us against 209 after the others)
     size_t clearing = ((beside ? src.sums_bytes() : 0) + src.clear_size() + (128u << 10) - 1) >> 17;
     if (!room) clearing = 0;
     clearing = std::min<size_t>(clearing, 2u * sm_count);
