@@ -31,7 +31,7 @@ CUDA_SOURCES = ["msda_capi.cu", "resident_ctas.cu", "msda_fwd_sm100.cu", "msda_b
                 "gemm_tc_sm100.cu"]
 EXT_SOURCES = ["binding.cpp", "autograd.cpp"]
 CUDA_HEADERS = ["msda_common.cuh", "msda_tile.cuh", "msda_launch.h", "resident_ctas.h", "msda_fwd_kernel.cuh",
-                "msda_bwd_kernel.cuh", "msda_bwd_sorted.cuh", "cell_sort.cuh", "da_params.h", "gemm_sm100.h",
+                "msda_bwd_kernel.cuh", "msda_bwd_sorted.cuh", "cell_sort.cuh", "sort_plan.h", "da_params.h", "gemm_sm100.h",
                 "gemm_common.cuh", "gemm_split.h", "split_scale.cuh", "dcn_common.cuh", "dcn_split.h",
                 "range_gate.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

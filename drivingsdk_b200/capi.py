@@ -28,6 +28,7 @@ SIGNATURES = {
     "msda_sm100_backward_sorted_workspace_bytes": (_sz, _DIMS7 + [_i]),
     "msda_sm100_fused_backward_sorted_workspace_bytes": (_sz, _DIMS7 + [_i]),
     "gka_sm100_backward_sorted_workspace_bytes": (_sz, _DIMS7 + [_i]),
+    "msda_sm100_sort_form": (_i, [_i] * 6),
     "msda_sm100_backward_ws": (_i, [_vp, _ip, _ip, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz]
                                + _DIMS7 + [_i, _vp]),
     "msda_sm100_fused_forward": (_i, [_vp, _ip, _ip, _vp, _vp, _vp, _vp] + _DIMS7 + [_i, _vp]),

@@ -8,12 +8,10 @@
 
 #include "msda_common.cuh"
 #include "msda_launch.h"
+#include "sort_plan.h"
 
 namespace msda {
 
-constexpr int kSortThreads = 1024;
-constexpr uint32_t kSortCells = 24 * 1024;   // counters of one CTA: 96 KB, two CTAs per SM
-constexpr uint32_t kSortRoom = 28 * 1024;    // ... and the most that two CTAs per SM may have
 constexpr uint32_t kMaxStream = 256;         // most consecutive sorted samples in one stream
 
 template <typename TL>
@@ -97,7 +95,6 @@ __device__ __forceinline__ void cluster_barrier() {
 //           first positions for all (cell by cell, a cell's parts by CTA): three remote accesses, side
 //           by side, per cell and CTA;
 //   alone   many samples per cell: every CTA sorts its samples on its own, the results follow each other.
-enum class Counters { kSplit, kMerged, kAlone };
 
 // One CTA's part of the sort of a map; returns how many of the map's samples have a place.
 template <Counters KEPT, typename Source>
@@ -246,14 +243,6 @@ __device__ __forceinline__ uint32_t sort_map(const Source& src, const SortParams
     return placed;
 }
 
-// How the counters of a map are kept. Two levels of 14 and 53 samples per cell in two parts took 80 us split,
-// 32 merged; at 5 per cell the two are equal. Alone from 16 samples per cell and CTA on.
-__host__ __device__ __forceinline__ Counters counters_of(uint32_t parts, uint32_t samples, uint32_t cells) {
-    const bool fits = cells <= kSortCells;
-    if (parts == 1 || (fits && samples / parts >= 16u * cells)) return Counters::kAlone;
-    return fits && 2u * samples >= parts * cells ? Counters::kMerged : Counters::kSplit;
-}
-
 // KEPT: the one way, for maps that are all alike (a kernel that holds all three spills more; 18 and 12
 // convolution maps of 13 K samples: 26.6 and 26.0 us, now 13.7 and 10.0); -1: chosen map by map.
 template <typename Source, int KEPT>
@@ -386,25 +375,10 @@ static cudaError_t plan_tickets(const void* kernel, int streams, SortParams& sp,
 template <typename Source>
 static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp, int sm_count,
                                cudaStream_t stream) {
-    // The cluster that is done first, by a model of the time in ns: an SM works on two CTAs at a time, 1.5
-    // per sample of both (one alone takes 0.65 of the time of two); a cluster costs 8 us, and 3.1 per
-    // cell and other CTA (merged) or 2.8 per sample (split). More parts have to gain a tenth: apart,
-    // they leave shorter runs. (Samples alone, us: 256 maps of 80 K 258 / 227 / 208 in 1 / 4 / 8 parts,
-    // 192 of 20 K 67 / 56 / 57 in 1 / 2 / 4, 96 of 107 K 111 / 127 / 95 / 84 in 1 / 2 / 4 / 8; 144 of
-    // 5 K, whole sort: 17 / 28 in 1 / 2.) In a kernel that holds one way only a cluster costs 5 us (12 and 18
-    // maps of 13 K samples on 1.5 K cells: 15.6 and 15.5 us in 1 part, 11.5 and 11.6 in 4, 10.2 and 13.5 in 8).
-    const double cluster = Source::kMapsAlike ? 5000.0 : 8000.0;
-    double least = 0.0;
-    for (uint32_t parts = 1; parts <= kMaxSortParts; parts *= 2) {
-        const uint32_t per_sm = (maps * parts + sm_count - 1) / sm_count;
-        const double share = (per_sm / 2 + 0.65 * (per_sm % 2)) / parts;
-        const double between = std::min(3.1 * src.mean_cells * (parts - 1), 2.8 * src.samples);
-        const double ns = share * (1.5 * src.samples + (parts > 1 ? between : 0.0)) + (parts > 1 ? cluster : 0.0);
-        if (parts == 1 || ns < 0.9 * least) {
-            least = ns;
-            sp.parts = parts;
-        }
-    }
+    const SortChoice choice = choose_sort({maps, src.samples, src.mean_cells, src.most_cells},
+                                          static_cast<uint32_t>(sm_count), Source::kMapsAlike);
+    sp.parts = choice.parts;
+    sp.room = choice.room;
     sp.nregions = maps;
     void (*kern)(const Source, const SortParams) = nullptr;
     if constexpr (Source::kMapsAlike) {
@@ -415,10 +389,6 @@ static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp,
     } else {
         kern = sort_cells_kernel<Source, -1>;
     }
-    // more room only where that lets every map's samples be staged (it costs L1: the encoder shape's
-    // sort takes 82 instead of 69 us; one in a hundred of the whole backward where it is not needed)
-    const uint32_t part = (src.samples - 1) / sp.parts + 1, staged = part + src.most_cells;
-    sp.room = staged > kSortCells && staged <= kSortRoom && part >= 16u * src.most_cells ? kSortRoom : kSortCells;
     const size_t smem = sp.room * sizeof(uint32_t);
     int resident = 0;   // (asked for the shared-memory limit that the call sets)
     const cudaError_t e = resident_ctas(reinterpret_cast<const void*>(kern), kSortThreads, smem, &resident);
@@ -427,7 +397,7 @@ static cudaError_t launch_sort(const Source& src, uint32_t maps, SortParams& sp,
     // long (192 maps of 20 K samples, 189 MB: 51 + 32 -> 61 us; 16 of 160 K, 82 MB: 59 + 15 -> 60), and
     // by a memset otherwise (256 of 80 K, 490 MB: 194 + 79 -> 314; key points, 553 MB: 17 + 104 -> 123).
     const bool room = maps * sp.parts <= 3u * sm_count / 2u;
-    const bool beside = room && src.sums_bytes() / 6e3 <= 1.5 * least;
+    const bool beside = room && src.sums_bytes() / 6e3 <= 1.5 * choice.ns;
     sp.clear_sums = beside ? 1u : 0u;
     if (!beside && src.sums_bytes() > 0) {
         const cudaError_t err = cudaMemsetAsync(src.sums(), 0, src.sums_bytes(), stream);

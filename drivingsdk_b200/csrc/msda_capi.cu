@@ -9,6 +9,7 @@
 
 #include "../../include/msda_sm100.h"
 #include "msda_launch.h"
+#include "sort_plan.h"
 
 namespace {
 
@@ -640,6 +641,19 @@ int msda_sm100_device_status(int clear) {
         if (ce != cudaSuccess) return fail_cuda(ce);
     }
     return word;
+}
+
+int msda_sm100_sort_form(int maps, int samples, int mean_cells, int most_cells, int cells, int sm_count) {
+    if (maps <= 0 || samples <= 0 || mean_cells < 0 || most_cells <= 0 || cells <= 0 || sm_count <= 0)
+        return MSDA_ERR_DIMS;
+    const uint32_t n = static_cast<uint32_t>(samples), c = static_cast<uint32_t>(cells);
+    const msda::SortChoice s = msda::choose_sort(
+        {static_cast<uint32_t>(maps), n, static_cast<uint32_t>(mean_cells), static_cast<uint32_t>(most_cells)},
+        static_cast<uint32_t>(sm_count), false);
+    const msda::Counters kept = msda::counters_of(s.parts, n, c);
+    const bool staged = kept == msda::Counters::kAlone && c + (n - 1) / s.parts + 1 <= s.room;
+    return static_cast<int>(s.parts) | static_cast<int>(kept) << 4 | (staged ? 64 : 0) |
+           (s.room > msda::kSortCells ? 128 : 0);
 }
 
 int msda_sm100_tune(int knob, int value) {

@@ -65,7 +65,6 @@ cudaError_t launch_gka_backward(const Params& p, int dtype, int acc_f32, const R
 
 // Scratch of the backward over cell-sorted samples (msda_bwd_sorted.cuh); device memory, part of
 // the caller's workspace.
-constexpr uint32_t kMaxSortParts = 8;
 struct SortParams {
     uint32_t* ticket;       // next ticket of the main kernel
     uint2* regions;         // [B * H * L] {first position, samples} of each sorted region

@@ -313,11 +313,18 @@ typedef enum msda_tune {
 } msda_tune;
 int msda_sm100_tune(int knob, int value);
 
+/* How the sort behind the sorted attention backwards divides its work, for tests; launches nothing. `maps`
+ * (batch entries x heads x levels) of `samples` samples each on a GPU of sm_count SMs: CTAs per map, plus for a
+ * map of `cells` cells 16 * (0: counters split over the cluster's CTAs, 1: merged, 2: each on its own), 64 if
+ * sorted numbers are staged in shared memory, 128 if the CTAs take the larger amount of it for that. */
+int msda_sm100_sort_form(int maps, int samples, int mean_cells, int most_cells, int cells, int sm_count);
+
 /* Optional timing hook for benchmarks, per host thread. While set, every
  * forward call records (fwd_start, fwd_stop) and every backward call records
  * (bwd_start, bwd_stop) — all cudaEvent_t created by the caller — immediately
  * around its main kernel launch, on the launch stream, so that the kernel can
- * be timed without the zero-fill or the down-conversion. Pass NULLs to clear.
+ * be timed without the zero-fill or the down-conversion. Around all but the
+ * down-conversion in the sorted backward, whose sort fills with zeros as well. Pass NULLs to clear.
  * An event pair must not be reused before the caller has read it. */
 void msda_sm100_profile_events(void* fwd_start, void* fwd_stop, void* bwd_start, void* bwd_stop);
 

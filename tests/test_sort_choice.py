@@ -1,9 +1,11 @@
 """Which calls the backward over cell-sorted samples takes: the size of the workspace says it. Calls on either
 side of the lines, at widths that fill their lanes and widths that do not; 16-bit rows of 8 bytes, which the
-unsorted kernel takes one channel at a time, are sorted from 0.1 M samples on."""
+unsorted kernel takes one channel at a time, are sorted from 0.1 M samples on. And how the sorts of the GPU
+tests divide their work, so that a change of the rules cannot move a test to another path unseen."""
 import pytest
 
 from drivingsdk_b200 import capi
+from tests.test_cell_sort_gpu import CASES as SORTS
 
 # operator, type, B, K, H, D, L, Q, P, sorted
 CALLS = [
@@ -52,3 +54,12 @@ def test_more_samples_never_leave_the_sorted_form(D, dtype):
         chosen = [size(2, 3000, 8, D, 4, Q, 4, code) > lib.msda_sm100_backward_workspace_bytes(2, 3000, 8, D, code)
                   for Q in (100, 390, 400, 1000, 2000, 4000, 8000, 20000, 50000)]
         assert chosen == sorted(chosen)
+
+
+@pytest.mark.parametrize("case", SORTS)
+def test_sorts_take_the_form_they_are_tested_for(case):
+    B, Q, H, _, levels, P, _, forms = SORTS[case]
+    K, L = sum(h * w for h, w in levels), len(levels)
+    for (h, w), (parts, kept, staged, large) in zip(levels, forms):
+        got = capi.load().msda_sm100_sort_form(B * H * L, Q * P, K // L, 2 * (K + 1), (h + 1) * (w + 1), 148)
+        assert (got & 15, got >> 4 & 3, bool(got & 64), bool(got & 128)) == (parts, kept, staged, large)
