@@ -8,8 +8,8 @@
 //   * gradients are once-differentiable: using them in a graph raises;
 //   * while torch.jit.trace records, the calls go through those classes, which the tracer sees (a
 //     call that it does not see becomes a constant: the result for the example input).
-// A call whose gradient nobody asks for runs the forward without a node: building one takes 1.5 of the
-// 6.5 us of host time of a small inference call.
+// A call of the attention operators, the aggregation or max pooling whose gradient nobody asks for runs the
+// forward without a node: building one takes 1.4 of the 9.2 us of a small inference call.
 #include <ATen/FuncTorchTLS.h>
 #include <ATen/autocast_mode.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>

@@ -8,7 +8,7 @@
 // at the operator's test shape, and reduces as many: 168 and 385 us, bound by the return path of
 // 128-bit loads and by the reductions. With a 3 x 3 kernel some nine samples share a cell: sorted
 // by cell, corner rows and their sums stay in registers and what is left is to write or read the
-// columns once (481 MB): 98 and 156 us, plus 21 us for the sort, which both directions use.
+// columns once (481 MB): 98 and 159 us, plus 14 us for the sort, which both directions use.
 // One sample at a time per warp, lane = channel quads j and j + 32 of a slice of NV * 128 channels;
 // backward slices add their parts of the t_c up with atomics.
 #include "cell_sort.cuh"
@@ -257,7 +257,7 @@ template <int NV>
 __global__ void __launch_bounds__(kThreadsPerCta, NV > 1 ? 2 : 3)
 scatter_sorted_kernel(const __grid_constant__ DcnParams p, const __grid_constant__ SortParams sp,
                       uint32_t slices) {
-    constexpr int U = 4;    // samples in flight (512 channels: 181 us with two, 156 with four)
+    constexpr int U = 4;    // samples in flight (512 channels: 180 us with two, 159 with four, though 52 bytes spill)
     __shared__ __align__(16) Record s_rec[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t units = static_cast<uint32_t>(p.C) / 4, step_y = static_cast<uint32_t>(p.W) * units;
