@@ -535,8 +535,9 @@ msda_bwd_sorted_kernel(const __grid_constant__ Params p, const __grid_constant__
 }
 
 // Nearest-pixel main kernel: one row per sample. LPR lanes cover a row (four channels each, NV
-// times), 32 / LPR samples of one pixel are worked on at a time and share its row. Bound by its
-// instructions and by shared memory and L1 together (with grad_out rows from L1 7 % faster): records
+// times), 32 / LPR samples of one pixel are worked on at a time and share its row. Bound by shared memory
+// and L1 and by its own chains together (64 % of the load/store wavefronts, 55 % of the issue slots; with
+// grad_out rows from L1 7 % faster): records
 // in shared memory instead of two shuffles per row, and no guards for groups within their pixel,
 // took 10.3 M samples on 375 pixels, 64 channels, from 317 to 287 us (bf16 327 to 260).
 template <typename T, typename TL, int NV, int LPR, bool RAGGED>

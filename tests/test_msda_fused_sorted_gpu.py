@@ -17,6 +17,8 @@ CASES = {   # B, Q, H, D, levels, P
     "lp16": (1, 300, 8, 64, ((32, 32), (16, 16), (8, 8), (4, 4)), 4),
     "lp32": (2, 200, 4, 16, ((29, 50), (15, 25), (8, 13), (4, 7)), 8),
     "few": (1, 1, 1, 4, ((3, 2),), 3),
+    "d256": (1, 150, 2, 256, ((12, 10), (6, 5)), 4),
+    "d100": (1, 150, 2, 100, ((12, 10), (6, 5)), 4),
 }
 
 

@@ -18,7 +18,7 @@ def _same(name, got, want):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("D", [32, 24])
+@pytest.mark.parametrize("D", [32, 24, 96, 256])
 def test_sorted_backward_with_an_infinite_gradient(D, dtype):
     import drivingsdk_b200 as sdk
     w = workloads.Workload("inf", 1, 60, 2, D, ((3, 4), (1, 1)), 4, (-0.2, 1.2), seed=D)
@@ -36,6 +36,38 @@ def test_sorted_backward_with_an_infinite_gradient(D, dtype):
             capi.load().msda_sm100_tune(capi.TUNE_SORT, old)
     assert any(torch.isinf(g).any() for g in grads[0][1:])
     for name, want, got in zip(("value", "loc", "attn"), *grads):
+        _same(name, got.float(), want.float())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [24, 32, 96, 256])
+def test_sorted_fused_backward_with_values_that_are_not_finite(D, dtype):
+    """Infinite gradients, reference points nowhere, masked logits (one task has no other), an infinite value."""
+    import drivingsdk_b200 as sdk
+    w = workloads.Workload("inf", 1, 60, 2, D, ((3, 4), (1, 1)), 4, (-0.2, 1.2), seed=D)
+    dev = parity.to_device(workloads.make_inputs(w, dtype), dtype)
+    g = torch.Generator(device="cuda").manual_seed(D)
+    ref = torch.rand(1, 60, 2, 2, generator=g, device="cuda").to(dtype)
+    ref[0, 7, 0, 0], ref[0, 8, 1, 1], ref[0, 9] = float("nan"), float("inf"), -float("inf")
+    logits = torch.randn(1, 60, 2, 2, 4, generator=g, device="cuda").to(dtype)
+    logits[0, ::5, :, 0, 1:] = -float("inf")
+    logits[0, 11, 1] = -float("inf")
+    value = dev["value"].abs() + 0.1
+    value[0, 5, 1, D - 1] = float("inf")
+    go = torch.ones(1, 60, 2 * D, dtype=dtype, device="cuda")
+    go[0, ::3, 5] = float("inf")
+    off = torch.randn(1, 60, 2, 2, 4, 2, generator=g, device="cuda").to(dtype)
+    grads = []
+    for sort in (0, 2):
+        old = capi.load().msda_sm100_tune(capi.TUNE_SORT, sort)
+        try:
+            ts = [t.detach().requires_grad_() for t in (value, ref, off, logits)]
+            out = sdk.multi_scale_deformable_attn_fused(ts[0], dev["shapes"], dev["starts"], *ts[1:])
+            grads.append(torch.autograd.grad(out, ts, go))
+        finally:
+            capi.load().msda_sm100_tune(capi.TUNE_SORT, old)
+    assert not torch.isfinite(grads[0][0]).all()
+    for name, want, got in zip(("value", "ref", "off", "logits"), *grads):
         _same(name, got.float(), want.float())
 
 
